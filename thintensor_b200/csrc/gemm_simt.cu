@@ -11,111 +11,225 @@
 // thinruntime/triton_kernels.py:484-535, 2959-2986, 3022-3083.
 #include "common.cuh"
 
-#define GS_BM 64
-#define GS_BN 64
-#define GS_BK 16
-#define GS_THREADS 256
+// Tiles of 64 x 128 outputs by 128 threads, an 8 x 8 square of outputs in each thread's registers, so that an operand number
+// read from shared memory serves eight multiply-adds; two shared-memory stages of 16 k, the next stage's numbers on their way
+// from global memory while this one is multiplied.  Neighbouring outputs of a row are one packed instruction (two multiply-adds,
+// each rounded as ever): no faster on the FMA pipe, but half the instructions, and the form with single ones lost a sixth of its
+// issue slots to register conflicts.  Warps whose 32 rows all lie behind m skip the arithmetic.  Bound by issue: 1,000 x 4,096 x
+// 4,096 runs at 51 TFLOP/s of the pipe's 74 (single multiply-adds on stages filled by asynchronous copies: 43).  4 x 4 outputs a
+// thread and one stage, the form before, was bound by shared memory and the loads' latency: at 193 rows 16,384 features of 2,048 took
+// 695 us against 334 (in 4 slices of k), 2,048 of 8,192 574 against 203 (8 slices), 3,072 of 2,048 216 against 72 (6 slices).
+constexpr int GS_BM = 64, GS_BN = 128, GS_BK = 16, GS_THREADS = 128;
+constexpr int GS_XLD = GS_BM + 4, GS_WLD = GS_BN + 4;
+
+__device__ __forceinline__ void gs_fma2(unsigned long long& d, unsigned long long a, unsigned long long b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+
+// four neighbouring numbers, widened; vec: they lie on a boundary of their own size
+__device__ __forceinline__ void gs_load4(float (&v)[4], const float* p, int count, bool vec) {
+    if (vec && count == 4) {
+        const float4 q = __ldg(reinterpret_cast<const float4*>(p));
+        v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+    } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] = e < count ? __ldg(p + e) : 0.0f;
+    }
+}
+__device__ __forceinline__ void gs_load4(float (&v)[4], const __nv_bfloat16* p, int count, bool vec) {
+    if (vec && count == 4) {
+        const uint2 q = __ldg(reinterpret_cast<const uint2*>(p));
+        v[0] = __uint_as_float(q.x << 16); v[1] = __uint_as_float(q.x & 0xffff0000u);
+        v[2] = __uint_as_float(q.y << 16); v[3] = __uint_as_float(q.y & 0xffff0000u);
+    } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] = e < count ? __bfloat162float(p[e]) : 0.0f;
+    }
+}
 
 template <typename TX, typename TW>
 __global__ void __launch_bounds__(GS_THREADS)
 gemm_simt_kernel(const TX* __restrict__ x, long long ldx, const TW* __restrict__ w, long long ldw,
                  const float* __restrict__ bias, float* __restrict__ out, long long ldo, long long split_stride,
-                 int m, int n, int k, int k_per_split) {
-    __shared__ float xs[GS_BK][GS_BM + 4];
-    __shared__ float ws[GS_BK][GS_BN + 4];
+                 int m, int n, int k, int k_per_split, int vec_x, int vec_w, int vec_o) {
+    __shared__ __align__(16) float xs[2][GS_BK][GS_XLD];
+    __shared__ __align__(16) float ws[2][GS_BK][GS_WLD];
+    tt_pdl_launch_dependents();
     const int m0 = blockIdx.y * GS_BM, n0 = blockIdx.x * GS_BN;
     const int split = blockIdx.z;
     const int k_begin = split * k_per_split;
     const int k_end = min(k, k_begin + k_per_split);
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;  // 16 x 16 threads, 4 x 4 outputs each
-    float acc[4][4];
+    // warps 2 x 2 over the tile (32 rows x 64 columns each), lanes 4 x 8; a thread's rows are two runs of four 16 apart, its
+    // columns two runs of four 32 apart, so that the lanes' 16-byte reads lie side by side
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int row = (warp >> 1) * 32 + (lane >> 3) * 4, col = (warp & 1) * 64 + (lane & 7) * 4;
+    const bool busy = m0 + (warp >> 1) * 32 < m;
+    unsigned long long acc[8][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
 
-    // loader mapping: 256 threads fetch 64 rows x 16 k = 1024 numbers, 4 consecutive k each
+    // piece i of a thread: row (threadIdx.x + i * 128) / 4 of the operand's tile, four k from 4 * (threadIdx.x % 4)
     const int load_row = threadIdx.x >> 2, load_k = (threadIdx.x & 3) * 4;
-    for (int kk = k_begin; kk < k_end; kk += GS_BK) {
+    float xr[2][4], wr[4][4];
+    auto fetch = [&](int kk) {
+        const int count = max(0, min(4, k_end - kk - load_k));
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int gn = n0 + load_row + 32 * i;
+            gs_load4(wr[i], w + (size_t)gn * ldw + kk + load_k, gn < n ? count : 0, vec_w);
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int gm = m0 + load_row + 32 * i;
+            gs_load4(xr[i], x + (size_t)gm * ldx + kk + load_k, gm < m ? count : 0, vec_x);
+        }
+    };
+    auto put = [&](int stage) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            const int kx = kk + load_k + e;
-            const int gm = m0 + load_row, gn = n0 + load_row;
-            xs[load_k + e][load_row] = (gm < m && kx < k_end) ? tt_to_float(x[(size_t)gm * ldx + kx]) : 0.0f;
-            ws[load_k + e][load_row] = (gn < n && kx < k_end) ? tt_to_float(w[(size_t)gn * ldw + kx]) : 0.0f;
+#pragma unroll
+            for (int i = 0; i < 2; ++i) xs[stage][load_k + e][load_row + 32 * i] = xr[i][e];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) ws[stage][load_k + e][load_row + 32 * i] = wr[i][e];
         }
-        __syncthreads();
+    };
+    tt_pdl_wait();                                              // before either operand: a caller's weights may be fresh
+    fetch(k_begin);
+    put(0);
+    __syncthreads();
+    int stage = 0;
+    for (int kk = k_begin; kk < k_end; kk += GS_BK, stage ^= 1) {
+        const bool more = kk + GS_BK < k_end;
+        if (more) fetch(kk + GS_BK);
+        if (busy) {
 #pragma unroll
-        for (int e = 0; e < GS_BK; ++e) {
-            float a[4], b[4];
+            for (int e = 0; e < GS_BK; ++e) {
+                const float4 a0 = *reinterpret_cast<const float4*>(&xs[stage][e][row]), a1 = *reinterpret_cast<const float4*>(&xs[stage][e][row + 16]);
+                const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(&ws[stage][e][col]), b1 = *reinterpret_cast<const ulonglong2*>(&ws[stage][e][col + 32]);
+                const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
 #pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = xs[e][ty * 4 + i];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = ws[e][tx * 4 + j];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+                for (int i = 0; i < 8; ++i) {
+                    const unsigned long long twice = ((unsigned long long)__float_as_uint(a[i]) << 32) | __float_as_uint(a[i]);
+                    gs_fma2(acc[i][0], twice, b0.x);
+                    gs_fma2(acc[i][1], twice, b0.y);
+                    gs_fma2(acc[i][2], twice, b1.x);
+                    gs_fma2(acc[i][3], twice, b1.y);
+                }
+            }
         }
-        __syncthreads();
+        if (more) {
+            put(stage ^ 1);                                     // the stage that the round before read: everyone has passed its barrier
+            __syncthreads();
+        }
     }
     float* o = out + (size_t)split * split_stride;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int gm = m0 + ty * 4 + i;
+    for (int i = 0; i < 8; ++i) {
+        const int gm = m0 + row + (i & 3) + 16 * (i >> 2);
         if (gm >= m) continue;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int gn = n0 + tx * 4 + j;
-            if (gn >= n) continue;
-            float v = acc[i][j];
-            if (bias && split == 0) v += bias[gn];
-            o[(size_t)gm * ldo + gn] = v;
+        for (int j = 0; j < 2; ++j) {
+            const int gn = n0 + col + 32 * j;
+            float v[4] = {__uint_as_float((unsigned)acc[i][2 * j]), __uint_as_float((unsigned)(acc[i][2 * j] >> 32)),
+                          __uint_as_float((unsigned)acc[i][2 * j + 1]), __uint_as_float((unsigned)(acc[i][2 * j + 1] >> 32))};
+            if (bias && split == 0) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) v[e] += gn + e < n ? bias[gn + e] : 0.0f;
+            }
+            float* to = o + (size_t)gm * ldo + gn;
+            if (vec_o && gn + 4 <= n) {
+                *reinterpret_cast<float4*>(to) = make_float4(v[0], v[1], v[2], v[3]);
+                continue;
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (gn + e < n) to[e] = v[e];
         }
     }
 }
 
-// Skinny form for few rows of x (decoding): one warp per output column n and up to 8
-// rows of x at a time, lanes stride over k, so the weights are read once per 8 rows.
+// Skinny form for few rows of x (decoding, the few wanted rows of a head): a warp takes four output columns and up to 8 rows of x
+// at a time, its lanes stride over k four numbers each, so that a lane has four 16-byte loads of weights in flight, a round ahead
+// of their use, and a number of x that it fetched (from the L1) serves four columns.  Bound by reading the weights where there are enough
+// columns: 4 rows of 128,256 x 2,048 float32 weights 793 -> 254 us (4.1 TB/s) against a warp per column with 4-byte loads.
+constexpr int GR_COLS = 4, GR_ROWS = 8, GR_WARPS = 4;
+
 template <typename TX, typename TW>
-__global__ void gemm_rows_kernel(const TX* __restrict__ x, long long ldx, const TW* __restrict__ w, long long ldw,
-                                 const float* __restrict__ bias, float* __restrict__ out, long long ldo, int m, int n,
-                                 int k) {
+__global__ void __launch_bounds__(GR_WARPS * 32)
+gemm_rows_kernel(const TX* __restrict__ x, long long ldx, const TW* __restrict__ w, long long ldw,
+                 const float* __restrict__ bias, float* __restrict__ out, long long ldo, int m, int n,
+                 int k, int vec_x, int vec_w) {
+    tt_pdl_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int col = blockIdx.x * (blockDim.x >> 5) + warp;
+    const int col = (blockIdx.x * GR_WARPS + warp) * GR_COLS;
     if (col >= n) return;
-    const TW* wrow = w + (size_t)col * ldw;
-    for (int m0 = 0; m0 < m; m0 += 8) {
-        float acc[8];
+    float wv[GR_COLS][4];
+    auto weights = [&](int kk) {
+        const int count = max(0, min(4, k - kk));
 #pragma unroll
-        for (int i = 0; i < 8; ++i) acc[i] = 0.0f;
-        for (int kk = lane; kk < k; kk += 32) {
-            const float wv = tt_to_float(wrow[kk]);
+        for (int c = 0; c < GR_COLS; ++c) gs_load4(wv[c], w + (size_t)min(col + c, n - 1) * ldw + kk, count, vec_w);
+    };
+    tt_pdl_wait();
+    for (int m0 = 0; m0 < m; m0 += GR_ROWS) {
+        weights(lane * 4);
+        float acc[GR_ROWS][GR_COLS];
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
-                if (m0 + i < m) acc[i] = fmaf(tt_to_float(x[(size_t)(m0 + i) * ldx + kk]), wv, acc[i]);
+        for (int i = 0; i < GR_ROWS; ++i)
+#pragma unroll
+            for (int c = 0; c < GR_COLS; ++c) acc[i][c] = 0.0f;
+        for (int kk = lane * 4; kk < k; kk += 128) {
+            float now[GR_COLS][4];
+#pragma unroll
+            for (int c = 0; c < GR_COLS; ++c)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) now[c][e] = wv[c][e];
+            if (kk + 128 < k) weights(kk + 128);
+            const int count = min(4, k - kk);
+#pragma unroll
+            for (int i = 0; i < GR_ROWS; ++i) {
+                if (m0 + i >= m) break;
+                float xv[4];
+                gs_load4(xv, x + (size_t)(m0 + i) * ldx + kk, count, vec_x);
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+#pragma unroll
+                    for (int c = 0; c < GR_COLS; ++c) acc[i][c] = fmaf(xv[e], now[c][e], acc[i][c]);
+            }
         }
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const float total = tt_warp_sum(acc[i]);
-            if (lane == 0 && m0 + i < m) out[(size_t)(m0 + i) * ldo + col] = total + (bias ? bias[col] : 0.0f);
+        for (int i = 0; i < GR_ROWS; ++i) {
+            if (m0 + i >= m) break;
+#pragma unroll
+            for (int c = 0; c < GR_COLS; ++c) {
+                const float total = tt_warp_sum(acc[i][c]);
+                if (lane == 0 && col + c < n) out[(size_t)(m0 + i) * ldo + col + c] = total + (bias ? bias[col + c] : 0.0f);
+            }
         }
     }
 }
+
+// four neighbouring numbers of every row lie on a boundary of their size
+template <typename T>
+static int vec4(const void* p, long long ld) { return ((uintptr_t)p % (4 * sizeof(T))) == 0 && ld % 4 == 0; }
 
 template <typename TX, typename TW>
 static int launch(const void* x, long long ldx, const void* w, long long ldw, const float* bias, float* out,
                   long long ldo, long long split_stride, int m, int n, int k, int splits, cudaStream_t stream) {
+    const int vec_x = vec4<TX>(x, ldx), vec_w = vec4<TW>(w, ldw);
     if (m <= 16 && splits == 1) {
-        const int warps = 8;
-        gemm_rows_kernel<TX, TW><<<(n + warps - 1) / warps, warps * 32, 0, stream>>>((const TX*)x, ldx, (const TW*)w, ldw, bias, out, ldo, m, n, k);
+        const int cols = GR_WARPS * GR_COLS;
+        tt_launch_pdl(gemm_rows_kernel<TX, TW>, dim3((n + cols - 1) / cols), dim3(GR_WARPS * 32), 0, stream, (const TX*)x, ldx, (const TW*)w, ldw, bias, out,
+                      ldo, m, n, k, vec_x, vec_w);
         TT_LAUNCH_CHECK();
     }
     int k_per_split = (k + splits - 1) / splits;
     k_per_split = (k_per_split + GS_BK - 1) / GS_BK * GS_BK;
     const dim3 grid((n + GS_BN - 1) / GS_BN, (m + GS_BM - 1) / GS_BM, splits);
     if (grid.y > 65535) return (int)cudaErrorInvalidValue;
-    gemm_simt_kernel<TX, TW><<<grid, GS_THREADS, 0, stream>>>((const TX*)x, ldx, (const TW*)w, ldw, bias, out, ldo, split_stride, m, n, k, k_per_split);
+    tt_launch_pdl(gemm_simt_kernel<TX, TW>, grid, dim3(GS_THREADS), 0, stream, (const TX*)x, ldx, (const TW*)w, ldw, bias, out, ldo, split_stride, m, n, k,
+                  k_per_split, vec_x, vec_w, vec4<float>(out, ldo) && split_stride % 4 == 0);
     TT_LAUNCH_CHECK();
 }
 
