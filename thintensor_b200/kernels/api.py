@@ -905,6 +905,59 @@ def mamba2_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_col: int, dt_bias: tor
               _ptr(cu), _ptr(slots), sequences, heads, head_dim, state_size, groups, SCAN_FORMS[form], _stream()), "mamba2_scan")
 
 
+CHUNK_TOKENS = 64           # tokens of a chunk of the recurrences with a decay per head (CK_TOKENS in csrc/recurrent_chunks.cu)
+CHUNK_MAX_ROWS = 128        # state rows (key size) the chunk kernels take
+_CHUNK_FACTORS = 836
+
+
+def chunk_slots(n_tokens: int, sequences: int) -> int:
+    """Chunks that a step's packed sequences can have at most, however its tokens are dealt out to them."""
+    return n_tokens // CHUNK_TOKENS + sequences
+
+
+def scan_chunks_scratch(n_tokens: int, sequences: int, heads: int, groups: int) -> tuple[tuple[int, ...], tuple[int, ...]]:
+    """Shapes of the float32 scratch that :func:`scan_chunks` takes as ``scores`` and ``factors``."""
+    slots = chunk_slots(n_tokens, sequences)
+    return (slots, groups, CHUNK_TOKENS, CHUNK_TOKENS), (slots, heads, _CHUNK_FACTORS)
+
+
+def scan_chunks(x: torch.Tensor, b: torch.Tensor, c: torch.Tensor, state: torch.Tensor, y: torch.Tensor, cu: torch.Tensor, slots: torch.Tensor,
+                sequences: int, heads: int, head_dim: int, state_size: int, groups: int, scores: torch.Tensor, factors: torch.Tensor,
+                steps: tuple[torch.Tensor, int, torch.Tensor, torch.Tensor, torch.Tensor] | None = None, fixed_decay: torch.Tensor | None = None) -> None:
+    """The recurrences of :func:`mamba2_scan` and :func:`decay_scan`, a chunk of 64 tokens at a time (for prompts).  ``x``, ``b``, ``c``:
+    float32 ``[tokens, columns]`` of ``heads * head_dim`` and ``groups * state_size`` columns, views of one matrix (equal row
+    strides).  Either ``steps`` = (projection partial sums, first column of the raw step sizes, dt_bias, A_log, D) or ``fixed_decay``
+    (float32 ``[heads]``, step sizes one).  States of up to 128 rows.  ``scores`` and ``factors``: see :func:`scan_chunks_scratch`."""
+    for t, cols, name in ((x, heads * head_dim, "x"), (b, groups * state_size, "B"), (c, groups * state_size, "C")):
+        if t.dtype != torch.float32 or t.dim() != 2 or t.stride(1) != 1 or t.stride(0) != x.stride(0) or tuple(t.shape) != (x.shape[0], cols):
+            raise KernelError(f"scan_chunks: {name} must be float32 [tokens, {cols}] with the row stride of x")
+    for t, name in ((state, "recurrent state"), (y, "recurrence output"), (scores, "scores"), (factors, "factors")):
+        _need(t, torch.float32, name)
+    if (steps is None) == (fixed_decay is None):
+        raise KernelError("scan_chunks: decays come from step sizes or are fixed")
+    want_scores, want_factors = scan_chunks_scratch(x.shape[0], sequences, heads, groups)
+    if (state_size > CHUNK_MAX_ROWS or heads % groups or tuple(state.shape[1:]) != (heads, head_dim, state_size) or tuple(y.shape) != (x.shape[0], heads * head_dim)
+            or tuple(scores.shape) != want_scores or tuple(factors.shape) != want_factors):
+        raise KernelError("scan_chunks: shapes do not fit the sizes")
+    p, splits, stride, cols, dt_col, vectors = c_void_p(0), 0, 0, 0, 0, (None, None, None)
+    if steps is not None:
+        p, splits, stride, cols = _projection(steps[0])
+        dt_col, vectors = int(steps[1]), steps[2:]
+        if dt_col < 0 or dt_col + heads > cols:
+            raise KernelError("scan_chunks: the step sizes lie outside the projection")
+    for t, name in ((*zip(vectors, ("dt_bias", "A_log", "D")), (fixed_decay, "decay"))):
+        if t is not None:
+            _need(t, torch.float32, name)
+            if t.numel() != heads:
+                raise KernelError(f"scan_chunks: {name} has a number per head")
+    fn = _fn("recurrent_chunks", "tt_scan_chunks", [c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_longlong, c_int, c_int, c_void_p, c_void_p,
+                                                    c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
+                                                    c_int, c_int, c_int, c_int, c_void_p])
+    _check(fn(_ptr(x), _ptr(b), _ptr(c), x.stride(0), p, splits, stride, cols, dt_col, _ptr(vectors[0]), _ptr(vectors[1]), _ptr(vectors[2]),
+              _ptr(fixed_decay), _ptr(state), _ptr(y), _ptr(scores), _ptr(factors), _ptr(cu), _ptr(slots), sequences, want_scores[0], heads, groups,
+              head_dim, state_size, sm_count(x.device), _stream()), "scan_chunks", 2)
+
+
 def delta_scan(qkv: torch.Tensor, proj: torch.Tensor, b_col: int, a_col: int, dt_bias: torch.Tensor | None, a_log: torch.Tensor | None,
                state: torch.Tensor, out: torch.Tensor, cu: torch.Tensor, slots: torch.Tensor, sequences: int, heads: int, qk_heads: int,
                key_dim: int, value_dim: int, form: str = "auto", row_decay: torch.Tensor | None = None) -> None:

@@ -38,6 +38,7 @@ SOURCES: dict[str, list[str]] = {
     "attention_mma": [],
     "attention_tcgen05": [],
     "recurrent": [],
+    "recurrent_chunks": [],
     "latent_attention": [],
     "routing": [],
     "streams": [],

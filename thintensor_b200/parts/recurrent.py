@@ -110,6 +110,24 @@ def in_blocks(ctx) -> bool:
     return not ctx.decode and ctx.n_tokens >= 4 * ctx.sequences
 
 
+def in_chunks(ctx, heads: int, columns: int, rows: int) -> bool:
+    """Whether a recurrence with a decay per head takes its tokens in chunks of 64 (decided by the step's shape alone, like
+    :func:`in_blocks`): prompts of at least a chunk's length on average do, while the grid of a CTA per sequence, head and 32 columns
+    is at most four rounds of the SMs.  Measured on a B200 (us, chunks against token by token): 64 heads of 64 x 128, one sequence
+    of 64 tokens 23 and 33, of 40 tokens 22 and 22; two of 48 33 and 28; four of 731 332 and 545 (512 CTAs), 16 of 700 (2,048 CTAs)
+    1,060 and 1,035; 24 heads of 256 x 128, five of 96 (960 CTAs) 131 and 84: many CTAs keep the form that goes token by token busy."""
+    ctas = heads * ctx.sequences * -(-columns // 32)
+    return (not ctx.decode and rows <= api.CHUNK_MAX_ROWS and ctx.n_tokens >= api.CHUNK_TOKENS * ctx.sequences
+            and ctas <= 4 * api.sm_count(ctx.status.device))
+
+
+def scan_chunks(ctx, x, b, c, state, y, heads: int, head_dim: int, rows: int, groups: int, **decays) -> None:
+    """:func:`api.scan_chunks` on scratch memory of the step's."""
+    scores, factors = api.scan_chunks_scratch(ctx.n_tokens, ctx.sequences, heads, groups)
+    api.scan_chunks(x, b, c, state, y, ctx.cu, ctx.slots, ctx.sequences, heads, head_dim, rows, groups,
+                    ctx.scratch("chunks.scores", scores, torch.float32), ctx.scratch("chunks.factors", factors, torch.float32), **decays)
+
+
 @MIXERS.register("mamba2")
 class Mamba2(Mixer):
     NAMES = {"in": "in_proj.weight", "conv": "conv1d.weight", "conv_bias": "conv1d.bias", "dt_bias": "dt_bias", "A_log": "A_log",
@@ -173,8 +191,14 @@ class Mamba2(Mixer):
         api.causal_conv(proj, self.inner, self.channels, self.conv_weight, self.conv_bias, True, tail, xbc, ctx.cu, ctx.slots,
                         ctx.sequences, tokens, ctx.decode)
         y = ctx.scratch("mamba2.y", (tokens, self.inner), torch.float32)
-        api.mamba2_scan(xbc, proj, self.inner + self.channels, self.dt_bias, self.a_log, self.d_skip, recurrent, y, ctx.cu, ctx.slots,
-                        ctx.sequences, self.heads, self.head_dim, self.state, self.groups)
+        dt_col = self.inner + self.channels
+        if in_chunks(ctx, self.heads, self.head_dim, self.state):
+            x, b, c = xbc.split((self.inner, self.groups * self.state, self.groups * self.state), dim=1)
+            scan_chunks(ctx, x, b, c, recurrent, y, self.heads, self.head_dim, self.state, self.groups,
+                        steps=(proj, dt_col, self.dt_bias, self.a_log, self.d_skip))
+        else:
+            api.mamba2_scan(xbc, proj, dt_col, self.dt_bias, self.a_log, self.d_skip, recurrent, y, ctx.cu, ctx.slots, ctx.sequences, self.heads,
+                            self.head_dim, self.state, self.groups)
         gated = ctx.scratch("mamba2.gated", (tokens, self.inner))
         api.gated_group_norm(y, self.inner // self.norm_groups, proj, 0, self.norm, self.eps, True, gated)
         return self.out.delta(ctx, gated, "mamba2.out")
@@ -399,6 +423,9 @@ class DecayLinearAttention(Mixer):
                                  self.value_dim, 1.0)
         elif decay is not None:
             api.row_decay_scan(vkq, decay, recurrent, read, ctx.cu, ctx.slots, ctx.sequences, self.heads, self.key_dim, self.value_dim)
+        elif in_chunks(ctx, self.heads, self.value_dim, self.key_dim):
+            v, k, q = vkq.split((self.v, self.qk, self.qk), dim=1)
+            scan_chunks(ctx, v, k, q, recurrent, read, self.heads, self.value_dim, self.key_dim, self.heads, fixed_decay=self.decays)
         else:
             api.decay_scan(vkq, self.decays, recurrent, read, ctx.cu, ctx.slots, ctx.sequences, self.heads, self.key_dim, self.value_dim)
         return self.finish(ctx, proj, read)
