@@ -97,3 +97,45 @@ def test_recurrence_in_chunks(heads, groups, P, N, pad, fixed):
             assert float((y[span].double().reshape(-1, heads, P) - want).abs().max()) <= 2e-5 * max(1.0, float(want.abs().max()))
         assert float((state[slot].double() - last).abs().max()) <= 2e-5 * max(1.0, float(last.abs().max()))
     assert torch.equal(state[[3, 7]], before[[3, 7]])
+
+
+@pytest.mark.parametrize("heads,qk_heads,D,V", [(2, 1, 128, 128), (3, 3, 65, 33), (4, 2, 64, 30), (64, 32, 24, 64), (40, 40, 128, 72), (2, 2, 3, 7)])
+def test_delta_rule_in_chunks(heads, qk_heads, D, V):
+    """As above for the gated delta rule; the last token of the longest sequence repeats the keys before it (a system whose
+    off-diagonal numbers are as large as they get)."""
+    from thintensor_b200.kernels import api
+
+    news, slot_ids = [63, 64, 0, 1, 130, 65], [4, 0, 6, 2, 1, 5]
+    tokens, sequences, qk = sum(news), len(news), qk_heads * D
+    qkv = randn(tokens, 2 * qk + heads * V, seed=15)
+    cu = [sum(news[:i]) for i in range(sequences + 1)]
+    qkv[cu[5] - 20:cu[5], qk:2 * qk] = qkv[cu[5] - 1, qk:2 * qk]
+    state = randn(8, heads, V, D, seed=16)
+    before = state.clone()
+    out = torch.full((tokens, heads * V), 7.0, device=DEV)
+    a_log, dt_bias = randn(heads, seed=17, scale=2.0), randn(heads, seed=18)
+    raw = randn(2, tokens, 2 * heads + 3, seed=19)
+    scratch = torch.full(api.delta_chunks_scratch(tokens, sequences, heads, D, V), float("nan"), device=DEV)
+    api.delta_chunks(qkv, raw, 1, heads + 2, dt_bias, a_log, state, out, i32(cu), i32(slot_ids), sequences, heads, qk_heads, D, V, scratch)
+    z = raw.double().sum(0)
+    beta = torch.sigmoid(z[:, 1:1 + heads])
+    decay = torch.exp(-torch.exp(a_log.double()) * torch.nn.functional.softplus(z[:, heads + 2:2 * heads + 2] + dt_bias.double()))
+    unit = lambda y: y / (y.square().sum(-1, keepdim=True) + 1e-6).sqrt()
+    share = heads // qk_heads
+    q = (unit(qkv[:, :qk].double().reshape(-1, qk_heads, D)) * D ** -0.5).repeat_interleave(share, 1)
+    k = unit(qkv[:, qk:2 * qk].double().reshape(-1, qk_heads, D)).repeat_interleave(share, 1)
+    v = qkv[:, 2 * qk:].double().reshape(-1, heads, V)
+    for s, slot in enumerate(slot_ids):
+        S = before[slot].double()
+        want = torch.empty(news[s], heads, V, dtype=torch.float64, device=DEV)
+        for i in range(news[s]):
+            t = cu[s] + i
+            S = decay[t][:, None, None] * S
+            u = beta[t][:, None] * (v[t] - (S @ k[t][:, :, None])[..., 0])
+            S = S + u[:, :, None] * k[t][:, None, :]
+            want[i] = (S @ q[t][:, :, None])[..., 0]
+        if news[s]:
+            got = out[cu[s]:cu[s + 1]].double().reshape(-1, heads, V)
+            assert float((got - want).abs().max()) <= 2e-5 * max(1.0, float(want.abs().max()))
+        assert float((state[slot].double() - S).abs().max()) <= 2e-5 * max(1.0, float(S.abs().max()))
+    assert torch.equal(state[[3, 7]], before[[3, 7]])

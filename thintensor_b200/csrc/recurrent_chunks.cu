@@ -150,7 +150,7 @@ __device__ __forceinline__ void ck_factors(float* __restrict__ out, float a0, fl
 }
 
 template <int NP>
-__global__ void __launch_bounds__(CK_THREADS)
+__global__ void __launch_bounds__(CK_THREADS, 2)
 scan_chunks_prepare_kernel(const ScanChunks a) {
     tt_pdl_launch_dependents();
     tt_pdl_wait();
@@ -287,6 +287,128 @@ __device__ __forceinline__ void ck_product(unsigned long long (&acc)[4][2], cons
     }
 }
 
+// Two such products with the same B (k0 .. k0 + K - 1 in sums of 32, which are added up: a long chain of additions loses more)
+template <int RL, int K>
+__device__ __forceinline__ void ck_two_products(unsigned long long (&acc0)[4][2], const float* __restrict__ A0, unsigned long long (&acc1)[4][2],
+                                                const float* __restrict__ A1, int lda, const float* __restrict__ B, int ldb, int k0) {
+    constexpr int SUM = K < 32 ? K : 32;
+    float4 x0[2][4], x1[2][4];
+    ulonglong2 y[2][4];
+    auto load = [&](int at, int k) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            x0[at][r] = *reinterpret_cast<const float4*>(A0 + r * RL * lda + k);
+            x1[at][r] = *reinterpret_cast<const float4*>(A1 + r * RL * lda + k);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) y[at][e] = *reinterpret_cast<const ulonglong2*>(B + (k + e) * ldb);
+    };
+    load(0, k0);
+#pragma unroll 1
+    for (int ks = 0; ks < K; ks += SUM) {
+        unsigned long long p0[4][2], p1[4][2];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) p0[r][0] = p0[r][1] = p1[r][0] = p1[r][1] = 0ull;
+#pragma unroll
+        for (int step = 0; step < SUM / 4; ++step) {
+            const int at = step & 1, next = ks + 4 * (step + 1);
+            if (next < K) load(at ^ 1, k0 + next);
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const float v0 = e == 0 ? x0[at][r].x : e == 1 ? x0[at][r].y : e == 2 ? x0[at][r].z : x0[at][r].w;
+                    const float v1 = e == 0 ? x1[at][r].x : e == 1 ? x1[at][r].y : e == 2 ? x1[at][r].z : x1[at][r].w;
+                    const unsigned long long t0 = ck_pair(v0, v0), t1 = ck_pair(v1, v1);
+                    ck_fma2(p0[r][0], t0, y[at][e].x);
+                    ck_fma2(p0[r][1], t0, y[at][e].y);
+                    ck_fma2(p1[r][0], t1, y[at][e].x);
+                    ck_fma2(p1[r][1], t1, y[at][e].y);
+                }
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                acc0[r][c] = ck_pair(ck_lo(acc0[r][c]) + ck_lo(p0[r][c]), ck_hi(acc0[r][c]) + ck_hi(p0[r][c]));
+                acc1[r][c] = ck_pair(ck_lo(acc1[r][c]) + ck_lo(p1[r][c]), ck_hi(acc1[r][c]) + ck_hi(p1[r][c]));
+            }
+    }
+}
+
+// acc += A * B over K numbers of k from k0 on, in sums of 32 (a long chain of additions loses more)
+template <int RL, int K>
+__device__ __forceinline__ void ck_state_product(unsigned long long (&acc)[4][2], const float* __restrict__ A, int lda, const float* __restrict__ B, int ldb, int k0) {
+    constexpr int SUM = K < 32 ? K : 32;
+#pragma unroll 1
+    for (int k = k0; k < k0 + K; k += SUM) {
+        unsigned long long part[4][2];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) part[r][0] = part[r][1] = 0ull;
+        ck_product<RL>(part, A, lda, B, ldb, k, 4, k + SUM);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            acc[r][0] = ck_pair(ck_lo(acc[r][0]) + ck_lo(part[r][0]), ck_hi(acc[r][0]) + ck_hi(part[r][0]));
+            acc[r][1] = ck_pair(ck_lo(acc[r][1]) + ck_lo(part[r][1]), ck_hi(acc[r][1]) + ck_hi(part[r][1]));
+        }
+    }
+}
+
+// S <- all S + sum over the chunk's tokens of B[j] (w x)[j]^T: NL state rows and four columns of a lane; B: row j at j * NP
+template <int NP, int NL>
+__device__ __forceinline__ void ck_update(unsigned long long (&s)[NL][2], float all, const float* __restrict__ B, const float* __restrict__ XW, int ldx) {
+#pragma unroll
+    for (int i = 0; i < NL; ++i) {
+        s[i][0] = ck_pair(ck_lo(s[i][0]) * all, ck_hi(s[i][0]) * all);
+        s[i][1] = ck_pair(ck_lo(s[i][1]) * all, ck_hi(s[i][1]) * all);
+    }
+#pragma unroll 8
+    for (int j = 0; j < CK_TOKENS; ++j) {
+        float bv[NL];
+        if constexpr (NL == 4) {
+            const float4 q = *reinterpret_cast<const float4*>(B + j * NP);
+            bv[0] = q.x; bv[1] = q.y; bv[2] = q.z; bv[3] = q.w;
+        } else if constexpr (NL == 2) {
+            const float2 q = *reinterpret_cast<const float2*>(B + j * NP);
+            bv[0] = q.x; bv[1] = q.y;
+        } else {
+            bv[0] = B[j * NP];
+        }
+        const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(XW + j * ldx);
+#pragma unroll
+        for (int i = 0; i < NL; ++i) {
+            const unsigned long long twice = ck_pair(bv[i], bv[i]);
+            ck_fma2(s[i][0], twice, x.x);
+            ck_fma2(s[i][1], twice, x.y);
+        }
+    }
+}
+
+// A chunk's outputs: this lane's sums and the other slices'; rows from `left` on do not exist
+template <int RL, int SLICES>
+__device__ __forceinline__ void ck_outputs(const unsigned long long (&acc)[4][2], const float* __restrict__ parts, int ldx, int row, int col, int width, int left,
+                                           bool vec, float* __restrict__ out, int stride) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const int i = row + RL * r;
+        float o[4] = {ck_lo(acc[r][0]), ck_hi(acc[r][0]), ck_lo(acc[r][1]), ck_hi(acc[r][1])};
+#pragma unroll
+        for (int k = 0; k < SLICES - 1; ++k) {
+            const float4 q = *reinterpret_cast<const float4*>(parts + (k * CK_TOKENS + i) * ldx + col);
+            o[0] += q.x; o[1] += q.y; o[2] += q.z; o[3] += q.w;
+        }
+        if (i >= left || col >= width) continue;
+        float* to = out + (size_t)i * stride + col;
+        if (vec) {
+            *reinterpret_cast<float4*>(to) = make_float4(o[0], o[1], o[2], o[3]);
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (col + e < width) to[e] = o[e];
+        }
+    }
+}
+
 template <int NP, int TP>
 struct CkLayout {
     static constexpr int LDA = NP + 4, LDX = TP + 4;
@@ -403,7 +525,7 @@ scan_chunks_kernel(const ScanChunks a) {
 #pragma unroll
         for (int r = 0; r < 4; ++r) acc[r][0] = acc[r][1] = 0ull;
         constexpr int K = NP / L::SLICES;
-        ck_product<RL>(acc, As + row * L::LDA, L::LDA, Ss + col, L::LDX, slice * K, 4, slice * K + K);
+        ck_state_product<RL, K>(acc, As + row * L::LDA, L::LDA, Ss + col, L::LDX, slice * K);
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
             const float e = F[CK_E + row + RL * r];
@@ -427,58 +549,14 @@ scan_chunks_kernel(const ScanChunks a) {
             }
         }
         // S <- e_63 S + B^T (w x)
-        const float all = F[CK_ALL];
-#pragma unroll
-        for (int i = 0; i < NL; ++i) {
-            s[i][0] = ck_pair(ck_lo(s[i][0]) * all, ck_hi(s[i][0]) * all);
-            s[i][1] = ck_pair(ck_lo(s[i][1]) * all, ck_hi(s[i][1]) * all);
-        }
-        const float* B = stage + L::B + srow;
-#pragma unroll 8
-        for (int j = 0; j < CK_TOKENS; ++j) {
-            float bv[NL];
-            if constexpr (NL == 4) {
-                const float4 q = *reinterpret_cast<const float4*>(B + j * NP);
-                bv[0] = q.x; bv[1] = q.y; bv[2] = q.z; bv[3] = q.w;
-            } else if constexpr (NL == 2) {
-                const float2 q = *reinterpret_cast<const float2*>(B + j * NP);
-                bv[0] = q.x; bv[1] = q.y;
-            } else {
-                bv[0] = B[j * NP];
-            }
-            const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(XW + j * L::LDX + col);
-#pragma unroll
-            for (int i = 0; i < NL; ++i) {
-                const unsigned long long twice = ck_pair(bv[i], bv[i]);
-                ck_fma2(s[i][0], twice, x.x);
-                ck_fma2(s[i][1], twice, x.y);
-            }
-        }
+        ck_update<NP, NL>(s, F[CK_ALL], stage + L::B + srow, XW + col, L::LDX);
 #pragma unroll
         for (int i = 0; i < NL; ++i)
             *reinterpret_cast<float4*>(Ss + (srow + i) * L::LDX + col) = make_float4(ck_lo(s[i][0]), ck_hi(s[i][0]), ck_lo(s[i][1]), ck_hi(s[i][1]));
         __syncthreads();                                        // this stage may be filled again, the weighted rows be written again
-        if (slice == 0) {                                       // the other slices' sums are there: the chunk's outputs
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const int i = row + RL * r, t = chunk * CK_TOKENS + i;
-                float o[4] = {ck_lo(acc[r][0]), ck_hi(acc[r][0]), ck_lo(acc[r][1]), ck_hi(acc[r][1])};
-#pragma unroll
-                for (int k = 0; k < L::SLICES - 1; ++k) {
-                    const float4 q = *reinterpret_cast<const float4*>(ck_shared + L::PARTS + (k * CK_TOKENS + i) * L::LDX + col);
-                    o[0] += q.x; o[1] += q.y; o[2] += q.z; o[3] += q.w;
-                }
-                if (t >= n || col >= width) continue;
-                float* to = a.y + (size_t)(first + t) * inner + (size_t)h * P + p0 + col;
-                if (vec_x) {
-                    *reinterpret_cast<float4*>(to) = make_float4(o[0], o[1], o[2], o[3]);
-                } else {
-#pragma unroll
-                    for (int e = 0; e < 4; ++e)
-                        if (col + e < width) to[e] = o[e];
-                }
-            }
-        }
+        if (slice == 0)                                         // the other slices' sums are there: the chunk's outputs
+            ck_outputs<RL, L::SLICES>(acc, ck_shared + L::PARTS, L::LDX, row, col, width, n - chunk * CK_TOKENS, vec_x,
+                                      a.y + (size_t)(first + chunk * CK_TOKENS) * inner + (size_t)h * P + p0, inner);
     }
     ck_wait<0>();
 #pragma unroll
@@ -524,4 +602,397 @@ extern "C" int tt_scan_chunks(const float* x, const float* b, const float* c, lo
     const bool narrow = (long long)heads * sequences * ((P + 31) / 32) * 2 <= sms + sms / 4;
     if (N <= 64) return narrow ? scan_chunks_launch<64, 16>(a, max_slots, stream) : scan_chunks_launch<64, 32>(a, max_slots, stream);
     return narrow ? scan_chunks_launch<128, 16>(a, max_slots, stream) : scan_chunks_launch<128, 32>(a, max_slots, stream);
+}
+
+// ------------------------------------------------------------------------------------------------------ the gated delta rule
+//   q = q / |q| * scale, k = k / |k|;  S <- a_t S;  u_t = beta_t (v_t - S^T k_t);  S <- S + k_t u_t^T;  o_t = S^T q_t
+// (lengths with 1e-6 under the root, scale = D^-1/2).  Inside a chunk that starts from state S
+//   u_i = beta_i v_i - beta_i e_i S^T k_i - sum_(j<i) beta_i f(i, j) (k_i . k_j) u_j
+// is a unit lower triangular system, (I + A) U = beta V - (beta e K) S, whose solution is U = U0 - W S with (I + A) U0 = beta V and
+// (I + A) W = beta e K: neither needs the state, so the first kernel solves for both, parallel over chunks and heads, and the second
+// walks the chunks with   U = U0 - W S,   o = e Q S + P U (P_ij = f(i, j) q_i . k_j, j <= i),   S <- e_63 S + (w K)^T U.
+// Everything is float32 multiply-adds; the systems are solved by forward substitution, a column a thread.  16 heads of 128 x 128 on 4,097
+// tokens: 1,950 us token by token, now 478: the first kernel 130 (bound by issue and shared memory; two columns a thread and half the
+// threads 229, the whole substitution unrolled 278), the second 345 (bound like the one above; the two products with the state,
+// W S and Q S, take an operand of S from shared memory once for both: one after the other 408).
+constexpr int CD_THREADS = 256;
+constexpr int CD_E = 0, CD_W = 64, CD_ALL = 128, CD_FACTORS = 136;        // of a chunk and head, for the second kernel
+
+struct DeltaChunks {
+    const float* qkv;           // float32 rows [q | k | v]: query/key head g at g * D, value head h at 2 * qk_heads * D + h * V
+    size_t stride;
+    const float* proj;          // columns b_col + h and a_col + h of the partial sums: raw write strength, raw decay input
+    int splits, cols, b_col, a_col;
+    size_t split_stride;
+    const float* dt_bias;
+    const float* a_log;
+    float* state;               // [slots][heads][V][D]
+    float* out;                 // [tokens][heads * V]
+    float* scratch;             // [slots][heads]: W [64][D], U0 [64][V], P [64][64], factors [CD_FACTORS]
+    const int* cu;
+    const int* slots;
+    int sequences, heads, qk_heads, D, V, vec, vec_v;
+    __host__ __device__ size_t chunk_floats() const { return (size_t)CK_TOKENS * (D + V + CK_TOKENS) + CD_FACTORS; }
+    __device__ float* chunk_scratch(int slot, int h) const { return scratch + ((size_t)slot * heads + h) * chunk_floats(); }
+};
+
+template <int NP>
+__global__ void __launch_bounds__(CD_THREADS, 2)
+delta_chunks_prepare_kernel(const DeltaChunks a) {
+    tt_pdl_launch_dependents();
+    tt_pdl_wait();
+    constexpr int LD = NP + 4;
+    extern __shared__ __align__(16) float ck_shared[];
+    float* ks = ck_shared;                                      // [64][LD]
+    float* qs = ks + CK_TOKENS * LD;                            // [64][LD]
+    float* As = qs + CK_TOKENS * LD;                            // [64][CK_MLD]
+    float* f = As + CK_TOKENS * CK_MLD;                         // [CK_FACTORS]
+    float* nq = f + CK_FACTORS;                                 // [64] each: 1 / |q|, 1 / |k|, beta
+    float* nk = nq + CK_TOKENS;
+    float* beta = nk + CK_TOKENS;
+    float* scalars = beta + CK_TOKENS;                          // [2][64]
+    const int slot = blockIdx.x, h = blockIdx.y, D = a.D, V = a.V;
+    int lo = 0, hi = a.sequences;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (ck_first_slot(a.cu, mid) <= slot) lo = mid; else hi = mid;
+    }
+    const int first = a.cu[lo], n = a.cu[lo + 1] - first, c0 = (slot - ck_first_slot(a.cu, lo)) * CK_TOKENS;
+    if (c0 >= n) return;
+    const int count = min(CK_TOKENS, n - c0), g = h / (a.heads / a.qk_heads);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (D < NP) {
+        for (int e = threadIdx.x; e < 2 * CK_TOKENS * LD; e += CD_THREADS) ck_shared[e] = 0.0f;
+        __syncthreads();
+    }
+    const float* rows = a.qkv + (size_t)(first + c0) * a.stride;
+    ck_stage<NP, CD_THREADS>(qs, LD, rows + (size_t)g * D, a.stride, count, D, a.vec);
+    ck_stage<NP, CD_THREADS>(ks, LD, rows + (size_t)(a.qk_heads + g) * D, a.stride, count, D, a.vec);
+    ck_commit();
+    if (warp == 0) {
+        float decay[2];
+        const float neg_a = -expf(__ldg(a.a_log + h)), bias = __ldg(a.dt_bias + h);
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            const int i = lane + 32 * half;
+            const float* row = a.proj + (size_t)(first + c0 + i) * a.cols + h;
+            decay[half] = 1.0f;
+            float write = 0.0f;
+            if (i < count) {
+                const float raw = ck_sum_slices(row + a.a_col, a.splits, a.split_stride) + bias;
+                decay[half] = expf(neg_a * (raw > 20.0f ? raw : log1pf(expf(raw))));
+                write = 1.0f / (1.0f + expf(-ck_sum_slices(row + a.b_col, a.splits, a.split_stride)));
+            }
+            beta[i] = write;
+        }
+        ck_factors(f, decay[0], decay[1], 1.0f, 1.0f, lane, scalars, scalars + CK_TOKENS);
+    }
+    ck_wait<0>();
+    __syncthreads();
+    // lengths: four lanes a row
+    for (int item = threadIdx.x >> 2; item < 2 * CK_TOKENS; item += CD_THREADS / 4) {
+        const float* row = (item < CK_TOKENS ? qs : ks) + (item & (CK_TOKENS - 1)) * LD;
+        float sum = 0.0f;
+        for (int c = threadIdx.x & 3; c < D; c += 4) sum = fmaf(row[c], row[c], sum);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+        if (!(threadIdx.x & 3)) (item < CK_TOKENS ? nq : nk)[item & (CK_TOKENS - 1)] = rsqrtf(sum + 1e-6f) * (item < CK_TOKENS ? rsqrtf((float)D) : 1.0f);
+    }
+    __syncthreads();
+    float* scratch = a.chunk_scratch(slot, h);
+    float* P = scratch + (size_t)CK_TOKENS * (D + V);
+    // k . k and q . k: 16 x 16 threads, rows and columns 16 apart
+    {
+        const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+        float kk[4][4], qk[4][4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) kk[r][c] = qk[r][c] = 0.0f;
+#pragma unroll 1
+        for (int k0 = 0; k0 < NP; k0 += 32) {                   // short sums, added up
+            float pk[4][4], pq[4][4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) pk[r][c] = pq[r][c] = 0.0f;
+#pragma unroll 2
+            for (int k = k0; k < k0 + 32; k += 4) {
+                float4 b[4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) b[c] = *reinterpret_cast<const float4*>(ks + (tx + 16 * c) * LD + k);
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const float4 x = *reinterpret_cast<const float4*>(ks + (ty + 16 * r) * LD + k), y = *reinterpret_cast<const float4*>(qs + (ty + 16 * r) * LD + k);
+#pragma unroll
+                    for (int c = 0; c <= r; ++c) {              // the others lie above the diagonal
+                        pk[r][c] = fmaf(x.x, b[c].x, pk[r][c]); pk[r][c] = fmaf(x.y, b[c].y, pk[r][c]);
+                        pk[r][c] = fmaf(x.z, b[c].z, pk[r][c]); pk[r][c] = fmaf(x.w, b[c].w, pk[r][c]);
+                        pq[r][c] = fmaf(y.x, b[c].x, pq[r][c]); pq[r][c] = fmaf(y.y, b[c].y, pq[r][c]);
+                        pq[r][c] = fmaf(y.z, b[c].z, pq[r][c]); pq[r][c] = fmaf(y.w, b[c].w, pq[r][c]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int c = 0; c <= r; ++c) { kk[r][c] += pk[r][c]; qk[r][c] += pq[r][c]; }
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int i = ty + 16 * r, bi = i >> 3;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int j = tx + 16 * c, bj = j >> 3;
+                const float fij = bi > bj ? f[CK_U + i] * f[CK_BLOCKS + bi * 8 + bj] * f[CK_V + j] : bi == bj ? f[CK_DIAG + bi * 64 + (i & 7) * 8 + (j & 7)] : 0.0f;
+                As[i * CK_MLD + j] = j < i ? -beta[i] * fij * (nk[i] * nk[j] * kk[r][c]) : 0.0f;         // -A
+                P[i * CK_TOKENS + j] = j <= i ? fij * (nq[i] * nk[j] * qk[r][c]) : 0.0f;
+            }
+        }
+    }
+    if (threadIdx.x < CK_TOKENS) {
+        float* factors = P + CK_TOKENS * CK_TOKENS;
+        factors[CD_E + threadIdx.x] = f[CK_E + threadIdx.x] * nq[threadIdx.x];
+        factors[CD_W + threadIdx.x] = f[CK_W + threadIdx.x] * nk[threadIdx.x];
+        if (threadIdx.x == 0) factors[CD_ALL] = f[CK_ALL];
+    }
+    __syncthreads();
+    // (I + A) x = r for the columns of beta e K (made W) and of beta V (made U0), one a thread, 16 rows at a time: what the rows
+    // before contribute as a product (sums of 16 added up), then the triangle of the 16.  Half of the CTA takes the keys'
+    // columns, in place, and every second tile of NP value columns; the other half the other tiles, where the queries lay.
+    const int half = threadIdx.x / (CD_THREADS / 2), col = threadIdx.x % (CD_THREADS / 2);
+    float* xs = (half ? qs : ks) + col;
+    const float* values = rows + (size_t)2 * a.qk_heads * D + (size_t)h * V;
+    for (int job = half; (job - 1) * NP < V; job += 2) {       // job 0: the keys; job t: value columns from (t - 1) * NP on
+        const int c = (job ? (job - 1) * NP : 0) + col, width = job ? V : D;
+        if (col >= NP || c >= width) continue;
+        float* to = scratch + (job ? (size_t)CK_TOKENS * D : 0) + c;
+        float raw[16];                                          // the next 16 rows' values, fetched ahead
+        auto fetch = [&](int i0) {
+            if (!job) return;
+#pragma unroll
+            for (int r = 0; r < 16; ++r) raw[r] = i0 + r < count ? __ldg(values + (size_t)(i0 + r) * a.stride + c) : 0.0f;
+        };
+        fetch(0);
+#pragma unroll 1
+        for (int i0 = 0; i0 < CK_TOKENS; i0 += 16) {
+            float x[16];
+#pragma unroll
+            for (int r = 0; r < 16; ++r) {
+                const int i = i0 + r;
+                x[r] = job ? beta[i] * raw[r] : beta[i] * f[CK_E + i] * nk[i] * xs[i * LD];
+            }
+            if (i0 + 16 < CK_TOKENS) fetch(i0 + 16);
+#pragma unroll 1
+            for (int j0 = 0; j0 < i0; j0 += 16) {
+                float sum[16];
+#pragma unroll
+                for (int r = 0; r < 16; ++r) sum[r] = 0.0f;
+#pragma unroll
+                for (int j = j0; j < j0 + 16; j += 4) {
+                    float y[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) y[e] = xs[(j + e) * LD];
+#pragma unroll
+                    for (int r = 0; r < 16; ++r) {
+                        const float4 m = *reinterpret_cast<const float4*>(As + (i0 + r) * CK_MLD + j);
+                        sum[r] = fmaf(m.x, y[0], sum[r]);
+                        sum[r] = fmaf(m.y, y[1], sum[r]);
+                        sum[r] = fmaf(m.z, y[2], sum[r]);
+                        sum[r] = fmaf(m.w, y[3], sum[r]);
+                    }
+                }
+#pragma unroll
+                for (int r = 0; r < 16; ++r) x[r] += sum[r];
+            }
+#pragma unroll
+            for (int r = 1; r < 16; ++r) {
+#pragma unroll
+                for (int j = 0; j < r; j += 4) {
+                    const float4 m = *reinterpret_cast<const float4*>(As + (i0 + r) * CK_MLD + i0 + j);
+                    x[r] = fmaf(m.x, x[j], x[r]);
+                    if (j + 1 < r) x[r] = fmaf(m.y, x[j + 1], x[r]);
+                    if (j + 2 < r) x[r] = fmaf(m.z, x[j + 2], x[r]);
+                    if (j + 3 < r) x[r] = fmaf(m.w, x[j + 3], x[r]);
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < 16; ++r) {
+                xs[(i0 + r) * LD] = x[r];
+                to[(size_t)(i0 + r) * width] = x[r];
+            }
+        }
+    }
+}
+
+template <int NP, int TP>
+struct CdLayout {
+    using L = CkLayout<NP, TP>;                                 // lanes, rows and slices as above
+    static constexpr int LDA = L::LDA, LDX = L::LDX;
+    static constexpr int Q = 0, W = Q + CK_TOKENS * LDA, S = W + CK_TOKENS * LDA, XW = S + NP * LDX, PARTS = XW + CK_TOKENS * LDX;
+    static constexpr int STAGE = PARTS + (L::SLICES - 1) * CK_TOKENS * LDX;
+    static constexpr int K = 0, X = K + CK_TOKENS * NP, M = X + CK_TOKENS * LDX, F = M + CK_TOKENS * CK_MLD, STAGE_FLOATS = F + CD_FACTORS;
+    static constexpr size_t BYTES = (size_t)(STAGE + 2 * STAGE_FLOATS) * sizeof(float);
+};
+
+template <int NP, int TP>
+__global__ void __launch_bounds__(CK_THREADS, 1)
+delta_chunks_kernel(const DeltaChunks a) {
+    using D_ = CdLayout<NP, TP>;
+    using L = CkLayout<NP, TP>;
+    constexpr int PL = L::PL, RL = L::RL, ROW_BLOCKS = CK_TOKENS / L::ROWS, SLICE_K = NP / L::SLICES;
+    constexpr int NL = NP * TP / (CK_THREADS * 4);              // state rows of a lane
+    extern __shared__ __align__(16) float ck_shared[];
+    tt_pdl_launch_dependents();
+    tt_pdl_wait();
+    const int h = blockIdx.x, b = blockIdx.y, p0 = blockIdx.z * TP;
+    const int first = a.cu[b], n = a.cu[b + 1] - first;
+    if (n <= 0) return;
+    const int g = h / (a.heads / a.qk_heads), V = a.V, D = a.D;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int col = 4 * (lane % PL), width = min(TP, V - p0);
+    const int slice = warp / ROW_BLOCKS, block = (warp + (warp >> 2)) % ROW_BLOCKS;
+    const int row = block * L::ROWS + lane / PL;
+    const int srow = warp * (NP / CK_WARPS) + (lane / PL) * NL;
+    float* Qs = ck_shared + D_::Q;
+    float* Ws = ck_shared + D_::W;
+    float* Ss = ck_shared + D_::S;
+    float* XW = ck_shared + D_::XW;
+    const int chunks = (n + CK_TOKENS - 1) / CK_TOKENS, slot0 = ck_first_slot(a.cu, b);
+    const bool vec_x = a.vec_v && (width & 3) == 0;
+
+    for (int e = threadIdx.x; e < D_::STAGE + 2 * D_::STAGE_FLOATS; e += CK_THREADS) ck_shared[e] = 0.0f;
+    __syncthreads();
+    auto fetch_first = [&](int chunk) {                         // what meets the state: q and W
+        if (chunk < chunks) {
+            const int c0 = chunk * CK_TOKENS;
+            ck_stage<NP>(Qs, D_::LDA, a.qkv + (size_t)(first + c0) * a.stride + (size_t)g * D, a.stride, min(CK_TOKENS, n - c0), D, a.vec);
+            ck_stage<NP>(Ws, D_::LDA, a.chunk_scratch(slot0 + chunk, h), D, CK_TOKENS, D, !(D & 3));
+        }
+        ck_commit();
+    };
+    auto fetch_rest = [&](int chunk) {
+        if (chunk < chunks) {
+            const int c0 = chunk * CK_TOKENS;
+            float* stage = ck_shared + D_::STAGE + (chunk & 1) * D_::STAGE_FLOATS;
+            const float* scratch = a.chunk_scratch(slot0 + chunk, h);
+            ck_stage<NP>(stage + D_::K, NP, a.qkv + (size_t)(first + c0) * a.stride + (size_t)(a.qk_heads + g) * D, a.stride, min(CK_TOKENS, n - c0), D, a.vec);
+            ck_stage<TP>(stage + D_::X, D_::LDX, scratch + (size_t)CK_TOKENS * D + p0, V, CK_TOKENS, width, vec_x);
+            const float* P = scratch + (size_t)CK_TOKENS * (D + V);
+            ck_stage<CK_TOKENS>(stage + D_::M, CK_MLD, P, CK_TOKENS, CK_TOKENS, CK_TOKENS, true);
+            for (int e = threadIdx.x; e < CD_FACTORS / 4; e += CK_THREADS) ck_copy16(stage + D_::F + 4 * e, P + CK_TOKENS * CK_TOKENS + 4 * e, true);
+        }
+        ck_commit();
+    };
+    fetch_rest(0);
+    fetch_first(0);
+
+    float* S = a.state + (((size_t)a.slots[b] * a.heads + h) * V + p0 + col) * D;
+    unsigned long long s[NL][2];
+#pragma unroll
+    for (int i = 0; i < NL; ++i) {
+        float v[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] = srow + i < D && p0 + col + e < V ? S[(size_t)e * D + srow + i] : 0.0f;
+        s[i][0] = ck_pair(v[0], v[1]);
+        s[i][1] = ck_pair(v[2], v[3]);
+        *reinterpret_cast<float4*>(Ss + (srow + i) * D_::LDX + col) = make_float4(v[0], v[1], v[2], v[3]);
+    }
+
+    for (int chunk = 0; chunk < chunks; ++chunk) {
+        float* stage = ck_shared + D_::STAGE + (chunk & 1) * D_::STAGE_FLOATS;
+        float* X = stage + D_::X;
+        const float* M = stage + D_::M;
+        const float* F = stage + D_::F;
+        fetch_rest(chunk + 1);
+        ck_wait<1>();
+        __syncthreads();                                        // this chunk's numbers and the state are there
+        unsigned long long acc[4][2], ws[4][2];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) acc[r][0] = acc[r][1] = ws[r][0] = ws[r][1] = 0ull;
+        ck_two_products<RL, SLICE_K>(ws, Ws + row * D_::LDA, acc, Qs + row * D_::LDA, D_::LDA, Ss + col, D_::LDX, slice * SLICE_K);
+        {                                                       // W S: the first slice's sums lie where the weighted rows will
+            float* to = slice == 0 ? XW : ck_shared + D_::PARTS + (slice - 1) * CK_TOKENS * D_::LDX;
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+                *reinterpret_cast<float4*>(to + (row + RL * r) * D_::LDX + col) = make_float4(ck_lo(ws[r][0]), ck_hi(ws[r][0]), ck_lo(ws[r][1]), ck_hi(ws[r][1]));
+        }
+        __syncthreads();                                        // W S is whole; q, W and the old state are read
+        fetch_first(chunk + 1);
+        for (int e = threadIdx.x; e < CK_TOKENS * PL; e += CK_THREADS) {           // U = U0 - W S, and the rows the update adds
+            const int t = e / PL, c = 4 * (e % PL);
+            float4 u = *reinterpret_cast<const float4*>(X + t * D_::LDX + c);
+            float4 ws = *reinterpret_cast<const float4*>(XW + t * D_::LDX + c);
+#pragma unroll
+            for (int k = 0; k < L::SLICES - 1; ++k) {
+                const float4 q = *reinterpret_cast<const float4*>(ck_shared + D_::PARTS + (k * CK_TOKENS + t) * D_::LDX + c);
+                ws.x += q.x; ws.y += q.y; ws.z += q.z; ws.w += q.w;
+            }
+            u.x -= ws.x; u.y -= ws.y; u.z -= ws.z; u.w -= ws.w;
+            const float w = F[CD_W + t];
+            *reinterpret_cast<float4*>(X + t * D_::LDX + c) = u;
+            *reinterpret_cast<float4*>(XW + t * D_::LDX + c) = make_float4(w * u.x, w * u.y, w * u.z, w * u.w);
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const float e = F[CD_E + row + RL * r];
+            acc[r][0] = ck_pair(ck_lo(acc[r][0]) * e, ck_hi(acc[r][0]) * e);
+            acc[r][1] = ck_pair(ck_lo(acc[r][1]) * e, ck_hi(acc[r][1]) * e);
+        }
+        __syncthreads();                                        // U is there
+        ck_product<RL>(acc, M + row * CK_MLD, CK_MLD, X + col, D_::LDX, 4 * slice, 4 * L::SLICES, block * L::ROWS + L::ROWS);
+        if (slice > 0) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+                *reinterpret_cast<float4*>(ck_shared + D_::PARTS + ((slice - 1) * CK_TOKENS + row + RL * r) * D_::LDX + col) =
+                    make_float4(ck_lo(acc[r][0]), ck_hi(acc[r][0]), ck_lo(acc[r][1]), ck_hi(acc[r][1]));
+        }
+        const float all = F[CD_ALL];
+        ck_update<NP, NL>(s, all, stage + D_::K + srow, XW + col, D_::LDX);
+#pragma unroll
+        for (int i = 0; i < NL; ++i)
+            *reinterpret_cast<float4*>(Ss + (srow + i) * D_::LDX + col) = make_float4(ck_lo(s[i][0]), ck_hi(s[i][0]), ck_lo(s[i][1]), ck_hi(s[i][1]));
+        __syncthreads();
+        if (slice == 0)
+            ck_outputs<RL, L::SLICES>(acc, ck_shared + D_::PARTS, D_::LDX, row, col, width, n - chunk * CK_TOKENS, vec_x,
+                                      a.out + (size_t)(first + chunk * CK_TOKENS) * (a.heads * V) + (size_t)h * V + p0, a.heads * V);
+    }
+    ck_wait<0>();
+#pragma unroll
+    for (int i = 0; i < NL; ++i) {
+        const float v[4] = {ck_lo(s[i][0]), ck_hi(s[i][0]), ck_lo(s[i][1]), ck_hi(s[i][1])};
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (srow + i < D && p0 + col + e < V) S[(size_t)e * D + srow + i] = v[e];
+    }
+}
+
+template <int NP, int TP>
+static int delta_chunks_launch(const DeltaChunks& a, int max_slots, cudaStream_t stream) {
+    constexpr size_t prepare_bytes = (size_t)(2 * CK_TOKENS * (NP + 4) + CK_TOKENS * CK_MLD + CK_FACTORS + 5 * CK_TOKENS) * sizeof(float);
+    static bool allowed = false;
+    if (!allowed) {
+        cudaError_t code = ck_allow(delta_chunks_prepare_kernel<NP>, prepare_bytes);
+        if (code == cudaSuccess) code = ck_allow(delta_chunks_kernel<NP, TP>, CdLayout<NP, TP>::BYTES);
+        if (code != cudaSuccess) return (int)code;
+        allowed = true;
+    }
+    tt_launch_pdl(delta_chunks_prepare_kernel<NP>, dim3(max_slots, a.heads), dim3(CD_THREADS), prepare_bytes, stream, a);
+    tt_launch_pdl(delta_chunks_kernel<NP, TP>, dim3(a.heads, a.sequences, (a.V + TP - 1) / TP), dim3(CK_THREADS), CdLayout<NP, TP>::BYTES, stream, a);
+    TT_LAUNCH_CHECK();
+}
+
+// scratch: max_slots * heads * (64 * (D + V + 64) + CD_FACTORS) floats; max_slots as for tt_scan_chunks
+extern "C" int tt_delta_chunks(const float* qkv, int qkv_cols, const float* proj, int splits, long long split_stride, int cols, int b_col, int a_col,
+                               const float* dt_bias, const float* a_log, float* state, float* out, float* scratch, const int* cu, const int* slots,
+                               int sequences, int max_slots, int heads, int qk_heads, int D, int V, int sms, cudaStream_t stream) {
+    if (sequences <= 0 || max_slots <= 0) return 0;
+    if (D <= 0 || D > 128 || V <= 0 || qk_heads <= 0 || heads % qk_heads || heads > 65535 || sequences > 65535) return (int)cudaErrorInvalidValue;
+    if (!qkv || !proj || !dt_bias || !a_log || !scratch) return (int)cudaErrorInvalidValue;
+    const int vec = ((uintptr_t)qkv & 15) == 0 && !(qkv_cols & 3) && !(D & 3);
+    const DeltaChunks a{qkv, (size_t)qkv_cols, proj, splits, cols, b_col, a_col, (size_t)split_stride, dt_bias, a_log, state, out, scratch, cu, slots,
+                        sequences, heads, qk_heads, D, V, vec, ((uintptr_t)out & 15) == 0 && ((uintptr_t)scratch & 15) == 0 && !(V & 3) ? 1 : 0};
+    const bool narrow = (long long)heads * sequences * ((V + 31) / 32) * 2 <= sms + sms / 4;        // as for tt_scan_chunks
+    if (D <= 64) return narrow ? delta_chunks_launch<64, 16>(a, max_slots, stream) : delta_chunks_launch<64, 32>(a, max_slots, stream);
+    return narrow ? delta_chunks_launch<128, 16>(a, max_slots, stream) : delta_chunks_launch<128, 32>(a, max_slots, stream);
 }

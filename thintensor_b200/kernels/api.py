@@ -908,6 +908,7 @@ def mamba2_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_col: int, dt_bias: tor
 CHUNK_TOKENS = 64           # tokens of a chunk of the recurrences with a decay per head (CK_TOKENS in csrc/recurrent_chunks.cu)
 CHUNK_MAX_ROWS = 128        # state rows (key size) the chunk kernels take
 _CHUNK_FACTORS = 836
+_DELTA_CHUNK_FACTORS = 136
 
 
 def chunk_slots(n_tokens: int, sequences: int) -> int:
@@ -956,6 +957,32 @@ def scan_chunks(x: torch.Tensor, b: torch.Tensor, c: torch.Tensor, state: torch.
     _check(fn(_ptr(x), _ptr(b), _ptr(c), x.stride(0), p, splits, stride, cols, dt_col, _ptr(vectors[0]), _ptr(vectors[1]), _ptr(vectors[2]),
               _ptr(fixed_decay), _ptr(state), _ptr(y), _ptr(scores), _ptr(factors), _ptr(cu), _ptr(slots), sequences, want_scores[0], heads, groups,
               head_dim, state_size, sm_count(x.device), _stream()), "scan_chunks", 2)
+
+
+def delta_chunks_scratch(n_tokens: int, sequences: int, heads: int, key_dim: int, value_dim: int) -> tuple[int, ...]:
+    """Shape of the float32 scratch that :func:`delta_chunks` takes."""
+    return chunk_slots(n_tokens, sequences), heads, CHUNK_TOKENS * (key_dim + value_dim + CHUNK_TOKENS) + _DELTA_CHUNK_FACTORS
+
+
+def delta_chunks(qkv: torch.Tensor, proj: torch.Tensor, b_col: int, a_col: int, dt_bias: torch.Tensor, a_log: torch.Tensor, state: torch.Tensor,
+                 out: torch.Tensor, cu: torch.Tensor, slots: torch.Tensor, sequences: int, heads: int, qk_heads: int, key_dim: int, value_dim: int,
+                 scratch: torch.Tensor) -> None:
+    """:func:`delta_scan` with a decay per head, a chunk of 64 tokens at a time (for prompts; key sizes of up to 128).  ``scratch``:
+    see :func:`delta_chunks_scratch`."""
+    for t, name in ((qkv, "q/k/v"), (dt_bias, "dt_bias"), (a_log, "A_log"), (state, "recurrent state"), (out, "recurrence output"), (scratch, "scratch")):
+        _need(t, torch.float32, name)
+    shape = delta_chunks_scratch(qkv.shape[0], sequences, heads, key_dim, value_dim)
+    if (qkv.shape[1] != 2 * qk_heads * key_dim + heads * value_dim or tuple(state.shape[1:]) != (heads, value_dim, key_dim) or heads % qk_heads
+            or tuple(out.shape) != (qkv.shape[0], heads * value_dim) or key_dim > CHUNK_MAX_ROWS or tuple(scratch.shape) != shape
+            or dt_bias.numel() != heads or a_log.numel() != heads):
+        raise KernelError("delta_chunks: shapes do not fit the sizes")
+    p, splits, stride, cols = _projection(proj)
+    if min(b_col, a_col) < 0 or max(b_col, a_col) + heads > cols:
+        raise KernelError("delta_chunks: write strengths or decays lie outside the projection")
+    fn = _fn("recurrent_chunks", "tt_delta_chunks", [c_void_p, c_int, c_void_p, c_int, c_longlong, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p,
+                                                     c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p])
+    _check(fn(_ptr(qkv), qkv.shape[1], p, splits, stride, cols, b_col, a_col, _ptr(dt_bias), _ptr(a_log), _ptr(state), _ptr(out), _ptr(scratch),
+              _ptr(cu), _ptr(slots), sequences, shape[0], heads, qk_heads, key_dim, value_dim, sm_count(qkv.device), _stream()), "delta_chunks", 2)
 
 
 def delta_scan(qkv: torch.Tensor, proj: torch.Tensor, b_col: int, a_col: int, dt_bias: torch.Tensor | None, a_log: torch.Tensor | None,
