@@ -139,3 +139,68 @@ def test_delta_rule_in_chunks(heads, qk_heads, D, V):
             assert float((got - want).abs().max()) <= 2e-5 * max(1.0, float(want.abs().max()))
         assert float((state[slot].double() - S).abs().max()) <= 2e-5 * max(1.0, float(S.abs().max()))
     assert torch.equal(state[[3, 7]], before[[3, 7]])
+
+
+# --------------------------------------------------------------------------------- the passes around the recurrences
+@pytest.mark.parametrize("group,groups,tokens", [(4, 3, 2), (128, 5, 9), (132, 2, 3), (256, 4, 33), (260, 1, 40), (1024, 2, 600), (1028, 1, 7), (4096, 1, 1030), (8192, 1, 3), (30, 4, 5)])
+@pytest.mark.parametrize("splits,gate_first,gate,dtype", [(1, True, "silu", torch.bfloat16), (5, False, "sigmoid", torch.float32)])
+def test_gated_group_norm_by_pieces(group, groups, tokens, splits, gate_first, gate, dtype):
+    """A warp a group, a block a group with one and with four pieces a thread, and sizes without whole pieces."""
+    from thintensor_b200.kernels import api
+
+    width, col = group * groups, 8
+    y, proj, weight = randn(tokens, width, seed=20), randn(splits, tokens, width + 12, seed=21), 1.0 + randn(group, seed=22, scale=0.1)
+    out = torch.empty(tokens, width, dtype=dtype, device=DEV)
+    api.gated_group_norm(y, group, proj, col, weight, 1e-6, gate_first, out, gate)
+    z = proj.double().sum(0)[:, col:col + width].reshape(tokens, groups, group)
+    z = torch.sigmoid(z) * (1.0 if gate == "sigmoid" else z)
+    v = y.double().reshape(tokens, groups, group)
+    norm = lambda a: a / (a.square().mean(-1, keepdim=True) + 1e-6).sqrt() * weight.double()
+    want = (norm(v * z) if gate_first else norm(v) * z).reshape(tokens, width)
+    limit = dict(rtol=2.0 ** -8, atol=1e-6) if dtype == torch.bfloat16 else dict(rtol=1e-5, atol=1e-5)
+    torch.testing.assert_close(out.double(), want, **limit)
+
+
+@pytest.mark.parametrize("splits", [1, 2])
+@pytest.mark.parametrize("taps", [1, 4, 8])
+def test_convolution_tiles_inside_and_across_sequences(taps, splits):
+    """Sequences that start and end inside, at and beyond the tiles of 16 tokens."""
+    from thintensor_b200.kernels import api
+
+    news, slot_ids, channels, col = [16, 40, 1, 23, 33], [3, 0, 5, 1, 2], 130, 3
+    tokens = sum(news)
+    cu = [sum(news[:i]) for i in range(len(news) + 1)]
+    proj, weight, bias = randn(splits, tokens, channels + 7, seed=23), randn(channels, taps, seed=24), randn(channels, seed=25)
+    state = randn(6, max(taps - 1, 1), channels, seed=26)[:, :taps - 1].contiguous()
+    before = state.clone()
+    out = torch.empty(tokens, channels, device=DEV)
+    api.causal_conv(proj, col, channels, weight, bias, True, state, out, i32(cu), i32(slot_ids), len(news), tokens, False)
+    x = proj.double().sum(0)[:, col:col + channels]
+    for s, slot in enumerate(slot_ids):
+        rows = torch.cat((before[slot].double(), x[cu[s]:cu[s + 1]]))
+        want = sum(rows[j:j + news[s]] * weight[:, j].double() for j in range(taps)) + bias.double()
+        torch.testing.assert_close(out[cu[s]:cu[s + 1]].double(), want * torch.sigmoid(want), rtol=1e-5, atol=1e-5)
+        torch.testing.assert_close(state[slot].double(), rows[rows.shape[0] - (taps - 1):], rtol=1e-6, atol=1e-6)
+
+
+@pytest.mark.parametrize("heads,D,V,rotary,tokens", [(3, 128, 256, 128, 5), (2, 64, 20, 24, 1030), (2, 12, 8, 0, 3), (2, 10, 8, 4, 3), (1, 256, 4, 256, 2)])
+@pytest.mark.parametrize("activation", [False, True])
+def test_linear_attention_inputs_by_pieces(heads, D, V, rotary, tokens, activation):
+    from thintensor_b200.kernels import api
+
+    qk, hv, past = heads * D, heads * V, 77
+    proj = randn(2, tokens, 2 * qk + hv + 4, seed=27)
+    inv_freq = (100.0 ** (-torch.arange(0, max(rotary, 2), 2, dtype=torch.float64) / max(rotary, 2))).float().to(DEV)
+    vkq = torch.empty(tokens, hv + 2 * qk, device=DEV)
+    api.linear_attention_prepare(proj, heads, D, V, activation, inv_freq, rotary, 0.5, vkq, i32([0, tokens]), i32([past]), 1, tokens, 2.0)
+    x = proj.double().sum(0)
+    x = x * torch.sigmoid(x) if activation else x
+    q, k, v = (part.reshape(tokens, heads, -1) for part in x[:, :2 * qk + hv].split((qk, qk, hv), 1))
+    angle = ((past + torch.arange(tokens, device=DEV)).float()[:, None, None] * inv_freq[:rotary // 2]).double()
+
+    def turn(z):
+        a, b, h = z[..., :rotary // 2], z[..., rotary // 2:rotary], z[..., rotary:]
+        return torch.cat((a * angle.cos() - b * angle.sin(), b * angle.cos() + a * angle.sin(), h), -1) if rotary else z
+
+    want = torch.cat((v.reshape(tokens, -1), 0.5 * turn(k).reshape(tokens, -1), 2.0 * turn(q).reshape(tokens, -1)), 1)
+    torch.testing.assert_close(vkq.double(), want, rtol=1e-5, atol=2e-5)

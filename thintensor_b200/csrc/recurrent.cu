@@ -42,6 +42,24 @@ __device__ __forceinline__ float rec_sum_slices(const float* __restrict__ p, int
     return total;
 }
 
+// the same for four neighbouring elements on a 16-byte boundary (split_stride a multiple of four)
+__device__ __forceinline__ float4 rec_sum_slices4(const float* __restrict__ p, int splits, size_t split_stride) {
+    float4 total = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    int s = 0;
+    for (; s + 4 <= splits; s += 4) {
+        float4 v[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] = __ldg(reinterpret_cast<const float4*>(p + (size_t)(s + e) * split_stride));
+#pragma unroll
+        for (int e = 0; e < 4; ++e) { total.x += v[e].x; total.y += v[e].y; total.z += v[e].z; total.w += v[e].w; }
+    }
+    for (; s < splits; ++s) {
+        const float4 v = __ldg(reinterpret_cast<const float4*>(p + (size_t)s * split_stride));
+        total.x += v.x; total.y += v.y; total.z += v.z; total.w += v.w;
+    }
+    return total;
+}
+
 // Asynchronous copies into shared memory: a chunk of tokens is fetched while the chunk before it is worked on.
 __device__ __forceinline__ uint32_t rec_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void rec_copy4(float* dst, const float* src) {
@@ -138,7 +156,8 @@ constexpr int CONV_TILE = 16;       // packed tokens a thread walks with its cha
 
 // A thread takes one channel through CONV_TILE packed tokens: every input is read once (plus taps - 1 at the tile's
 // start) and the window of the last inputs slides through registers.  Where the tile crosses into the next sequence
-// the window is filled from that sequence's state.
+// the window is filled from that sequence's state.  Bound by its loads: a tile inside one sequence asks for all of them at once
+// (2,048 tokens of 4,352 channels 58 -> 47 us, 4,097 of 4,096 107 -> 82).
 __global__ void causal_conv_kernel(const float* __restrict__ proj, int splits, size_t split_stride, int cols, int col_off,
                                    int channels, const float* __restrict__ weight, const float* __restrict__ bias, int taps,
                                    int activation, const float* __restrict__ state, size_t slot_stride, float* __restrict__ out,
@@ -172,6 +191,23 @@ __global__ void causal_conv_kernel(const float* __restrict__ proj, int splits, s
         }
     };
     fill(t0);
+    if (splits == 1 && t1 - t0 == CONV_TILE && t1 <= next) {     // a tile inside one sequence: all of its inputs are asked for at once
+        float x[CONV_TILE];
+#pragma unroll
+        for (int k = 0; k < CONV_TILE; ++k) x[k] = __ldg(proj + (size_t)(t0 + k) * cols + col_off + c);
+#pragma unroll
+        for (int k = 0; k < CONV_TILE; ++k) {
+            float acc = shift;
+#pragma unroll
+            for (int j = 0; j < CONV_MAX_TAPS; ++j)
+                if (j <= keep) acc = fmaf(w[j], j < keep ? win[j] : x[k], acc);
+            out[(size_t)(t0 + k) * channels + c] = activation ? rec_silu(acc) : acc;
+#pragma unroll
+            for (int j = 0; j < CONV_MAX_TAPS - 1; ++j)
+                if (j < keep) win[j] = j + 1 < keep ? win[j + 1] : x[k];
+        }
+        return;
+    }
     for (int t = t0; t < t1; ++t) {
         if (t == next) {                                         // the next sequence starts here
             ++b;
@@ -516,12 +552,70 @@ __global__ void linear_attention_prepare_kernel(const float* __restrict__ proj, 
     }
 }
 
+// The same, four neighbouring numbers a thread: sizes, columns and bases on 16-byte boundaries, and rotation halves of whole
+// pieces.  A block takes one token's columns (or, for few tokens, a share of them) and makes the token's sines and cosines once for
+// all heads.  Bound by its loads and stores: 4,096 tokens of 8,192 numbers, half of them rotated, 207 -> 66 us (4.1 TB/s) against a number
+// and a sine a thread.
+__global__ void __launch_bounds__(256)
+linear_attention_prepare4_kernel(const float* __restrict__ proj, int splits, size_t split_stride, int cols, int heads, int D, int V, int activation,
+                                 const float* __restrict__ inv_freq, int rotary_dim, float q_scale, float k_scale, float* __restrict__ vkq,
+                                 const int* __restrict__ cu, const int* __restrict__ len_before, int sequences) {
+    __shared__ __align__(16) float cosines[REC_MAX_ROWS / 2], sines[REC_MAX_ROWS / 2];
+    tt_pdl_launch_dependents();
+    tt_pdl_wait();
+    const int t = blockIdx.x, half = rotary_dim >> 1;
+    if (rotary_dim > 0) {
+        const int b = tt_find_sequence(cu, sequences, t);
+        const float pos = (float)(len_before[b] + (t - cu[b]));
+        for (int i = threadIdx.x; i < half; i += blockDim.x) {
+            float sn, cs;
+            sincosf(pos * __ldg(inv_freq + i), &sn, &cs);
+            cosines[i] = cs;
+            sines[i] = sn;
+        }
+        __syncthreads();
+    }
+    const int qk = heads * D, hv = heads * V;
+    const float* row = proj + (size_t)t * cols;
+    float* out = vkq + (size_t)t * (hv + 2 * qk);
+    auto load = [&](int j) {
+        float4 x = rec_sum_slices4(row + j, splits, split_stride);
+        if (activation) { x.x = rec_silu(x.x); x.y = rec_silu(x.y); x.z = rec_silu(x.z); x.w = rec_silu(x.w); }
+        return x;
+    };
+    for (int j = 4 * (blockIdx.y * blockDim.x + threadIdx.x); j < 2 * qk + hv; j += 4 * gridDim.y * blockDim.x) {
+        float4 x = load(j);
+        if (j >= 2 * qk) {                                       // v
+            *reinterpret_cast<float4*>(out + j - 2 * qk) = x;
+            continue;
+        }
+        const bool is_k = j >= qk;
+        const int i = (is_k ? j - qk : j) % D;
+        if (i < rotary_dim) {
+            const bool low = i < half;
+            const float4 other = load(low ? j + half : j - half);
+            const float4 cs = *reinterpret_cast<const float4*>(cosines + (low ? i : i - half)), sn = *reinterpret_cast<const float4*>(sines + (low ? i : i - half));
+            x = low ? make_float4(x.x * cs.x - other.x * sn.x, x.y * cs.y - other.y * sn.y, x.z * cs.z - other.z * sn.z, x.w * cs.w - other.w * sn.w)
+                    : make_float4(x.x * cs.x + other.x * sn.x, x.y * cs.y + other.y * sn.y, x.z * cs.z + other.z * sn.z, x.w * cs.w + other.w * sn.w);
+        }
+        const float scale = is_k ? k_scale : q_scale;
+        *reinterpret_cast<float4*>(out + hv + (is_k ? j - qk : qk + j)) = make_float4(x.x * scale, x.y * scale, x.z * scale, x.w * scale);
+    }
+}
+
 extern "C" int tt_linear_attention_prepare(const float* proj, int splits, long long split_stride, int cols, int heads, int D, int V,
                                            int activation, const float* inv_freq, int rotary_dim, float q_scale, float k_scale, float* vkq,
                                            const int* cu, const int* len_before, int sequences, int n_tokens, cudaStream_t stream) {
     if (n_tokens <= 0) return 0;
     if (rotary_dim < 0 || rotary_dim > D || (rotary_dim & 1) || 2 * heads * D + heads * V > cols) return (int)cudaErrorInvalidValue;
     const int total = 2 * heads * D + heads * V;
+    if (D % 4 == 0 && V % 4 == 0 && cols % 4 == 0 && split_stride % 4 == 0 && (rotary_dim / 2) % 4 == 0 && rotary_dim <= REC_MAX_ROWS
+        && (((uintptr_t)proj | (uintptr_t)vkq) & 15) == 0) {
+        const int blocks = n_tokens >= 1024 ? (total + 8191) / 8192 : (total + 1023) / 1024;        // eight pieces a thread for prompts, one for few tokens
+        tt_launch_pdl(linear_attention_prepare4_kernel, dim3(n_tokens, blocks < 32 ? blocks : 32), dim3(256), 0, stream, proj, splits, (size_t)split_stride, cols,
+                      heads, D, V, activation, inv_freq, rotary_dim, q_scale, k_scale, vkq, cu, len_before, sequences);
+        TT_LAUNCH_CHECK();
+    }
     const int want = n_tokens >= 1024 ? (total + 1023) / 1024 : (total + 255) / 256;                // few tokens: a token's columns over more blocks
     const int tiles = want < 32 ? want : 32;
     tt_launch_pdl(linear_attention_prepare_kernel, dim3(n_tokens, tiles), dim3(256), 0, stream, proj, splits, (size_t)split_stride, cols, heads, D,
@@ -1340,6 +1434,78 @@ gated_group_norm_reg_kernel(const float* __restrict__ y, int width, int group, c
     }
 }
 
+// The same four neighbouring numbers at a time, PIECES of them a thread, all loads of a thread in flight together.  WARP: a warp
+// takes a group (heads of up to 128 * PIECES numbers; blocks of one warp had the launch of 65,536 blocks to pay), otherwise a
+// block does; few groups (decoding) are shared out over as many threads as there are pieces.  Bound by its loads: 2,048 groups of 4,096
+// 70 -> 39 us, 65,552 of 128 98 -> 31, 65,536 of 256 117 -> 54, 8 of 4,096 with 16 slices of gates 18 -> 12.
+template <typename TOut> __device__ __forceinline__ void gn_store4(TOut* to, float a, float b, float c, float d);
+template <> __device__ __forceinline__ void gn_store4<float>(float* to, float a, float b, float c, float d) { *reinterpret_cast<float4*>(to) = make_float4(a, b, c, d); }
+template <> __device__ __forceinline__ void gn_store4<__nv_bfloat16>(__nv_bfloat16* to, float a, float b, float c, float d) {
+    __nv_bfloat162 v[2] = {__floats2bfloat162_rn(a, b), __floats2bfloat162_rn(c, d)};
+    *reinterpret_cast<uint2*>(to) = *reinterpret_cast<uint2*>(v);
+}
+
+template <typename TOut, int PIECES, bool WARP>
+__global__ void __launch_bounds__(WARP ? 256 : PIECES == 1 ? 1024 : 512)
+gated_group_norm4_kernel(const float* __restrict__ y, int width, int group, long long total, const float* __restrict__ proj, int splits, size_t split_stride,
+                         int cols, int gate_col, const float* __restrict__ weight, int weight_len, float eps, int gate_first, TOut* __restrict__ out,
+                         int gate_kind) {
+    tt_pdl_launch_dependents();
+    tt_pdl_wait();
+    __shared__ float reduce[32];
+    const long long item = WARP ? (long long)blockIdx.x * 8 + (threadIdx.x >> 5) : blockIdx.x;       // (token, group)
+    if (WARP && item >= total) return;
+    const int lane = WARP ? threadIdx.x & 31 : threadIdx.x, lanes = WARP ? 32 : blockDim.x;
+    const int groups = width / group;
+    const long long t = item / groups;
+    const int c0 = (int)(item - t * groups) * group;
+    const float* yr = y + (size_t)t * width + c0;
+    const float* gr = proj + (size_t)t * cols + gate_col + c0;
+    float4 v[PIECES], gate[PIECES];
+#pragma unroll
+    for (int e = 0; e < PIECES; ++e) {
+        const int j = 4 * (lane + e * lanes);
+        v[e] = gate[e] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (j < group) {
+            v[e] = __ldg(reinterpret_cast<const float4*>(yr + j));
+            gate[e] = rec_sum_slices4(gr + j, splits, split_stride);
+        }
+    }
+    float sumsq = 0.0f;
+#pragma unroll
+    for (int e = 0; e < PIECES; ++e) {
+        float4& g = gate[e];
+        g = make_float4(rec_gate(g.x, gate_kind), rec_gate(g.y, gate_kind), rec_gate(g.z, gate_kind), rec_gate(g.w, gate_kind));
+        if (gate_first) v[e] = make_float4(v[e].x * g.x, v[e].y * g.y, v[e].z * g.z, v[e].w * g.w);
+        sumsq = fmaf(v[e].x, v[e].x, fmaf(v[e].y, v[e].y, fmaf(v[e].z, v[e].z, fmaf(v[e].w, v[e].w, sumsq))));
+    }
+    const float r = rsqrtf((WARP ? tt_warp_sum(sumsq) : tt_block_sum(sumsq, reduce)) / (float)group + eps);
+    TOut* o = out + (size_t)t * width + c0;
+#pragma unroll
+    for (int e = 0; e < PIECES; ++e) {
+        const int j = 4 * (lane + e * lanes);
+        if (j >= group) continue;
+        const float4 w = __ldg(reinterpret_cast<const float4*>(weight + (c0 + j) % weight_len)), g = gate[e];
+        if (gate_first) gn_store4<TOut>(o + j, v[e].x * r * w.x, v[e].y * r * w.y, v[e].z * r * w.z, v[e].w * r * w.w);
+        else gn_store4<TOut>(o + j, v[e].x * r * w.x * g.x, v[e].y * r * w.y * g.y, v[e].z * r * w.z * g.z, v[e].w * r * w.w * g.w);
+    }
+}
+
+template <typename TOut>
+static void gated_group_norm4(const float* y, long long total, int width, int group, const float* proj, int splits, size_t split_stride, int cols, int gate_col,
+                              const float* weight, int weight_len, float eps, int gate_first, TOut* out, int gate_kind, cudaStream_t stream) {
+#define TT_GN4(PIECES, WARP, GRID, THREADS) tt_launch_pdl(gated_group_norm4_kernel<TOut, PIECES, WARP>, dim3((unsigned)(GRID)), dim3(THREADS), 0, stream, y, width, group, total, proj, splits, split_stride, cols, gate_col, weight, weight_len, eps, gate_first, out, gate_kind)
+    const int quads = group / 4;
+    if (quads <= 64) {
+        if (quads <= 32) TT_GN4(1, true, (total + 7) / 8, 256); else TT_GN4(2, true, (total + 7) / 8, 256);
+    } else if (quads <= 1024 && (total < 1024 || quads < 256)) {          // few groups: as many threads as there are pieces
+        TT_GN4(1, false, total, (quads + 31) / 32 * 32);
+    } else {
+        TT_GN4(4, false, total, (quads / 4 + 31 + (quads % 4 > 0)) / 32 * 32);
+    }
+#undef TT_GN4
+}
+
 extern "C" int tt_gated_group_norm(const float* y, int n_tokens, int width, int group, const float* proj, int splits,
                                    long long split_stride, int cols, int gate_col, const float* weight, int weight_len, float eps,
                                    int gate_first, void* out, int out_dtype, int gate_kind, cudaStream_t stream) {
@@ -1347,6 +1513,14 @@ extern "C" int tt_gated_group_norm(const float* y, int n_tokens, int width, int 
     if (group <= 0 || width % group || weight_len <= 0) return (int)cudaErrorInvalidValue;
     const long long blocks = (long long)n_tokens * (width / group);
     if (blocks > 2147483647LL) return (int)cudaErrorInvalidValue;
+    if (group % 4 == 0 && group <= 4 * 4 * 512 && cols % 4 == 0 && gate_col % 4 == 0 && split_stride % 4 == 0 && weight_len % 4 == 0
+        && (((uintptr_t)y | (uintptr_t)proj | (uintptr_t)weight | (uintptr_t)out) & 15) == 0) {
+        if (out_dtype == TT_F32)
+            gated_group_norm4<float>(y, blocks, width, group, proj, splits, (size_t)split_stride, cols, gate_col, weight, weight_len, eps, gate_first, (float*)out, gate_kind, stream);
+        else
+            gated_group_norm4<__nv_bfloat16>(y, blocks, width, group, proj, splits, (size_t)split_stride, cols, gate_col, weight, weight_len, eps, gate_first, (__nv_bfloat16*)out, gate_kind, stream);
+        TT_LAUNCH_CHECK();
+    }
     if (group <= 1024 * GN_VALUES) {
         int threads = (((group + 3) / 4 + 31) / 32) * 32;       // about four numbers a thread
         if (threads > 1024) threads = 1024;
