@@ -204,3 +204,68 @@ def test_linear_attention_inputs_by_pieces(heads, D, V, rotary, tokens, activati
 
     want = torch.cat((v.reshape(tokens, -1), 0.5 * turn(k).reshape(tokens, -1), 2.0 * turn(q).reshape(tokens, -1)), 1)
     torch.testing.assert_close(vkq.double(), want, rtol=1e-5, atol=2e-5)
+
+
+# ------------------------------------------------------------------------------------ exact attention in tiles of 32 queries
+@pytest.mark.parametrize("heads,kv_heads,D,V", [(4, 2, 64, 64), (3, 1, 128, 128), (2, 2, 48, 80), (2, 1, 16, 112), (2, 1, 30, 17)])
+@pytest.mark.parametrize("window,sink,cap", [(0, False, 0.0), (40, True, 5.0), (-48, False, 0.0)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_exact_attention_tiles(heads, kv_heads, D, V, window, sink, cap, dtype):
+    """Sequences that end inside, at and behind tiles and cache blocks, with and without a past; whatever lies in the cache beside what
+    is seen is no number, and one late value is not either: only its own query and the later ones may meet it."""
+    from thintensor_b200.kernels import api
+
+    news, past = [31, 64, 1, 33, 65], [0, 40, 63, 64, 5]
+    tokens, sequences = sum(news), len(news)
+    cu = [sum(news[:i]) for i in range(sequences + 1)]
+    width = 4
+    blocks = sequences * width
+    order = torch.randperm(blocks, generator=torch.Generator().manual_seed(1)).tolist()
+    k_pool = torch.full((blocks, kv_heads, 64, D), float("nan"), dtype=dtype, device=DEV)
+    v_pool = torch.full((blocks, kv_heads, V, 64), float("nan"), dtype=dtype, device=DEV)
+    table = [[order[s * width + i] if i * 64 < past[s] + news[s] else -1 for i in range(width)] for s in range(sequences)]
+    q = randn(tokens, heads * D, seed=30, dtype=dtype)
+    sinks = randn(heads, seed=31) if sink else None
+    slopes = randn(heads, seed=32).abs() * 0.01 if cap else None
+    gate = randn(2, tokens, heads * V, seed=33) if window > 0 else None
+    values, keys = [], []
+    for s in range(sequences):
+        n = past[s] + news[s]
+        k, v = randn(n, kv_heads, D, seed=40 + s, dtype=dtype), randn(n, kv_heads, V, seed=50 + s, dtype=dtype)
+        keys.append(k)
+        values.append(v)
+        for i in range(-(-n // 64)):
+            part = slice(64 * i, min(n, 64 * i + 64))
+            k_pool[table[s][i], :, :part.stop - part.start] = k[part].transpose(0, 1)
+            v_pool[table[s][i], :, :, :part.stop - part.start] = v[part].permute(1, 2, 0)
+    poisoned = past[1] + 20                                     # a place of the second sequence
+    v_pool[table[1][poisoned // 64], :, :, poisoned % 64] = float("nan")
+    out = torch.full((tokens, heads * V), 7.0, dtype=dtype, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    api.attention(q, k_pool, v_pool, i32(table), i32(cu), i32(past), sequences, tokens, heads, kv_heads, D, D ** -0.5, window, 1, out, None, None, status,
+                  value_dim=V, sinks=sinks, softcap=cap, slopes=slopes, gate=gate)
+    assert int(status) == 0
+    for s in range(sequences):
+        n = past[s] + news[s]
+        for h in range(heads):
+            place = past[s] + torch.arange(news[s], device=DEV)
+            key = torch.arange(n, device=DEV)
+            score = q[cu[s]:cu[s + 1]].double().reshape(-1, heads, D)[:, h] @ keys[s][:, h // (heads // kv_heads)].double().T * D ** -0.5
+            if cap:
+                score = cap * torch.tanh(score / cap) - slopes[h].double() * (place[:, None] - key[None])
+            seen = key[None] <= place[:, None]
+            if window > 0:
+                seen &= key[None] > place[:, None] - window
+            if window < 0:
+                seen &= key[None] >= (place - place % -window)[:, None]
+            score = score.masked_fill(~seen, -float("inf"))
+            if sink:
+                score = torch.cat((score, sinks[h].double().expand(news[s], 1)), 1)
+            want = torch.softmax(score, -1)[:, :n] @ values[s][:, h // (heads // kv_heads)].double()
+            if gate is not None:
+                want = want * torch.sigmoid(gate.double().sum(0)[cu[s]:cu[s + 1], h * V:(h + 1) * V])
+            got = out[cu[s]:cu[s + 1]].double().reshape(-1, heads, V)[:, h]
+            clean = ~seen[:, poisoned] if s == 1 else torch.ones(news[s], dtype=torch.bool, device=DEV)
+            limit = dict(rtol=2e-5, atol=2e-5) if dtype == torch.float32 else dict(rtol=2.0 ** -8, atol=1e-4)
+            torch.testing.assert_close(got[clean], want[clean], **limit)
+            assert bool(got[~clean].isnan().all())

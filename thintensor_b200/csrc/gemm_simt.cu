@@ -152,19 +152,24 @@ gemm_simt_kernel(const TX* __restrict__ x, long long ldx, const TW* __restrict__
 
 // Skinny form for few rows of x (decoding, the few wanted rows of a head): a warp takes four output columns and up to 8 rows of x
 // at a time, its lanes stride over k four numbers each, so that a lane has four 16-byte loads of weights in flight, a round ahead
-// of their use, and a number of x that it fetched (from the L1) serves four columns.  Bound by reading the weights where there are enough
-// columns: 4 rows of 128,256 x 2,048 float32 weights 793 -> 254 us (4.1 TB/s) against a warp per column with 4-byte loads.
-constexpr int GR_COLS = 4, GR_ROWS = 8, GR_WARPS = 4;
+// of their use, and a number of x that it fetched (from the L1) serves four columns.  Where there are too few columns for eight warps an SM,
+// the four warps of a block take the same columns and walk k by turns.  Bound by reading the weights (us against a warp per
+// column with 4-byte loads, float32): 1 and 4 rows of 128,256 x 2,048 761 -> 157 (6.7 TB/s) and 823 -> 205, 8 of 16,384 x 2,048 181 -> 92,
+// 8 of 2,048 x 8,192 238 -> 34, 3 of 3,072 x 2,048 35 -> 11.
+// GR_ROWS: rows of x at a time (1, 4 or 8, the least that holds m: fewer sums a lane, more warps an SM).
+constexpr int GR_COLS = 4, GR_WARPS = 4;
 
-template <typename TX, typename TW>
+template <typename TX, typename TW, int GR_ROWS>
 __global__ void __launch_bounds__(GR_WARPS * 32)
 gemm_rows_kernel(const TX* __restrict__ x, long long ldx, const TW* __restrict__ w, long long ldw,
                  const float* __restrict__ bias, float* __restrict__ out, long long ldo, int m, int n,
-                 int k, int vec_x, int vec_w) {
+                 int k, int vec_x, int vec_w, int k_warps) {
+    __shared__ float sums[GR_WARPS][GR_ROWS][GR_COLS];
     tt_pdl_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int col = (blockIdx.x * GR_WARPS + warp) * GR_COLS;
-    if (col >= n) return;
+    // k_warps (1 or all): so many warps share four columns and walk k by turns
+    const int col = (k_warps > 1 ? (int)blockIdx.x : (int)blockIdx.x * GR_WARPS + warp) * GR_COLS, k0 = (k_warps > 1 ? warp * 128 : 0) + lane * 4, step = 128 * k_warps;
+    if (col >= n) return;                                       // with shared columns the whole block leaves
     float wv[GR_COLS][4];
     auto weights = [&](int kk) {
         const int count = max(0, min(4, k - kk));
@@ -173,19 +178,19 @@ gemm_rows_kernel(const TX* __restrict__ x, long long ldx, const TW* __restrict__
     };
     tt_pdl_wait();
     for (int m0 = 0; m0 < m; m0 += GR_ROWS) {
-        weights(lane * 4);
+        weights(k0);
         float acc[GR_ROWS][GR_COLS];
 #pragma unroll
         for (int i = 0; i < GR_ROWS; ++i)
 #pragma unroll
             for (int c = 0; c < GR_COLS; ++c) acc[i][c] = 0.0f;
-        for (int kk = lane * 4; kk < k; kk += 128) {
+        for (int kk = k0; kk < k; kk += step) {
             float now[GR_COLS][4];
 #pragma unroll
             for (int c = 0; c < GR_COLS; ++c)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) now[c][e] = wv[c][e];
-            if (kk + 128 < k) weights(kk + 128);
+            if (kk + step < k) weights(kk + step);
             const int count = min(4, k - kk);
 #pragma unroll
             for (int i = 0; i < GR_ROWS; ++i) {
@@ -198,13 +203,26 @@ gemm_rows_kernel(const TX* __restrict__ x, long long ldx, const TW* __restrict__
                     for (int c = 0; c < GR_COLS; ++c) acc[i][c] = fmaf(xv[e], now[c][e], acc[i][c]);
             }
         }
+        if (k_warps > 1) __syncthreads();                       // the rows before are written
 #pragma unroll
         for (int i = 0; i < GR_ROWS; ++i) {
             if (m0 + i >= m) break;
 #pragma unroll
             for (int c = 0; c < GR_COLS; ++c) {
                 const float total = tt_warp_sum(acc[i][c]);
-                if (lane == 0 && col + c < n) out[(size_t)(m0 + i) * ldo + col + c] = total + (bias ? bias[col + c] : 0.0f);
+                if (lane) continue;
+                if (k_warps > 1) sums[warp][i][c] = total;
+                else if (col + c < n) out[(size_t)(m0 + i) * ldo + col + c] = total + (bias ? bias[col + c] : 0.0f);
+            }
+        }
+        if (k_warps > 1) {
+            __syncthreads();
+            const int i = threadIdx.x / GR_COLS, c = threadIdx.x % GR_COLS;
+            if (i < GR_ROWS && m0 + i < m && col + c < n) {
+                float total = 0.0f;
+#pragma unroll
+                for (int s = 0; s < GR_WARPS; ++s) total += sums[s][i][c];
+                out[(size_t)(m0 + i) * ldo + col + c] = total + (bias ? bias[col + c] : 0.0f);
             }
         }
     }
@@ -219,9 +237,11 @@ static int launch(const void* x, long long ldx, const void* w, long long ldw, co
                   long long ldo, long long split_stride, int m, int n, int k, int splits, cudaStream_t stream) {
     const int vec_x = vec4<TX>(x, ldx), vec_w = vec4<TW>(w, ldw);
     if (m <= 16 && splits == 1) {
-        const int cols = GR_WARPS * GR_COLS;
-        tt_launch_pdl(gemm_rows_kernel<TX, TW>, dim3((n + cols - 1) / cols), dim3(GR_WARPS * 32), 0, stream, (const TX*)x, ldx, (const TW*)w, ldw, bias, out,
-                      ldo, m, n, k, vec_x, vec_w);
+        // fewer than eight warps an SM: the four warps of a block share its columns
+        const int k_warps = n < 8 * GR_COLS * 148 ? GR_WARPS : 1, cols = k_warps > 1 ? GR_COLS : GR_WARPS * GR_COLS;
+#define TT_ROWS(ROWS) tt_launch_pdl(gemm_rows_kernel<TX, TW, ROWS>, dim3((n + cols - 1) / cols), dim3(GR_WARPS * 32), 0, stream, (const TX*)x, ldx, (const TW*)w, ldw, bias, out, ldo, m, n, k, vec_x, vec_w, k_warps)
+        if (m == 1) TT_ROWS(1); else if (m <= 4) TT_ROWS(4); else TT_ROWS(8);
+#undef TT_ROWS
         TT_LAUNCH_CHECK();
     }
     int k_per_split = (k + splits - 1) / splits;
