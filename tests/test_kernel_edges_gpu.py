@@ -70,21 +70,22 @@ def test_recurrence_in_chunks(heads, groups, P, N, pad, fixed):
     tokens, inner, sequences = sum(news), heads * P, len(news)
     width = inner + 2 * groups * N + pad
     rows = randn(tokens, width, seed=5)
-    x, b, c = rows[:, :inner], rows[:, inner:inner + groups * N], rows[:, inner + groups * N:inner + 2 * groups * N]
+    x, b, c = rows[:, pad:pad + inner], rows[:, pad + inner:pad + inner + groups * N], rows[:, pad + inner + groups * N:pad + inner + 2 * groups * N]
+    places = (pad, pad + inner, pad + inner + groups * N)
     state = randn(8, heads, P, N, seed=6)
     before = state.clone()
     cu = [sum(news[:i]) for i in range(sequences + 1)]
     y = torch.full((tokens, inner), 7.0, device=DEV)
     a_log, dt_bias, skip = randn(heads, seed=7, scale=2.0), randn(heads, seed=8), randn(heads, seed=9)
     raw = randn(2, tokens, heads + 3, seed=10)
-    scores, factors = (torch.full(shape, float("nan"), device=DEV) for shape in api.scan_chunks_scratch(tokens, sequences, heads, groups))
+    scratch = torch.full(api.scan_chunks_scratch(tokens, sequences, heads, groups), float("nan"), device=DEV)
     if fixed:
         constant = torch.tensor([0.97, 0.0, 1.0, -0.8], device=DEV).repeat(heads)[:heads].contiguous()
-        api.scan_chunks(x, b, c, state, y, i32(cu), i32(slot_ids), sequences, heads, P, N, groups, scores, factors, fixed_decay=constant)
+        api.scan_chunks(rows, *places, state, y, i32(cu), i32(slot_ids), sequences, heads, P, N, groups, scratch, fixed_decay=constant)
         dt = torch.ones(tokens, heads, device=DEV, dtype=torch.float64)
         decay, skip = constant.double().expand(tokens, heads), torch.zeros(heads, device=DEV)
     else:
-        api.scan_chunks(x, b, c, state, y, i32(cu), i32(slot_ids), sequences, heads, P, N, groups, scores, factors, steps=(raw, 2, dt_bias, a_log, skip))
+        api.scan_chunks(rows, *places, state, y, i32(cu), i32(slot_ids), sequences, heads, P, N, groups, scratch, steps=(raw, 2, dt_bias, a_log, skip))
         dt = torch.nn.functional.softplus(raw.double().sum(0)[:, 2:2 + heads] + dt_bias.double())
         decay = torch.exp(-torch.exp(a_log.double()) * dt)
     each = heads // groups
@@ -269,3 +270,50 @@ def test_exact_attention_tiles(heads, kv_heads, D, V, window, sink, cap, dtype):
             limit = dict(rtol=2e-5, atol=2e-5) if dtype == torch.float32 else dict(rtol=2.0 ** -8, atol=1e-4)
             torch.testing.assert_close(got[clean], want[clean], **limit)
             assert bool(got[~clean].isnan().all())
+
+
+# ------------------------------------------------------------------------- latent attention: several tokens of a head together
+@pytest.mark.parametrize("heads,dim,rot,V,rank,dtype,tensor_cores", [
+    (16, 64, 64, 128, 512, torch.bfloat16, True), (5, 24, 16, 20, 48, torch.bfloat16, True), (20, 9, 32, 33, 144, torch.bfloat16, True),
+    (3, 20, 10, 17, 40, torch.float32, False), (2, 16, 8, 12, 20, torch.float32, False),
+])
+@pytest.mark.parametrize("tokens", [1, 7, 8, 13])
+@pytest.mark.parametrize("gate", [None, "head", "each"])
+def test_latent_decode_groups(heads, dim, rot, V, rank, dtype, tensor_cores, tokens, gate):
+    """One token for each of as many sequences: fewer than a group, a whole one, and one and a part; slices that lie in one cache block and in
+    two, empty ones, and heads that do not fill sixteen rows."""
+    from thintensor_b200.kernels import api
+
+    window, scale, row = 100, (dim + rot) ** -0.5, rank + rot
+    past = [(37 * i + 63) % 190 for i in range(tokens)]
+    width = 3
+    pool = randn(tokens * width, 1, 64, row, seed=60, dtype=dtype)
+    order = torch.randperm(tokens * width, generator=torch.Generator().manual_seed(2)).tolist()
+    table = [order[i * width:(i + 1) * width] for i in range(tokens)]
+    q = randn(2, tokens, heads * (dim + rot), seed=61)
+    w_key, w_value = (randn(heads * n, rank, seed=62 + i, scale=rank ** -0.5, dtype=dtype) for i, n in enumerate((dim, V)))
+    gates = None if gate is None else randn(3, tokens, heads if gate == "head" else heads * V, seed=64)
+    inv_freq = torch.tensor([1.0, 0.1, 0.01, 0.001], device=DEV)
+    out = torch.full((tokens, heads * V), 7.0, dtype=dtype, device=DEV)
+    splits = 2 if tensor_cores else 3
+    scratch = lambda n: torch.full((n,), float("nan"), device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    api.latent_attention(q, w_key, w_value, pool, i32(table), i32(list(range(tokens + 1))), i32(past), tokens, tokens, heads, dim, rot, V, rank, inv_freq, 8, scale,
+                         window, splits, out, scratch(tokens * heads * row), scratch(tokens * heads * splits * rank), scratch(tokens * heads * splits * 2), status,
+                         tensor_cores, gate=gates)
+    assert int(status) == 0
+    z = q.double().sum(0).reshape(tokens, heads, dim + rot)
+    for t in range(tokens):
+        angle = (past[t] * inv_freq).double()
+        a, b = z[t, :, dim:dim + 4], z[t, :, dim + 4:dim + 8]
+        turned = torch.cat((a * angle.cos() - b * angle.sin(), b * angle.cos() + a * angle.sin(), z[t, :, dim + 8:]), 1)
+        folded = torch.cat((torch.einsum("hd,hdr->hr", z[t, :, :dim], w_key.double().reshape(heads, dim, rank)), turned), 1) * scale
+        rows = pool[torch.tensor(table[t], device=DEV)].double().reshape(-1, row)[max(0, past[t] + 1 - window):past[t] + 1]
+        mixed = torch.softmax(folded @ rows.T, -1) @ rows[:, :rank]
+        want = torch.einsum("hr,hvr->hv", mixed, w_value.double().reshape(heads, V, rank)).reshape(-1)
+        if gate is not None:
+            g = torch.sigmoid(gates.double().sum(0)[t])
+            want = want * (g.repeat_interleave(V) if gate == "head" else g)
+        # bfloat16: folded queries, probabilities and the result are narrowed, each to eight bits
+        error = float((out[t].double() - want).norm() / want.norm())
+        assert error <= (2e-5 if dtype == torch.float32 else 3 * 2.0 ** -8), (t, error)

@@ -49,6 +49,20 @@ __device__ __forceinline__ float lat_rotate(const float* __restrict__ part, int 
     return first ? part[j] * cs - part[pair] * sn : part[j] * cs + part[pair] * sn;
 }
 
+// sum over the k-slices of a projection, in slice order, sixteen loads in flight together
+__device__ __forceinline__ float lat_sum_slices(const float* __restrict__ p, int splits, size_t stride) {
+    float total = 0.0f;
+    for (int s0 = 0; s0 < splits; s0 += 16) {
+        float v[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = s0 + i < splits ? __ldg(p + (size_t)(s0 + i) * stride) : 0.0f;
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+            if (s0 + i < splits) total += v[i];
+    }
+    return total;
+}
+
 template <typename TOut, typename TC>
 __global__ void latent_prepare_kernel(const float* __restrict__ down, int splits, size_t split_stride, int row_stride, int q_rank, int rank,
                                       int rot, const float* __restrict__ q_weight, const float* __restrict__ kv_weight, float eps,
@@ -68,8 +82,7 @@ __global__ void latent_prepare_kernel(const float* __restrict__ down, int splits
     const float* src = down + (size_t)t * row_stride;
     float sq_q = 0.0f, sq_c = 0.0f;
     for (int j = threadIdx.x; j < cols; j += blockDim.x) {
-        float x = 0.0f;
-        for (int s = 0; s < splits; ++s) x += src[(size_t)s * split_stride + j];
+        const float x = lat_sum_slices(src + j, splits, split_stride);
         lat_row[j] = x;
         if (j < q_rank) sq_q = fmaf(x, x, sq_q);
         else if (j < q_rank + rank) sq_c = fmaf(x, x, sq_c);
@@ -113,13 +126,14 @@ template <> struct LatVec<__nv_bfloat16> {
     }
 };
 
-// The query a head's scores are taken with, one block per (token, head): [Wk_h^T q_plain | rotated q_rot] * scale, float32
-// [tokens][heads][rank + rot].  Threads run across the latent, so that a row of Wk_h is read side by side.
-template <typename TW>
+// The query a head's scores are taken with, one block per (token, head): [Wk_h^T q_plain | rotated q_rot] * scale,
+// [tokens][heads][rank + rot] (float32, or narrowed for the tensor-core form, which multiplies bfloat16).  Threads run across
+// the latent, so that a row of Wk_h is read side by side.
+template <typename TW, typename TA>
 __global__ void latent_absorb_kernel(const float* __restrict__ q, int q_splits, size_t q_stride, int q_row, const TW* __restrict__ w_key,
                                      const int* __restrict__ cu, const int* __restrict__ len_before, int sequences, int heads, int dim,
                                      int rot, int rank, const float* __restrict__ inv_freq, int rotary_dim, int interleaved,
-                                     float rot_scale, float scale, float* __restrict__ absorbed) {
+                                     float rot_scale, float scale, TA* __restrict__ absorbed) {
     tt_pdl_launch_dependents();
     const int t = blockIdx.x / heads, h = blockIdx.x - t * heads;
     int pos = 0;
@@ -131,15 +145,13 @@ __global__ void latent_absorb_kernel(const float* __restrict__ q, int q_splits, 
     extern __shared__ float lat_shared[];                       // dim + rot
     const float* qsrc = q + (size_t)t * q_row + (size_t)h * (dim + rot);
     for (int d = threadIdx.x; d < dim + rot; d += blockDim.x) {
-        float x = 0.0f;
-        for (int s = 0; s < q_splits; ++s) x += qsrc[(size_t)s * q_stride + d];
-        lat_shared[d] = x;
+        lat_shared[d] = lat_sum_slices(qsrc + d, q_splits, q_stride);
     }
     __syncthreads();
-    float* out = absorbed + ((size_t)t * heads + h) * (rank + rot);
+    TA* out = absorbed + ((size_t)t * heads + h) * (rank + rot);
     const float* qr = lat_shared + dim;
     for (int i = threadIdx.x; i < rot; i += blockDim.x)
-        out[rank + i] = lat_rotate(qr, i, rotary_dim, interleaved, pos, inv_freq, rot_scale) * scale;
+        out[rank + i] = tt_from_float<TA>(lat_rotate(qr, i, rotary_dim, interleaved, pos, inv_freq, rot_scale) * scale);
     for (int r = threadIdx.x; r < rank; r += blockDim.x) {
         const TW* col = w_key + (size_t)h * dim * rank + r;
         float a[8];
@@ -154,7 +166,7 @@ __global__ void latent_absorb_kernel(const float* __restrict__ q, int q_splits, 
             for (int i = 0; i < 8; ++i) a[i] = fmaf(w[i], lat_shared[d + i], a[i]);
         }
         for (; d < dim; ++d) a[0] = fmaf(lat_weight(col + (size_t)d * rank), lat_shared[d], a[0]);
-        out[r] = (((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]))) * scale;
+        out[r] = tt_from_float<TA>((((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]))) * scale);
     }
 }
 
@@ -404,18 +416,20 @@ __global__ void latent_attention_rows_kernel(const float* __restrict__ absorbed,
 // of LT_KEYS keys, group of 16 heads).  All heads of a token read the same cache rows, so the heads are the 16 rows of the
 // products: S [heads x keys] = A [heads x (rank + rot)] K^T with A the folded queries, then O [heads x rank] = P C with C
 // the latent part of the same rows.  The slice's rows and the folded queries are staged in shared memory once and serve
-// both products; the slice's maximum is known before the second product, so nothing is rescaled.  Every warp takes 16 of
-// the keys in the first product and every fourth 16-column piece of the latent in the second (warp-level
-// mma.sync through the wmma interface).  Slices are combined by latent_merge_expand_kernel.
-constexpr int LT_KEYS = 64, LT_HEADS = 16, LT_S_LD = LT_KEYS + 4, LT_P_LD = LT_KEYS + 8, LT_O_LD = 20;
+// both products; the slice's maximum is known before the second product, so nothing is rescaled.  Of the eight warps four take 16 of
+// the keys each over the first half of a row in the first product and four over the second half, and every warp takes every eighth
+// 16-column piece of the latent in the second (warp-level mma.sync through the wmma interface).  Slices are combined by the merge kernels.
+// What bounds it is the latency of a CTA's chain (rows, scores, softmax, sums), two CTAs an SM: 48 sequences of 1,024 visible rows of 576,
+// 16 heads: 59 -> 37 us with a cold L2 (four warps, the queries in float32 and narrowed here, an integer division for every 16 bytes copied).
+constexpr int LT_KEYS = 64, LT_HEADS = 16, LT_S_LD = LT_KEYS + 4, LT_P_LD = LT_KEYS + 8, LT_WARPS = 8;
 
 static size_t latent_decode_shared(int row_len) {
-    return (size_t)(LT_HEADS + LT_KEYS) * (row_len + 8) * sizeof(__nv_bfloat16) + (size_t)LT_HEADS * LT_S_LD * sizeof(float) +
-           (size_t)LT_HEADS * LT_P_LD * sizeof(__nv_bfloat16) + (size_t)4 * LT_HEADS * LT_O_LD * sizeof(float);
+    return (size_t)(LT_HEADS + LT_KEYS) * (row_len + 8) * sizeof(__nv_bfloat16) + (size_t)2 * LT_HEADS * LT_S_LD * sizeof(float) +
+           (size_t)LT_HEADS * LT_P_LD * sizeof(__nv_bfloat16);
 }
 
-__global__ void __launch_bounds__(128)
-latent_decode_mma_kernel(const float* __restrict__ absorbed, const __nv_bfloat16* __restrict__ pool, const int* __restrict__ table,
+__global__ void __launch_bounds__(32 * LT_WARPS)
+latent_decode_mma_kernel(const __nv_bfloat16* __restrict__ absorbed, const __nv_bfloat16* __restrict__ pool, const int* __restrict__ table,
                          int table_width, int pool_blocks, const int* __restrict__ len_before, int heads, int rot, int rank,
                          int window, int splits, float* __restrict__ part_acc, float* __restrict__ part_ml, unsigned* status) {
     using namespace nvcuda;
@@ -424,9 +438,8 @@ latent_decode_mma_kernel(const float* __restrict__ absorbed, const __nv_bfloat16
     const int row_len = rank + rot, ld = row_len + 8;           // rows 16 bytes apart modulo 128: no bank is met twice
     __nv_bfloat16* q_s = reinterpret_cast<__nv_bfloat16*>(lat_bytes);               // [16][ld]
     __nv_bfloat16* k_s = q_s + LT_HEADS * ld;                                       // [64][ld]
-    float* s_s = reinterpret_cast<float*>(k_s + LT_KEYS * ld);                      // [16][LT_S_LD]
-    __nv_bfloat16* p_s = reinterpret_cast<__nv_bfloat16*>(s_s + LT_HEADS * LT_S_LD);  // [16][LT_P_LD]
-    float* o_s = reinterpret_cast<float*>(p_s + LT_HEADS * LT_P_LD);                // [4][16][LT_O_LD]
+    float* s_s = reinterpret_cast<float*>(k_s + LT_KEYS * ld);                      // [2][16][LT_S_LD]: the row's two halves
+    __nv_bfloat16* p_s = reinterpret_cast<__nv_bfloat16*>(s_s + 2 * LT_HEADS * LT_S_LD);  // [16][LT_P_LD]
     const int t = blockIdx.x, split = blockIdx.y, h0 = blockIdx.z * LT_HEADS;       // one token per sequence: token t is sequence t
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int pos = len_before[t];
@@ -435,74 +448,70 @@ latent_decode_mma_kernel(const float* __restrict__ absorbed, const __nv_bfloat16
     const int end = min(begin + LT_KEYS, pos + 1);
     const int* table_row = table + (size_t)t * table_width;
     const int pieces = row_len >> 3;                            // 16-byte pieces of a row
+    // the slice lies in one or two cache blocks
+    const long long off0 = begin < end ? tt_cache_offset(table_row, begin, 0, 1, row_len, pool_blocks, status) : -1;
+    const int in_first = min(LT_KEYS, TT_BLOCK_TOKENS - begin % TT_BLOCK_TOKENS);   // rows of the slice in the first of them
+    const long long off1 = begin + in_first < end ? tt_cache_offset(table_row, begin + in_first, 0, 1, row_len, pool_blocks, status) : -1;
     tt_pdl_wait();
-    // the slice's rows: asynchronous 16-byte copies, all of a thread's in flight together (one after the other they cost a
-    // round trip to the L2 each: 36 of them for a row of 576 numbers)
-    for (int e = threadIdx.x; e < LT_KEYS * pieces; e += blockDim.x) {
-        const int r = e / pieces, c = e - r * pieces;
-        long long off = -1;
-        if (begin + r < end) off = tt_cache_offset(table_row, begin + r, 0, 1, row_len, pool_blocks, status);
-        __nv_bfloat16* dst = k_s + r * ld + 8 * c;
-        if (off >= 0) {
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(pool + off + 8 * c) : "memory");
+    // asynchronous 16-byte copies, all of a thread's in flight together: the folded queries, then the slice's rows
+    const int step_r = blockDim.x / pieces, step_c = blockDim.x - step_r * pieces;
+    int r = threadIdx.x / pieces, c = threadIdx.x - r * pieces;
+    for (; r < LT_HEADS + LT_KEYS; r += step_r, c += step_c) {
+        if (c >= pieces) { c -= pieces; ++r; }
+        if (r >= LT_HEADS + LT_KEYS) break;
+        const __nv_bfloat16* from = nullptr;
+        if (r < LT_HEADS) {
+            if (h0 + r < heads) from = absorbed + ((size_t)t * heads + h0 + r) * row_len + 8 * c;
         } else {
-            *reinterpret_cast<uint4*>(dst) = make_uint4(0u, 0u, 0u, 0u);
-        }
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    // the folded queries: eight 16-byte loads asked for before the first is narrowed
-    const int quads = row_len >> 2;
-    for (int e0 = threadIdx.x; e0 < LT_HEADS * quads; e0 += 8 * blockDim.x) {
-        float4 v[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int e = e0 + i * blockDim.x, r = e / quads, c = e - r * quads;
-            v[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (e < LT_HEADS * quads && h0 + r < heads)
-                v[i] = *reinterpret_cast<const float4*>(absorbed + ((size_t)t * heads + h0 + r) * row_len + 4 * c);
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int e = e0 + i * blockDim.x, r = e / quads, c = e - r * quads;
-            if (e < LT_HEADS * quads) {
-                __nv_bfloat162* dst = reinterpret_cast<__nv_bfloat162*>(q_s + r * ld + 4 * c);
-                dst[0] = __floats2bfloat162_rn(v[i].x, v[i].y);
-                dst[1] = __floats2bfloat162_rn(v[i].z, v[i].w);
+            const int k = r - LT_HEADS;
+            if (begin + k < end) {
+                if (k < in_first) { if (off0 >= 0) from = pool + off0 + (size_t)k * row_len + 8 * c; }
+                else if (off1 >= 0) from = pool + off1 + (size_t)(k - in_first) * row_len + 8 * c;
             }
         }
+        __nv_bfloat16* dst = q_s + r * ld + 8 * c;              // the rows follow the queries
+        if (from) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(from) : "memory");
+        else *reinterpret_cast<uint4*>(dst) = make_uint4(0u, 0u, 0u, 0u);
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
-    {   // S = A K^T: this warp's 16 keys
+    {   // S = A K^T: 16 of the keys, half of the row
+        const int tile = warp & 3, half = warp >> 2, steps = row_len >> 4, middle = (steps + 1) >> 1;
         wmma::fragment<wmma::accumulator, 16, 16, 16, float> acc;
         wmma::fill_fragment(acc, 0.0f);
-        for (int k = 0; k < row_len; k += 16) {
+#pragma unroll 4
+        for (int k = half ? middle : 0; k < (half ? steps : middle); ++k) {
             wmma::fragment<wmma::matrix_a, 16, 16, 16, __nv_bfloat16, wmma::row_major> a;
             wmma::fragment<wmma::matrix_b, 16, 16, 16, __nv_bfloat16, wmma::col_major> b;
-            wmma::load_matrix_sync(a, q_s + k, ld);
-            wmma::load_matrix_sync(b, k_s + (16 * warp) * ld + k, ld);
+            wmma::load_matrix_sync(a, q_s + 16 * k, ld);
+            wmma::load_matrix_sync(b, k_s + (16 * tile) * ld + 16 * k, ld);
             wmma::mma_sync(acc, a, b, acc);
         }
-        wmma::store_matrix_sync(s_s + 16 * warp, acc, LT_S_LD, wmma::mem_row_major);
+        wmma::store_matrix_sync(s_s + half * LT_HEADS * LT_S_LD + 16 * tile, acc, LT_S_LD, wmma::mem_row_major);
     }
     __syncthreads();
-    for (int r = 4 * warp; r < 4 * warp + 4; ++r) {            // softmax of a head's row over the slice, float32
-        const float s0 = begin + lane < end ? s_s[r * LT_S_LD + lane] : -INFINITY;
-        const float s1 = begin + lane + 32 < end ? s_s[r * LT_S_LD + lane + 32] : -INFINITY;
+    for (int row = 2 * warp; row < 2 * warp + 2; ++row) {       // softmax of a head's row over the slice, float32
+        const float* s0_s = s_s + row * LT_S_LD;
+        const float* s1_s = s0_s + LT_HEADS * LT_S_LD;
+        const float s0 = begin + lane < end ? s0_s[lane] + s1_s[lane] : -INFINITY;
+        const float s1 = begin + lane + 32 < end ? s0_s[lane + 32] + s1_s[lane + 32] : -INFINITY;
         const float m = tt_warp_max(fmaxf(s0, s1));
         const float p0 = s0 == -INFINITY ? 0.0f : expf(s0 - m), p1 = s1 == -INFINITY ? 0.0f : expf(s1 - m);
         const float l = tt_warp_sum(p0 + p1);
-        p_s[r * LT_P_LD + lane] = __float2bfloat16_rn(p0);
-        p_s[r * LT_P_LD + lane + 32] = __float2bfloat16_rn(p1);
-        if (lane == 0 && h0 + r < heads) {
-            const size_t slot = ((size_t)t * heads + h0 + r) * splits + split;
+        p_s[row * LT_P_LD + lane] = __float2bfloat16_rn(p0);
+        p_s[row * LT_P_LD + lane + 32] = __float2bfloat16_rn(p1);
+        if (lane == 0 && h0 + row < heads) {
+            const size_t slot = ((size_t)t * heads + h0 + row) * splits + split;
             part_ml[slot * 2] = m;
             part_ml[slot * 2 + 1] = l;
         }
     }
     __syncthreads();
-    float* mine = o_s + warp * LT_HEADS * LT_O_LD;
-    for (int f = warp; f < (rank >> 4); f += 4) {               // O = P C: 16 columns of the latent at a time
+    const bool whole = h0 + LT_HEADS <= heads;                  // sixteen heads: the sums go to their places as they are
+    float* out = part_acc + (((size_t)t * heads + h0) * splits + split) * rank;
+    float* mine = s_s + warp * (2 * LT_HEADS * LT_S_LD / LT_WARPS);                 // 272 floats: a tile of 16 x 16, in the scores' place
+    for (int f = warp; f < (rank >> 4); f += LT_WARPS) {        // O = P C: 16 columns of the latent at a time
         wmma::fragment<wmma::accumulator, 16, 16, 16, float> acc;
         wmma::fill_fragment(acc, 0.0f);
 #pragma unroll
@@ -513,12 +522,14 @@ latent_decode_mma_kernel(const float* __restrict__ absorbed, const __nv_bfloat16
             wmma::load_matrix_sync(b, k_s + kk * ld + 16 * f, ld);
             wmma::mma_sync(acc, a, b, acc);
         }
-        wmma::store_matrix_sync(mine, acc, LT_O_LD, wmma::mem_row_major);
-        __syncwarp();
-        for (int e = lane; e < LT_HEADS * 16; e += 32) {
-            const int r = e >> 4, c = e & 15;
-            if (h0 + r < heads) part_acc[(((size_t)t * heads + h0 + r) * splits + split) * rank + 16 * f + c] = mine[r * LT_O_LD + c];
+        if (whole) {
+            wmma::store_matrix_sync(out + 16 * f, acc, splits * rank, wmma::mem_row_major);
+            continue;
         }
+        wmma::store_matrix_sync(mine, acc, 16, wmma::mem_row_major);
+        __syncwarp();
+        for (int e = lane; e < LT_HEADS * 16; e += 32)
+            if (h0 + (e >> 4) < heads) out[(size_t)(e >> 4) * splits * rank + 16 * f + (e & 15)] = mine[e];
         __syncwarp();
     }
 }
@@ -594,6 +605,86 @@ __global__ void latent_merge_expand_kernel(const float* __restrict__ part_acc, c
     }
 }
 
+// The same for LM_TOKENS tokens of a head at a time, so that Wv_h crosses from the L2 once for them; slices of a token are
+// combined by a quarter of the block, four neighbouring numbers a thread.  Bound by the slices' sums and Wv_h out of the L2: 48 tokens, 16
+// heads of 128, 16 slices of latents of 512: 45 -> 28 us with a cold L2.  rank a multiple of 8 (16 bytes of a bfloat16 row).
+constexpr int LM_TOKENS = 4, LM_THREADS = 512;
+
+template <typename TOut, typename TW>
+__global__ void __launch_bounds__(LM_THREADS, 2)
+latent_merge_expand_group_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml, int splits, int rank, int vdim, int heads, int n_tokens,
+                                 const TW* __restrict__ w_value, TOut* __restrict__ out, const float* __restrict__ gate, int gate_splits, size_t gate_stride,
+                                 int gate_row, int gate_each) {
+    tt_pdl_launch_dependents();
+    tt_pdl_wait();
+    extern __shared__ __align__(16) float lat_group[];          // [LM_TOKENS][rank], then [LM_TOKENS][splits]
+    const int h = blockIdx.x, t0 = blockIdx.y * LM_TOKENS, count = min(LM_TOKENS, n_tokens - t0);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float* weight = lat_group + LM_TOKENS * rank;
+    auto opened = [&](int t, int column) { return 1.0f / (1.0f + expf(-lat_sum_slices(gate + (size_t)t * gate_row + column, gate_splits, gate_stride))); };
+    if (warp < count) {                                         // a slice's share: exp(m_s - m) / l
+        const float* ml = part_ml + ((size_t)(t0 + warp) * heads + h) * splits * 2;
+        float m = -INFINITY;
+        for (int s = lane; s < splits; s += 32) m = fmaxf(m, ml[2 * s]);
+        m = tt_warp_max(m);
+        float l = 0.0f;
+        for (int s = lane; s < splits; s += 32)
+            if (ml[2 * s] != -INFINITY) l += ml[2 * s + 1] * expf(ml[2 * s] - m);
+        l = tt_warp_sum(l);
+        const float inv = l > 0.0f ? 1.0f / l : 0.0f;
+        for (int s = lane; s < splits; s += 32) weight[warp * splits + s] = ml[2 * s] != -INFINITY ? expf(ml[2 * s] - m) * inv : 0.0f;
+    }
+    __syncthreads();
+    {
+        const int g = threadIdx.x / (LM_THREADS / LM_TOKENS);
+        for (int r = 4 * (threadIdx.x % (LM_THREADS / LM_TOKENS)); r < rank; r += 4 * (LM_THREADS / LM_TOKENS)) {
+            float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (g < count) {
+                const float* from = part_acc + ((size_t)(t0 + g) * heads + h) * splits * rank + r;
+#pragma unroll 16
+                for (int s = 0; s < splits; ++s) {
+                    const float4 v = __ldg(reinterpret_cast<const float4*>(from + (size_t)s * rank));
+                    const float w = weight[g * splits + s];
+                    acc.x = fmaf(v.x, w, acc.x); acc.y = fmaf(v.y, w, acc.y); acc.z = fmaf(v.z, w, acc.z); acc.w = fmaf(v.w, w, acc.w);
+                }
+            }
+            *reinterpret_cast<float4*>(lat_group + g * rank + r) = acc;
+        }
+    }
+    __syncthreads();
+    constexpr int VEC = LatVec<TW>::N, ROWS = 4;                // a warp takes four output numbers, lanes across the latent
+    for (int v0 = ROWS * warp; v0 < vdim; v0 += ROWS * (LM_THREADS / 32)) {
+        float o[ROWS * LM_TOKENS];
+#pragma unroll
+        for (int i = 0; i < ROWS * LM_TOKENS; ++i) o[i] = 0.0f;
+        for (int r = lane * VEC; r < rank; r += 32 * VEC) {
+            float w[ROWS][VEC];
+#pragma unroll
+            for (int i = 0; i < ROWS; ++i) LatVec<TW>::load(w_value + ((size_t)h * vdim + min(v0 + i, vdim - 1)) * rank + r, w[i]);
+#pragma unroll
+            for (int g = 0; g < LM_TOKENS; ++g) {
+                float c[VEC];
+#pragma unroll
+                for (int e = 0; e < VEC; e += 4) {
+                    const float4 q = *reinterpret_cast<const float4*>(lat_group + g * rank + r + e);
+                    c[e] = q.x; c[e + 1] = q.y; c[e + 2] = q.z; c[e + 3] = q.w;
+                }
+#pragma unroll
+                for (int i = 0; i < ROWS; ++i)
+#pragma unroll
+                    for (int e = 0; e < VEC; ++e) o[i * LM_TOKENS + g] = fmaf(w[i][e], c[e], o[i * LM_TOKENS + g]);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < ROWS * LM_TOKENS; ++i) {
+            const float total = tt_warp_sum(o[i]);
+            const int v = v0 + i / LM_TOKENS, t = t0 + i % LM_TOKENS;
+            if (lane == i && v < vdim && t < n_tokens)
+                out[((size_t)t * heads + h) * vdim + v] = tt_from_float<TOut>(gate ? total * opened(t, gate_each ? h * vdim + v : h) : total);
+        }
+    }
+}
+
 extern "C" int tt_latent_prepare(const float* down, int splits, long long split_stride, int row_stride, int q_rank, int rank, int rot,
                                  const float* q_weight, const float* kv_weight, float eps, const float* inv_freq, int rotary_dim,
                                  int interleaved, float rot_scale, void* q_latent, int act_dtype, void* pool, int cache_dtype, const int* table, int table_width,
@@ -606,7 +697,7 @@ extern "C" int tt_latent_prepare(const float* down, int splits, long long split_
         return (int)cudaErrorInvalidValue;
     const size_t shared = (size_t)(cols + 32) * sizeof(float);
     if (shared > 48 * 1024) return (int)cudaErrorInvalidValue;
-    const int threads = cols >= 1024 ? 256 : 128;
+    const int threads = n_tokens <= 148 && cols >= 1024 ? 512 : cols >= 1024 ? 256 : 128;        // few tokens: a row over more threads
 #define TT_PREP(T) tt_launch_pdl(latent_prepare_kernel<T, T>, dim3(n_tokens), dim3(threads), shared, stream, down, splits, (size_t)split_stride, row_stride, q_rank, rank, rot, q_weight, kv_weight, eps, inv_freq, rotary_dim, interleaved, rot_scale, (T*)q_latent, (T*)pool, table, table_width, pool_blocks, cu, len_before, sequences, status)
     if (act_dtype == TT_F32) TT_PREP(float); else TT_PREP(__nv_bfloat16);
 #undef TT_PREP
@@ -629,9 +720,17 @@ extern "C" int tt_latent_attention(const float* q, int q_splits, long long q_str
     if (rows > 2147483647LL) return (int)cudaErrorInvalidValue;
     const size_t shared = (size_t)LAT_WARPS * (rank + rot) * sizeof(float);
     const dim3 grid((unsigned)blocks, splits), block(LAT_WARPS * 32);
-#define TT_ABSORB(TW) tt_launch_pdl(latent_absorb_kernel<TW>, dim3((unsigned)rows), dim3(rank >= 512 ? 512 : rank >= 256 ? 256 : 128), (size_t)(dim + rot) * sizeof(float), stream, q, q_splits, (size_t)q_stride, q_row, (const TW*)w_key, cu, len_before, sequences, heads, dim, rot, rank, inv_freq, rotary_dim, interleaved, rot_scale, scale, absorbed)
+    // Wv_h is fetched for several tokens at a time from eight tokens on (fewer leave too few blocks).  The same for Wk_h measured
+    // no difference (48 tokens, 16 heads: 122.4 and 122.6 us for the layer): the queries' k-slices are what that kernel waits for.
+    const bool grouped = n_tokens >= 8 && (n_tokens + LM_TOKENS - 1) / LM_TOKENS <= 65535;
+    const bool narrow = one_token_each == 2;                    // the tensor-core form takes the folded queries in bfloat16
+#define TT_ABSORB_AS(TW, TA) tt_launch_pdl(latent_absorb_kernel<TW, TA>, dim3((unsigned)rows), dim3(rank >= 512 ? 512 : rank >= 256 ? 256 : 128), (size_t)(dim + rot) * sizeof(float), stream, q, q_splits, (size_t)q_stride, q_row, (const TW*)w_key, cu, len_before, sequences, heads, dim, rot, rank, inv_freq, rotary_dim, interleaved, rot_scale, scale, (TA*)(void*)absorbed)
+#define TT_ABSORB(TW) do { if (narrow) TT_ABSORB_AS(TW, __nv_bfloat16); else TT_ABSORB_AS(TW, float); } while (0)
 #define TT_ATT(TA) tt_launch_pdl(latent_attention_kernel<TA>, grid, block, shared, stream, (const float*)absorbed, (const TA*)pool, table, table_width, pool_blocks, cu, len_before, sequences, n_tokens, heads, rot, rank, window, splits, part_acc, part_ml, status)
-#define TT_MERGE(TA, TW) tt_launch_pdl(latent_merge_expand_kernel<TA, TW>, dim3((unsigned)rows), dim3(256), (size_t)(rank + splits) * sizeof(float), stream, (const float*)part_acc, (const float*)part_ml, splits, rank, vdim, heads, (const TW*)w_value, (TA*)out, gate, gate_splits, (size_t)gate_stride, gate_row, gate_each)
+#define TT_MERGE(TA, TW) do { \
+        const size_t group_shared = (size_t)LM_TOKENS * (rank + splits) * sizeof(float); \
+        if (grouped && rank % 8 == 0 && group_shared <= 48 * 1024 && ((uintptr_t)w_value & 15) == 0) tt_launch_pdl(latent_merge_expand_group_kernel<TA, TW>, dim3(heads, (n_tokens + LM_TOKENS - 1) / LM_TOKENS), dim3(LM_THREADS), group_shared, stream, (const float*)part_acc, (const float*)part_ml, splits, rank, vdim, heads, n_tokens, (const TW*)w_value, (TA*)out, gate, gate_splits, (size_t)gate_stride, gate_row, gate_each); \
+        else tt_launch_pdl(latent_merge_expand_kernel<TA, TW>, dim3((unsigned)rows), dim3(256), (size_t)(rank + splits) * sizeof(float), stream, (const float*)part_acc, (const float*)part_ml, splits, rank, vdim, heads, (const TW*)w_value, (TA*)out, gate, gate_splits, (size_t)gate_stride, gate_row, gate_each); } while (0)
     if (weight_dtype == TT_F32) TT_ABSORB(float); else TT_ABSORB(__nv_bfloat16);
 #define TT_ATT_ROWS(TA) tt_launch_pdl(latent_attention_rows_kernel<TA>, grid, block, 0, stream, (const float*)absorbed, (const TA*)pool, table, table_width, pool_blocks, cu, len_before, sequences, n_tokens, heads, rot, rank, window, splits, part_acc, part_ml, status)
     const int piece = act_dtype == TT_F32 ? 4 : 8;              // numbers in 16 bytes of a cache row
@@ -643,8 +742,8 @@ extern "C" int tt_latent_attention(const float* q, int q_splits, long long q_str
             if (e != cudaSuccess) return (int)e;
             allowed = need;
         }
-        tt_launch_pdl(latent_decode_mma_kernel, dim3(n_tokens, splits, (heads + LT_HEADS - 1) / LT_HEADS), dim3(128), need, stream,
-                      (const float*)absorbed, (const __nv_bfloat16*)pool, table, table_width, pool_blocks, len_before, heads, rot, rank, window,
+        tt_launch_pdl(latent_decode_mma_kernel, dim3(n_tokens, splits, (heads + LT_HEADS - 1) / LT_HEADS), dim3(32 * LT_WARPS), need, stream,
+                      (const __nv_bfloat16*)(const void*)absorbed, (const __nv_bfloat16*)pool, table, table_width, pool_blocks, len_before, heads, rot, rank, window,
                       splits, part_acc, part_ml, status);
     } else if (rank % piece == 0 && rot % piece == 0) {
         if (act_dtype == TT_F32) TT_ATT_ROWS(float); else TT_ATT_ROWS(__nv_bfloat16);
@@ -657,6 +756,7 @@ extern "C" int tt_latent_attention(const float* q, int q_splits, long long q_str
     else if (weight_dtype == TT_F32) TT_MERGE(__nv_bfloat16, float);
     else TT_MERGE(__nv_bfloat16, __nv_bfloat16);
 #undef TT_ABSORB
+#undef TT_ABSORB_AS
 #undef TT_ATT
 #undef TT_MERGE
     TT_LAUNCH_CHECK();

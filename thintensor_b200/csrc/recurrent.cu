@@ -158,6 +158,8 @@ constexpr int CONV_TILE = 16;       // packed tokens a thread walks with its cha
 // start) and the window of the last inputs slides through registers.  Where the tile crosses into the next sequence
 // the window is filled from that sequence's state.  Bound by its loads: a tile inside one sequence asks for all of them at once
 // (2,048 tokens of 4,352 channels 58 -> 47 us, 4,097 of 4,096 107 -> 82).
+// ONE_SLICE: the projection is not cut into slices, so that this holds (the registers it takes cost the other form's blocks their place).
+template <bool ONE_SLICE>
 __global__ void causal_conv_kernel(const float* __restrict__ proj, int splits, size_t split_stride, int cols, int col_off,
                                    int channels, const float* __restrict__ weight, const float* __restrict__ bias, int taps,
                                    int activation, const float* __restrict__ state, size_t slot_stride, float* __restrict__ out,
@@ -191,7 +193,7 @@ __global__ void causal_conv_kernel(const float* __restrict__ proj, int splits, s
         }
     };
     fill(t0);
-    if (splits == 1 && t1 - t0 == CONV_TILE && t1 <= next) {     // a tile inside one sequence: all of its inputs are asked for at once
+    if (ONE_SLICE && t1 - t0 == CONV_TILE && t1 <= next) {       // a tile inside one sequence: all of its inputs are asked for at once
         float x[CONV_TILE];
 #pragma unroll
         for (int k = 0; k < CONV_TILE; ++k) x[k] = __ldg(proj + (size_t)(t0 + k) * cols + col_off + c);
@@ -272,8 +274,9 @@ extern "C" int tt_causal_conv(const float* proj, int splits, long long split_str
     const unsigned bx = (unsigned)((channels + threads - 1) / threads);
     if (taps < 1 || taps > CONV_MAX_TAPS || bx > 65535) return (int)cudaErrorInvalidValue;
     if (!one_token_each) {
-        tt_launch_pdl(causal_conv_kernel, dim3((n_tokens + CONV_TILE - 1) / CONV_TILE, bx), dim3(threads), 0, stream, proj, splits, (size_t)split_stride, cols, col_off,
-                      channels, weight, bias, taps, activation, (const float*)state, (size_t)slot_stride, out, cu, slots, sequences, n_tokens);
+#define TT_CONVOLVE(ONE) tt_launch_pdl(causal_conv_kernel<ONE>, dim3((n_tokens + CONV_TILE - 1) / CONV_TILE, bx), dim3(threads), 0, stream, proj, splits, (size_t)split_stride, cols, col_off, channels, weight, bias, taps, activation, (const float*)state, (size_t)slot_stride, out, cu, slots, sequences, n_tokens)
+        if (splits == 1) TT_CONVOLVE(true); else TT_CONVOLVE(false);
+#undef TT_CONVOLVE
     }
     if (taps > 1 || one_token_each)
         tt_launch_pdl(causal_conv_state_kernel, dim3(sequences, bx), dim3(threads), 0, stream, proj, splits, (size_t)split_stride, cols,

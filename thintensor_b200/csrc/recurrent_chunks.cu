@@ -586,18 +586,20 @@ static int scan_chunks_launch(const ScanChunks& a, int max_slots, cudaStream_t s
     TT_LAUNCH_CHECK();
 }
 
-// x, b, c: rows of `stride` numbers (see ScanChunks).  max_slots: n_tokens / 64 + sequences (scratch for scores and factors holds as many).
-// sms: the device's multiprocessors.
-extern "C" int tt_scan_chunks(const float* x, const float* b, const float* c, long long stride, const float* proj, int splits, long long split_stride,
+// rows: [tokens][width] with x, B and C from the given columns on (see ScanChunks).  max_slots: n_tokens / 64 + sequences.  scratch: so many
+// times the scores of every group (64 * 64 numbers) and the factors of every head (CK_FACTORS).  sms: the device's multiprocessors.
+extern "C" int tt_scan_chunks(const float* rows, int width, int x_col, int b_col, int c_col, const float* proj, int splits, long long split_stride,
                               int cols, int dt_col, const float* dt_bias, const float* a_log, const float* d_skip, const float* fixed_decay, float* state,
-                              float* y, float* scores, float* factors, const int* cu, const int* slots, int sequences, int max_slots, int heads,
+                              float* y, float* scratch, const int* cu, const int* slots, int sequences, int max_slots, int heads,
                               int groups, int P, int N, int sms, cudaStream_t stream) {
     if (sequences <= 0 || max_slots <= 0) return 0;
     if (N <= 0 || N > 128 || P <= 0 || groups <= 0 || groups > 65535 || heads % groups || sequences > 65535) return (int)cudaErrorInvalidValue;
-    if (!fixed_decay && (!proj || !dt_bias || !a_log)) return (int)cudaErrorInvalidValue;
+    if (!rows || !scratch || (!fixed_decay && (!proj || !dt_bias || !a_log))) return (int)cudaErrorInvalidValue;
+    const float *x = rows + x_col, *b = rows + b_col, *c = rows + c_col;
+    float *scores = scratch, *factors = scratch + (size_t)max_slots * groups * CK_TOKENS * CK_TOKENS;
     const uintptr_t bases = (uintptr_t)x | (uintptr_t)b | (uintptr_t)c | (uintptr_t)y;
-    const ScanChunks a{x, b, c, (size_t)stride, proj, splits, cols, dt_col, (size_t)split_stride, dt_bias, a_log, d_skip, fixed_decay, state, y, scores, factors,
-                       cu, slots, sequences, heads, groups, P, N, (bases & 15) == 0 && !(stride & 3) && !(N & 3) && !(P & 3) ? 1 : 0};
+    const ScanChunks a{x, b, c, (size_t)width, proj, splits, cols, dt_col, (size_t)split_stride, dt_bias, a_log, d_skip, fixed_decay, state, y, scores, factors,
+                       cu, slots, sequences, heads, groups, P, N, (bases & 15) == 0 && !(width & 3) && !(N & 3) && !(P & 3) ? 1 : 0};
     // 32 columns a CTA use a number of C twice; 16 where that grid would leave half of the SMs without one
     const bool narrow = (long long)heads * sequences * ((P + 31) / 32) * 2 <= sms + sms / 4;
     if (N <= 64) return narrow ? scan_chunks_launch<64, 16>(a, max_slots, stream) : scan_chunks_launch<64, 32>(a, max_slots, stream);

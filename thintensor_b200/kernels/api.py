@@ -916,52 +916,49 @@ def chunk_slots(n_tokens: int, sequences: int) -> int:
     return n_tokens // CHUNK_TOKENS + sequences
 
 
-def scan_chunks_scratch(n_tokens: int, sequences: int, heads: int, groups: int) -> tuple[tuple[int, ...], tuple[int, ...]]:
-    """Shapes of the float32 scratch that :func:`scan_chunks` takes as ``scores`` and ``factors``."""
-    slots = chunk_slots(n_tokens, sequences)
-    return (slots, groups, CHUNK_TOKENS, CHUNK_TOKENS), (slots, heads, _CHUNK_FACTORS)
+def scan_chunks_scratch(n_tokens: int, sequences: int, heads: int, groups: int) -> tuple[int]:
+    """Shape of the float32 scratch that :func:`scan_chunks` takes: scores for every chunk and group, factors for every chunk and head."""
+    return (chunk_slots(n_tokens, sequences) * (groups * CHUNK_TOKENS * CHUNK_TOKENS + heads * _CHUNK_FACTORS),)
 
 
-def scan_chunks(x: torch.Tensor, b: torch.Tensor, c: torch.Tensor, state: torch.Tensor, y: torch.Tensor, cu: torch.Tensor, slots: torch.Tensor,
-                sequences: int, heads: int, head_dim: int, state_size: int, groups: int, scores: torch.Tensor, factors: torch.Tensor,
+def scan_chunks(rows: torch.Tensor, x_col: int, b_col: int, c_col: int, state: torch.Tensor, y: torch.Tensor, cu: torch.Tensor, slots: torch.Tensor,
+                sequences: int, heads: int, head_dim: int, state_size: int, groups: int, scratch: torch.Tensor,
                 steps: tuple[torch.Tensor, int, torch.Tensor, torch.Tensor, torch.Tensor] | None = None, fixed_decay: torch.Tensor | None = None) -> None:
-    """The recurrences of :func:`mamba2_scan` and :func:`decay_scan`, a chunk of 64 tokens at a time (for prompts).  ``x``, ``b``, ``c``:
-    float32 ``[tokens, columns]`` of ``heads * head_dim`` and ``groups * state_size`` columns, views of one matrix (equal row
-    strides).  Either ``steps`` = (projection partial sums, first column of the raw step sizes, dt_bias, A_log, D) or ``fixed_decay``
-    (float32 ``[heads]``, step sizes one).  States of up to 128 rows.  ``scores`` and ``factors``: see :func:`scan_chunks_scratch`."""
-    for t, cols, name in ((x, heads * head_dim, "x"), (b, groups * state_size, "B"), (c, groups * state_size, "C")):
-        if t.dtype != torch.float32 or t.dim() != 2 or t.stride(1) != 1 or t.stride(0) != x.stride(0) or tuple(t.shape) != (x.shape[0], cols):
-            raise KernelError(f"scan_chunks: {name} must be float32 [tokens, {cols}] with the row stride of x")
-    for t, name in ((state, "recurrent state"), (y, "recurrence output"), (scores, "scores"), (factors, "factors")):
+    """The recurrences of :func:`mamba2_scan` and :func:`decay_scan`, a chunk of 64 tokens at a time (for prompts).  ``rows``: float32
+    ``[tokens, columns]`` with x (``heads * head_dim`` columns), B and C (``groups * state_size`` columns each) from the given columns on.
+    Either ``steps`` = (projection partial sums, first column of the raw step sizes, dt_bias, A_log, D) or ``fixed_decay``
+    (float32 ``[heads]``, step sizes one).  States of up to 128 rows.  ``scratch``: see :func:`scan_chunks_scratch`."""
+    for t, name in ((rows, "x/B/C"), (state, "recurrent state"), (y, "recurrence output"), (scratch, "scratch")):
         _need(t, torch.float32, name)
     if (steps is None) == (fixed_decay is None):
         raise KernelError("scan_chunks: decays come from step sizes or are fixed")
-    want_scores, want_factors = scan_chunks_scratch(x.shape[0], sequences, heads, groups)
-    if (state_size > CHUNK_MAX_ROWS or heads % groups or tuple(state.shape[1:]) != (heads, head_dim, state_size) or tuple(y.shape) != (x.shape[0], heads * head_dim)
-            or tuple(scores.shape) != want_scores or tuple(factors.shape) != want_factors):
+    tokens, width = rows.shape
+    if (state_size > CHUNK_MAX_ROWS or heads % groups or state.shape[1:] != (heads, head_dim, state_size) or y.shape != (tokens, heads * head_dim)
+            or min(x_col, b_col, c_col) < 0 or x_col + heads * head_dim > width or max(b_col, c_col) + groups * state_size > width
+            or scratch.numel() < scan_chunks_scratch(tokens, sequences, heads, groups)[0]):
         raise KernelError("scan_chunks: shapes do not fit the sizes")
-    p, splits, stride, cols, dt_col, vectors = c_void_p(0), 0, 0, 0, 0, (None, None, None)
+    p, splits, stride, cols, dt_col, vectors = None, 0, 0, 0, 0, (None, None, None)
     if steps is not None:
         p, splits, stride, cols = _projection(steps[0])
         dt_col, vectors = int(steps[1]), steps[2:]
         if dt_col < 0 or dt_col + heads > cols:
             raise KernelError("scan_chunks: the step sizes lie outside the projection")
-    for t, name in ((*zip(vectors, ("dt_bias", "A_log", "D")), (fixed_decay, "decay"))):
+    for t in (*vectors, fixed_decay):
         if t is not None:
-            _need(t, torch.float32, name)
+            _need(t, torch.float32, "number per head")
             if t.numel() != heads:
-                raise KernelError(f"scan_chunks: {name} has a number per head")
-    fn = _fn("recurrent_chunks", "tt_scan_chunks", [c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_longlong, c_int, c_int, c_void_p, c_void_p,
-                                                    c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
+                raise KernelError("scan_chunks: decays, biases and skips have a number per head")
+    fn = _fn("recurrent_chunks", "tt_scan_chunks", [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_longlong, c_int, c_int, c_void_p, c_void_p,
+                                                    c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                                                     c_int, c_int, c_int, c_int, c_void_p])
-    _check(fn(_ptr(x), _ptr(b), _ptr(c), x.stride(0), p, splits, stride, cols, dt_col, _ptr(vectors[0]), _ptr(vectors[1]), _ptr(vectors[2]),
-              _ptr(fixed_decay), _ptr(state), _ptr(y), _ptr(scores), _ptr(factors), _ptr(cu), _ptr(slots), sequences, want_scores[0], heads, groups,
-              head_dim, state_size, sm_count(x.device), _stream()), "scan_chunks", 2)
+    _check(fn(rows.data_ptr(), width, x_col, b_col, c_col, p, splits, stride, cols, dt_col, *(None if t is None else t.data_ptr() for t in vectors),
+              None if fixed_decay is None else fixed_decay.data_ptr(), state.data_ptr(), y.data_ptr(), scratch.data_ptr(), _ptr(cu), _ptr(slots), sequences,
+              chunk_slots(tokens, sequences), heads, groups, head_dim, state_size, sm_count(rows.device), _stream()), "scan_chunks", 2)
 
 
-def delta_chunks_scratch(n_tokens: int, sequences: int, heads: int, key_dim: int, value_dim: int) -> tuple[int, ...]:
+def delta_chunks_scratch(n_tokens: int, sequences: int, heads: int, key_dim: int, value_dim: int) -> tuple[int]:
     """Shape of the float32 scratch that :func:`delta_chunks` takes."""
-    return chunk_slots(n_tokens, sequences), heads, CHUNK_TOKENS * (key_dim + value_dim + CHUNK_TOKENS) + _DELTA_CHUNK_FACTORS
+    return (chunk_slots(n_tokens, sequences) * heads * (CHUNK_TOKENS * (key_dim + value_dim + CHUNK_TOKENS) + _DELTA_CHUNK_FACTORS),)
 
 
 def delta_chunks(qkv: torch.Tensor, proj: torch.Tensor, b_col: int, a_col: int, dt_bias: torch.Tensor, a_log: torch.Tensor, state: torch.Tensor,
@@ -971,18 +968,19 @@ def delta_chunks(qkv: torch.Tensor, proj: torch.Tensor, b_col: int, a_col: int, 
     see :func:`delta_chunks_scratch`."""
     for t, name in ((qkv, "q/k/v"), (dt_bias, "dt_bias"), (a_log, "A_log"), (state, "recurrent state"), (out, "recurrence output"), (scratch, "scratch")):
         _need(t, torch.float32, name)
-    shape = delta_chunks_scratch(qkv.shape[0], sequences, heads, key_dim, value_dim)
-    if (qkv.shape[1] != 2 * qk_heads * key_dim + heads * value_dim or tuple(state.shape[1:]) != (heads, value_dim, key_dim) or heads % qk_heads
-            or tuple(out.shape) != (qkv.shape[0], heads * value_dim) or key_dim > CHUNK_MAX_ROWS or tuple(scratch.shape) != shape
-            or dt_bias.numel() != heads or a_log.numel() != heads):
+    tokens = qkv.shape[0]
+    if (qkv.shape[1] != 2 * qk_heads * key_dim + heads * value_dim or state.shape[1:] != (heads, value_dim, key_dim) or heads % qk_heads
+            or out.shape != (tokens, heads * value_dim) or key_dim > CHUNK_MAX_ROWS or dt_bias.numel() != heads or a_log.numel() != heads
+            or scratch.numel() < delta_chunks_scratch(tokens, sequences, heads, key_dim, value_dim)[0]):
         raise KernelError("delta_chunks: shapes do not fit the sizes")
     p, splits, stride, cols = _projection(proj)
     if min(b_col, a_col) < 0 or max(b_col, a_col) + heads > cols:
         raise KernelError("delta_chunks: write strengths or decays lie outside the projection")
     fn = _fn("recurrent_chunks", "tt_delta_chunks", [c_void_p, c_int, c_void_p, c_int, c_longlong, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p,
                                                      c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p])
-    _check(fn(_ptr(qkv), qkv.shape[1], p, splits, stride, cols, b_col, a_col, _ptr(dt_bias), _ptr(a_log), _ptr(state), _ptr(out), _ptr(scratch),
-              _ptr(cu), _ptr(slots), sequences, shape[0], heads, qk_heads, key_dim, value_dim, sm_count(qkv.device), _stream()), "delta_chunks", 2)
+    _check(fn(qkv.data_ptr(), qkv.shape[1], p, splits, stride, cols, b_col, a_col, dt_bias.data_ptr(), a_log.data_ptr(), state.data_ptr(), out.data_ptr(),
+              scratch.data_ptr(), _ptr(cu), _ptr(slots), sequences, chunk_slots(tokens, sequences), heads, qk_heads, key_dim, value_dim, sm_count(qkv.device),
+              _stream()), "delta_chunks", 2)
 
 
 def delta_scan(qkv: torch.Tensor, proj: torch.Tensor, b_col: int, a_col: int, dt_bias: torch.Tensor | None, a_log: torch.Tensor | None,

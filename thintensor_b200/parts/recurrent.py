@@ -110,22 +110,18 @@ def in_blocks(ctx) -> bool:
     return not ctx.decode and ctx.n_tokens >= 4 * ctx.sequences
 
 
+CHUNKS_FROM = 160
+
+
 def in_chunks(ctx, heads: int, columns: int, rows: int) -> bool:
     """Whether a recurrence with a decay per head takes its tokens in chunks of 64 (decided by the step's shape alone, like
-    :func:`in_blocks`): prompts of at least a chunk's length on average do, while the grid of a CTA per sequence, head and 32 columns
+    :func:`in_blocks`): prompts of at least ``CHUNKS_FROM`` tokens on average do (for fewer a launch more eats the gain: a layer of 16 heads of
+    128 x 128 on 130 tokens took 97 us token by token and 112 in chunks, on 200 141 and 104), while the grid of a CTA per sequence, head and 32 columns
     is at most four rounds of the SMs.  Measured on a B200 (us, chunks against token by token): 64 heads of 64 x 128, one sequence
     of 64 tokens 23 and 33, of 40 tokens 22 and 22; two of 48 33 and 28; four of 731 332 and 545 (512 CTAs), 16 of 700 (2,048 CTAs)
     1,060 and 1,035; 24 heads of 256 x 128, five of 96 (960 CTAs) 131 and 84: many CTAs keep the form that goes token by token busy."""
-    ctas = heads * ctx.sequences * -(-columns // 32)
-    return (not ctx.decode and rows <= api.CHUNK_MAX_ROWS and ctx.n_tokens >= api.CHUNK_TOKENS * ctx.sequences
-            and ctas <= 4 * api.sm_count(ctx.status.device))
-
-
-def scan_chunks(ctx, x, b, c, state, y, heads: int, head_dim: int, rows: int, groups: int, **decays) -> None:
-    """:func:`api.scan_chunks` on scratch memory of the step's."""
-    scores, factors = api.scan_chunks_scratch(ctx.n_tokens, ctx.sequences, heads, groups)
-    api.scan_chunks(x, b, c, state, y, ctx.cu, ctx.slots, ctx.sequences, heads, head_dim, rows, groups,
-                    ctx.scratch("chunks.scores", scores, torch.float32), ctx.scratch("chunks.factors", factors, torch.float32), **decays)
+    return (not ctx.decode and rows <= api.CHUNK_MAX_ROWS and ctx.n_tokens >= CHUNKS_FROM * ctx.sequences
+            and heads * ctx.sequences * -(-columns // 32) <= 4 * api.sm_count(ctx.status.device))
 
 
 @MIXERS.register("mamba2")
@@ -193,9 +189,9 @@ class Mamba2(Mixer):
         y = ctx.scratch("mamba2.y", (tokens, self.inner), torch.float32)
         dt_col = self.inner + self.channels
         if in_chunks(ctx, self.heads, self.head_dim, self.state):
-            x, b, c = xbc.split((self.inner, self.groups * self.state, self.groups * self.state), dim=1)
-            scan_chunks(ctx, x, b, c, recurrent, y, self.heads, self.head_dim, self.state, self.groups,
-                        steps=(proj, dt_col, self.dt_bias, self.a_log, self.d_skip))
+            scratch = ctx.scratch("chunks.scan", api.scan_chunks_scratch(tokens, ctx.sequences, self.heads, self.groups), torch.float32)
+            api.scan_chunks(xbc, 0, self.inner, self.inner + self.groups * self.state, recurrent, y, ctx.cu, ctx.slots, ctx.sequences, self.heads,
+                            self.head_dim, self.state, self.groups, scratch, steps=(proj, dt_col, self.dt_bias, self.a_log, self.d_skip))
         else:
             api.mamba2_scan(xbc, proj, dt_col, self.dt_bias, self.a_log, self.d_skip, recurrent, y, ctx.cu, ctx.slots, ctx.sequences, self.heads,
                             self.head_dim, self.state, self.groups)
@@ -214,7 +210,7 @@ class GatedDelta(Mixer):
     # Prompts of at least so many tokens on average go in chunks of 64 (decays per head; decided by the step's shape alone).  Measured on
     # a B200, 16 heads of 128 x 128 (us, chunks against token by token): one sequence of 64 tokens 42 and 35, five of 64 69 and 70, one of
     # 700 (8 heads) 96 and 315, one of 4,097 478 and 1,950, 16 of 500 671 and 869.
-    CHUNKS_FROM = 96
+    CHUNKS_FROM = 128
 
     def __init__(self, hidden: int, heads: int, qk_heads: int, key_dim: int, value_dim: int, conv: int = 4, eps: float = 1e-6,
                  names: dict | None = None, channel_decay: int | None = None, low_rank_gate: int | None = None, gate: str = "silu"):
@@ -433,8 +429,9 @@ class DecayLinearAttention(Mixer):
         elif decay is not None:
             api.row_decay_scan(vkq, decay, recurrent, read, ctx.cu, ctx.slots, ctx.sequences, self.heads, self.key_dim, self.value_dim)
         elif in_chunks(ctx, self.heads, self.value_dim, self.key_dim):
-            v, k, q = vkq.split((self.v, self.qk, self.qk), dim=1)
-            scan_chunks(ctx, v, k, q, recurrent, read, self.heads, self.value_dim, self.key_dim, self.heads, fixed_decay=self.decays)
+            scratch = ctx.scratch("chunks.scan", api.scan_chunks_scratch(tokens, ctx.sequences, self.heads, self.heads), torch.float32)
+            api.scan_chunks(vkq, 0, self.v, self.v + self.qk, recurrent, read, ctx.cu, ctx.slots, ctx.sequences, self.heads, self.value_dim, self.key_dim,
+                            self.heads, scratch, fixed_decay=self.decays)
         else:
             api.decay_scan(vkq, self.decays, recurrent, read, ctx.cu, ctx.slots, ctx.sequences, self.heads, self.key_dim, self.value_dim)
         return self.finish(ctx, proj, read)
