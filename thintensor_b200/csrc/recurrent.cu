@@ -157,9 +157,10 @@ constexpr int CONV_TILE = 16;       // packed tokens a thread walks with its cha
 // A thread takes one channel through CONV_TILE packed tokens: every input is read once (plus taps - 1 at the tile's
 // start) and the window of the last inputs slides through registers.  Where the tile crosses into the next sequence
 // the window is filled from that sequence's state.  Bound by its loads: a tile inside one sequence asks for all of them at once
-// (2,048 tokens of 4,352 channels 58 -> 47 us, 4,097 of 4,096 107 -> 82).
+// (2,048 tokens of 4,352 channels 50 -> 39 us, 4,097 of 4,096 100 -> 74; 650 of 4,352, in tiles of half the length so that there are blocks
+// enough, 30 -> 21, in whole ones 33).
 // ONE_SLICE: the projection is not cut into slices, so that this holds (the registers it takes cost the other form's blocks their place).
-template <bool ONE_SLICE>
+template <bool ONE_SLICE, int TILE>
 __global__ void causal_conv_kernel(const float* __restrict__ proj, int splits, size_t split_stride, int cols, int col_off,
                                    int channels, const float* __restrict__ weight, const float* __restrict__ bias, int taps,
                                    int activation, const float* __restrict__ state, size_t slot_stride, float* __restrict__ out,
@@ -176,7 +177,7 @@ __global__ void causal_conv_kernel(const float* __restrict__ proj, int splits, s
     }
     tt_pdl_wait();
     if (c >= channels) return;
-    const int t0 = blockIdx.x * CONV_TILE, t1 = min(t0 + CONV_TILE, n_tokens);
+    const int t0 = blockIdx.x * TILE, t1 = min(t0 + TILE, n_tokens);
     int b = tt_find_sequence(cu, sequences, t0);
     int first = cu[b], next = cu[b + 1];
     float win[CONV_MAX_TAPS];                                    // win[j], j < keep: the input (keep - j) tokens back
@@ -193,12 +194,12 @@ __global__ void causal_conv_kernel(const float* __restrict__ proj, int splits, s
         }
     };
     fill(t0);
-    if (ONE_SLICE && t1 - t0 == CONV_TILE && t1 <= next) {       // a tile inside one sequence: all of its inputs are asked for at once
-        float x[CONV_TILE];
+    if (ONE_SLICE && t1 - t0 == TILE && t1 <= next) {       // a tile inside one sequence: all of its inputs are asked for at once
+        float x[TILE];
 #pragma unroll
-        for (int k = 0; k < CONV_TILE; ++k) x[k] = __ldg(proj + (size_t)(t0 + k) * cols + col_off + c);
+        for (int k = 0; k < TILE; ++k) x[k] = __ldg(proj + (size_t)(t0 + k) * cols + col_off + c);
 #pragma unroll
-        for (int k = 0; k < CONV_TILE; ++k) {
+        for (int k = 0; k < TILE; ++k) {
             float acc = shift;
 #pragma unroll
             for (int j = 0; j < CONV_MAX_TAPS; ++j)
@@ -274,8 +275,8 @@ extern "C" int tt_causal_conv(const float* proj, int splits, long long split_str
     const unsigned bx = (unsigned)((channels + threads - 1) / threads);
     if (taps < 1 || taps > CONV_MAX_TAPS || bx > 65535) return (int)cudaErrorInvalidValue;
     if (!one_token_each) {
-#define TT_CONVOLVE(ONE) tt_launch_pdl(causal_conv_kernel<ONE>, dim3((n_tokens + CONV_TILE - 1) / CONV_TILE, bx), dim3(threads), 0, stream, proj, splits, (size_t)split_stride, cols, col_off, channels, weight, bias, taps, activation, (const float*)state, (size_t)slot_stride, out, cu, slots, sequences, n_tokens)
-        if (splits == 1) TT_CONVOLVE(true); else TT_CONVOLVE(false);
+#define TT_CONVOLVE(ONE, TILE) tt_launch_pdl(causal_conv_kernel<ONE, TILE>, dim3((n_tokens + TILE - 1) / TILE, bx), dim3(threads), 0, stream, proj, splits, (size_t)split_stride, cols, col_off, channels, weight, bias, taps, activation, (const float*)state, (size_t)slot_stride, out, cu, slots, sequences, n_tokens)
+        if (splits == 1 && n_tokens < 1024) TT_CONVOLVE(true, CONV_TILE / 2); else if (splits == 1) TT_CONVOLVE(true, CONV_TILE); else TT_CONVOLVE(false, CONV_TILE);
 #undef TT_CONVOLVE
     }
     if (taps > 1 || one_token_each)
@@ -1501,7 +1502,7 @@ static void gated_group_norm4(const float* y, long long total, int width, int gr
     const int quads = group / 4;
     if (quads <= 64) {
         if (quads <= 32) TT_GN4(1, true, (total + 7) / 8, 256); else TT_GN4(2, true, (total + 7) / 8, 256);
-    } else if (quads <= 1024 && (total < 1024 || quads < 256)) {          // few groups: as many threads as there are pieces
+    } else if (quads <= 1024 && (total < 296 || quads < 256)) {          // few groups: as many threads as there are pieces
         TT_GN4(1, false, total, (quads + 31) / 32 * 32);
     } else {
         TT_GN4(4, false, total, (quads / 4 + 31 + (quads % 4 > 0)) / 32 * 32);
