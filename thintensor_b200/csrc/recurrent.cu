@@ -158,7 +158,7 @@ constexpr int CONV_TILE = 16;       // packed tokens a thread walks with its cha
 // start) and the window of the last inputs slides through registers.  Where the tile crosses into the next sequence
 // the window is filled from that sequence's state.  Bound by its loads: a tile inside one sequence asks for all of them at once
 // (2,048 tokens of 4,352 channels 50 -> 39 us, 4,097 of 4,096 100 -> 74; 650 of 4,352, in tiles of half the length so that there are blocks
-// enough, 30 -> 21, in whole ones 33).
+// enough, 30 -> 25, in whole ones 33).
 // ONE_SLICE: the projection is not cut into slices, so that this holds (the registers it takes cost the other form's blocks their place).
 template <bool ONE_SLICE, int TILE>
 __global__ void causal_conv_kernel(const float* __restrict__ proj, int splits, size_t split_stride, int cols, int col_off,
@@ -275,7 +275,7 @@ extern "C" int tt_causal_conv(const float* proj, int splits, long long split_str
     const unsigned bx = (unsigned)((channels + threads - 1) / threads);
     if (taps < 1 || taps > CONV_MAX_TAPS || bx > 65535) return (int)cudaErrorInvalidValue;
     if (!one_token_each) {
-#define TT_CONVOLVE(ONE, TILE) tt_launch_pdl(causal_conv_kernel<ONE, TILE>, dim3((n_tokens + TILE - 1) / TILE, bx), dim3(threads), 0, stream, proj, splits, (size_t)split_stride, cols, col_off, channels, weight, bias, taps, activation, (const float*)state, (size_t)slot_stride, out, cu, slots, sequences, n_tokens)
+#define TT_CONVOLVE(ONE, TILE) tt_launch_pdl(causal_conv_kernel<ONE, TILE>, dim3((n_tokens + (TILE) - 1) / (TILE), bx), dim3(threads), 0, stream, proj, splits, (size_t)split_stride, cols, col_off, channels, weight, bias, taps, activation, (const float*)state, (size_t)slot_stride, out, cu, slots, sequences, n_tokens)
         if (splits == 1 && n_tokens < 1024) TT_CONVOLVE(true, CONV_TILE / 2); else if (splits == 1) TT_CONVOLVE(true, CONV_TILE); else TT_CONVOLVE(false, CONV_TILE);
 #undef TT_CONVOLVE
     }
