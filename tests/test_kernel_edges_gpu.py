@@ -317,3 +317,27 @@ def test_latent_decode_groups(heads, dim, rot, V, rank, dtype, tensor_cores, tok
         # bfloat16: folded queries, probabilities and the result are narrowed, each to eight bits
         error = float((out[t].double() - want).norm() / want.norm())
         assert error <= (2e-5 if dtype == torch.float32 else 3 * 2.0 ** -8), (t, error)
+
+
+# --------------------------------------------------------------------------------------------- routing, a warp a token
+@pytest.mark.parametrize("hidden,experts,extra", [(8, 5, 0), (2048, 16, 1), (2056, 33, 0), (4096, 40, 2), (4104, 8, 0), (100, 8, 0)])
+@pytest.mark.parametrize("tokens", [1024, 1025, 1031])
+def test_routing_of_prompts(hidden, experts, extra, tokens):
+    """Rows of one piece a lane and of the most there are, rows that are no whole pieces, and too long ones (both forms)."""
+    from thintensor_b200.kernels import api
+
+    x = randn(tokens, hidden, seed=70, dtype=torch.bfloat16)
+    w = randn(experts + extra, hidden, seed=71, scale=hidden ** -0.5, dtype=torch.bfloat16)
+    top = 3
+    gates, chosen, weights = torch.empty(tokens, experts + extra, device=DEV), torch.empty(tokens, top, dtype=torch.int32, device=DEV), torch.empty(tokens, top, device=DEV)
+    api.route_rows(x, w, top, 1, 1, gates, chosen, weights, extra=extra)
+    logits = x.double() @ w.double().T
+    score = torch.softmax(logits[:, :experts], -1)
+    value, index = score.topk(top + 1, -1)
+    clear = (value[:, :-1] - value[:, 1:]).amin(1) > 1e-5           # float32 sums of up to 4,104 products decide closer calls as they fall
+    assert float(clear.double().mean()) > 0.95
+    assert torch.equal(chosen[clear].long(), index[clear, :top])
+    torch.testing.assert_close(weights[clear].double(), (value / value[:, :top].sum(1, keepdim=True))[clear, :top], rtol=1e-4, atol=1e-6)
+    torch.testing.assert_close(gates[:, experts:].double(), torch.sigmoid(logits[:, experts:]), rtol=1e-4, atol=1e-6)
+    dense = torch.zeros(tokens, experts, device=DEV).scatter_(1, chosen.long(), weights)
+    assert torch.equal(gates[:, :experts], dense)
