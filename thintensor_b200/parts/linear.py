@@ -49,8 +49,9 @@ class Linear:
                 out = ctx.scratch(name, (splits, tokens, self.out_features), torch.float32)
             api.gemm_tcgen05(x, self.weight, self.bias, out, ctx.status, operands_checked=True, shares=self.shares(ctx, tokens))
             return out
-        splits = api.gemm_simt_splits(tokens, self.out_features, self.in_features)
-        out = into.unsqueeze(0) if splits == 1 and into is not None else ctx.scratch(name, (splits, tokens, self.out_features), torch.float32)
+        # a caller that brings an output wants the product itself: no slices that it would have to add up
+        out = into.unsqueeze(0) if into is not None else ctx.scratch(
+            name, (api.gemm_simt_splits(tokens, self.out_features, self.in_features), tokens, self.out_features), torch.float32)
         api.gemm_simt(x, self.weight, self.bias, out)
         return out
 
