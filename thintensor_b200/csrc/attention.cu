@@ -116,11 +116,11 @@ attention_tiles_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, co
             for (int i = 0; i < N; i += 4) *reinterpret_cast<float4*>(Vs + d * AT_PLD + j + i) = make_float4(x[i], x[i + 1], x[i + 2], x[i + 3]);
         }
         __syncthreads();
-        float s[4][4];
+        float s[4][4], s2[4][4];                                // two sums a score, added up: a long chain of additions loses more
 #pragma unroll
         for (int r = 0; r < 4; ++r)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) s[r][c] = 0.0f;
+            for (int c = 0; c < 4; ++c) s[r][c] = s2[r][c] = 0.0f;
 #pragma unroll 4
         for (int d = 0; d < SIZE; d += 4) {
             float4 a[4], b[4];
@@ -134,8 +134,8 @@ attention_tiles_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, co
                 for (int c = 0; c < 4; ++c) {
                     s[r][c] = fmaf(a[r].x, b[c].x, s[r][c]);
                     s[r][c] = fmaf(a[r].y, b[c].y, s[r][c]);
-                    s[r][c] = fmaf(a[r].z, b[c].z, s[r][c]);
-                    s[r][c] = fmaf(a[r].w, b[c].w, s[r][c]);
+                    s2[r][c] = fmaf(a[r].z, b[c].z, s2[r][c]);
+                    s2[r][c] = fmaf(a[r].w, b[c].w, s2[r][c]);
                 }
         }
         bool whole = true;                                      // the warp's queries see every key of the block
@@ -145,7 +145,7 @@ attention_tiles_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, co
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 const int key = base + tx + 16 * c;
-                float v = s[r][c];
+                float v = s[r][c] + s2[r][c];
                 if (cap > 0.0f) v = cap * tanhf(v * inv_cap);
                 v -= slope * (float)(pos[r] - key);
                 const bool seen = key >= seen_from[r] && key <= pos[r];
@@ -173,7 +173,12 @@ attention_tiles_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, co
         }
         whole = __all_sync(0xffffffffu, whole);                 // a warp's rows and weights are its own
         __syncwarp();
-        auto weigh = [&](auto guarded) {
+        auto weigh = [&](auto guarded) {                        // the block's sums, then added to the running ones
+            float part[4][DIMS];
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int d = 0; d < DIMS; ++d) part[r][d] = 0.0f;
 #pragma unroll 2
             for (int j = 0; j < TT_BLOCK_TOKENS; j += 4) {
                 float4 p[4];
@@ -185,13 +190,17 @@ attention_tiles_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, co
 #pragma unroll
                     for (int r = 0; r < 4; ++r) {
                         // a weight of zero does not touch its value: what a query does not see may be no number
-                        if (!decltype(guarded)::value || p[r].x != 0.0f) acc[r][d] = fmaf(p[r].x, v.x, acc[r][d]);
-                        if (!decltype(guarded)::value || p[r].y != 0.0f) acc[r][d] = fmaf(p[r].y, v.y, acc[r][d]);
-                        if (!decltype(guarded)::value || p[r].z != 0.0f) acc[r][d] = fmaf(p[r].z, v.z, acc[r][d]);
-                        if (!decltype(guarded)::value || p[r].w != 0.0f) acc[r][d] = fmaf(p[r].w, v.w, acc[r][d]);
+                        if (!decltype(guarded)::value || p[r].x != 0.0f) part[r][d] = fmaf(p[r].x, v.x, part[r][d]);
+                        if (!decltype(guarded)::value || p[r].y != 0.0f) part[r][d] = fmaf(p[r].y, v.y, part[r][d]);
+                        if (!decltype(guarded)::value || p[r].z != 0.0f) part[r][d] = fmaf(p[r].z, v.z, part[r][d]);
+                        if (!decltype(guarded)::value || p[r].w != 0.0f) part[r][d] = fmaf(p[r].w, v.w, part[r][d]);
                     }
                 }
             }
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int d = 0; d < DIMS; ++d) acc[r][d] += part[r][d];
         };
         if (whole) weigh(AtBool<false>()); else weigh(AtBool<true>());
     }
