@@ -587,14 +587,15 @@ static int scan_chunks_launch(const ScanChunks& a, int max_slots, cudaStream_t s
 }
 
 // rows: [tokens][width] with x, B and C from the given columns on (see ScanChunks).  max_slots: n_tokens / 64 + sequences.  scratch: so many
-// times the scores of every group (64 * 64 numbers) and the factors of every head (CK_FACTORS).  sms: the device's multiprocessors.
+// times the scores of every group (64 * 64 numbers) and the factors of every head (CK_FACTORS), on a 16-byte boundary: the walk copies
+// it in 16-byte pieces whatever the rows' alignment.  sms: the device's multiprocessors.
 extern "C" int tt_scan_chunks(const float* rows, int width, int x_col, int b_col, int c_col, const float* proj, int splits, long long split_stride,
                               int cols, int dt_col, const float* dt_bias, const float* a_log, const float* d_skip, const float* fixed_decay, float* state,
                               float* y, float* scratch, const int* cu, const int* slots, int sequences, int max_slots, int heads,
                               int groups, int P, int N, int sms, cudaStream_t stream) {
     if (sequences <= 0 || max_slots <= 0) return 0;
     if (N <= 0 || N > 128 || P <= 0 || groups <= 0 || groups > 65535 || heads % groups || sequences > 65535) return (int)cudaErrorInvalidValue;
-    if (!rows || !scratch || (!fixed_decay && (!proj || !dt_bias || !a_log))) return (int)cudaErrorInvalidValue;
+    if (!rows || !scratch || ((uintptr_t)scratch & 15) || (!fixed_decay && (!proj || !dt_bias || !a_log))) return (int)cudaErrorInvalidValue;
     const float *x = rows + x_col, *b = rows + b_col, *c = rows + c_col;
     float *scores = scratch, *factors = scratch + (size_t)max_slots * groups * CK_TOKENS * CK_TOKENS;
     const uintptr_t bases = (uintptr_t)x | (uintptr_t)b | (uintptr_t)c | (uintptr_t)y;
@@ -984,16 +985,16 @@ static int delta_chunks_launch(const DeltaChunks& a, int max_slots, cudaStream_t
     TT_LAUNCH_CHECK();
 }
 
-// scratch: max_slots * heads * (64 * (D + V + 64) + CD_FACTORS) floats; max_slots as for tt_scan_chunks
+// scratch: max_slots * heads * (64 * (D + V + 64) + CD_FACTORS) floats on a 16-byte boundary; max_slots as for tt_scan_chunks
 extern "C" int tt_delta_chunks(const float* qkv, int qkv_cols, const float* proj, int splits, long long split_stride, int cols, int b_col, int a_col,
                                const float* dt_bias, const float* a_log, float* state, float* out, float* scratch, const int* cu, const int* slots,
                                int sequences, int max_slots, int heads, int qk_heads, int D, int V, int sms, cudaStream_t stream) {
     if (sequences <= 0 || max_slots <= 0) return 0;
     if (D <= 0 || D > 128 || V <= 0 || qk_heads <= 0 || heads % qk_heads || heads > 65535 || sequences > 65535) return (int)cudaErrorInvalidValue;
-    if (!qkv || !proj || !dt_bias || !a_log || !scratch) return (int)cudaErrorInvalidValue;
+    if (!qkv || !proj || !dt_bias || !a_log || !scratch || ((uintptr_t)scratch & 15)) return (int)cudaErrorInvalidValue;
     const int vec = ((uintptr_t)qkv & 15) == 0 && !(qkv_cols & 3) && !(D & 3);
     const DeltaChunks a{qkv, (size_t)qkv_cols, proj, splits, cols, b_col, a_col, (size_t)split_stride, dt_bias, a_log, state, out, scratch, cu, slots,
-                        sequences, heads, qk_heads, D, V, vec, ((uintptr_t)out & 15) == 0 && ((uintptr_t)scratch & 15) == 0 && !(V & 3) ? 1 : 0};
+                        sequences, heads, qk_heads, D, V, vec, ((uintptr_t)out & 15) == 0 && !(V & 3) ? 1 : 0};
     const bool narrow = (long long)heads * sequences * ((V + 31) / 32) * 2 <= sms + sms / 4;        // as for tt_scan_chunks
     if (D <= 64) return narrow ? delta_chunks_launch<64, 16>(a, max_slots, stream) : delta_chunks_launch<64, 32>(a, max_slots, stream);
     return narrow ? delta_chunks_launch<128, 16>(a, max_slots, stream) : delta_chunks_launch<128, 32>(a, max_slots, stream);

@@ -74,6 +74,12 @@ def _need(t: torch.Tensor, dtype: torch.dtype, name: str) -> None:
         raise KernelError(f"{name} must be contiguous")
 
 
+def _need_aligned(t: torch.Tensor, name: str) -> None:
+    """For memory that a kernel copies in 16-byte pieces."""
+    if t.data_ptr() % 16:
+        raise KernelError(f"{name} must start on a 16-byte boundary")
+
+
 def _need_columns(t: torch.Tensor, dtype: torch.dtype, name: str) -> None:
     """Like :func:`_need` for a product's output, which may be a range of the columns of a wider matrix."""
     if t.dtype != dtype:
@@ -927,9 +933,10 @@ def scan_chunks(rows: torch.Tensor, x_col: int, b_col: int, c_col: int, state: t
     """The recurrences of :func:`mamba2_scan` and :func:`decay_scan`, a chunk of 64 tokens at a time (for prompts).  ``rows``: float32
     ``[tokens, columns]`` with x (``heads * head_dim`` columns), B and C (``groups * state_size`` columns each) from the given columns on.
     Either ``steps`` = (projection partial sums, first column of the raw step sizes, dt_bias, A_log, D) or ``fixed_decay``
-    (float32 ``[heads]``, step sizes one).  States of up to 128 rows.  ``scratch``: see :func:`scan_chunks_scratch`."""
+    (float32 ``[heads]``, step sizes one).  States of up to 128 rows.  ``scratch``, on a 16-byte boundary: see :func:`scan_chunks_scratch`."""
     for t, name in ((rows, "x/B/C"), (state, "recurrent state"), (y, "recurrence output"), (scratch, "scratch")):
         _need(t, torch.float32, name)
+    _need_aligned(scratch, "scratch")
     if (steps is None) == (fixed_decay is None):
         raise KernelError("scan_chunks: decays come from step sizes or are fixed")
     tokens, width = rows.shape
@@ -964,10 +971,11 @@ def delta_chunks_scratch(n_tokens: int, sequences: int, heads: int, key_dim: int
 def delta_chunks(qkv: torch.Tensor, proj: torch.Tensor, b_col: int, a_col: int, dt_bias: torch.Tensor, a_log: torch.Tensor, state: torch.Tensor,
                  out: torch.Tensor, cu: torch.Tensor, slots: torch.Tensor, sequences: int, heads: int, qk_heads: int, key_dim: int, value_dim: int,
                  scratch: torch.Tensor) -> None:
-    """:func:`delta_scan` with a decay per head, a chunk of 64 tokens at a time (for prompts; key sizes of up to 128).  ``scratch``:
-    see :func:`delta_chunks_scratch`."""
+    """:func:`delta_scan` with a decay per head, a chunk of 64 tokens at a time (for prompts; key sizes of up to 128).  ``scratch``, on
+    a 16-byte boundary: see :func:`delta_chunks_scratch`."""
     for t, name in ((qkv, "q/k/v"), (dt_bias, "dt_bias"), (a_log, "A_log"), (state, "recurrent state"), (out, "recurrence output"), (scratch, "scratch")):
         _need(t, torch.float32, name)
+    _need_aligned(scratch, "scratch")
     tokens = qkv.shape[0]
     if (qkv.shape[1] != 2 * qk_heads * key_dim + heads * value_dim or state.shape[1:] != (heads, value_dim, key_dim) or heads % qk_heads
             or out.shape != (tokens, heads * value_dim) or key_dim > CHUNK_MAX_ROWS or dt_bias.numel() != heads or a_log.numel() != heads
