@@ -319,6 +319,31 @@ def test_latent_decode_groups(heads, dim, rot, V, rank, dtype, tensor_cores, tok
         assert error <= (2e-5 if dtype == torch.float32 else 3 * 2.0 ** -8), (t, error)
 
 
+@pytest.mark.parametrize("dtype,tensor_cores", [(torch.bfloat16, True), (torch.float32, False)])
+@pytest.mark.parametrize("off", [1, 4])
+def test_latent_slice_sums_off_their_boundary(dtype, tensor_cores, off):
+    """The slices' sums 4 and 16 bytes off: fragments are stored through shared memory, and at 4 bytes the kernel that combines slices
+    four numbers at a time leaves the call to the one that takes them singly."""
+    from thintensor_b200.kernels import api
+
+    tokens, heads, dim, rot, V, rank, splits, past = 9, 16, 16, 16, 24, 48, 2, 100
+    row = rank + rot
+    pool, table = randn(tokens * 2, 1, 64, row, seed=80, dtype=dtype), torch.arange(tokens * 2, dtype=torch.int32, device=DEV).reshape(tokens, 2)
+    q = randn(1, tokens, heads * (dim + rot), seed=81)
+    w_key, w_value = (randn(heads * n, rank, seed=82, scale=rank ** -0.5, dtype=dtype) for n in (dim, V))
+    outs = []
+    for shift in (0, off):
+        out, status = torch.full((tokens, heads * V), 7.0, dtype=dtype, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+        part = torch.full((tokens * heads * splits * rank + 8,), float("nan"), device=DEV)
+        api.latent_attention(q, w_key, w_value, pool, table, i32(list(range(tokens + 1))), i32([past] * tokens), tokens, tokens, heads, dim, rot, V, rank,
+                             torch.ones(rot // 2, device=DEV), rot, row ** -0.5, 0, splits, out, torch.empty(tokens * heads * row, device=DEV),
+                             part[shift:-8 + shift], torch.empty(tokens * heads * splits * 2, device=DEV), status, tensor_cores)
+        assert int(status) == 0
+        outs.append(out.double())
+    # the same numbers with the expansion's float32 sums in another order, then (bfloat16) narrowed once
+    assert float((outs[1] - outs[0]).norm() / outs[0].norm()) <= (1e-6 if dtype == torch.float32 else 2.0 ** -8)
+
+
 # --------------------------------------------------------------------------------------------- routing, a warp a token
 @pytest.mark.parametrize("hidden,experts,extra", [(8, 5, 0), (2048, 16, 1), (2056, 33, 0), (4096, 40, 2), (4104, 8, 0), (100, 8, 0)])
 @pytest.mark.parametrize("tokens", [1024, 1025, 1031])

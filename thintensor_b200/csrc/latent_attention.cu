@@ -508,8 +508,9 @@ latent_decode_mma_kernel(const __nv_bfloat16* __restrict__ absorbed, const __nv_
         }
     }
     __syncthreads();
-    const bool whole = h0 + LT_HEADS <= heads;                  // sixteen heads: the sums go to their places as they are
     float* out = part_acc + (((size_t)t * heads + h0) * splits + split) * rank;
+    // sixteen heads: the sums go to their places as they are (on 32-byte boundaries: a fragment's store needs them)
+    const bool whole = h0 + LT_HEADS <= heads && ((uintptr_t)part_acc & 31) == 0;
     float* mine = s_s + warp * (2 * LT_HEADS * LT_S_LD / LT_WARPS);                 // 272 floats: a tile of 16 x 16, in the scores' place
     for (int f = warp; f < (rank >> 4); f += LT_WARPS) {        // O = P C: 16 columns of the latent at a time
         wmma::fragment<wmma::accumulator, 16, 16, 16, float> acc;
@@ -729,7 +730,7 @@ extern "C" int tt_latent_attention(const float* q, int q_splits, long long q_str
 #define TT_ATT(TA) tt_launch_pdl(latent_attention_kernel<TA>, grid, block, shared, stream, (const float*)absorbed, (const TA*)pool, table, table_width, pool_blocks, cu, len_before, sequences, n_tokens, heads, rot, rank, window, splits, part_acc, part_ml, status)
 #define TT_MERGE(TA, TW) do { \
         const size_t group_shared = (size_t)LM_TOKENS * (rank + splits) * sizeof(float); \
-        if (grouped && rank % 8 == 0 && group_shared <= 48 * 1024 && ((uintptr_t)w_value & 15) == 0) tt_launch_pdl(latent_merge_expand_group_kernel<TA, TW>, dim3(heads, (n_tokens + LM_TOKENS - 1) / LM_TOKENS), dim3(LM_THREADS), group_shared, stream, (const float*)part_acc, (const float*)part_ml, splits, rank, vdim, heads, n_tokens, (const TW*)w_value, (TA*)out, gate, gate_splits, (size_t)gate_stride, gate_row, gate_each); \
+        if (grouped && rank % 8 == 0 && group_shared <= 48 * 1024 && (((uintptr_t)w_value | (uintptr_t)part_acc) & 15) == 0) tt_launch_pdl(latent_merge_expand_group_kernel<TA, TW>, dim3(heads, (n_tokens + LM_TOKENS - 1) / LM_TOKENS), dim3(LM_THREADS), group_shared, stream, (const float*)part_acc, (const float*)part_ml, splits, rank, vdim, heads, n_tokens, (const TW*)w_value, (TA*)out, gate, gate_splits, (size_t)gate_stride, gate_row, gate_each); \
         else tt_launch_pdl(latent_merge_expand_kernel<TA, TW>, dim3((unsigned)rows), dim3(256), (size_t)(rank + splits) * sizeof(float), stream, (const float*)part_acc, (const float*)part_ml, splits, rank, vdim, heads, (const TW*)w_value, (TA*)out, gate, gate_splits, (size_t)gate_stride, gate_row, gate_each); } while (0)
     if (weight_dtype == TT_F32) TT_ABSORB(float); else TT_ABSORB(__nv_bfloat16);
 #define TT_ATT_ROWS(TA) tt_launch_pdl(latent_attention_rows_kernel<TA>, grid, block, 0, stream, (const float*)absorbed, (const TA*)pool, table, table_width, pool_blocks, cu, len_before, sequences, n_tokens, heads, rot, rank, window, splits, part_acc, part_ml, status)

@@ -1272,8 +1272,9 @@ def latent_attention(q: torch.Tensor, w_key: torch.Tensor, w_value: torch.Tensor
     ``w_key`` ``[heads * dim, rank]`` and ``w_value`` ``[heads * vdim, rank]`` expand a latent into a head's keys and values;
     ``pool`` ``[blocks, 1, 64, rank + rot]`` holds per token the latent and the rotated key part all heads share.  Score of
     query i and key j: ``(q_plain . w_key_h c_j + q_rot . k_rot_j) * scale`` for ``0 <= i - j < window`` (``window`` 0: every
-    earlier key); ``out`` ``[tokens, heads * vdim]``.  Scratch memory, all float32: ``absorbed`` ``[tokens * heads * (rank +
-    rot)]`` for the queries with ``w_key`` folded in; ``part_acc`` ``[tokens * heads * splits * rank]`` and ``part_ml``
+    earlier key); ``out`` ``[tokens, heads * vdim]``.  Scratch memory, float32 tensors: ``absorbed`` ``[tokens * heads * (rank +
+    rot)]`` for the queries with ``w_key`` folded in (the tensor-core form narrows them: bfloat16 in the front half of it, which
+    must start on a 16-byte boundary); ``part_acc`` ``[tokens * heads * splits * rank]`` and ``part_ml``
     ``[tokens * heads * splits * 2]`` for the ``splits`` slices the keys are cut into.  ``tensor_cores``: a step of one token per
     sequence whose sizes :func:`latent_decode_tensor_cores` takes runs both products on the tensor cores, with the heads of a
     token as the rows; ``splits`` must then cover every key a token can see in slices of ``LATENT_DECODE_SLICE`` keys.
@@ -1299,6 +1300,8 @@ def latent_attention(q: torch.Tensor, w_key: torch.Tensor, w_value: torch.Tensor
         raise KernelError("latent_attention: shapes do not fit the sizes")
     for t, name in ((absorbed, "folded queries"), (part_acc, "slice sums"), (part_ml, "slice maxima")):
         _need(t, torch.float32, name)
+    if tensor_cores:
+        _need_aligned(absorbed, "folded queries")
     if (absorbed.numel() < n_tokens * heads * (rank + rot) or part_acc.numel() < n_tokens * heads * splits * rank
             or part_ml.numel() < n_tokens * heads * splits * 2):
         raise KernelError("latent_attention: scratch memory is too small")
