@@ -142,6 +142,72 @@ def test_delta_rule_in_chunks(heads, qk_heads, D, V):
     assert torch.equal(state[[3, 7]], before[[3, 7]])
 
 
+@pytest.mark.parametrize("heads,N", [(2, 128), (2, 24), (100, 128), (100, 64)])                     # 16 and 32 columns a CTA, both sizes of state
+@pytest.mark.parametrize("what", ["x", "b", "c", "dt"])
+@pytest.mark.parametrize("token,value", [(0, float("inf")), (30, float("inf")), (30, float("nan")), (63, float("-inf")), (81, float("nan"))])
+def test_recurrence_in_chunks_keeps_later_tokens_out(heads, N, what, token, value):
+    """A number that is not finite reaches what it reaches token by token: the earlier tokens' outputs, the other columns and the
+    other sequence keep their bits."""
+    from thintensor_b200.kernels import api
+
+    P, news = 20, [130, 70]
+    tokens, inner = sum(news), heads * P
+    cu, slots = i32([0, news[0], tokens]), i32([1, 0])
+    a_log, dt_bias, skip = randn(heads, seed=7, scale=2.0), randn(heads, seed=8), randn(heads, seed=9)
+    outs = []
+    for poisoned in (False, True):
+        rows, raw = randn(tokens, inner + 2 * N, seed=90), randn(1, tokens, heads, seed=91)
+        if poisoned:
+            place = {"x": 3, "b": inner + 2, "c": inner + N + 2, "dt": 1}[what]
+            (raw[0] if what == "dt" else rows)[token, place] = value
+        forms = []
+        for chunks in (True, False):
+            state, y = randn(2, heads, P, N, seed=92), torch.full((tokens, inner), 7.0, device=DEV)
+            if chunks:
+                scratch = torch.full(api.scan_chunks_scratch(tokens, 2, heads, 1), float("nan"), device=DEV)
+                api.scan_chunks(rows, 0, inner, inner + N, state, y, cu, slots, 2, heads, P, N, 1, scratch, steps=(raw, 0, dt_bias, a_log, skip))
+            else:
+                api.mamba2_scan(rows, raw, 0, dt_bias, a_log, skip, state, y, cu, slots, 2, heads, P, N, 1)
+            forms.append((y, state))
+        outs.append(forms)
+    (clean, clean_state), (y, state) = outs[0][0], outs[1][0]
+    by_token, by_token_state = outs[1][1]
+    assert torch.equal(y[:token], clean[:token]) and torch.equal(y[news[0]:], clean[news[0]:]) and torch.equal(state[0], clean_state[0])
+    assert torch.equal(y.isfinite(), by_token.isfinite()) and torch.equal(state.isfinite(), by_token_state.isfinite())
+
+
+@pytest.mark.parametrize("heads,D", [(2, 128), (2, 24), (100, 128), (100, 64)])
+@pytest.mark.parametrize("what", ["q", "k", "v", "beta", "decay"])
+@pytest.mark.parametrize("token,value", [(0, float("inf")), (30, float("inf")), (30, float("nan")), (63, float("-inf")), (81, float("nan"))])
+def test_delta_rule_in_chunks_keeps_later_tokens_out(heads, D, what, token, value):
+    from thintensor_b200.kernels import api
+
+    V, news = 20, [130, 70]
+    tokens, qk = sum(news), heads * D
+    cu, slots = i32([0, news[0], tokens]), i32([1, 0])
+    a_log, dt_bias = randn(heads, seed=17, scale=2.0), randn(heads, seed=18)
+    outs = []
+    for poisoned in (False, True):
+        qkv, raw = randn(tokens, 2 * qk + heads * V, seed=93), randn(1, tokens, 2 * heads, seed=94)
+        if poisoned:
+            place = {"q": 2, "k": qk + 2, "v": 2 * qk + 3, "beta": 1, "decay": heads + 1}[what]
+            (raw[0] if what in ("beta", "decay") else qkv)[token, place] = value
+        forms = []
+        for chunks in (True, False):
+            state, out = randn(2, heads, V, D, seed=95), torch.full((tokens, heads * V), 7.0, device=DEV)
+            if chunks:
+                scratch = torch.full(api.delta_chunks_scratch(tokens, 2, heads, D, V), float("nan"), device=DEV)
+                api.delta_chunks(qkv, raw, 0, heads, dt_bias, a_log, state, out, cu, slots, 2, heads, heads, D, V, scratch)
+            else:
+                api.delta_scan(qkv, raw, 0, heads, dt_bias, a_log, state, out, cu, slots, 2, heads, heads, D, V)
+            forms.append((out, state))
+        outs.append(forms)
+    (clean, clean_state), (out, state) = outs[0][0], outs[1][0]
+    by_token, by_token_state = outs[1][1]
+    assert torch.equal(out[:token], clean[:token]) and torch.equal(out[news[0]:], clean[news[0]:]) and torch.equal(state[0], clean_state[0])
+    assert torch.equal(out.isfinite(), by_token.isfinite()) and torch.equal(state.isfinite(), by_token_state.isfinite())
+
+
 # --------------------------------------------------------------------------------- the passes around the recurrences
 @pytest.mark.parametrize("group,groups,tokens", [(4, 3, 2), (128, 5, 9), (132, 2, 3), (256, 4, 33), (260, 1, 40), (1024, 2, 600), (1028, 1, 7), (4096, 1, 1030), (8192, 1, 3), (30, 4, 5)])
 @pytest.mark.parametrize("splits,gate_first,gate,dtype", [(1, True, "silu", torch.bfloat16), (5, False, "sigmoid", torch.float32)])

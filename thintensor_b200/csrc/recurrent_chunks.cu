@@ -246,7 +246,8 @@ scan_chunks_prepare_kernel(const ScanChunks a) {
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) out[(ty + 16 * i) * CK_TOKENS + tx + 16 * j] = j <= i ? total[i][j] : 0.0f;
+        for (int j = 0; j < 4; ++j)                             // zeros above the diagonal: a later token's score may be no number
+            out[(ty + 16 * i) * CK_TOKENS + tx + 16 * j] = tx + 16 * j <= ty + 16 * i ? total[i][j] : 0.0f;
 }
 
 // -------------------------------------------------------------------------------------------------- the walk over the chunks
@@ -286,6 +287,28 @@ __device__ __forceinline__ void ck_product(unsigned long long (&acc)[4][2], cons
         multiply(an, bn);
     }
 }
+
+// The same with what lies behind a row left out instead of multiplied by the zeros that stand there: for a chunk with numbers in B
+// that are not finite, which must not reach the tokens before them (0 * inf is no number).  row: this lane's first.
+template <int RL>
+__device__ __forceinline__ void ck_causal_product(unsigned long long (&acc)[4][2], const float* __restrict__ A, int lda, const float* __restrict__ B, int ldb, int k0, int stride, int k_end, int row) {
+#pragma unroll 1
+    for (int k = k0; k < k_end; k += stride)
+#pragma unroll 1
+        for (int e = 0; e < 4; ++e) {
+            const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(B + (k + e) * ldb);
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                if (k + e > row + RL * r) continue;
+                const float v = A[r * RL * lda + k + e];
+                const unsigned long long twice = ck_pair(v, v);
+                ck_fma2(acc[r][0], twice, y.x);
+                ck_fma2(acc[r][1], twice, y.y);
+            }
+        }
+}
+// zero for finite numbers, no number otherwise
+__device__ __forceinline__ float ck_not_finite(const float4& x) { return fmaf(x.x, 0.0f, fmaf(x.y, 0.0f, fmaf(x.z, 0.0f, x.w * 0.0f))); }
 
 // Two such products with the same B (k0 .. k0 + K - 1 in sums of 32, which are added up: a long chain of additions loses more)
 template <int RL, int K>
@@ -493,6 +516,7 @@ scan_chunks_kernel(const ScanChunks a) {
         __syncthreads();                                        // this chunk's numbers and the state are there
 
         // the decays into the scores, and the rows the update adds
+        float odd = 0.0f;                                       // no longer zero: an x of the chunk is not finite
         {
             const int j = 4 * (threadIdx.x & 15), bj = j >> 3;
             const float4 v = *reinterpret_cast<const float4*>(F + CK_V + j);
@@ -518,6 +542,7 @@ scan_chunks_kernel(const ScanChunks a) {
                 const int t = e / PL, c = 4 * (e - t * PL);
                 const float4 x = *reinterpret_cast<const float4*>(X + t * L::LDX + c);
                 const float w = F[CK_W + t];
+                odd += ck_not_finite(x);
                 *reinterpret_cast<float4*>(XW + t * L::LDX + c) = make_float4(w * x.x, w * x.y, w * x.z, w * x.w);
             }
         }
@@ -532,9 +557,10 @@ scan_chunks_kernel(const ScanChunks a) {
             acc[r][0] = ck_pair(ck_lo(acc[r][0]) * e, ck_hi(acc[r][0]) * e);
             acc[r][1] = ck_pair(ck_lo(acc[r][1]) * e, ck_hi(acc[r][1]) * e);
         }
-        __syncthreads();                                        // scores and weighted rows are written, C and the old state are read
+        const bool finite = !__syncthreads_or(odd != 0.0f);     // scores and weighted rows are written, C and the old state are read
         fetch_a(chunk + 1);
-        ck_product<RL>(acc, M + row * CK_MLD, CK_MLD, X + col, L::LDX, 4 * slice, 4 * L::SLICES, block * L::ROWS + L::ROWS);
+        if (finite) ck_product<RL>(acc, M + row * CK_MLD, CK_MLD, X + col, L::LDX, 4 * slice, 4 * L::SLICES, block * L::ROWS + L::ROWS);
+        else ck_causal_product<RL>(acc, M + row * CK_MLD, CK_MLD, X + col, L::LDX, 4 * slice, 4 * L::SLICES, block * L::ROWS + L::ROWS, row);
         if (slice > 0) {
 #pragma unroll
             for (int r = 0; r < 4; ++r)
@@ -922,6 +948,7 @@ delta_chunks_kernel(const DeltaChunks a) {
         }
         __syncthreads();                                        // W S is whole; q, W and the old state are read
         fetch_first(chunk + 1);
+        float odd = 0.0f;                                       // no longer zero: a number of U is not finite
         for (int e = threadIdx.x; e < CK_TOKENS * PL; e += CK_THREADS) {           // U = U0 - W S, and the rows the update adds
             const int t = e / PL, c = 4 * (e % PL);
             float4 u = *reinterpret_cast<const float4*>(X + t * D_::LDX + c);
@@ -933,6 +960,7 @@ delta_chunks_kernel(const DeltaChunks a) {
             }
             u.x -= ws.x; u.y -= ws.y; u.z -= ws.z; u.w -= ws.w;
             const float w = F[CD_W + t];
+            odd += ck_not_finite(u);
             *reinterpret_cast<float4*>(X + t * D_::LDX + c) = u;
             *reinterpret_cast<float4*>(XW + t * D_::LDX + c) = make_float4(w * u.x, w * u.y, w * u.z, w * u.w);
         }
@@ -942,8 +970,9 @@ delta_chunks_kernel(const DeltaChunks a) {
             acc[r][0] = ck_pair(ck_lo(acc[r][0]) * e, ck_hi(acc[r][0]) * e);
             acc[r][1] = ck_pair(ck_lo(acc[r][1]) * e, ck_hi(acc[r][1]) * e);
         }
-        __syncthreads();                                        // U is there
-        ck_product<RL>(acc, M + row * CK_MLD, CK_MLD, X + col, D_::LDX, 4 * slice, 4 * L::SLICES, block * L::ROWS + L::ROWS);
+        const bool finite = !__syncthreads_or(odd != 0.0f);     // U is there
+        if (finite) ck_product<RL>(acc, M + row * CK_MLD, CK_MLD, X + col, D_::LDX, 4 * slice, 4 * L::SLICES, block * L::ROWS + L::ROWS);
+        else ck_causal_product<RL>(acc, M + row * CK_MLD, CK_MLD, X + col, D_::LDX, 4 * slice, 4 * L::SLICES, block * L::ROWS + L::ROWS, row);
         if (slice > 0) {
 #pragma unroll
             for (int r = 0; r < 4; ++r)
