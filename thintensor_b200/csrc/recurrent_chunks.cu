@@ -594,19 +594,16 @@ scan_chunks_kernel(const ScanChunks a) {
     }
 }
 
+// on every launch: it holds for the current device alone, and an engine may run on any of the process's
 template <typename Kernel>
 static cudaError_t ck_allow(Kernel kernel, size_t bytes) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); }
 
 template <int NP, int TP>
 static int scan_chunks_launch(const ScanChunks& a, int max_slots, cudaStream_t stream) {
     constexpr size_t prepare_bytes = (size_t)2 * CK_TOKENS * (NP + 4) * sizeof(float);
-    static bool allowed = false;
-    if (!allowed) {
-        cudaError_t code = ck_allow(scan_chunks_prepare_kernel<NP>, prepare_bytes);
-        if (code == cudaSuccess) code = ck_allow(scan_chunks_kernel<NP, TP>, CkLayout<NP, TP>::BYTES);
-        if (code != cudaSuccess) return (int)code;
-        allowed = true;
-    }
+    cudaError_t code = ck_allow(scan_chunks_prepare_kernel<NP>, prepare_bytes);
+    if (code == cudaSuccess) code = ck_allow(scan_chunks_kernel<NP, TP>, CkLayout<NP, TP>::BYTES);
+    if (code != cudaSuccess) return (int)code;
     tt_launch_pdl(scan_chunks_prepare_kernel<NP>, dim3(max_slots, a.groups, (a.heads / a.groups + CK_WARPS - 1) / CK_WARPS), dim3(CK_THREADS), prepare_bytes, stream, a);
     tt_launch_pdl(scan_chunks_kernel<NP, TP>, dim3(a.heads, a.sequences, (a.P + TP - 1) / TP), dim3(CkLayout<NP, TP>::THREADS), CkLayout<NP, TP>::BYTES, stream, a);
     TT_LAUNCH_CHECK();
@@ -1002,13 +999,9 @@ delta_chunks_kernel(const DeltaChunks a) {
 template <int NP, int TP>
 static int delta_chunks_launch(const DeltaChunks& a, int max_slots, cudaStream_t stream) {
     constexpr size_t prepare_bytes = (size_t)(2 * CK_TOKENS * (NP + 4) + CK_TOKENS * CK_MLD + CK_FACTORS + 5 * CK_TOKENS) * sizeof(float);
-    static bool allowed = false;
-    if (!allowed) {
-        cudaError_t code = ck_allow(delta_chunks_prepare_kernel<NP>, prepare_bytes);
-        if (code == cudaSuccess) code = ck_allow(delta_chunks_kernel<NP, TP>, CdLayout<NP, TP>::BYTES);
-        if (code != cudaSuccess) return (int)code;
-        allowed = true;
-    }
+    cudaError_t code = ck_allow(delta_chunks_prepare_kernel<NP>, prepare_bytes);
+    if (code == cudaSuccess) code = ck_allow(delta_chunks_kernel<NP, TP>, CdLayout<NP, TP>::BYTES);
+    if (code != cudaSuccess) return (int)code;
     tt_launch_pdl(delta_chunks_prepare_kernel<NP>, dim3(max_slots, a.heads), dim3(CD_THREADS), prepare_bytes, stream, a);
     tt_launch_pdl(delta_chunks_kernel<NP, TP>, dim3(a.heads, a.sequences, (a.V + TP - 1) / TP), dim3(CK_THREADS), CdLayout<NP, TP>::BYTES, stream, a);
     TT_LAUNCH_CHECK();
