@@ -234,11 +234,11 @@ static int vec4(const void* p, long long ld) { return ((uintptr_t)p % (4 * sizeo
 
 template <typename TX, typename TW>
 static int launch(const void* x, long long ldx, const void* w, long long ldw, const float* bias, float* out,
-                  long long ldo, long long split_stride, int m, int n, int k, int splits, cudaStream_t stream) {
+                  long long ldo, long long split_stride, int m, int n, int k, int splits, int sms, cudaStream_t stream) {
     const int vec_x = vec4<TX>(x, ldx), vec_w = vec4<TW>(w, ldw);
     if (m <= 16 && splits == 1) {
         // fewer than eight warps an SM: the four warps of a block share its columns
-        const int k_warps = n < 8 * GR_COLS * 148 ? GR_WARPS : 1, cols = k_warps > 1 ? GR_COLS : GR_WARPS * GR_COLS;
+        const int k_warps = n < 8 * GR_COLS * sms ? GR_WARPS : 1, cols = k_warps > 1 ? GR_COLS : GR_WARPS * GR_COLS;
 #define TT_ROWS(ROWS) tt_launch_pdl(gemm_rows_kernel<TX, TW, ROWS>, dim3((n + cols - 1) / cols), dim3(GR_WARPS * 32), 0, stream, (const TX*)x, ldx, (const TW*)w, ldw, bias, out, ldo, m, n, k, vec_x, vec_w, k_warps)
         if (m == 1) TT_ROWS(1); else if (m <= 4) TT_ROWS(4); else TT_ROWS(8);
 #undef TT_ROWS
@@ -253,14 +253,15 @@ static int launch(const void* x, long long ldx, const void* w, long long ldw, co
     TT_LAUNCH_CHECK();
 }
 
+// sms: the device's multiprocessors
 extern "C" int tt_gemm_simt(const void* x, int x_dtype, long long ldx, const void* w, int w_dtype, long long ldw,
                             const float* bias, float* out, long long ldo, long long split_stride, int m, int n, int k,
-                            int splits, cudaStream_t stream) {
+                            int splits, int sms, cudaStream_t stream) {
     if (m <= 0 || n <= 0) return 0;
     if (k <= 0 || splits < 1 || splits > 64) return (int)cudaErrorInvalidValue;
-    if (x_dtype == TT_F32 && w_dtype == TT_F32) return launch<float, float>(x, ldx, w, ldw, bias, out, ldo, split_stride, m, n, k, splits, stream);
-    if (x_dtype == TT_BF16 && w_dtype == TT_BF16) return launch<__nv_bfloat16, __nv_bfloat16>(x, ldx, w, ldw, bias, out, ldo, split_stride, m, n, k, splits, stream);
-    if (x_dtype == TT_BF16 && w_dtype == TT_F32) return launch<__nv_bfloat16, float>(x, ldx, w, ldw, bias, out, ldo, split_stride, m, n, k, splits, stream);
-    if (x_dtype == TT_F32 && w_dtype == TT_BF16) return launch<float, __nv_bfloat16>(x, ldx, w, ldw, bias, out, ldo, split_stride, m, n, k, splits, stream);
+    if (x_dtype == TT_F32 && w_dtype == TT_F32) return launch<float, float>(x, ldx, w, ldw, bias, out, ldo, split_stride, m, n, k, splits, sms, stream);
+    if (x_dtype == TT_BF16 && w_dtype == TT_BF16) return launch<__nv_bfloat16, __nv_bfloat16>(x, ldx, w, ldw, bias, out, ldo, split_stride, m, n, k, splits, sms, stream);
+    if (x_dtype == TT_BF16 && w_dtype == TT_F32) return launch<__nv_bfloat16, float>(x, ldx, w, ldw, bias, out, ldo, split_stride, m, n, k, splits, sms, stream);
+    if (x_dtype == TT_F32 && w_dtype == TT_BF16) return launch<float, __nv_bfloat16>(x, ldx, w, ldw, bias, out, ldo, split_stride, m, n, k, splits, sms, stream);
     return (int)cudaErrorInvalidValue;
 }

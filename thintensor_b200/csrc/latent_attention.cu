@@ -689,7 +689,7 @@ latent_merge_expand_group_kernel(const float* __restrict__ part_acc, const float
 extern "C" int tt_latent_prepare(const float* down, int splits, long long split_stride, int row_stride, int q_rank, int rank, int rot,
                                  const float* q_weight, const float* kv_weight, float eps, const float* inv_freq, int rotary_dim,
                                  int interleaved, float rot_scale, void* q_latent, int act_dtype, void* pool, int cache_dtype, const int* table, int table_width,
-                                 int pool_blocks, const int* cu, const int* len_before, int sequences, int n_tokens, unsigned* status,
+                                 int pool_blocks, const int* cu, const int* len_before, int sequences, int n_tokens, unsigned* status, int sms,
                                  cudaStream_t stream) {
     if (n_tokens <= 0) return 0;
     const int cols = q_rank + rank + rot;
@@ -698,7 +698,7 @@ extern "C" int tt_latent_prepare(const float* down, int splits, long long split_
         return (int)cudaErrorInvalidValue;
     const size_t shared = (size_t)(cols + 32) * sizeof(float);
     if (shared > 48 * 1024) return (int)cudaErrorInvalidValue;
-    const int threads = n_tokens <= 148 && cols >= 1024 ? 512 : cols >= 1024 ? 256 : 128;        // few tokens: a row over more threads
+    const int threads = n_tokens <= sms && cols >= 1024 ? 512 : cols >= 1024 ? 256 : 128;        // few tokens: a row over more threads
 #define TT_PREP(T) tt_launch_pdl(latent_prepare_kernel<T, T>, dim3(n_tokens), dim3(threads), shared, stream, down, splits, (size_t)split_stride, row_stride, q_rank, rank, rot, q_weight, kv_weight, eps, inv_freq, rotary_dim, interleaved, rot_scale, (T*)q_latent, (T*)pool, table, table_width, pool_blocks, cu, len_before, sequences, status)
     if (act_dtype == TT_F32) TT_PREP(float); else TT_PREP(__nv_bfloat16);
 #undef TT_PREP

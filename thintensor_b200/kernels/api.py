@@ -1253,12 +1253,12 @@ def latent_prepare(down: torch.Tensor, q_rank: int, rank: int, rot: int, q_weigh
         raise KernelError(f"latent_prepare: {cols} projected numbers per token are more than the kernel stages")
     fn = _fn("latent_attention", "tt_latent_prepare", [c_void_p, c_int, c_longlong, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_float,
                                                        c_void_p, c_int, c_int, c_float, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int,
-                                                       c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p])
+                                                       c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p])
     code = dtype_code(q_latent.dtype if q_rank else pool.dtype)
     _check(fn(p, splits, stride, row_stride, q_rank, rank, rot, _ptr(q_weight), _ptr(kv_weight), eps, _ptr(inv_freq), rotary_dim,
               1 if interleaved else 0, float(rot_scale), _ptr(q_latent), code,
               _ptr(pool), code, _ptr(table), table.shape[1], 0 if pool is None else pool.shape[0], _ptr(cu), _ptr(len_before), sequences,
-              n_tokens, _ptr(status), _stream()), "latent_prepare")
+              n_tokens, _ptr(status), sm_count(down.device), _stream()), "latent_prepare")
 
 
 def latent_attention(q: torch.Tensor, w_key: torch.Tensor, w_value: torch.Tensor, pool: torch.Tensor, table: torch.Tensor, cu: torch.Tensor,
@@ -1593,9 +1593,9 @@ def gemm_simt(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None, out: 
     if bias is not None:
         _need(bias, torch.float32, "bias")
     fn = _fn("gemm_simt", "tt_gemm_simt", [c_void_p, c_int, c_longlong, c_void_p, c_int, c_longlong, c_void_p, c_void_p, c_longlong,
-                                           c_longlong, c_int, c_int, c_int, c_int, c_void_p])
+                                           c_longlong, c_int, c_int, c_int, c_int, c_int, c_void_p])
     _check(fn(_ptr(x), dtype_code(x.dtype), x.stride(0), _ptr(w), dtype_code(w.dtype), w.stride(0), _ptr(bias), _ptr(out), out.stride(1),
-              out.stride(0), m, n, k, out.shape[0], _stream()), "gemm_simt")
+              out.stride(0), m, n, k, out.shape[0], sm_count(x.device), _stream()), "gemm_simt")
 
 
 def gemm_simt_splits(tokens: int, features: int, k: int, sms: int | None = None) -> int:
