@@ -110,18 +110,39 @@ def in_blocks(ctx) -> bool:
     return not ctx.decode and ctx.n_tokens >= 4 * ctx.sequences
 
 
-CHUNKS_FROM = 160
+def scan_chunks_pay(n_tokens: int, sequences: int, ctas: int, sms: int) -> bool:
+    """Whether a Mamba-2 or fixed-decay recurrence runs faster in chunks of 64 tokens than token by token.  A CTA of the walk over the
+    chunks (a sequence, head and 32 columns) has an SM to itself, so that every ``sms`` of them cost a round of equal length, while the kernels that go token by
+    token share the SMs evenly from twice as many CTAs on.  Kernel times, chunks against token by token (us, one B200, 148 SMs): 64 CTAs, one
+    sequence of 160 tokens 29 and 55; 256, four of 160 61 and 79; 320, five of 160 83 and 87, five of 800 309 and 423; 512, eight of 160
+    112 and 96, eight of 320 177 and 188 (32 of 320 with 64 x 64 states 140 and 135), eight of 640 330 and 370; 1,024, eight of 640 537 and
+    530, 16 of 700 637 and 579.  640 CTAs of five sequences of 800 tokens took 452 and 621, in rounds that are nearly full; the line stays at four rounds."""
+    each = n_tokens // sequences
+    return each >= 160 and (ctas <= 3 * sms or (each >= 400 and ctas <= 4 * sms))
 
 
-def in_chunks(ctx, heads: int, columns: int, rows: int) -> bool:
+def delta_chunks_pay(n_tokens: int, sequences: int, ctas: int, key_dim: int, sms: int) -> bool:
+    """The same for the gated delta rule with a decay per head.  Keys of 128 numbers: 64 CTAs, one sequence of 128 tokens 44 and 61; 512, eight of
+    128 110 and 134; 768 (six rounds, the last a fifth full), eight of 128 166 and 143, of 320 363 and 348; 1,024 (seven, full), 16 of 320 445 and 558; 2,048 (14, full),
+    32 of 256 716 and 718; 4,096, 64 of 200 1,393 and 1,032.  Keys of 64: 256 CTAs, four of 128 53 and 71; 512, eight of 128 100 and 97, of 320 222 and 239;
+    1,024, 16 of 500 624 and 581; 4,096, 64 of 200 1,279 and 628."""
+    each, rounds = n_tokens // sequences, -(-ctas // sms)
+    if each < 128:
+        return False
+    if rounds <= 4:
+        return rounds <= 3 or key_dim > 64 or each >= 320
+    return key_dim > 64 and each >= 256 and rounds <= 14 and 10 * ctas >= 9 * rounds * sms      # the last round nearly full
+
+
+def in_chunks(ctx, heads: int, columns: int, rows: int, delta: bool = False) -> bool:
     """Whether a recurrence with a decay per head takes its tokens in chunks of 64 (decided by the step's shape alone, like
-    :func:`in_blocks`): prompts of at least ``CHUNKS_FROM`` tokens on average do (for fewer a launch more eats the gain: a layer of 16 heads of
-    128 x 128 on 130 tokens took 97 us token by token and 112 in chunks, on 200 141 and 104), while the grid of a CTA per sequence, head and 32 columns
-    is at most four rounds of the SMs.  Measured on a B200 (us, chunks against token by token): 64 heads of 64 x 128, one sequence
-    of 64 tokens 23 and 33, of 40 tokens 22 and 22; two of 48 33 and 28; four of 731 332 and 545 (512 CTAs), 16 of 700 (2,048 CTAs)
-    1,060 and 1,035; 24 heads of 256 x 128, five of 96 (960 CTAs) 131 and 84: many CTAs keep the form that goes token by token busy."""
-    return (not ctx.decode and rows <= api.CHUNK_MAX_ROWS and ctx.n_tokens >= CHUNKS_FROM * ctx.sequences
-            and heads * ctx.sequences * -(-columns // 32) <= 4 * api.sm_count(ctx.status.device))
+    :func:`in_blocks`, and so by the average of a step's lengths: a prompt among many sequences of one token goes token by token)."""
+    if ctx.decode or rows > api.CHUNK_MAX_ROWS:
+        return False
+    ctas, sms = heads * ctx.sequences * -(-columns // 32), api.sm_count(ctx.status.device)
+    if delta:
+        return delta_chunks_pay(ctx.n_tokens, ctx.sequences, ctas, rows, sms)
+    return scan_chunks_pay(ctx.n_tokens, ctx.sequences, ctas, sms)
 
 
 @MIXERS.register("mamba2")
@@ -206,11 +227,6 @@ class GatedDelta(Mixer):
              "v_conv": "v_conv1d.weight", "b": "b_proj.weight", "a": "a_proj.weight", "g": "g_proj.weight", "dt_bias": "dt_bias",
              "A_log": "A_log", "norm": "o_norm.weight", "out": "o_proj.weight", "a1": "a1_proj.weight", "a2": "a2_proj.weight",
              "g1": "g1_proj.weight", "g2": "g2_proj.weight"}
-
-    # Prompts of at least so many tokens on average go in chunks of 64 (decays per head; decided by the step's shape alone).  Measured on
-    # a B200, 16 heads of 128 x 128 (us, chunks against token by token): one sequence of 64 tokens 42 and 35, five of 64 69 and 70, one of
-    # 700 (8 heads) 96 and 315, one of 4,097 478 and 1,950, 16 of 500 671 and 869.
-    CHUNKS_FROM = 128
 
     def __init__(self, hidden: int, heads: int, qk_heads: int, key_dim: int, value_dim: int, conv: int = 4, eps: float = 1e-6,
                  names: dict | None = None, channel_decay: int | None = None, low_rank_gate: int | None = None, gate: str = "silu"):
@@ -302,7 +318,7 @@ class GatedDelta(Mixer):
         if decay is not None and in_blocks(ctx):
             api.row_decay_blocks(qkv[:, :self.qk], qkv[:, self.qk: 2 * self.qk], qkv[:, 2 * self.qk:], decay, recurrent, read, ctx.cu, ctx.slots,
                                  ctx.sequences, self.heads, self.qk_heads, self.key_dim, self.value_dim, self.key_dim ** -0.5, (proj, self.b_col))
-        elif decay is None and not ctx.decode and self.key_dim <= api.CHUNK_MAX_ROWS and tokens >= self.CHUNKS_FROM * ctx.sequences:
+        elif decay is None and in_chunks(ctx, self.heads, self.value_dim, self.key_dim, delta=True):
             shape = api.delta_chunks_scratch(tokens, ctx.sequences, self.heads, self.key_dim, self.value_dim)
             api.delta_chunks(qkv, proj, self.b_col, self.a_col, self.dt_bias, self.a_log, recurrent, read, ctx.cu, ctx.slots, ctx.sequences, self.heads,
                              self.qk_heads, self.key_dim, self.value_dim, ctx.scratch("chunks.delta", shape, torch.float32))
