@@ -43,3 +43,10 @@ def test_which_prompts_take_the_delta_rule_in_chunks(sequences, each, ctas, key_
     from thintensor_b200.parts.recurrent import delta_chunks_pay
 
     assert delta_chunks_pay(sequences * each, sequences, ctas, key_dim, 148) == chunks
+
+
+@pytest.mark.parametrize("decay,chunks", [((0.9, 1.0), True), ((-1.0, 0.0), True), ((0.9, 1.0001), False), ((-8.0, 0.5), False), ((float("nan"), 0.5), False)])
+def test_decays_beyond_one_go_token_by_token(decay, chunks):
+    from thintensor_b200.parts.recurrent import DecayLinearAttention
+
+    assert DecayLinearAttention(hidden=64, heads=2, key_dim=16, value_dim=16, decay=decay).chunks == chunks

@@ -346,6 +346,9 @@ class DecayLinearAttention(Mixer):
         self.decay = None if decay is None else tuple(float(d) for d in decay)
         if self.decay is not None and len(self.decay) != self.heads:
             raise ValueError(f"{len(self.decay)} decays for {self.heads} heads")
+        # Chunks multiply a state by the product of up to 64 decays at once: decays beyond one could overflow there where the recurrence does
+        # not (8^64 times a state of zero), so they go token by token.
+        self.chunks = self.decay is not None and all(abs(d) <= 1.0 for d in self.decay)
         self.rank = None if channel_decay is None else int(channel_decay["rank"])
         self.tau = None if channel_decay is None else float(channel_decay["tau"])
         self.query_scale = float(query_scale)
@@ -444,7 +447,7 @@ class DecayLinearAttention(Mixer):
                                  self.value_dim, 1.0)
         elif decay is not None:
             api.row_decay_scan(vkq, decay, recurrent, read, ctx.cu, ctx.slots, ctx.sequences, self.heads, self.key_dim, self.value_dim)
-        elif in_chunks(ctx, self.heads, self.value_dim, self.key_dim):
+        elif self.chunks and in_chunks(ctx, self.heads, self.value_dim, self.key_dim):
             scratch = ctx.scratch("chunks.scan", api.scan_chunks_scratch(tokens, ctx.sequences, self.heads, self.heads), torch.float32)
             api.scan_chunks(vkq, 0, self.v, self.v + self.qk, recurrent, read, ctx.cu, ctx.slots, ctx.sequences, self.heads, self.value_dim, self.key_dim,
                             self.heads, scratch, fixed_decay=self.decays)
