@@ -432,3 +432,10 @@ def test_routing_of_prompts(hidden, experts, extra, tokens):
     torch.testing.assert_close(gates[:, experts:].double(), torch.sigmoid(logits[:, experts:]), rtol=1e-4, atol=1e-6)
     dense = torch.zeros(tokens, experts, device=DEV).scatter_(1, chosen.long(), weights)
     assert torch.equal(gates[:, :experts], dense)
+
+
+@pytest.mark.parametrize("hidden,experts,extra,tokens", [(512, 6, 1, 1185), (504, 8, 0, 1185), (768, 16, 0, 1200), (1024, 40, 0, 1300), (1536, 5, 0, 1037), (1792, 7, 0, 1025),
+                                                         (2560, 16, 0, 1025), (2568, 9, 1, 1030), (3584, 20, 0, 1025), (3592, 8, 0, 1025)])
+def test_routing_at_row_lengths(hidden, experts, extra, tokens):
+    """Both forms on both sides of the shortest rows that a warp takes, and every instance at the ends of its row lengths."""
+    test_routing_of_prompts(hidden, experts, extra, tokens)

@@ -213,9 +213,10 @@ __global__ void route_rows_kernel(const TX* __restrict__ x, const TW* __restrict
     if (warp == 0) route_token(logits, 1, 0, t, experts, top, groups, keep, gates, chosen, weights, logits + experts + opt.extra, opt);
 }
 
-// The same for prompts in bfloat16: a warp a token, its row in the lanes' registers (16 bytes each, up to RT_PIECES of them), so that
+// The same for prompts in bfloat16: a warp a token, its row in the lanes' registers (16 bytes each, up to RT_PIECES of them; instances
+// for rows of up to 2,048, 2,560, 3,584 and 4,096 numbers, because pieces without numbers cost as much as others), so that
 // the router's rows, which the block's eight warps read together, come out of the L1 and no barrier stands between a token's steps.
-// 2,048 tokens of 2,048 numbers, 16 experts: 47 -> 33 us (a block a token staged its row and re-read the matrix from the L2).
+// 2,048 tokens of 2,048 numbers, 16 experts: 30 -> 16 us (a block a token staged its row and re-read the matrix from the L2).
 constexpr int RT_WARPS = 8, RT_PIECES = 16;                     // rows of up to 4,096 numbers
 
 template <int PIECES>
@@ -309,9 +310,10 @@ __global__ void scale_expert_columns_vec_kernel(T* __restrict__ act, int row_str
     *p = raw;
 }
 
+// sms: the device's multiprocessors
 extern "C" int tt_route_rows(const void* x, int x_dtype, const void* w, int w_dtype, int hidden, int n_tokens, int experts, int top,
                              int groups, int keep, float* gates, int* chosen, float* weights, int sigmoid, const float* correction,
-                             int group_top2, int plain_weights, int extra, float weight_scale, cudaStream_t stream) {
+                             int group_top2, int plain_weights, int extra, float weight_scale, int sms, cudaStream_t stream) {
     if (n_tokens <= 0) return 0;
     if (experts <= 0 || experts > ROUTE_MAX_EXPERTS || top < 1 || top > 32 || top > experts || groups < 1 || groups > 32 ||
         experts % groups || keep < 1 || keep > groups || extra < 0 || extra > 32)
@@ -319,11 +321,22 @@ extern "C" int tt_route_rows(const void* x, int x_dtype, const void* w, int w_dt
     const RouteOptions opt{sigmoid, correction, group_top2, plain_weights, extra, weight_scale};
     const size_t shared = (size_t)(hidden + experts + extra + 32) * sizeof(float);
     if (shared > 48 * 1024) return (int)cudaErrorInvalidValue;
-    // a warp a token from as many tokens on as fill two warps of every SM's schedulers (below that a token's experts are shared out over a block)
-    if (n_tokens > 1024 && x_dtype == TT_BF16 && w_dtype == TT_BF16 && hidden % 8 == 0 && hidden <= 32 * 8 * RT_PIECES && (((uintptr_t)x | (uintptr_t)w) & 15) == 0) {
+    // A warp a token.  It pays a reduction for every expert, so rows have to be long enough for their products to outweigh it, the longer the
+    // more experts there are; and tokens enough for a block of eight on every SM, or rows so long that 129 blocks do.  Measured, a block a
+    // token against a warp a token (us): 2,048 tokens of 2,048 numbers, 16 experts 30 and 16, 256 experts 321 and 167; 512 numbers, 8 experts
+    // 12.7 and 10.0, 64 experts 32 and 37; 768 numbers, 64 experts 43 and 38, but 3,000 tokens a sixth the other way; 1,024 numbers, 256 experts
+    // 169 and 133, 3,000 tokens 6 % the other way; 1,183 tokens of 1,536 numbers, 4 experts 9.0 and 7.1; 1,025 of them, 64 experts 7 % the other
+    // way, of 1,792 numbers a seventh less.
+    const int row_from = experts + extra <= 8 ? 512 : experts + extra <= 16 ? 768 : 1024;
+    const int row_least = n_tokens > RT_WARPS * sms ? row_from : n_tokens > (RT_WARPS - 1) * sms ? 1536 : 1792;
+    if (n_tokens > 1024 && hidden >= row_least && x_dtype == TT_BF16 && w_dtype == TT_BF16 && hidden % 8 == 0 && hidden <= 32 * 8 * RT_PIECES && (((uintptr_t)x | (uintptr_t)w) & 15) == 0) {
         const size_t each = (size_t)RT_WARPS * (experts + extra + 32) * sizeof(float);
 #define TT_ROUTE_TOKENS(PIECES) tt_launch_pdl(route_tokens_kernel<PIECES>, dim3((n_tokens + RT_WARPS - 1) / RT_WARPS), dim3(32 * RT_WARPS), each, stream, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, hidden, n_tokens, experts, top, groups, keep, gates, chosen, weights, opt)
-        if (hidden <= 32 * 8 * 8) TT_ROUTE_TOKENS(8); else TT_ROUTE_TOKENS(RT_PIECES);
+        const int pieces = (hidden + 255) / 256;
+        if (pieces <= 8) TT_ROUTE_TOKENS(8);
+        else if (pieces <= 10) TT_ROUTE_TOKENS(10);
+        else if (pieces <= 14) TT_ROUTE_TOKENS(14);
+        else TT_ROUTE_TOKENS(RT_PIECES);
 #undef TT_ROUTE_TOKENS
         TT_LAUNCH_CHECK();
     }

@@ -1505,9 +1505,9 @@ def route_rows(x: torch.Tensor, w: torch.Tensor, top: int, groups: int, keep: in
     if tuple(gates.shape) != (tokens, experts + extra) or tuple(chosen.shape) != (tokens, top) or tuple(weights.shape) != (tokens, top):
         raise KernelError("route_rows: outputs do not fit the sizes")
     fn = _fn("routing", "tt_route_rows", [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
-                                          c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_float, c_void_p])
+                                          c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_float, c_int, c_void_p])
     _check(fn(_ptr(x), dtype_code(x.dtype), _ptr(w), dtype_code(w.dtype), hidden, tokens, experts, top, groups, keep, _ptr(gates),
-              _ptr(chosen), _ptr(weights), *options, _stream()), "route_rows")
+              _ptr(chosen), _ptr(weights), *options, sm_count(x.device), _stream()), "route_rows")
 
 
 ROUTE_MAX_HIDDEN = 11000
