@@ -439,3 +439,24 @@ def test_routing_of_prompts(hidden, experts, extra, tokens):
 def test_routing_at_row_lengths(hidden, experts, extra, tokens):
     """Both forms on both sides of the shortest rows that a warp takes, and every instance at the ends of its row lengths."""
     test_routing_of_prompts(hidden, experts, extra, tokens)
+
+
+@pytest.mark.parametrize("width,shared", [(8, 0), (16, 24), (5, 0), (12, 3)])                       # whole 16-byte pieces, and single numbers
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("tokens", [1, 37, 700])
+def test_weights_of_experts(width, shared, dtype, tokens):
+    """What an expert made of a token that did not choose it is left out, be it a number or not; every other product is one
+    rounding of the exact one."""
+    from thintensor_b200.kernels import api
+
+    experts = 6
+    act = randn(tokens, experts * width + shared, seed=96, dtype=dtype)
+    gates = randn(tokens, experts + (1 if shared else 0), seed=97).abs() + 0.1
+    gates[:, :experts] *= torch.arange(experts, device=DEV) % 3 == torch.arange(tokens, device=DEV)[:, None] % 3
+    each = gates[:, :experts].repeat_interleave(width, 1)
+    each = torch.cat((each, gates[:, experts:].expand(tokens, shared)), 1) if shared else each
+    act[each == 0] = float("inf")
+    act[:, 1] = torch.where(each[:, 1] == 0, float("nan"), act[:, 1].float()).to(dtype)
+    want = torch.where(each == 0, torch.zeros((), device=DEV), act.float() * each).to(dtype)
+    api.scale_expert_columns(act, width, gates, experts, shared)
+    assert torch.equal(act, want)
