@@ -727,9 +727,12 @@ extern "C" int tt_latent_attention(const float* q, int q_splits, long long q_str
     if (rows > 2147483647LL) return (int)cudaErrorInvalidValue;
     const size_t shared = (size_t)LAT_WARPS * (rank + rot) * sizeof(float);
     const dim3 grid((unsigned)blocks, splits), block(LAT_WARPS * 32);
-    // Wv_h is fetched for several tokens at a time from eight tokens on (fewer leave too few blocks).  The same for Wk_h measured
-    // no difference (48 tokens, 16 heads: 122.4 and 122.6 us for the layer): the queries' k-slices are what that kernel waits for.
-    const bool grouped = n_tokens >= 8 && (n_tokens + LM_TOKENS - 1) / LM_TOKENS <= 65535;
+    // Wv_h is fetched for several tokens at a time in the tensor-core form, from eight tokens and 64 blocks on: fewer leave SMs idle (8 and 48 tokens
+    // of 4 heads with latents of 64: 12.2 us apart, 13.5 together; 16.8 and 16.6), and behind the other forms, whose slices are few, nothing was
+    // gained (16 heads, latents of 512, 8 tokens 48 and 51 us).  The same for Wk_h measured no difference (48 tokens, 16 heads: 122.4 and 122.6
+    // us for the layer): the queries' k-slices are what that kernel waits for.
+    const int groups = (n_tokens + LM_TOKENS - 1) / LM_TOKENS;
+    const bool grouped = one_token_each == 2 && n_tokens >= 8 && (long long)heads * groups >= 64 && groups <= 65535;
     const bool narrow = one_token_each == 2;                    // the tensor-core form takes the folded queries in bfloat16
 #define TT_ABSORB_AS(TW, TA) tt_launch_pdl(latent_absorb_kernel<TW, TA>, dim3((unsigned)rows), dim3(rank >= 512 ? 512 : rank >= 256 ? 256 : 128), (size_t)(dim + rot) * sizeof(float), stream, q, q_splits, (size_t)q_stride, q_row, (const TW*)w_key, cu, len_before, sequences, heads, dim, rot, rank, inv_freq, rotary_dim, interleaved, rot_scale, scale, (TA*)(void*)absorbed)
 #define TT_ABSORB(TW) do { if (narrow) TT_ABSORB_AS(TW, __nv_bfloat16); else TT_ABSORB_AS(TW, float); } while (0)
