@@ -460,3 +460,16 @@ def test_weights_of_experts(width, shared, dtype, tokens):
     want = torch.where(each == 0, torch.zeros((), device=DEV), act.float() * each).to(dtype)
     api.scale_expert_columns(act, width, gates, experts, shared)
     assert torch.equal(act, want)
+
+
+@pytest.mark.parametrize("group,groups,tokens", [(4, 700, 6), (32, 4, 1023), (32, 4, 1025), (60, 1, 4100), (64, 1, 5)])
+@pytest.mark.parametrize("splits,gate_first", [(1, True), (9, False)])
+def test_gated_group_norm_of_small_groups(group, groups, tokens, splits, gate_first):
+    """On both sides of the number of groups from which small ones go in pieces, with slices that do not fill a round of loads."""
+    test_gated_group_norm_by_pieces(group, groups, tokens, splits, gate_first, "silu", torch.float32)
+
+
+@pytest.mark.parametrize("heads,D,V,rotary,tokens", [(16, 128, 128, 128, 32), (16, 128, 128, 128, 33), (2, 256, 4, 256, 200), (2, 12, 8, 0, 3200), (3, 64, 20, 24, 1400)])
+def test_linear_attention_inputs_of_prompts(heads, D, V, rotary, tokens):
+    """On both sides of the size from which they are made in pieces."""
+    test_linear_attention_inputs_by_pieces(heads, D, V, rotary, tokens, True)

@@ -42,10 +42,18 @@ __device__ __forceinline__ float rec_sum_slices(const float* __restrict__ p, int
     return total;
 }
 
-// the same for four neighbouring elements on a 16-byte boundary (split_stride a multiple of four)
+// the same for four neighbouring elements on a 16-byte boundary (split_stride a multiple of four); LONG: eight loads in flight
+template <bool LONG>
 __device__ __forceinline__ float4 rec_sum_slices4(const float* __restrict__ p, int splits, size_t split_stride) {
     float4 total = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     int s = 0;
+    for (; LONG && s + 8 <= splits; s += 8) {
+        float4 v[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = __ldg(reinterpret_cast<const float4*>(p + (size_t)(s + e) * split_stride));
+#pragma unroll
+        for (int e = 0; e < 8; ++e) { total.x += v[e].x; total.y += v[e].y; total.z += v[e].z; total.w += v[e].w; }
+    }
     for (; s + 4 <= splits; s += 4) {
         float4 v[4];
 #pragma unroll
@@ -583,7 +591,7 @@ linear_attention_prepare4_kernel(const float* __restrict__ proj, int splits, siz
     const float* row = proj + (size_t)t * cols;
     float* out = vkq + (size_t)t * (hv + 2 * qk);
     auto load = [&](int j) {
-        float4 x = rec_sum_slices4(row + j, splits, split_stride);
+        float4 x = rec_sum_slices4<false>(row + j, splits, split_stride);
         if (activation) { x.x = rec_silu(x.x); x.y = rec_silu(x.y); x.z = rec_silu(x.z); x.w = rec_silu(x.w); }
         return x;
     };
@@ -613,8 +621,10 @@ extern "C" int tt_linear_attention_prepare(const float* proj, int splits, long l
     if (n_tokens <= 0) return 0;
     if (rotary_dim < 0 || rotary_dim > D || (rotary_dim & 1) || 2 * heads * D + heads * V > cols) return (int)cudaErrorInvalidValue;
     const int total = 2 * heads * D + heads * V;
-    if (D % 4 == 0 && V % 4 == 0 && cols % 4 == 0 && split_stride % 4 == 0 && (rotary_dim / 2) % 4 == 0 && rotary_dim <= REC_MAX_ROWS
-        && (((uintptr_t)proj | (uintptr_t)vkq) & 15) == 0) {
+    // pieces from 200,000 numbers on: below, a number a thread is the shorter chain (16 heads of 128 rotated whole, 8 tokens: 2.2 us against 2.9;
+    // 64 tokens: 4.3 against 4.1)
+    if ((long long)n_tokens * total >= 200000 && D % 4 == 0 && V % 4 == 0 && cols % 4 == 0 && split_stride % 4 == 0 && (rotary_dim / 2) % 4 == 0
+        && rotary_dim <= REC_MAX_ROWS && (((uintptr_t)proj | (uintptr_t)vkq) & 15) == 0) {
         const int blocks = n_tokens >= 1024 ? (total + 8191) / 8192 : (total + 1023) / 1024;        // eight pieces a thread for prompts, one for few tokens
         tt_launch_pdl(linear_attention_prepare4_kernel, dim3(n_tokens, blocks < 32 ? blocks : 32), dim3(256), 0, stream, proj, splits, (size_t)split_stride, cols,
                       heads, D, V, activation, inv_freq, rotary_dim, q_scale, k_scale, vkq, cu, len_before, sequences);
@@ -1449,7 +1459,7 @@ template <> __device__ __forceinline__ void gn_store4<__nv_bfloat16>(__nv_bfloat
     *reinterpret_cast<uint2*>(to) = *reinterpret_cast<uint2*>(v);
 }
 
-template <typename TOut, int PIECES, bool WARP>
+template <typename TOut, int PIECES, bool WARP, bool LONG>
 __global__ void __launch_bounds__(WARP ? 256 : PIECES == 1 ? 1024 : 512)
 gated_group_norm4_kernel(const float* __restrict__ y, int width, int group, long long total, const float* __restrict__ proj, int splits, size_t split_stride,
                          int cols, int gate_col, const float* __restrict__ weight, int weight_len, float eps, int gate_first, TOut* __restrict__ out,
@@ -1472,7 +1482,7 @@ gated_group_norm4_kernel(const float* __restrict__ y, int width, int group, long
         v[e] = gate[e] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (j < group) {
             v[e] = __ldg(reinterpret_cast<const float4*>(yr + j));
-            gate[e] = rec_sum_slices4(gr + j, splits, split_stride);
+            gate[e] = rec_sum_slices4<LONG>(gr + j, splits, split_stride);
         }
     }
     float sumsq = 0.0f;
@@ -1498,11 +1508,12 @@ gated_group_norm4_kernel(const float* __restrict__ y, int width, int group, long
 template <typename TOut>
 static void gated_group_norm4(const float* y, long long total, int width, int group, const float* proj, int splits, size_t split_stride, int cols, int gate_col,
                               const float* weight, int weight_len, float eps, int gate_first, TOut* out, int gate_kind, cudaStream_t stream) {
-#define TT_GN4(PIECES, WARP, GRID, THREADS) tt_launch_pdl(gated_group_norm4_kernel<TOut, PIECES, WARP>, dim3((unsigned)(GRID)), dim3(THREADS), 0, stream, y, width, group, total, proj, splits, split_stride, cols, gate_col, weight, weight_len, eps, gate_first, out, gate_kind)
+    // eight slices' loads in flight where there are as many and a thread has one piece (the registers cost other forms up to a quarter)
+#define TT_GN4(PIECES, WARP, GRID, THREADS) tt_launch_pdl(PIECES == 1 && splits >= 8 ? gated_group_norm4_kernel<TOut, PIECES, WARP, PIECES == 1> : gated_group_norm4_kernel<TOut, PIECES, WARP, false>, dim3((unsigned)(GRID)), dim3(THREADS), 0, stream, y, width, group, total, proj, splits, split_stride, cols, gate_col, weight, weight_len, eps, gate_first, out, gate_kind)
     const int quads = group / 4;
     if (quads <= 64) {
         if (quads <= 32) TT_GN4(1, true, (total + 7) / 8, 256); else TT_GN4(2, true, (total + 7) / 8, 256);
-    } else if (quads <= 1024 && (total < 296 || quads < 256)) {          // few groups: as many threads as there are pieces
+    } else if (quads <= 1024 && (total < 296 || quads < 256 || (splits >= 8 && total < 1184))) {         // few groups: as many threads as there are pieces
         TT_GN4(1, false, total, (quads + 31) / 32 * 32);
     } else {
         TT_GN4(4, false, total, (quads / 4 + 31 + (quads % 4 > 0)) / 32 * 32);
@@ -1517,7 +1528,9 @@ extern "C" int tt_gated_group_norm(const float* y, int n_tokens, int width, int 
     if (group <= 0 || width % group || weight_len <= 0) return (int)cudaErrorInvalidValue;
     const long long blocks = (long long)n_tokens * (width / group);
     if (blocks > 2147483647LL) return (int)cudaErrorInvalidValue;
-    if (group % 4 == 0 && group <= 4 * 4 * 512 && cols % 4 == 0 && gate_col % 4 == 0 && split_stride % 4 == 0 && weight_len % 4 == 0
+    // groups of fewer than 64 numbers leave half of a warp's lanes without a piece, which pays only where there are many of them (groups of 32:
+    // 256 of them 2.7 us and 2.9 in pieces, 1,200 3.0 and 3.0, with 16 slices of gates 3.1 and 3.7, 2,048 4.0 and 3.5)
+    if (group % 4 == 0 && (group >= 64 || blocks >= 2048) && group <= 4 * 4 * 512 && cols % 4 == 0 && gate_col % 4 == 0 && split_stride % 4 == 0 && weight_len % 4 == 0
         && (((uintptr_t)y | (uintptr_t)proj | (uintptr_t)weight | (uintptr_t)out) & 15) == 0) {
         if (out_dtype == TT_F32)
             gated_group_norm4<float>(y, blocks, width, group, proj, splits, (size_t)split_stride, cols, gate_col, weight, weight_len, eps, gate_first, (float*)out, gate_kind, stream);
