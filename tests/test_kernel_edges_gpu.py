@@ -473,3 +473,19 @@ def test_gated_group_norm_of_small_groups(group, groups, tokens, splits, gate_fi
 def test_linear_attention_inputs_of_prompts(heads, D, V, rotary, tokens):
     """On both sides of the size from which they are made in pieces."""
     test_linear_attention_inputs_by_pieces(heads, D, V, rotary, tokens, True)
+
+
+@pytest.mark.parametrize("m,n,k,pad,splits", [(17, 300, 500, 0, 1), (65, 63, 40, 0, 1), (100, 64, 64, 4, 1), (130, 129, 257, 1, 2), (9, 300, 130, 0, 1), (16, 64, 64, 0, 1),
+                                              (193, 2048, 512, 0, 1), (193, 3072, 512, 4, 2), (97, 300, 1000, 2, 8)])
+@pytest.mark.parametrize("x_dtype,w_dtype", [(torch.float32, torch.float32), (torch.float32, torch.bfloat16), (torch.bfloat16, torch.float32), (torch.bfloat16, torch.bfloat16)])
+def test_exact_product_is_exact_to_float32(m, n, k, pad, splits, x_dtype, w_dtype):
+    """Tiles of both widths, few rows in several passes.  A chain of k multiply-adds whose partial sums grow like sqrt(i) is off by about
+    2^-24 sqrt(k) / 2.4 of the result (2-norm); operands rounded to eleven or eight bits would be off by 2^-12 or more."""
+    from thintensor_b200.kernels import api
+
+    x, w = randn(m, k + pad, seed=1, dtype=x_dtype)[:, pad:], randn(n, k + pad, seed=2, dtype=w_dtype)[:, pad:]
+    wide = torch.full((splits, m, n + pad), 7.0, device=DEV)
+    api.gemm_simt(x, w, None, wide[:, :, :n])
+    want = x.double() @ w.double().T
+    assert float((wide[:, :, :n].double().sum(0) - want).norm() / want.norm()) <= 2.0 ** -24 * (2 * k ** 0.5 + 4)
+    assert bool((wide[:, :, n:] == 7.0).all())
