@@ -489,3 +489,32 @@ def test_exact_product_is_exact_to_float32(m, n, k, pad, splits, x_dtype, w_dtyp
     want = x.double() @ w.double().T
     assert float((wide[:, :, :n].double().sum(0) - want).norm() / want.norm()) <= 2.0 ** -24 * (2 * k ** 0.5 + 4)
     assert bool((wide[:, :, n:] == 7.0).all())
+
+
+@pytest.mark.parametrize("heads,kv_heads,D,V", [(4, 2, 64, 64), (32, 8, 48, 80), (3, 1, 128, 128)])
+@pytest.mark.parametrize("sequences,new,past", [(1, 8, 0), (1, 17, 40), (3, 31, 0), (3, 32, 32), (2, 47, 9), (2, 48, 0), (1, 64, 0)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_exact_attention_of_one_block(heads, kv_heads, D, V, sequences, new, past, dtype):
+    """Tables one block wide, on both sides of the line from which queries go in tiles; the block's places behind the last key hold no
+    numbers."""
+    from thintensor_b200.kernels import api
+
+    tokens, n = sequences * new, past + new
+    k_pool = torch.full((sequences, kv_heads, 64, D), float("nan"), dtype=dtype, device=DEV)
+    v_pool = torch.full((sequences, kv_heads, V, 64), float("nan"), dtype=dtype, device=DEV)
+    k_pool[:, :, :n] = randn(sequences, kv_heads, n, D, seed=110, dtype=dtype)
+    v_pool[:, :, :, :n] = randn(sequences, kv_heads, V, n, seed=111, dtype=dtype)
+    table = torch.arange(sequences, dtype=torch.int32, device=DEV).flip(0)[:, None].contiguous()
+    q, out = randn(tokens, heads * D, seed=112, dtype=dtype), torch.full((tokens, heads * V), 7.0, dtype=dtype, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    api.attention(q, k_pool, v_pool, table, i32([new * i for i in range(sequences + 1)]), i32([past] * sequences), sequences, tokens, heads, kv_heads, D, D ** -0.5,
+                  0, 1, out, None, None, status, value_dim=V)
+    assert int(status) == 0
+    each = heads // kv_heads
+    for s in range(sequences):
+        K, W = (pool[sequences - 1 - s].double() for pool in (k_pool, v_pool))
+        score = torch.einsum("thd,hnd->htn", q[s * new:(s + 1) * new].double().reshape(new, heads, D), K[:, :n].repeat_interleave(each, 0)) * D ** -0.5
+        score = score.masked_fill(torch.arange(n, device=DEV)[None] > past + torch.arange(new, device=DEV)[:, None], -float("inf"))
+        want = torch.einsum("htn,hvn->thv", torch.softmax(score, -1), W[:, :, :n].repeat_interleave(each, 0)).reshape(new, -1)
+        limit = dict(rtol=2e-5, atol=2e-5) if dtype == torch.float32 else dict(rtol=2.0 ** -8, atol=1e-4)
+        torch.testing.assert_close(out[s * new:(s + 1) * new].double(), want, **limit)

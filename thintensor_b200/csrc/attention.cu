@@ -234,9 +234,14 @@ static int attention_tiles_launch(const void* q, const void* k_pool, const void*
 }
 
 // Whether a step's queries go in tiles: prompts (eight tokens a sequence on average fill a quarter of a tile, which already pays), heads of up to
-// 128 numbers, the cache on 16-byte boundaries.
-static bool attention_in_tiles(const void* k_pool, const void* v_pool, int sequences, int n_tokens, int heads, int head_dim, int value_dim, int splits) {
-    return splits == 1 && n_tokens >= 8 * sequences && head_dim <= 128 && value_dim <= 128 && heads <= 65535
+// 128 numbers, the cache on 16-byte boundaries.  Where the block table is one block wide, a query meets so few keys that tiles have to be full, or a
+// query a warp has to keep the SMs busy, for tiles to be faster.  Measured without a past, a query a warp against tiles (us, heads of 64): one prompt of 16 tokens, 32
+// heads 9.0 and 10.8, of 24 10.9 and 10.2, of 40 24 and 13; 8 prompts of 16 17 and 14; 16 of 8 24 and 28, of 12 42 and 30; one of 32 tokens, 8 heads 12.3 and 13.1.
+static bool attention_in_tiles(const void* k_pool, const void* v_pool, int table_width, int sequences, int n_tokens, int heads, int head_dim, int value_dim, int splits) {
+    const long long warps = (long long)n_tokens * heads;
+    const bool enough = table_width > 1 ? n_tokens >= 8 * sequences : n_tokens >= 40 * sequences || (n_tokens >= 24 * sequences && warps >= 1024)
+        || (n_tokens >= 16 * sequences && warps >= 2048) || (n_tokens >= 12 * sequences && warps >= 6144);
+    return splits == 1 && enough && head_dim <= 128 && value_dim <= 128 && heads <= 65535
         && (((uintptr_t)k_pool | (uintptr_t)v_pool) & 15) == 0;
 }
 
@@ -253,7 +258,7 @@ extern "C" int tt_attention(const void* q, const void* k_pool, const void* v_poo
     if (head_dim <= 0 || head_dim > ATTN_MAX_HEAD_DIM || value_dim <= 0 || value_dim > ATTN_MAX_HEAD_DIM || heads % kv_heads || splits < 1 || splits > 65535)
         return (int)cudaErrorInvalidValue;
     if (splits > 1 && (!part_acc || !part_ml)) return (int)cudaErrorInvalidValue;
-    if (attention_in_tiles(k_pool, v_pool, sequences, n_tokens, heads, head_dim, value_dim, splits)) {
+    if (attention_in_tiles(k_pool, v_pool, table_width, sequences, n_tokens, heads, head_dim, value_dim, splits)) {
 #define TT_TILES(T, SIZE) attention_tiles_launch<T, SIZE>(q, k_pool, v_pool, table, table_width, pool_blocks, cu, len_before, sequences, n_tokens, heads, kv_heads, head_dim, value_dim, scale, sinks, window, out, status, extra, stream)
         const bool small = head_dim <= 64 && value_dim <= 64;
         if (dtype == TT_F32) return small ? TT_TILES(float, 64) : TT_TILES(float, 128);
