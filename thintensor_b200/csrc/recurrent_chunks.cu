@@ -673,10 +673,10 @@ delta_chunks_prepare_kernel(const DeltaChunks a) {
     float* qs = ks + CK_TOKENS * LD;                            // [64][LD]
     float* As = qs + CK_TOKENS * LD;                            // [64][CK_MLD]
     float* f = As + CK_TOKENS * CK_MLD;                         // [CK_FACTORS]
-    float* nq = f + CK_FACTORS;                                 // [64] each: 1 / |q|, 1 / |k|, beta
-    float* nk = nq + CK_TOKENS;
-    float* beta = nk + CK_TOKENS;
-    float* scalars = beta + CK_TOKENS;                          // [2][64]
+    double* nq = reinterpret_cast<double*>(f + CK_FACTORS);     // [64] each: D^-1/2 / |q|, 1 / |k|; then beta
+    double* nk = nq + CK_TOKENS;
+    float* beta = reinterpret_cast<float*>(nk + CK_TOKENS);
+    float* scalars = beta + CK_TOKENS;                          // [2][64]; then the rows' factors of W's right-hand side
     const int slot = blockIdx.x, h = blockIdx.y, D = a.D, V = a.V;
     int lo = 0, hi = a.sequences;
     while (hi - lo > 1) {
@@ -718,11 +718,11 @@ delta_chunks_prepare_kernel(const DeltaChunks a) {
     // lengths: four lanes a row
     for (int item = threadIdx.x >> 2; item < 2 * CK_TOKENS; item += CD_THREADS / 4) {
         const float* row = (item < CK_TOKENS ? qs : ks) + (item & (CK_TOKENS - 1)) * LD;
-        float sum = 0.0f;
-        for (int c = threadIdx.x & 3; c < D; c += 4) sum = fmaf(row[c], row[c], sum);
+        double sum = 0.0;
+        for (int c = threadIdx.x & 3; c < D; c += 4) sum = fma((double)row[c], (double)row[c], sum);
         sum += __shfl_xor_sync(0xffffffffu, sum, 1);
         sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-        if (!(threadIdx.x & 3)) (item < CK_TOKENS ? nq : nk)[item & (CK_TOKENS - 1)] = rsqrtf(sum + 1e-6f) * (item < CK_TOKENS ? rsqrtf((float)D) : 1.0f);
+        if (!(threadIdx.x & 3)) (item < CK_TOKENS ? nq : nk)[item & (CK_TOKENS - 1)] = 1.0 / sqrt((sum + 1e-6) * (item < CK_TOKENS ? (double)D : 1.0));
     }
     __syncthreads();
     float* scratch = a.chunk_scratch(slot, h);
@@ -736,33 +736,45 @@ delta_chunks_prepare_kernel(const DeltaChunks a) {
 #pragma unroll
             for (int c = 0; c < 4; ++c) kk[r][c] = qk[r][c] = 0.0f;
 #pragma unroll 1
-        for (int k0 = 0; k0 < NP; k0 += 32) {                   // short sums, added up
-            float pk[4][4], pq[4][4];
+        for (int k0 = 0; k0 < NP; k0 += 32) {                   // sums of 8, added up to 32, added up: long chains lose more
+            float hk[4][4], hq[4][4];
 #pragma unroll
             for (int r = 0; r < 4; ++r)
 #pragma unroll
-                for (int c = 0; c < 4; ++c) pk[r][c] = pq[r][c] = 0.0f;
-#pragma unroll 2
-            for (int k = k0; k < k0 + 32; k += 4) {
-                float4 b[4];
+                for (int c = 0; c < 4; ++c) hk[r][c] = hq[r][c] = 0.0f;
+#pragma unroll 1
+            for (int k1 = k0; k1 < k0 + 32; k1 += 8) {
+                float pk[4][4], pq[4][4];
 #pragma unroll
-                for (int c = 0; c < 4; ++c) b[c] = *reinterpret_cast<const float4*>(ks + (tx + 16 * c) * LD + k);
+                for (int r = 0; r < 4; ++r)
 #pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    const float4 x = *reinterpret_cast<const float4*>(ks + (ty + 16 * r) * LD + k), y = *reinterpret_cast<const float4*>(qs + (ty + 16 * r) * LD + k);
+                    for (int c = 0; c < 4; ++c) pk[r][c] = pq[r][c] = 0.0f;
 #pragma unroll
-                    for (int c = 0; c <= r; ++c) {              // the others lie above the diagonal
-                        pk[r][c] = fmaf(x.x, b[c].x, pk[r][c]); pk[r][c] = fmaf(x.y, b[c].y, pk[r][c]);
-                        pk[r][c] = fmaf(x.z, b[c].z, pk[r][c]); pk[r][c] = fmaf(x.w, b[c].w, pk[r][c]);
-                        pq[r][c] = fmaf(y.x, b[c].x, pq[r][c]); pq[r][c] = fmaf(y.y, b[c].y, pq[r][c]);
-                        pq[r][c] = fmaf(y.z, b[c].z, pq[r][c]); pq[r][c] = fmaf(y.w, b[c].w, pq[r][c]);
+                for (int k = k1; k < k1 + 8; k += 4) {
+                    float4 b[4];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) b[c] = *reinterpret_cast<const float4*>(ks + (tx + 16 * c) * LD + k);
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        const float4 x = *reinterpret_cast<const float4*>(ks + (ty + 16 * r) * LD + k), y = *reinterpret_cast<const float4*>(qs + (ty + 16 * r) * LD + k);
+#pragma unroll
+                        for (int c = 0; c <= r; ++c) {              // the others lie above the diagonal
+                            pk[r][c] = fmaf(x.x, b[c].x, pk[r][c]); pk[r][c] = fmaf(x.y, b[c].y, pk[r][c]);
+                            pk[r][c] = fmaf(x.z, b[c].z, pk[r][c]); pk[r][c] = fmaf(x.w, b[c].w, pk[r][c]);
+                            pq[r][c] = fmaf(y.x, b[c].x, pq[r][c]); pq[r][c] = fmaf(y.y, b[c].y, pq[r][c]);
+                            pq[r][c] = fmaf(y.z, b[c].z, pq[r][c]); pq[r][c] = fmaf(y.w, b[c].w, pq[r][c]);
+                        }
                     }
                 }
+#pragma unroll
+                for (int r = 0; r < 4; ++r)
+#pragma unroll
+                    for (int c = 0; c <= r; ++c) { hk[r][c] += pk[r][c]; hq[r][c] += pq[r][c]; }
             }
 #pragma unroll
             for (int r = 0; r < 4; ++r)
 #pragma unroll
-                for (int c = 0; c <= r; ++c) { kk[r][c] += pk[r][c]; qk[r][c] += pq[r][c]; }
+                for (int c = 0; c <= r; ++c) { kk[r][c] += hk[r][c]; qk[r][c] += hq[r][c]; }
         }
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
@@ -770,16 +782,23 @@ delta_chunks_prepare_kernel(const DeltaChunks a) {
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 const int j = tx + 16 * c, bj = j >> 3;
-                const float fij = bi > bj ? f[CK_U + i] * f[CK_BLOCKS + bi * 8 + bj] * f[CK_V + j] : bi == bj ? f[CK_DIAG + bi * 64 + (i & 7) * 8 + (j & 7)] : 0.0f;
-                As[i * CK_MLD + j] = j < i ? -beta[i] * fij * (nk[i] * nk[j] * kk[r][c]) : 0.0f;         // -A
-                P[i * CK_TOKENS + j] = j <= i ? fij * (nq[i] * nk[j] * qk[r][c]) : 0.0f;
+                if (c > r) {
+                    As[i * CK_MLD + j] = P[i * CK_TOKENS + j] = 0.0f;
+                    continue;
+                }
+                // products of the factors in float64, rounded once
+                const double fij = bi > bj ? (double)f[CK_U + i] * (double)f[CK_BLOCKS + bi * 8 + bj] * (double)f[CK_V + j] : bi == bj ? (double)f[CK_DIAG + bi * 64 + (i & 7) * 8 + (j & 7)] : 0.0;
+                const double fk = fij * nk[j];
+                As[i * CK_MLD + j] = j < i ? -(float)((double)beta[i] * nk[i] * fk * (double)kk[r][c]) : 0.0f;         // -A
+                P[i * CK_TOKENS + j] = j <= i ? (float)(nq[i] * fk * (double)qk[r][c]) : 0.0f;
             }
         }
     }
     if (threadIdx.x < CK_TOKENS) {
         float* factors = P + CK_TOKENS * CK_TOKENS;
-        factors[CD_E + threadIdx.x] = f[CK_E + threadIdx.x] * nq[threadIdx.x];
-        factors[CD_W + threadIdx.x] = f[CK_W + threadIdx.x] * nk[threadIdx.x];
+        factors[CD_E + threadIdx.x] = (float)((double)f[CK_E + threadIdx.x] * nq[threadIdx.x]);
+        factors[CD_W + threadIdx.x] = (float)((double)f[CK_W + threadIdx.x] * nk[threadIdx.x]);
+        scalars[threadIdx.x] = (float)((double)beta[threadIdx.x] * (double)f[CK_E + threadIdx.x] * nk[threadIdx.x]);
         if (threadIdx.x == 0) factors[CD_ALL] = f[CK_ALL];
     }
     __syncthreads();
@@ -802,11 +821,13 @@ delta_chunks_prepare_kernel(const DeltaChunks a) {
         fetch(0);
 #pragma unroll 1
         for (int i0 = 0; i0 < CK_TOKENS; i0 += 16) {
-            float x[16];
+            // the right-hand side, and what the rows before take off it, summed apart: many small terms added to x one by one would each round it
+            float x[16], before[16];
 #pragma unroll
             for (int r = 0; r < 16; ++r) {
                 const int i = i0 + r;
-                x[r] = job ? beta[i] * raw[r] : beta[i] * f[CK_E + i] * nk[i] * xs[i * LD];
+                before[r] = 0.0f;
+                x[r] = job ? beta[i] * raw[r] : scalars[i] * xs[i * LD];
             }
             if (i0 + 16 < CK_TOKENS) fetch(i0 + 16);
 #pragma unroll 1
@@ -829,18 +850,20 @@ delta_chunks_prepare_kernel(const DeltaChunks a) {
                     }
                 }
 #pragma unroll
-                for (int r = 0; r < 16; ++r) x[r] += sum[r];
+                for (int r = 0; r < 16; ++r) before[r] += sum[r];
             }
+            x[0] += before[0];
 #pragma unroll
             for (int r = 1; r < 16; ++r) {
 #pragma unroll
                 for (int j = 0; j < r; j += 4) {
                     const float4 m = *reinterpret_cast<const float4*>(As + (i0 + r) * CK_MLD + i0 + j);
-                    x[r] = fmaf(m.x, x[j], x[r]);
-                    if (j + 1 < r) x[r] = fmaf(m.y, x[j + 1], x[r]);
-                    if (j + 2 < r) x[r] = fmaf(m.z, x[j + 2], x[r]);
-                    if (j + 3 < r) x[r] = fmaf(m.w, x[j + 3], x[r]);
+                    before[r] = fmaf(m.x, x[j], before[r]);
+                    if (j + 1 < r) before[r] = fmaf(m.y, x[j + 1], before[r]);
+                    if (j + 2 < r) before[r] = fmaf(m.z, x[j + 2], before[r]);
+                    if (j + 3 < r) before[r] = fmaf(m.w, x[j + 3], before[r]);
                 }
+                x[r] += before[r];
             }
 #pragma unroll
             for (int r = 0; r < 16; ++r) {
@@ -998,7 +1021,7 @@ delta_chunks_kernel(const DeltaChunks a) {
 
 template <int NP, int TP>
 static int delta_chunks_launch(const DeltaChunks& a, int max_slots, cudaStream_t stream) {
-    constexpr size_t prepare_bytes = (size_t)(2 * CK_TOKENS * (NP + 4) + CK_TOKENS * CK_MLD + CK_FACTORS + 5 * CK_TOKENS) * sizeof(float);
+    constexpr size_t prepare_bytes = (size_t)(2 * CK_TOKENS * (NP + 4) + CK_TOKENS * CK_MLD + CK_FACTORS + 7 * CK_TOKENS) * sizeof(float);
     cudaError_t code = ck_allow(delta_chunks_prepare_kernel<NP>, prepare_bytes);
     if (code == cudaSuccess) code = ck_allow(delta_chunks_kernel<NP, TP>, CdLayout<NP, TP>::BYTES);
     if (code != cudaSuccess) return (int)code;
