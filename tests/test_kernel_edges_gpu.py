@@ -231,7 +231,7 @@ def test_gated_group_norm_by_pieces(group, groups, tokens, splits, gate_first, g
 @pytest.mark.parametrize("splits", [1, 2])
 @pytest.mark.parametrize("taps", [1, 4, 8])
 def test_convolution_tiles_inside_and_across_sequences(taps, splits):
-    """Sequences that start and end inside, at and beyond the tiles of 16 tokens."""
+    """Sequences that start and end inside, at and beyond the tiles (of 8 tokens in one slice, of 16 in two)."""
     from thintensor_b200.kernels import api
 
     news, slot_ids, channels, col = [16, 40, 1, 23, 33], [3, 0, 5, 1, 2], 130, 3
@@ -518,3 +518,58 @@ def test_exact_attention_of_one_block(heads, kv_heads, D, V, sequences, new, pas
         want = torch.einsum("htn,hvn->thv", torch.softmax(score, -1), W[:, :, :n].repeat_interleave(each, 0)).reshape(new, -1)
         limit = dict(rtol=2e-5, atol=2e-5) if dtype == torch.float32 else dict(rtol=2.0 ** -8, atol=1e-4)
         torch.testing.assert_close(out[s * new:(s + 1) * new].double(), want, **limit)
+
+
+# ------------------------------------------------------------------------------------------ long prompts through the tiles and chunks
+@pytest.mark.parametrize("taps", [1, 4, 8])
+def test_convolution_of_long_prompts(taps):
+    """One k-slice and at least 1,024 tokens: tiles of 16 tokens whose inputs are asked for at once.  Sequences that end inside, at and
+    across tiles, one of a single token, and a last tile that is not full."""
+    from thintensor_b200.kernels import api
+
+    news, slot_ids, channels, col = [16, 40, 1, 23, 911, 33, 15], [3, 0, 5, 1, 2, 6, 4], 130, 3
+    tokens = sum(news)
+    assert tokens >= 1024 and tokens % 16
+    cu = [sum(news[:i]) for i in range(len(news) + 1)]
+    proj, weight, bias = randn(1, tokens, channels + 7, seed=23), randn(channels, taps, seed=24), randn(channels, seed=25)
+    state = randn(8, max(taps - 1, 1), channels, seed=26)[:, :taps - 1].contiguous()
+    before = state.clone()
+    out = torch.full((tokens, channels), 7.0, device=DEV)
+    api.causal_conv(proj, col, channels, weight, bias, True, state, out, i32(cu), i32(slot_ids), len(news), tokens, False)
+    x = proj[0].double()[:, col:col + channels]
+    for s, slot in enumerate(slot_ids):
+        rows = torch.cat((before[slot].double(), x[cu[s]:cu[s + 1]]))
+        want = sum(rows[j:j + news[s]] * weight[:, j].double() for j in range(taps)) + bias.double()
+        torch.testing.assert_close(out[cu[s]:cu[s + 1]].double(), want * torch.sigmoid(want), rtol=1e-5, atol=1e-5)
+        assert torch.equal(state[slot].double(), rows[rows.shape[0] - (taps - 1):])
+    assert torch.equal(state[7], before[7])
+
+
+@pytest.mark.parametrize("heads,qk_heads,D,V", [(2, 1, 64, 130), (2, 2, 128, 257), (3, 3, 24, 70), (40, 20, 64, 130)])
+def test_delta_rule_in_chunks_in_several_value_tiles(heads, qk_heads, D, V):
+    """Value columns beyond a tile of 64 or 128: the first kernel's halves take further tiles in the keys' and queries' place."""
+    test_delta_rule_in_chunks(heads, qk_heads, D, V)
+
+
+@pytest.mark.parametrize("heads,P,N", [(2, 32, 128), (70, 64, 64)])
+def test_recurrence_in_many_chunks(heads, P, N):
+    """Seventeen chunks, so that both stages of shared memory are filled many times; among the constant decays some beyond one."""
+    from thintensor_b200.kernels import api
+
+    news = [1027, 200]
+    tokens, inner = sum(news), heads * P
+    cu, slots = i32([0, news[0], tokens]), i32([1, 0])
+    rows, state = randn(tokens, inner + 2 * heads * N, seed=100, scale=0.5), randn(2, heads, P, N, seed=101)
+    before, y = state.clone(), torch.full((tokens, inner), 7.0, device=DEV)
+    decays = torch.tensor([0.99, 1.003, -1.002, 0.5], device=DEV).repeat(heads)[:heads].contiguous()
+    scratch = torch.full(api.scan_chunks_scratch(tokens, 2, heads, heads), float("nan"), device=DEV)
+    api.scan_chunks(rows, 0, inner, inner + heads * N, state, y, cu, slots, 2, heads, P, N, heads, scratch, fixed_decay=decays)
+    x, b, c = (z.double().reshape(tokens, heads, -1) for z in rows.split((inner, heads * N, heads * N), 1))
+    for s, slot in enumerate((1, 0)):
+        span = slice(int(cu[s]), int(cu[s + 1]))
+        ones = torch.ones(news[s], heads, dtype=torch.float64, device=DEV)
+        want, last = recurrence(x[span], b[span], c[span], decays.double() * ones, ones, torch.zeros(heads, dtype=torch.float64, device=DEV), before[slot].double())
+        # heads grow by up to 1.003^1,027 = 22: each against its own size, as in the shorter test
+        for h in range(heads):
+            assert float((y[span].double().reshape(-1, heads, P)[:, h] - want[:, h]).abs().max()) <= 2e-5 * max(1.0, float(want[:, h].abs().max()))
+            assert float((state[slot, h].double() - last[h]).abs().max()) <= 2e-5 * max(1.0, float(last[h].abs().max()))
