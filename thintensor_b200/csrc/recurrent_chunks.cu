@@ -213,34 +213,46 @@ scan_chunks_prepare_kernel(const ScanChunks a) {
     for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) total[i][j] = 0.0f;
-    for (int k0 = 0; k0 < NP; k0 += 32) {                       // short sums, added up: a long chain of additions loses more
-        float acc[4][4];
+    for (int k0 = 0; k0 < NP; k0 += 32) {                       // sums of 8, added up to 32, added up: long chains lose more
+        float part[4][4];
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
-#pragma unroll 4
-        for (int k = k0; k < k0 + 32; k += 4) {
-            float4 c[4], b[4];
+            for (int j = 0; j < 4; ++j) part[i][j] = 0.0f;
+#pragma unroll 2
+        for (int k1 = k0; k1 < k0 + 32; k1 += 8) {
+            float acc[4][4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                c[i] = *reinterpret_cast<const float4*>(cs + (ty + 16 * i) * LD + k);
-                b[i] = *reinterpret_cast<const float4*>(bs + (tx + 16 * i) * LD + k);
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
+#pragma unroll
+            for (int k = k1; k < k1 + 8; k += 4) {
+                float4 c[4], b[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    c[i] = *reinterpret_cast<const float4*>(cs + (ty + 16 * i) * LD + k);
+                    b[i] = *reinterpret_cast<const float4*>(bs + (tx + 16 * i) * LD + k);
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j <= i; ++j) {              // columns behind the row's block are not used
+                        acc[i][j] = fmaf(c[i].x, b[j].x, acc[i][j]);
+                        acc[i][j] = fmaf(c[i].y, b[j].y, acc[i][j]);
+                        acc[i][j] = fmaf(c[i].z, b[j].z, acc[i][j]);
+                        acc[i][j] = fmaf(c[i].w, b[j].w, acc[i][j]);
+                    }
             }
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll
-                for (int j = 0; j <= i; ++j) {                  // columns behind the row's block are not used
-                    acc[i][j] = fmaf(c[i].x, b[j].x, acc[i][j]);
-                    acc[i][j] = fmaf(c[i].y, b[j].y, acc[i][j]);
-                    acc[i][j] = fmaf(c[i].z, b[j].z, acc[i][j]);
-                    acc[i][j] = fmaf(c[i].w, b[j].w, acc[i][j]);
-                }
+                for (int j = 0; j <= i; ++j) part[i][j] += acc[i][j];
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-            for (int j = 0; j <= i; ++j) total[i][j] += acc[i][j];
+            for (int j = 0; j <= i; ++j) total[i][j] += part[i][j];
     }
     float* out = a.scores + ((size_t)slot * a.groups + g) * CK_TOKENS * CK_TOKENS;
 #pragma unroll
@@ -407,10 +419,10 @@ __device__ __forceinline__ void ck_update(unsigned long long (&s)[NL][2], float 
     }
 }
 
-// A chunk's outputs: this lane's sums and the other slices'; rows from `left` on do not exist
+// A chunk's outputs: this lane's sums and the other slices', then skip times own (if there is one); rows from `left` on do not exist
 template <int RL, int SLICES>
 __device__ __forceinline__ void ck_outputs(const unsigned long long (&acc)[4][2], const float* __restrict__ parts, int ldx, int row, int col, int width, int left,
-                                           bool vec, float* __restrict__ out, int stride) {
+                                           bool vec, float skip, const float4* own, float* __restrict__ out, int stride) {
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
         const int i = row + RL * r;
@@ -419,6 +431,10 @@ __device__ __forceinline__ void ck_outputs(const unsigned long long (&acc)[4][2]
         for (int k = 0; k < SLICES - 1; ++k) {
             const float4 q = *reinterpret_cast<const float4*>(parts + (k * CK_TOKENS + i) * ldx + col);
             o[0] += q.x; o[1] += q.y; o[2] += q.z; o[3] += q.w;
+        }
+        if (own) {
+            o[0] = fmaf(skip, own[r].x, o[0]); o[1] = fmaf(skip, own[r].y, o[1]);
+            o[2] = fmaf(skip, own[r].z, o[2]); o[3] = fmaf(skip, own[r].w, o[3]);
         }
         if (i >= left || col >= width) continue;
         float* to = out + (size_t)i * stride + col;
@@ -566,14 +582,10 @@ scan_chunks_kernel(const ScanChunks a) {
             for (int r = 0; r < 4; ++r)
                 *reinterpret_cast<float4*>(ck_shared + L::PARTS + ((slice - 1) * CK_TOKENS + row + RL * r) * L::LDX + col) =
                     make_float4(ck_lo(acc[r][0]), ck_hi(acc[r][0]), ck_lo(acc[r][1]), ck_hi(acc[r][1]));
-        } else {
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const float4 x = *reinterpret_cast<const float4*>(X + (row + RL * r) * L::LDX + col);
-                acc[r][0] = ck_pair(fmaf(skip, x.x, ck_lo(acc[r][0])), fmaf(skip, x.y, ck_hi(acc[r][0])));
-                acc[r][1] = ck_pair(fmaf(skip, x.z, ck_lo(acc[r][1])), fmaf(skip, x.w, ck_hi(acc[r][1])));
-            }
         }
+        float4 own[4];                                          // added last, to the whole sum: one rounding at its size
+#pragma unroll
+        for (int r = 0; r < 4; ++r) own[r] = slice == 0 ? *reinterpret_cast<const float4*>(X + (row + RL * r) * L::LDX + col) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         // S <- e_63 S + B^T (w x)
         ck_update<NP, NL>(s, F[CK_ALL], stage + L::B + srow, XW + col, L::LDX);
 #pragma unroll
@@ -581,7 +593,7 @@ scan_chunks_kernel(const ScanChunks a) {
             *reinterpret_cast<float4*>(Ss + (srow + i) * L::LDX + col) = make_float4(ck_lo(s[i][0]), ck_hi(s[i][0]), ck_lo(s[i][1]), ck_hi(s[i][1]));
         __syncthreads();                                        // this stage may be filled again, the weighted rows be written again
         if (slice == 0)                                         // the other slices' sums are there: the chunk's outputs
-            ck_outputs<RL, L::SLICES>(acc, ck_shared + L::PARTS, L::LDX, row, col, width, n - chunk * CK_TOKENS, vec_x,
+            ck_outputs<RL, L::SLICES>(acc, ck_shared + L::PARTS, L::LDX, row, col, width, n - chunk * CK_TOKENS, vec_x, skip, own,
                                       a.y + (size_t)(first + chunk * CK_TOKENS) * inner + (size_t)h * P + p0, inner);
     }
     ck_wait<0>();
@@ -1006,7 +1018,7 @@ delta_chunks_kernel(const DeltaChunks a) {
             *reinterpret_cast<float4*>(Ss + (srow + i) * D_::LDX + col) = make_float4(ck_lo(s[i][0]), ck_hi(s[i][0]), ck_lo(s[i][1]), ck_hi(s[i][1]));
         __syncthreads();
         if (slice == 0)
-            ck_outputs<RL, L::SLICES>(acc, ck_shared + D_::PARTS, D_::LDX, row, col, width, n - chunk * CK_TOKENS, vec_x,
+            ck_outputs<RL, L::SLICES>(acc, ck_shared + D_::PARTS, D_::LDX, row, col, width, n - chunk * CK_TOKENS, vec_x, 0.0f, nullptr,
                                       a.out + (size_t)(first + chunk * CK_TOKENS) * (a.heads * V) + (size_t)h * V + p0, a.heads * V);
     }
     ck_wait<0>();
