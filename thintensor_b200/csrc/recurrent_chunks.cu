@@ -208,12 +208,12 @@ scan_chunks_prepare_kernel(const ScanChunks a) {
     __syncthreads();
     // G: 16 x 16 threads, rows and columns 16 apart
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    float total[4][4];
+    double total[4][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) total[i][j] = 0.0f;
-    for (int k0 = 0; k0 < NP; k0 += 32) {                       // sums of 8, added up to 32, added up: long chains lose more
+        for (int j = 0; j < 4; ++j) total[i][j] = 0.0;
+    for (int k0 = 0; k0 < NP; k0 += 32) {                       // sums of 8, added up to 32, those in float64: long chains lose more
         float part[4][4];
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -252,14 +252,14 @@ scan_chunks_prepare_kernel(const ScanChunks a) {
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-            for (int j = 0; j <= i; ++j) total[i][j] += part[i][j];
+            for (int j = 0; j <= i; ++j) total[i][j] += (double)part[i][j];
     }
     float* out = a.scores + ((size_t)slot * a.groups + g) * CK_TOKENS * CK_TOKENS;
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j)                             // zeros above the diagonal: a later token's score may be no number
-            out[(ty + 16 * i) * CK_TOKENS + tx + 16 * j] = tx + 16 * j <= ty + 16 * i ? total[i][j] : 0.0f;
+            out[(ty + 16 * i) * CK_TOKENS + tx + 16 * j] = tx + 16 * j <= ty + 16 * i ? (float)total[i][j] : 0.0f;
 }
 
 // -------------------------------------------------------------------------------------------------- the walk over the chunks
