@@ -573,3 +573,64 @@ def test_recurrence_in_many_chunks(heads, P, N):
         for h in range(heads):
             assert float((y[span].double().reshape(-1, heads, P)[:, h] - want[:, h]).abs().max()) <= 2e-5 * max(1.0, float(want[:, h].abs().max()))
             assert float((state[slot, h].double() - last[h]).abs().max()) <= 2e-5 * max(1.0, float(last[h].abs().max()))
+
+
+@pytest.mark.parametrize("heads,groups,P,N", [(4, 1, 32, 128), (4, 2, 24, 64)])
+def test_recurrence_in_chunks_is_as_close_as_token_by_token(heads, groups, P, N):
+    """Outputs against 64 bits, 2-norm: no further off than token by token but for a twentieth (the scores' sums of 32 in one chain, which a
+    chunk's outputs are made of, were a quarter to a third further off)."""
+    from thintensor_b200.kernels import api
+
+    tokens, inner = 900, heads * P
+    rows, raw = randn(tokens, inner + 2 * groups * N, seed=120), randn(1, tokens, heads, seed=121)
+    a_log, dt_bias, skip = randn(heads, seed=122), randn(heads, seed=123), randn(heads, seed=124)
+    cu, slots = i32([0, tokens]), i32([0])
+    outs = []
+    for chunks in (True, False):
+        state, y = torch.zeros(1, heads, P, N, device=DEV), torch.empty(tokens, inner, device=DEV)
+        if chunks:
+            scratch = torch.empty(api.scan_chunks_scratch(tokens, 1, heads, groups), device=DEV)
+            api.scan_chunks(rows, 0, inner, inner + groups * N, state, y, cu, slots, 1, heads, P, N, groups, scratch, steps=(raw, 0, dt_bias, a_log, skip))
+        else:
+            api.mamba2_scan(rows, raw, 0, dt_bias, a_log, skip, state, y, cu, slots, 1, heads, P, N, groups)
+        outs.append((y.double().reshape(tokens, heads, P), state[0].double()))
+    x, b, c = rows.double().split((inner, groups * N, groups * N), 1)
+    wide = lambda z: z.reshape(tokens, groups, N).repeat_interleave(heads // groups, 1)
+    dt = torch.nn.functional.softplus(raw[0].double() + dt_bias.double())
+    want, last = recurrence(x.reshape(tokens, heads, P), wide(b), wide(c), torch.exp(-torch.exp(a_log.double()) * dt), dt, skip.double(),
+                            torch.zeros(heads, P, N, dtype=torch.float64, device=DEV))
+    for i, exact in enumerate((want, last)):
+        chunked, by_token = (float((o[i] - exact).norm() / exact.norm()) for o in outs)
+        assert chunked <= 1.05 * by_token, (i, chunked, by_token)
+
+
+@pytest.mark.parametrize("heads,D,V", [(4, 128, 128), (4, 64, 64)])
+def test_delta_rule_in_chunks_is_as_close_as_token_by_token(heads, D, V):
+    """As above: with lengths, factors and scores in float32 throughout the outputs were a seventh to a third further off."""
+    from thintensor_b200.kernels import api
+
+    tokens, qk = 900, heads * D
+    qkv, raw = randn(tokens, 2 * qk + heads * V, seed=125), randn(1, tokens, 2 * heads, seed=126)
+    a_log, dt_bias = randn(heads, seed=127), randn(heads, seed=128)
+    cu, slots = i32([0, tokens]), i32([0])
+    outs = []
+    for chunks in (True, False):
+        state, out = torch.zeros(1, heads, V, D, device=DEV), torch.empty(tokens, heads * V, device=DEV)
+        if chunks:
+            scratch = torch.empty(api.delta_chunks_scratch(tokens, 1, heads, D, V), device=DEV)
+            api.delta_chunks(qkv, raw, 0, heads, dt_bias, a_log, state, out, cu, slots, 1, heads, heads, D, V, scratch)
+        else:
+            api.delta_scan(qkv, raw, 0, heads, dt_bias, a_log, state, out, cu, slots, 1, heads, heads, D, V)
+        outs.append(out.double().reshape(tokens, heads, V))
+    z = raw[0].double()
+    beta, decay = torch.sigmoid(z[:, :heads]), torch.exp(-torch.exp(a_log.double()) * torch.nn.functional.softplus(z[:, heads:] + dt_bias.double()))
+    unit = lambda y: y / (y.square().sum(-1, keepdim=True) + 1e-6).sqrt()
+    q, k = (unit(part.double().reshape(tokens, heads, D)) for part in qkv[:, :2 * qk].split(qk, 1))
+    v, S, want = qkv[:, 2 * qk:].double().reshape(tokens, heads, V), torch.zeros(heads, V, D, dtype=torch.float64, device=DEV), []
+    for t in range(tokens):
+        S = decay[t][:, None, None] * S
+        S = S + (beta[t][:, None] * (v[t] - (S @ k[t][:, :, None])[..., 0]))[:, :, None] * k[t][:, None, :]
+        want.append((S @ q[t][:, :, None])[..., 0] * D ** -0.5)
+    want = torch.stack(want)
+    chunked, by_token = (float((out - want).norm() / want.norm()) for out in outs)
+    assert chunked <= 1.05 * by_token, (chunked, by_token)

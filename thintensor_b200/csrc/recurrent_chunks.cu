@@ -213,14 +213,16 @@ scan_chunks_prepare_kernel(const ScanChunks a) {
     for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) total[i][j] = 0.0;
-    for (int k0 = 0; k0 < NP; k0 += 32) {                       // sums of 8, added up to 32, those in float64: long chains lose more
+    // sums of 8, for states of 128 rows added up to 32, those in float64: long chains lose more
+    constexpr int MIDDLE = NP > 64 ? 32 : 8;
+    for (int k0 = 0; k0 < NP; k0 += MIDDLE) {
         float part[4][4];
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
             for (int j = 0; j < 4; ++j) part[i][j] = 0.0f;
 #pragma unroll 2
-        for (int k1 = k0; k1 < k0 + 32; k1 += 8) {
+        for (int k1 = k0; k1 < k0 + MIDDLE; k1 += 8) {
             float acc[4][4];
 #pragma unroll
             for (int i = 0; i < 4; ++i)
