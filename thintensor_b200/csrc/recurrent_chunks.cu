@@ -5,10 +5,14 @@
 //
 // With f(i, j) = a_(j+1) * .. * a_i, e_i = a_0 * .. * a_i and w_j = f(63, j) dt_j, a chunk that starts from state S gives
 //   y_i = e_i (S^T C_i) + sum_(j<=i) f(i, j) dt_j (C_i . B_j) x_j + D x_i,     S <- e_63 S + sum_j w_j B_j x_j^T
-// so the token-by-token chain of row products becomes four matrix products a chunk, all of them float32 multiply-adds.  The
-// decays only ever enter as products of decays (never as quotients, never as differences of sums of logarithms): nothing can
-// overflow that does not overflow in the recurrence, nothing cancels, and a constant decay may have any sign.  The products are
-// formed in float64 from the float32 decays and rounded once.
+// so the token-by-token chain of row products becomes four matrix products a chunk, all of them float32 multiply-adds (the scores' short sums
+// are added in float64, so that outputs are as close to 64 bits as token by token: 30 runs, at most 3 % further off, 7 % closer in the mean).  The
+// decays only ever enter as products of decays (never as quotients, never as differences of sums of logarithms): nothing cancels, and a
+// constant decay may have any sign.  Up to 64 of them are multiplied before they meet a state, so none may exceed one (callers see to
+// it), and the scores C_i . B_j are formed undecayed: they overflow where |C| |B| does, which the recurrence, that meets dt x and the decays
+// in between, need not.  Numbers that are not finite reach the tokens they reach in the recurrence and no others.  Products of decays are
+// formed in float64 from the float32 decays and rounded once inside an 8-token block and in e, w and e_63; across blocks f(i, j) dt_j is
+// the product of three such numbers (in float32 here: five roundings; in float64, rounded once, for the delta rule below).
 //
 // Two kernels.  The first, parallel over chunks, makes what the columns of a head share: G_ij = C_i . B_j for every chunk and
 // group, and the factors of every chunk and head (u, v, E, diagonal blocks: f(i, j) is a product of three numbers across
@@ -18,8 +22,8 @@
 // What bounds it: shared memory's delivery of operands and the latency of two warps a scheduler (one CTA of 8 warps an SM; the
 // multiply-add pipe is 43 % busy); the copies of the next chunk run under this one's products.  16 warps with half the registers
 // spilled and were slower (348 against 227 us at the first size below), rows of operands used for two instead of four outputs
-// too (305).  Against the kernels that go token by token, whose chain of row products a token bounds them (us, one B200): 64 heads of
-// 64 x 128, one sequence of 2,048 tokens 895 -> 228, four of 731 545 -> 332; 16 heads of 256 x 128, four of 1,024 740 -> 455.
+// too (305).  Against the kernels that go token by token, whose chain of row products a token bounds them (us, one B200, back to back):
+// 64 heads of 64 x 128, one sequence of 2,048 tokens 748 -> 226, four of 731 423 -> 340; 16 heads of 256 x 128, four of 1,024 590 -> 476.
 #include "common.cuh"
 
 constexpr int CK_TOKENS = 64, CK_THREADS = 256, CK_WARPS = 8;          // threads: of the first kernel
@@ -651,8 +655,9 @@ extern "C" int tt_scan_chunks(const float* rows, int width, int x_col, int b_col
 // is a unit lower triangular system, (I + A) U = beta V - (beta e K) S, whose solution is U = U0 - W S with (I + A) U0 = beta V and
 // (I + A) W = beta e K: neither needs the state, so the first kernel solves for both, parallel over chunks and heads, and the second
 // walks the chunks with   U = U0 - W S,   o = e Q S + P U (P_ij = f(i, j) q_i . k_j, j <= i),   S <- e_63 S + (w K)^T U.
-// Everything is float32 multiply-adds; the systems are solved by forward substitution, a column a thread.  16 heads of 128 x 128 on 4,097
-// tokens: 1,950 us token by token, now 478: the first kernel 130 (bound by issue and shared memory; two columns a thread and half the
+// Products and sums are float32 multiply-adds (lengths, and products of factors with scores, float64 rounded once: in float32 throughout the
+// outputs were 14 % further from 64 bits than token by token, now 15 % closer, for 2 % of the time); the systems are solved by forward
+// substitution, a column a thread.  16 heads of 128 x 128 on 4,097 tokens: 1,900 us token by token, now 486: the first kernel 130 (bound by issue and shared memory; two columns a thread and half the
 // threads 229, the whole substitution unrolled 278), the second 345 (bound like the one above; the two products with the state,
 // W S and Q S, take an operand of S from shared memory once for both: one after the other 408).
 constexpr int CD_THREADS = 256;
