@@ -604,6 +604,49 @@ def test_recurrence_in_chunks_is_as_close_as_token_by_token(heads, groups, P, N)
         assert chunked <= 1.05 * by_token, (i, chunked, by_token)
 
 
+@pytest.mark.parametrize("heads,groups,P,N", [(40, 40, 130, 128), (40, 20, 130, 64), (40, 8, 70, 128), (40, 40, 70, 40), (3, 3, 50, 128), (5, 1, 90, 64)])
+@pytest.mark.parametrize("fixed", [False, True])
+def test_recurrence_in_chunks_in_wide_tiles(heads, groups, P, N, fixed):
+    """Grids whose CTAs hold 64 and 128 columns, whole and in part, and 16 and 32 columns with several tiles."""
+    test_recurrence_in_chunks(heads, groups, P, N, 0, fixed)
+
+
+@pytest.mark.parametrize("heads,P,N", [(100, 130, 128), (100, 130, 64), (100, 70, 128), (1, 20, 128)])
+@pytest.mark.parametrize("what", ["x", "c", "state"])
+def test_recurrence_in_chunks_keeps_other_columns(heads, P, N, what):
+    """A number that is not finite, in the widths of a CTA's columns: what it does not reach keeps its bits, what it reaches is what it is token by token."""
+    from thintensor_b200.kernels import api
+
+    news, inner = [150, 70], heads * P
+    tokens = sum(news)
+    cu, slots, decays = i32([0, news[0], tokens]), i32([1, 0]), torch.full((heads,), 0.9, device=DEV)
+    outs = []
+    for poisoned, chunks in ((False, True), (True, True), (True, False)):
+        rows, state = randn(tokens, inner + 2 * heads * N, seed=130), randn(2, heads, P, N, seed=131)
+        if poisoned and what == "state":
+            state[1, 0, 5, 1] = float("inf")
+        elif poisoned:
+            rows[100, 5 if what == "x" else inner + heads * N + 2] = float("nan")
+        y = torch.full((tokens, inner), 7.0, device=DEV)
+        if chunks:
+            scratch = torch.full(api.scan_chunks_scratch(tokens, 2, heads, heads, N), float("nan"), device=DEV)
+            api.scan_chunks(rows, 0, inner, inner + heads * N, state, y, cu, slots, 2, heads, P, N, heads, scratch, fixed_decay=decays)
+        else:
+            api.decay_scan(rows, decays, state, y, cu, slots, 2, heads, N, P)
+        outs.append((y, state))
+    (clean, clean_state), (y, state), (by_token, by_token_state) = outs
+    assert torch.equal(y.isfinite(), by_token.isfinite()) and torch.equal(state.isfinite(), by_token_state.isfinite())
+    reached = torch.zeros(tokens, inner, dtype=torch.bool, device=DEV)
+    if what == "c":
+        reached[100:news[0], :P] = True           # the token's outputs; the tokens behind it in the chunk are taken one by one
+    else:
+        reached[100 if what == "x" else 0:news[0], 5] = True
+    assert torch.equal(y[~reached], clean[~reached])
+    keeps = torch.ones_like(state, dtype=torch.bool)
+    keeps[1, 0, :P if what == "c" else 6] = False
+    assert torch.equal(state[keeps], clean_state[keeps])
+
+
 @pytest.mark.parametrize("heads,D,V", [(4, 128, 128), (4, 64, 64)])
 def test_delta_rule_in_chunks_is_as_close_as_token_by_token(heads, D, V):
     """As above: with lengths, factors and scores in float32 throughout the outputs were a seventh to a third further off."""

@@ -5,26 +5,28 @@
 //
 // With f(i, j) = a_(j+1) * .. * a_i, e_i = a_0 * .. * a_i and w_j = f(63, j) dt_j, a chunk that starts from state S gives
 //   y_i = e_i (S^T C_i) + sum_(j<=i) f(i, j) dt_j (C_i . B_j) x_j + D x_i,     S <- e_63 S + sum_j w_j B_j x_j^T
-// so the token-by-token chain of row products becomes four matrix products a chunk, all of them float32 multiply-adds (the scores' short sums
-// are added in float64, so that outputs are as close to 64 bits as token by token: 30 runs, at most 3 % further off, 7 % closer in the mean).  The
-// decays only ever enter as products of decays (never as quotients, never as differences of sums of logarithms): nothing cancels, and a
-// constant decay may have any sign.  Up to 64 of them are multiplied before they meet a state, so none may exceed one (callers see to
-// it), and the scores C_i . B_j are formed undecayed: they overflow where |C| |B| does, which the recurrence, that meets dt x and the decays
-// in between, need not.  Numbers that are not finite reach the tokens they reach in the recurrence and no others.  Products of decays are
-// formed in float64 from the float32 decays and rounded once inside an 8-token block and in e, w and e_63; across blocks f(i, j) dt_j is
-// the product of three such numbers (in float32 here: five roundings; in float64, rounded once, for the delta rule below).
+// so the token-by-token chain of row products becomes four matrix products a chunk.  They run on the tensor cores with every operand in three
+// bfloat16 parts (split_mma.cuh), which keeps them float32 products: against 64 bits, 30 runs, the outputs' error is 0.75 and the states' 0.81 of
+// token by token in the mean (float32 multiply-adds in chunks: 0.93 and 0.94; states that hold only the last few tokens are up to a third
+// further off).  The decays only ever enter as products of decays (never as quotients, never as differences of sums of logarithms): nothing cancels,
+// and a constant decay may have any sign.  Up to 64 of them are multiplied before they meet a state, so none may exceed one (callers see to
+// it).  Products of decays are formed in float64 from the float32 decays and rounded once inside an 8-token block and in e, w and e_63; across
+// blocks f(i, j) dt_j is the product of three such numbers (in float32 here: five roundings; in float64, rounded once, for the delta rule below).
+// Numbers that are not finite reach the tokens they reach in the recurrence and no others: the first kernel leaves them out and says which
+// token of a chunk is the first with one, the walk takes the columns they reach from that token on one by one.
 //
-// Two kernels.  The first, parallel over chunks, makes what the columns of a head share: G_ij = C_i . B_j for every chunk and
-// group, and the factors of every chunk and head (u, v, E, diagonal blocks: f(i, j) is a product of three numbers across
-// 8-token blocks, and is stored inside one).  The second walks a sequence's chunks with the state of TP columns of one head in
-// registers (256 threads) and, for the products that read it, in shared memory.
+// Two kernels.  The first, parallel over chunks, makes what the columns of a head share: C and B of every chunk and group, and the scores times
+// the factors f(i, j) dt_j of every chunk and head, in parts and in the order in which the walk's lanes take them, and e, w, e_63.  The second
+// walks a sequence's chunks with the state of 16 to 128 columns of one head in its warps' accumulators.
 //
-// What bounds it: shared memory's delivery of operands and the latency of two warps a scheduler (one CTA of 8 warps an SM; the
-// multiply-add pipe is 43 % busy); the copies of the next chunk run under this one's products.  16 warps with half the registers
-// spilled and were slower (348 against 227 us at the first size below), rows of operands used for two instead of four outputs
-// too (305).  Against the kernels that go token by token, whose chain of row products a token bounds them (us, one B200, back to back):
-// 64 heads of 64 x 128, one sequence of 2,048 tokens 748 -> 226, four of 731 423 -> 340; 16 heads of 256 x 128, four of 1,024 590 -> 476.
+// What bounds it: issue around the tensor cores (two warps a scheduler; half of a chunk's time is their products, the rest splitting states and x,
+// adding up outputs and waiting for one another).  16 warps with half the registers were slower at every size (64 heads of 64 x 128, 2,048
+// tokens: 222 against 169 us), as was fetching the operands with 16-byte copies by all threads instead of the copy engine (198).
+// Token by token, in chunks of float32 multiply-adds, and now (us, one B200, back to back): 64 heads of 64 x 128, one sequence of 2,048 tokens
+// 748, 227, 170, four of 731 423, 340, 236; 16 heads of 256 x 128, four of 1,024 590, 476, 311.
 #include "common.cuh"
+#include "split_mma.cuh"
+#include "tcgen05.cuh"
 
 constexpr int CK_TOKENS = 64, CK_THREADS = 256, CK_WARPS = 8;          // threads: of the first kernel
 constexpr int CK_MLD = CK_TOKENS + 4;
@@ -85,6 +87,11 @@ __device__ __forceinline__ float ck_sum_slices(const float* __restrict__ p, int 
     return total;
 }
 
+constexpr int CK_MBLOCKS = 10;                                  // blocks of 16 x 16 on and below the diagonal of 64 x 64
+// a chunk's record for one head: e [64], w [64] (times dt), decay [64], dt [64], then e_63 and the first token with a number that is not finite
+constexpr int CK_R_E = 0, CK_R_W = 64, CK_R_DECAY = 128, CK_R_DT = 192, CK_R_ALL = 256, CK_R_BAD = 257, CK_RECORD = 260;
+
+
 struct ScanChunks {
     const float* x;             // float32 rows of `stride` numbers: x of head h at + h * P, B and C of group g at + g * N
     const float* b;
@@ -99,58 +106,101 @@ struct ScanChunks {
     const float* fixed_decay;   // a constant decay per head (then step sizes are one), or null
     float* state;               // [slots][heads][P][N]
     float* y;                   // [tokens][heads * P]
-    float* scores;              // scratch: [slots][groups][64][64]
-    float* factors;             // scratch: [slots][heads][CK_FACTORS]
+    unsigned* status;           // or null
+    unsigned char* scratch;     // [slots][groups]: C and B as operands of the walk; [slots][heads]: scores times factors as an operand, the record
+    int max_slots;
     const int* cu;
     const int* slots;
-    int sequences, heads, groups, P, N, vec;
+    int sequences, heads, groups, P, N, vec, together;
+    static __host__ __device__ constexpr size_t group_bytes(int padded) { return (size_t)2 * padded / 16 * 4 * SPLIT_BLOCK_BYTES; }
+    static __host__ __device__ constexpr size_t head_bytes() { return (size_t)CK_MBLOCKS * SPLIT_BLOCK_BYTES + CK_RECORD * sizeof(float); }
+    template <int NP> __device__ uint4* group_scratch(int slot, int g) const {
+        return reinterpret_cast<uint4*>(scratch + ((size_t)slot * groups + g) * group_bytes(NP));
+    }
+    template <int NP> __device__ uint4* head_scratch(int slot, int h) const {
+        return reinterpret_cast<uint4*>(scratch + (size_t)max_slots * groups * group_bytes(NP) + ((size_t)slot * heads + h) * head_bytes());
+    }
 };
 
 // ------------------------------------------------------------------------------------------- what a chunk's columns share
-// The factors of one chunk and head, by one warp; lane l brings the decays and step sizes of tokens l and l + 32.
-__device__ __forceinline__ void ck_factors(float* __restrict__ out, float a0, float a1, float dt0, float dt1, int lane, float* decay, float* step) {
+// the rows of outputs of a block of scores: blocks 0; 1, 2; 3 .. 5; 6 .. 9
+__device__ __forceinline__ int ck_block_row(int block) { return block < 1 ? 0 : block < 3 ? 1 : block < 6 ? 2 : 3; }
+// finite, and its first bfloat16 part too
+__device__ __forceinline__ bool ck_usable(float x) { return fabsf(x) <= 3.3e38f; }
+
+// The factors of one chunk and head, by one warp, into shared memory; lane l brings the decays and step sizes of tokens l and l + 32.
+__device__ __forceinline__ void ck_factors(float* out, float a0, float a1, float dt0, float dt1, int lane, float* decay, float* step) {
     decay[lane] = a0; decay[lane + 32] = a1;
     step[lane] = dt0; step[lane + 32] = dt1;
     __syncwarp();
-    // lane l < 8: its block's product; then everyone has all eight
-    double mine = 1.0;
-    if (lane < 8)
-        for (int t = 0; t < 8; ++t) mine *= (double)decay[8 * lane + t];
-    double block[8];
+    // products inside a block of 8 tokens: of the decays up to the token's (u) and of those behind it (v)
+    const int t = lane & 7;
+    double u[2] = {(double)a0, (double)a1}, v[2] = {1.0, 1.0}, block[8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) block[k] = __shfl_sync(0xffffffffu, mine, k);
+    for (int o = 1; o < 8; o <<= 1)
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            const double other = __shfl_up_sync(0xffffffffu, u[half], o, 8);
+            if (t >= o) u[half] *= other;
+        }
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
-        const int i = lane + 32 * half, b = i >> 3, t = i & 7;
-        double u = 1.0, v = 1.0, before = 1.0, after = 1.0;
-        for (int k = 0; k <= t; ++k) u *= (double)decay[8 * b + k];
-        for (int k = t + 1; k < 8; ++k) v *= (double)decay[8 * b + k];
+        const double next = __shfl_down_sync(0xffffffffu, half ? (double)a1 : (double)a0, 1, 8);
+        if (t < 7) v[half] = next;
+    }
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            if (k < b) before *= block[k];
-            if (k > b) after *= block[k];
-        }
-        const double dt = (double)step[i];
-        out[CK_U + i] = (float)u;
-        out[CK_V + i] = (float)(v * dt);
-        out[CK_E + i] = (float)(before * u);
-        out[CK_W + i] = (float)(v * after * dt);
-        // column t of the diagonal block: f(i', i) dt_i for i' = 0 .. 7 (zero above the diagonal)
-        double p = dt;
-        for (int k = 0; k < 8; ++k) {
-            if (k > t) p *= (double)decay[8 * b + k];
-            out[CK_DIAG + b * 64 + k * 8 + t] = k < t ? 0.0f : (float)p;
-        }
-        // E[bi][bj]: the blocks strictly between
-        const int bi = i >> 3, bj = i & 7;
-        double e = 1.0;
+    for (int o = 1; o < 8; o <<= 1)
 #pragma unroll
-        for (int k = 0; k < 8; ++k)
-            if (k > bj && k < bi) e *= block[k];
-        out[CK_BLOCKS + i] = (float)e;
-        if (i == CK_TOKENS - 1) out[CK_ALL] = (float)(before * u);
+        for (int half = 0; half < 2; ++half) {
+            const double other = __shfl_down_sync(0xffffffffu, v[half], o, 8);
+            if (t + o < 8) v[half] *= other;
+        }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) block[k] = __shfl_sync(0xffffffffu, u[k >> 2], 8 * (k & 3) + 7);
+    double before[2] = {1.0, 1.0}, after[2] = {1.0, 1.0}, e[2] = {1.0, 1.0}, p[2] = {(double)dt0, (double)dt1};
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            const int i = lane + 32 * half, b = i >> 3;
+            if (k < b) before[half] *= block[k];
+            if (k > b) after[half] *= block[k];
+            // E[b][t]: the blocks strictly between; column t of the diagonal block b: f(i', i) dt_i for i' = 0 .. 7 (zero above the diagonal)
+            if (k > t && k < b) e[half] *= block[k];
+            if (k > t) p[half] *= (double)decay[8 * b + k];
+            out[CK_DIAG + b * 64 + k * 8 + t] = k < t ? 0.0f : (float)p[half];
+        }
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        const int i = lane + 32 * half;
+        const double dt = half ? (double)dt1 : (double)dt0;
+        out[CK_U + i] = (float)u[half];
+        out[CK_V + i] = (float)(v[half] * dt);
+        out[CK_E + i] = (float)(before[half] * u[half]);
+        out[CK_W + i] = (float)(v[half] * after[half] * dt);
+        out[CK_BLOCKS + i] = (float)e[half];
+        if (i == CK_TOKENS - 1) out[CK_ALL] = (float)(before[half] * u[half]);
     }
     __syncwarp();
+}
+
+template <int NP>
+struct CkPrepare {
+    // C and B in parts: [C, B][hi, mid, lo][64][PITCH bytes] (rows 16 bytes further than a multiple of 128: no bank conflicts); then, in their place,
+    // the scores and the factors of CK_WARPS heads; a lone head's factors, formed while C and B are on their way
+    static constexpr int PITCH = 2 * NP + 16, PART = CK_TOKENS * PITCH, ONE = 6 * PART, BYTES = ONE + CK_FACTORS * 4;
+    static_assert((CK_TOKENS * CK_MLD + CK_WARPS * CK_FACTORS) * 4 <= ONE, "scores and factors lie where C and B were");
+};
+// four 8 x 8 matrices of bfloat16; lane l names row l % 8 of matrix l / 8
+__device__ __forceinline__ uint4 ck_matrices(uint32_t at) {
+    uint4 v;
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(at) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint4 ck_matrices_turned(uint32_t at) {
+    uint4 v;
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(at) : "memory");
+    return v;
 }
 
 template <int NP>
@@ -158,12 +208,15 @@ __global__ void __launch_bounds__(CK_THREADS, 2)
 scan_chunks_prepare_kernel(const ScanChunks a) {
     tt_pdl_launch_dependents();
     tt_pdl_wait();
-    constexpr int LD = NP + 4;
+    using L = CkPrepare<NP>;
+    constexpr int KS = NP / 16;
     extern __shared__ __align__(16) float ck_shared[];
-    float* cs = ck_shared;
-    float* bs = cs + CK_TOKENS * LD;
+    float* gs = ck_shared;
+    float* factors = ck_shared + CK_TOKENS * CK_MLD;
+    float* one = ck_shared + L::ONE / 4;
     __shared__ float scalars[CK_WARPS][2][CK_TOKENS];
-    // blockIdx.z: the scores and the first CK_WARPS heads' factors, or the factors of CK_WARPS further heads of the group
+    __shared__ int bad, bad_head[CK_WARPS];
+    // blockIdx.z: `together` heads of the group (each of these CTAs forms the scores for itself)
     const int slot = blockIdx.x, g = blockIdx.y;
     int lo = 0, hi = a.sequences;                               // the sequence whose slots reach this one
     while (hi - lo > 1) {
@@ -173,102 +226,634 @@ scan_chunks_prepare_kernel(const ScanChunks a) {
     const int first = a.cu[lo], n = a.cu[lo + 1] - first, c0 = (slot - ck_first_slot(a.cu, lo)) * CK_TOKENS;
     if (c0 >= n) return;
     const int count = min(CK_TOKENS, n - c0);
-    if (blockIdx.z == 0 && a.N < NP) {
-        for (int e = threadIdx.x; e < 2 * CK_TOKENS * LD; e += CK_THREADS) ck_shared[e] = 0.0f;
-        __syncthreads();
-    }
-    const size_t row = (size_t)(first + c0) * a.stride;
-    if (blockIdx.z == 0) {
-        ck_stage<NP>(cs, LD, a.c + row + (size_t)g * a.N, a.stride, count, a.N, a.vec);
-        ck_stage<NP>(bs, LD, a.b + row + (size_t)g * a.N, a.stride, count, a.N, a.vec);
-        ck_commit();
-    }
-
-    // the factors of the group's heads, while the rows are on their way
+    if (threadIdx.x == 0) bad = CK_TOKENS;
+    __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, per_group = a.heads / a.groups;
-    if (const int k = blockIdx.z * CK_WARPS + warp; k < per_group) {
-        const int h = g * per_group + k;
-        float decay[2], step[2];
+    // the warps' heads; a lone head is the last warp's, which has one block of scores
+    const bool lone = a.together == 1;
+    const int own = lone ? CK_WARPS - 1 - warp : warp, h0 = g * per_group + blockIdx.z * a.together, h = h0 + own;
+    const int here = min(a.together, per_group - (int)blockIdx.z * a.together);            // heads of this CTA
+    float decay[2] = {1.0f, 1.0f}, step[2] = {0.0f, 0.0f};      // first the raw step sizes
+    if (own < here && !a.fixed_decay)
+#pragma unroll
+        for (int half = 0; half < 2; ++half)
+            if (lane + 32 * half < count) step[half] = ck_sum_slices(a.proj + (size_t)(first + c0 + lane + 32 * half) * a.cols + a.dt_col + h, a.splits, a.split_stride);
+    // C and B into their parts.  Numbers that are not finite are left out: the walk takes such a token and what follows it in the chunk one by one.
+    {
+        constexpr int PIECES = NP / 4, EACH = CK_TOKENS * PIECES / CK_THREADS;
+        const size_t row = (size_t)(first + c0) * a.stride + (size_t)g * a.N;
+        float4 v[2][EACH];
+#pragma unroll
+        for (int matrix = 0; matrix < 2; ++matrix)
+#pragma unroll
+            for (int e = 0; e < EACH; ++e) {
+                const int r = (threadIdx.x + e * CK_THREADS) / PIECES, c = 4 * ((threadIdx.x + e * CK_THREADS) % PIECES);
+                const float* at = (matrix ? a.b : a.c) + row + (size_t)r * a.stride + c;
+                float4& x = v[matrix][e];
+                x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (r >= count || c >= a.N) continue;
+                if (a.vec) x = __ldg(reinterpret_cast<const float4*>(at));
+                else {
+                    x.x = __ldg(at);
+                    if (c + 1 < a.N) x.y = __ldg(at + 1);
+                    if (c + 2 < a.N) x.z = __ldg(at + 2);
+                    if (c + 3 < a.N) x.w = __ldg(at + 3);
+                }
+            }
+#pragma unroll
+        for (int matrix = 0; matrix < 2; ++matrix)
+#pragma unroll
+            for (int e = 0; e < EACH; ++e) {
+                const int r = (threadIdx.x + e * CK_THREADS) / PIECES, c = 4 * ((threadIdx.x + e * CK_THREADS) % PIECES);
+                float4& x = v[matrix][e];
+                if (!(ck_usable(x.x) && ck_usable(x.y) && ck_usable(x.z) && ck_usable(x.w))) {
+                    atomicMin(&bad, r);
+                    x = make_float4(ck_usable(x.x) ? x.x : 0.0f, ck_usable(x.y) ? x.y : 0.0f, ck_usable(x.z) ? x.z : 0.0f, ck_usable(x.w) ? x.w : 0.0f);
+                }
+                uint2 hi, mid, lo;
+                split_pair(x.x, x.y, hi.x, mid.x, lo.x);
+                split_pair(x.z, x.w, hi.y, mid.y, lo.y);
+                unsigned char* at = reinterpret_cast<unsigned char*>(ck_shared) + matrix * 3 * L::PART + r * L::PITCH + 2 * c;
+                *reinterpret_cast<uint2*>(at) = hi;
+                *reinterpret_cast<uint2*>(at + L::PART) = mid;
+                *reinterpret_cast<uint2*>(at + 2 * L::PART) = lo;
+            }
+    }
+    if (own < here) {
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            if (lane + 32 * half >= count) continue;
+            if (a.fixed_decay) {
+                decay[half] = __ldg(a.fixed_decay + h);
+                step[half] = 1.0f;
+            } else {
+                const float raw = step[half] + __ldg(a.dt_bias + h);
+                step[half] = raw > 20.0f ? raw : log1pf(expf(raw));
+                decay[half] = expf(-expf(__ldg(a.a_log + h)) * step[half]);
+            }
+        }
+    }
+    float* f = lone ? one : factors + own * CK_FACTORS;
+    __syncthreads();                                            // C and B are there
+    if (lone && own == 0) ck_factors(f, decay[0], decay[1], step[0], step[1], lane, scalars[0][0], scalars[0][1]);
+    const int t2 = 2 * (lane & 3), gq = lane >> 2;
+    const uint32_t c_parts = tc::smem_u32(ck_shared), b_parts = c_parts + 3 * L::PART;
+    // rows 16 q .. of a matrix and 16 of its columns: as an operand whose columns the rows are (pieces x, y, z, w; as one whose rows they are: x, z, y, w)
+    const uint32_t plain = ((lane & 7) + 8 * (lane >> 4)) * L::PITCH + 16 * ((lane >> 3) & 1), turned = (lane & 15) * L::PITCH + 16 * (lane >> 4);
+    // the scores C B^T on and below the diagonal, in tiles of 16 x 8 (two or three a warp); sums of 32 are added in float64: long chains lose more
+    constexpr int TILES = (2 * CK_MBLOCKS + CK_WARPS - 1) / CK_WARPS;
+    const uint32_t columns = (lane & 7) * L::PITCH + 16 * (lane >> 3);
+    float scores[TILES][4];
+#pragma unroll
+    for (int mine = 0; mine < TILES; ++mine) {
+        const int block = (warp + CK_WARPS * mine) >> 1, tile = warp & 1;
+        if (block >= CK_MBLOCKS) continue;
+        const int q = ck_block_row(block), s = block - q * (q + 1) / 2;
+        double total[4] = {};
+        float rest[2][4] = {};
+#pragma unroll
+        for (int ks = 0; ks < KS; ks += 2) {
+            float sum[2][4];
+            SplitA A[2];
+            uint4 v[3];                                         // columns' parts: x and y of 16 k, z and w of the next
+#pragma unroll
+            for (int part = 0; part < 3; ++part) {
+                v[part] = ck_matrices(b_parts + part * L::PART + (16 * s + 8 * tile) * L::PITCH + 32 * ks + columns);
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    const uint4 x = ck_matrices(c_parts + part * L::PART + 16 * q * L::PITCH + 32 * (ks + k) + plain);
+                    uint32_t (&to)[4] = part == 0 ? A[k].hi : part == 1 ? A[k].mid : A[k].lo;
+                    to[0] = x.x; to[1] = x.z; to[2] = x.y; to[3] = x.w;
+                }
+            }
+            split_mma(rest[0], A[0].lo, v[0].x, v[0].y);
+            split_mma(rest[1], A[1].lo, v[0].z, v[0].w);
+            split_mma_zero(sum[0], A[0].hi, v[0].x, v[0].y);
+            split_mma_zero(sum[1], A[1].hi, v[0].z, v[0].w);
+            split_mma(rest[0], A[0].hi, v[2].x, v[2].y);
+            split_mma(rest[1], A[1].hi, v[2].z, v[2].w);
+            split_mma(rest[0], A[0].mid, v[1].x, v[1].y);
+            split_mma(rest[1], A[1].mid, v[1].z, v[1].w);
+            split_mma(rest[0], A[0].mid, v[0].x, v[0].y);
+            split_mma(rest[1], A[1].mid, v[0].z, v[0].w);
+            split_mma(rest[0], A[0].hi, v[1].x, v[1].y);
+            split_mma(rest[1], A[1].hi, v[1].z, v[1].w);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) total[e] += (double)(sum[0][e] + sum[1][e]);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) scores[mine][e] = (float)(total[e] + (double)(rest[0][e] + rest[1][e]));
+    }
+    if (blockIdx.z == 0) {
+        // C: k = state rows, columns = tokens; B: k = tokens, columns = state rows
+        uint4* out = a.group_scratch<NP>(slot, g) + lane;
+#pragma unroll 2
+        for (int item = warp; item < KS * 8; item += CK_WARPS) {
+            const int s = (item - KS * 4) / KS, q = (item - KS * 4) % KS;
+            uint4 v[3];
+#pragma unroll
+            for (int part = 0; part < 3; ++part)
+                v[part] = item < KS * 4 ? ck_matrices(c_parts + part * L::PART + 16 * (item & 3) * L::PITCH + 32 * (item >> 2) + plain)
+                                        : ck_matrices_turned(b_parts + part * L::PART + 16 * s * L::PITCH + 32 * q + turned);
+#pragma unroll
+            for (int part = 0; part < 3; ++part) out[item * (SPLIT_BLOCK_BYTES / 16) + 32 * part] = v[part];
+        }
+    }
+    __syncthreads();                                            // C and B are read
+#pragma unroll
+    for (int mine = 0; mine < TILES; ++mine) {
+        const int block = (warp + CK_WARPS * mine) >> 1;
+        if (block >= CK_MBLOCKS) continue;
+        const int q = ck_block_row(block), s = block - q * (q + 1) / 2;
+#pragma unroll
+        for (int half = 0; half < 2; ++half)
+            *reinterpret_cast<float2*>(gs + (16 * q + gq + 8 * half) * CK_MLD + 16 * s + 8 * (warp & 1) + t2) = make_float2(scores[mine][2 * half], scores[mine][2 * half + 1]);
+    }
+    if (!lone && own < here) ck_factors(f, decay[0], decay[1], step[0], step[1], lane, scalars[own][0], scalars[own][1]);
+    if (own < here) {
+        int first_bad = bad;
+#pragma unroll
+        for (int half = 0; half < 2; ++half)
+            if (!ck_usable(decay[half]) || !ck_usable(step[half])) first_bad = min(first_bad, lane + 32 * half);
+        first_bad = __reduce_min_sync(0xffffffffu, first_bad);
+        float* record = reinterpret_cast<float*>(a.head_scratch<NP>(slot, h) + CK_MBLOCKS * (SPLIT_BLOCK_BYTES / 16));
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
             const int i = lane + 32 * half;
-            decay[half] = 1.0f;
-            step[half] = 0.0f;
-            if (i < count) {
-                if (a.fixed_decay) {
-                    decay[half] = __ldg(a.fixed_decay + h);
-                    step[half] = 1.0f;
-                } else {
-                    const float raw = ck_sum_slices(a.proj + (size_t)(first + c0 + i) * a.cols + a.dt_col + h, a.splits, a.split_stride) + __ldg(a.dt_bias + h);
-                    step[half] = raw > 20.0f ? raw : log1pf(expf(raw));
-                    decay[half] = expf(-expf(__ldg(a.a_log + h)) * step[half]);
-                }
-            }
+            record[CK_R_E + i] = f[CK_E + i];
+            record[CK_R_W + i] = f[CK_W + i];
+            record[CK_R_DECAY + i] = decay[half];
+            record[CK_R_DT + i] = step[half];
         }
-        ck_factors(a.factors + ((size_t)slot * a.heads + h) * CK_FACTORS, decay[0], decay[1], step[0], step[1], lane, scalars[warp][0], scalars[warp][1]);
+        if (lane == 0) {
+            record[CK_R_ALL] = f[CK_ALL];
+            bad_head[own] = first_bad;
+        }
     }
-    if (blockIdx.z) return;
-    ck_wait<0>();
     __syncthreads();
-    // G: 16 x 16 threads, rows and columns 16 apart
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    double total[4][4];
+    // scores times factors, in blocks of 16 x 16 (q: tokens of the outputs, s: tokens they see)
+    for (int item = warp; item < here * CK_MBLOCKS; item += CK_WARPS) {
+        const int head = item / CK_MBLOCKS, block = item - head * CK_MBLOCKS, q = ck_block_row(block), s = block - q * (q + 1) / 2;
+        const float* f = lone ? one : factors + head * CK_FACTORS;
+        int first_bad = CK_TOKENS;
+        float v[2][4], odd = 0.0f;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+        for (int tile = 0; tile < 2; ++tile) {
+            const int i = 16 * q + 8 * tile + gq, bi = 2 * q + tile;
+            const float2 e = *reinterpret_cast<const float2*>(f + CK_BLOCKS + bi * 8 + 2 * s);
+            const float u = f[CK_U + i];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) total[i][j] = 0.0;
-    // sums of 8, for states of 128 rows added up to 32, those in float64: long chains lose more
-    constexpr int MIDDLE = NP > 64 ? 32 : 8;
-    for (int k0 = 0; k0 < NP; k0 += MIDDLE) {
-        float part[4][4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) part[i][j] = 0.0f;
-#pragma unroll 2
-        for (int k1 = k0; k1 < k0 + MIDDLE; k1 += 8) {
-            float acc[4][4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
-#pragma unroll
-            for (int k = k1; k < k1 + 8; k += 4) {
-                float4 c[4], b[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    c[i] = *reinterpret_cast<const float4*>(cs + (ty + 16 * i) * LD + k);
-                    b[i] = *reinterpret_cast<const float4*>(bs + (tx + 16 * i) * LD + k);
+            for (int half = 0; half < 2; ++half) {
+                const int j = 16 * s + 8 * half + t2;
+                const float2 score = *reinterpret_cast<const float2*>(gs + i * CK_MLD + j);
+                float2 m;
+                if (q > s) {
+                    const float2 step = *reinterpret_cast<const float2*>(f + CK_V + j);
+                    const float between = u * (half ? e.y : e.x);
+                    m = make_float2(score.x * (between * step.x), score.y * (between * step.y));
+                } else if (tile > half) {
+                    const float2 step = *reinterpret_cast<const float2*>(f + CK_V + j);
+                    const float between = u * e.x;
+                    m = make_float2(score.x * (between * step.x), score.y * (between * step.y));
+                } else if (tile == half) {                      // (the scores above the diagonal need not be finite)
+                    const float2 factor = *reinterpret_cast<const float2*>(f + CK_DIAG + bi * 64 + (i & 7) * 8 + t2);
+                    m = make_float2(j <= i ? score.x * factor.x : 0.0f, j + 1 <= i ? score.y * factor.y : 0.0f);
+                } else {
+                    m = make_float2(0.0f, 0.0f);
                 }
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-#pragma unroll
-                    for (int j = 0; j <= i; ++j) {              // columns behind the row's block are not used
-                        acc[i][j] = fmaf(c[i].x, b[j].x, acc[i][j]);
-                        acc[i][j] = fmaf(c[i].y, b[j].y, acc[i][j]);
-                        acc[i][j] = fmaf(c[i].z, b[j].z, acc[i][j]);
-                        acc[i][j] = fmaf(c[i].w, b[j].w, acc[i][j]);
-                    }
+                odd = fmaxf(odd, fmaxf(ck_usable(m.x) ? 0.0f : 1.0f, ck_usable(m.y) ? 0.0f : 1.0f));
+                v[tile][2 * half] = m.x;
+                v[tile][2 * half + 1] = m.y;
             }
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j <= i; ++j) part[i][j] += acc[i][j];
         }
+        if (odd != 0.0f) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+            for (int tile = 0; tile < 2; ++tile)
 #pragma unroll
-            for (int j = 0; j <= i; ++j) total[i][j] += (double)part[i][j];
+                for (int e = 0; e < 4; ++e)
+                    if (!ck_usable(v[tile][e])) {
+                        first_bad = min(first_bad, 16 * q + 8 * tile + gq);
+                        v[tile][e] = 0.0f;
+                    }
+        }
+        split_store(a.head_scratch<NP>(slot, h0 + head) + block * (SPLIT_BLOCK_BYTES / 16), lane, v);
+        if (first_bad < CK_TOKENS) atomicMin(bad_head + head, first_bad);
     }
-    float* out = a.scores + ((size_t)slot * a.groups + g) * CK_TOKENS * CK_TOKENS;
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j)                             // zeros above the diagonal: a later token's score may be no number
-            out[(ty + 16 * i) * CK_TOKENS + tx + 16 * j] = tx + 16 * j <= ty + 16 * i ? (float)total[i][j] : 0.0f;
+    __syncthreads();
+    if (threadIdx.x < here)
+        reinterpret_cast<int*>(a.head_scratch<NP>(slot, h0 + threadIdx.x) + CK_MBLOCKS * (SPLIT_BLOCK_BYTES / 16))[CK_R_BAD] = bad_head[threadIdx.x];
 }
 
 // -------------------------------------------------------------------------------------------------- the walk over the chunks
+// All products are transposed: 16 value columns on the rows of a tile (x^T, S^T), tokens or state rows on its columns, so that the state
+// S^T [columns x rows] that the update leaves in a warp's accumulators is, split, the operand with which the next chunk's tokens read it.
+// A warp holds 16 columns and a slice of NP / NS state rows; the NS warps of 16 columns add their parts of the outputs through
+// shared memory, PB times 16 columns are a CTA's.
+template <int NP, int PB, int NS>
+struct CkWalk {
+    static constexpr int THREADS = 32 * PB * NS, TP = 16 * PB, LDX = TP + 4, KS = NP / 16, KL = KS / NS;
+    static constexpr int C = 0, B = C + KS * 4 * SPLIT_BLOCK_BYTES, M = B + KS * 4 * SPLIT_BLOCK_BYTES, X = M + CK_MBLOCKS * SPLIT_BLOCK_BYTES;
+    static constexpr int X_BYTES = CK_TOKENS * LDX * 4, R = X + 2 * X_BYTES, PARTS = R + 2 * CK_RECORD * 4;
+    static constexpr int W = PARTS + (NS > 1 ? PB * (NS - 1) * 8 * 512 : 0), BAD = W + (NS > 1 ? PB * 4 * SPLIT_BLOCK_BYTES : 0), BAR = BAD + TP * 4, BYTES = BAR + 16;
+    static constexpr int FIRST_BYTES = CK_RECORD * 4 + CK_MBLOCKS * SPLIT_BLOCK_BYTES + KS * 4 * SPLIT_BLOCK_BYTES, B_BYTES = KS * 4 * SPLIT_BLOCK_BYTES;
+    // Which 16 tokens' x (j) a warp multiplies with the scores of which outputs (q >= j): a block each, about as many for the warps of
+    // every scheduler
+    static constexpr int XA = NS >= 4 ? 1 : 4 / NS;
+    static __device__ __forceinline__ int x_block(int pb, int ns, int at) {
+        if (NS == 1) return at;
+        if (NS == 2) return ns == 0 ? 3 * at : 1 + at;
+        const int w = pb & 1 ? NS - 1 - ns : ns;
+        return NS == 4 ? w : w < 3 ? 0 : w < 5 ? 1 : w < 7 ? 2 : 3;
+    }
+    static __device__ __forceinline__ bool takes(int pb, int ns, int q, int at) {
+        if (x_block(pb, ns, at) > q) return false;
+        if (NS < 8) return true;
+        const int w = pb & 1 ? NS - 1 - ns : ns;
+        return w == 0 ? q < 2 : w == 3 ? q < 3 : w == 1 ? q == 2 : w == 5 ? q == 2 : q == 3;
+    }
+};
+
+// a piece of memory by the copy engine (both addresses on 16 bytes); its bytes are counted on the barrier
+__device__ __forceinline__ void ck_fetch(void* to, const void* from, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(tc::smem_u32(to)), "l"(from), "r"(bytes), "r"(bar) : "memory");
+}
+// whether one of the numbers that this thread copied with ck_stage is not finite (after its copies have arrived)
+template <int WIDTH, int THREADS>
+__device__ __forceinline__ bool ck_staged_odd(const float* to, int to_stride, int width, bool vec) {
+    bool odd = false;
+    if (vec) {
+        constexpr int PER_ROW = WIDTH / 4, STEP = THREADS / PER_ROW, EACH = (CK_TOKENS + STEP - 1) / STEP;
+        const int r0 = threadIdx.x / PER_ROW, c = 4 * (threadIdx.x % PER_ROW);
+        if (c < width && (STEP <= CK_TOKENS || r0 < CK_TOKENS)) {
+#pragma unroll
+            for (int k = 0; k < EACH; ++k) {
+                const float4 v = *reinterpret_cast<const float4*>(to + (r0 + k * STEP) * to_stride + c);
+                odd |= !(ck_usable(v.x) && ck_usable(v.y) && ck_usable(v.z) && ck_usable(v.w));
+            }
+        }
+    } else {
+        for (int e = threadIdx.x; e < CK_TOKENS * WIDTH; e += THREADS)
+            if (e % WIDTH < width) odd |= !ck_usable(to[e / WIDTH * to_stride + e % WIDTH]);
+    }
+    return odd;
+}
+
+// One column's chunk token by token, by one warp: for chunks with numbers that are not finite.  Outputs from token `from` on.
+__device__ __noinline__ void ck_scan_column(const ScanChunks& a, const float* record, int token, int count, int h, int g, int p, float* S, int from) {
+    const int lane = threadIdx.x & 31;
+    const float skip = a.d_skip ? __ldg(a.d_skip + h) : 0.0f;
+    float s[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) s[k] = lane + 32 * k < a.N ? S[lane + 32 * k] : 0.0f;
+    for (int i = 0; i < count; ++i) {
+        const size_t row = (size_t)(token + i) * a.stride;
+        const float x = a.x[row + (size_t)h * a.P + p], decay = record[CK_R_DECAY + i], dx = record[CK_R_DT + i] * x;
+        float sum = 0.0f;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int n = lane + 32 * k;
+            if (n < a.N) {
+                s[k] = fmaf(dx, a.b[row + (size_t)g * a.N + n], decay * s[k]);
+                sum = fmaf(s[k], a.c[row + (size_t)g * a.N + n], sum);
+            }
+        }
+        sum = tt_warp_sum(sum);
+        if (lane == 0 && i >= from) a.y[(size_t)(token + i) * a.heads * a.P + (size_t)h * a.P + p] = fmaf(skip, x, sum);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        if (lane + 32 * k < a.N) S[lane + 32 * k] = s[k];
+}
+
+template <int NP, int PB, int NS>
+__global__ void __launch_bounds__(32 * PB * NS, 1)
+scan_chunks_kernel(const ScanChunks a) {
+    using L = CkWalk<NP, PB, NS>;
+    constexpr int THREADS = L::THREADS, TP = L::TP, LDX = L::LDX, KL = L::KL, PAIR = KL > 1 ? 2 : 1;
+    extern __shared__ __align__(16) unsigned char ck_bytes[];
+    tt_pdl_launch_dependents();
+    tt_pdl_wait();
+    const int h = blockIdx.x, b = blockIdx.y, p0 = blockIdx.z * TP;
+    const int first = a.cu[b], n = a.cu[b + 1] - first;
+    if (n <= 0) return;
+    const int g = h / (a.heads / a.groups), P = a.P, N = a.N, inner = a.heads * P, width = min(TP, P - p0);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, pb = warp / NS, ns = warp % NS;
+    const int t2 = 2 * (lane & 3), gq = lane >> 2;
+    const float skip = a.d_skip ? __ldg(a.d_skip + h) : 0.0f;
+    const int chunks = (n + CK_TOKENS - 1) / CK_TOKENS, slot0 = ck_first_slot(a.cu, b);
+    const bool vec_x = a.vec && (width & 3) == 0;
+    const uint4* Cs = reinterpret_cast<const uint4*>(ck_bytes + L::C) + ns * KL * 4 * (SPLIT_BLOCK_BYTES / 16);
+    const uint4* Bs = reinterpret_cast<const uint4*>(ck_bytes + L::B) + ns * KL * (SPLIT_BLOCK_BYTES / 16);
+    const uint4* Ms = reinterpret_cast<const uint4*>(ck_bytes + L::M);
+    uint4* Ws = reinterpret_cast<uint4*>(ck_bytes + L::W) + pb * 4 * (SPLIT_BLOCK_BYTES / 16);
+    float4* parts = reinterpret_cast<float4*>(ck_bytes + L::PARTS) + pb * (NS - 1) * 8 * 32 + lane;          // [another warp][tile of 8 tokens][lane]
+    int* bad_from = reinterpret_cast<int*>(ck_bytes + L::BAD);
+    for (int e = threadIdx.x; e < 2 * CK_TOKENS * LDX; e += THREADS) reinterpret_cast<float*>(ck_bytes + L::X)[e] = 0.0f;      // what no copy writes is zero
+    const uint32_t bar = tc::smem_u32(ck_bytes + L::BAR), bar_b = bar + 8;
+    if (threadIdx.x == 0) {
+        tc::mbar_init(bar, 1);
+        tc::mbar_init(bar_b, 1);
+        tc::fence_barrier_init();
+    }
+    __syncthreads();
+    bool in_time = true;                                        // no wait has run out
+
+    auto xs = [&](int chunk) { return reinterpret_cast<float*>(ck_bytes + L::X + (chunk & 1) * L::X_BYTES); };
+    auto records = [&](int chunk) { return reinterpret_cast<float*>(ck_bytes + L::R) + (chunk & 1) * CK_RECORD; };
+    auto fetch_first = [&](int chunk) {                         // x, C, scores and factors
+        if (chunk >= chunks) return;
+        const int c0 = chunk * CK_TOKENS;
+        const uint4* head = a.head_scratch<NP>(slot0 + chunk, h);
+        ck_stage<TP, THREADS>(xs(chunk), LDX, a.x + (size_t)(first + c0) * a.stride + (size_t)h * P + p0, a.stride, min(CK_TOKENS, n - c0), width, vec_x);
+        ck_commit();
+        if (threadIdx.x == 0) {
+            tc::mbar_expect_tx(bar, L::FIRST_BYTES);
+            ck_fetch(ck_bytes + L::C, a.group_scratch<NP>(slot0 + chunk, g), L::B_BYTES, bar);
+            ck_fetch(ck_bytes + L::M, head, CK_MBLOCKS * SPLIT_BLOCK_BYTES, bar);
+            ck_fetch(records(chunk), head + CK_MBLOCKS * (SPLIT_BLOCK_BYTES / 16), CK_RECORD * 4, bar);
+        }
+    };
+    fetch_first(0);
+
+    // this warp's state: tile k: columns pb * 16 + gq (and 8 further), rows row0 + 8 k + t2 and the next
+    const int row0 = ns * (NP / NS);
+    float* S = a.state + (((size_t)a.slots[b] * a.heads + h) * P + p0) * N;
+    float s[2 * KL][4];
+    auto load_state = [&](int half) {
+        const int p = pb * 16 + gq + 8 * half;
+#pragma unroll
+        for (int k = 0; k < 2 * KL; ++k)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int r = row0 + 8 * k + t2 + e;
+                s[k][2 * half + e] = p < width && r < N ? S[(size_t)p * N + r] : 0.0f;
+            }
+    };
+    auto store_state = [&]() {
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            const int p = pb * 16 + gq + 8 * half;
+#pragma unroll
+            for (int k = 0; k < 2 * KL; ++k)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int r = row0 + 8 * k + t2 + e;
+                    if (p < width && r < N) S[(size_t)p * N + r] = s[k][2 * half + e];
+                }
+        }
+    };
+    load_state(0);
+    load_state(1);
+    // 16 tokens' x (times w) of this warp's columns as an operand
+    auto split_x = [&](SplitA& A, const float* X, int j) {
+        const float* at = X + (16 * j + t2) * LDX + pb * 16 + gq;
+        split_pair(at[0], at[LDX], A.hi[0], A.mid[0], A.lo[0]);
+        split_pair(at[8], at[LDX + 8], A.hi[1], A.mid[1], A.lo[1]);
+        split_pair(at[8 * LDX], at[9 * LDX], A.hi[2], A.mid[2], A.lo[2]);
+        split_pair(at[8 * LDX + 8], at[9 * LDX + 8], A.hi[3], A.mid[3], A.lo[3]);
+    };
+    auto split_wx = [&](SplitA& A, const float* X, const float* F, int j) {
+        const float* at = X + (16 * j + t2) * LDX + pb * 16 + gq;
+        const float2 w = *reinterpret_cast<const float2*>(F + CK_R_W + 16 * j + t2), v = *reinterpret_cast<const float2*>(F + CK_R_W + 16 * j + t2 + 8);
+        split_pair(w.x * at[0], w.y * at[LDX], A.hi[0], A.mid[0], A.lo[0]);
+        split_pair(w.x * at[8], w.y * at[LDX + 8], A.hi[1], A.mid[1], A.lo[1]);
+        split_pair(v.x * at[8 * LDX], v.y * at[9 * LDX], A.hi[2], A.mid[2], A.lo[2]);
+        split_pair(v.x * at[8 * LDX + 8], v.y * at[9 * LDX + 8], A.hi[3], A.mid[3], A.lo[3]);
+    };
+
+    for (int chunk = 0; chunk < chunks; ++chunk) {
+        float* X = xs(chunk);
+        const float* F = records(chunk);
+        const int left = n - chunk * CK_TOKENS;
+        ck_wait<0>();
+        in_time = in_time && tc::mbar_wait(bar, chunk & 1);
+        bool odd = ck_staged_odd<TP, THREADS>(X, LDX, width, vec_x);
+#pragma unroll
+        for (int k = 0; k < 2 * KL; ++k)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) odd |= !ck_usable(s[k][e]);
+        // x, C, scores and factors are there; B, the weighted rows and the parts of the chunk before are read
+        bool some_bad = __syncthreads_or(odd);
+        some_bad |= __float_as_int(F[CK_R_BAD]) < CK_TOKENS;
+        if (threadIdx.x == 0) {
+            tc::mbar_expect_tx(bar_b, L::B_BYTES);
+            ck_fetch(ck_bytes + L::B, a.group_scratch<NP>(slot0 + chunk, g) + L::KS * 4 * (SPLIT_BLOCK_BYTES / 16), L::B_BYTES, bar_b);
+        }
+        if (some_bad) {
+            // columns from their first token on that is, or meets, a number that is not finite go token by token; the others as ever
+            for (int p = threadIdx.x; p < TP; p += THREADS) bad_from[p] = __float_as_int(F[CK_R_BAD]);
+            __syncthreads();
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                bool mine = false;
+#pragma unroll
+                for (int k = 0; k < 2 * KL; ++k) mine |= !ck_usable(s[k][2 * half]) || !ck_usable(s[k][2 * half + 1]);
+                if (mine) atomicMin(bad_from + pb * 16 + gq + 8 * half, 0);
+            }
+            for (int e = threadIdx.x; e < CK_TOKENS * TP; e += THREADS)
+                if (float* x = X + e / TP * LDX + e % TP; !ck_usable(*x)) {
+                    atomicMin(bad_from + e % TP, e / TP);
+                    *x = 0.0f;
+                }
+            store_state();
+            __syncthreads();
+            const int count = min(CK_TOKENS, left);
+            for (int p = warp; p < width; p += THREADS / 32)
+                if (bad_from[p] < count) ck_scan_column(a, F, first + chunk * CK_TOKENS, count, h, g, p0 + p, S + (size_t)p * N, bad_from[p]);
+            __syncthreads();
+        }
+        float* out = a.y + (size_t)(first + chunk * CK_TOKENS) * inner + (size_t)h * P + p0 + pb * 16 + gq;
+        const float* own = X + pb * 16 + gq;
+        const int limit[2] = {pb * 16 + gq < width ? min(left, some_bad ? bad_from[pb * 16 + gq] : CK_TOKENS) : 0,
+                              pb * 16 + gq + 8 < width ? min(left, some_bad ? bad_from[pb * 16 + gq + 8] : CK_TOKENS) : 0};
+        auto write = [&](int tile, const float (&o)[4]) {       // the outputs of 8 tokens: skip times x is added last
+            float* to = out + (size_t)(8 * tile + t2) * inner;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int i = 8 * tile + t2 + (e & 1), half = e >> 1;
+                const float v = a.d_skip ? fmaf(skip, own[i * LDX + 8 * half], o[e]) : o[e];
+                if (i < limit[half]) to[(e & 1 ? inner : 0) + 8 * half] = v;
+            }
+        };
+        float mine[NS > 1 ? 8 / NS : 1][4];
+        {
+            SplitA A, xa[L::XA];
+            if (NS > 1 && (NS <= 4 || ns < 4)) {                // the rows of the update, shared out among the warps that take them
+#pragma unroll
+                for (int j = 0; j < (NS < 4 ? 4 / NS : 1); ++j) {
+                    const int block = NS < 4 ? ns * (4 / NS) + j : ns;
+                    split_wx(A, X, F, block);
+                    split_store(Ws + block * (SPLIT_BLOCK_BYTES / 16), lane, A);
+                }
+            }
+            auto split_state = [&](SplitA& to, int k) {
+                split_pair(s[2 * k][0], s[2 * k][1], to.hi[0], to.mid[0], to.lo[0]);
+                split_pair(s[2 * k][2], s[2 * k][3], to.hi[1], to.mid[1], to.lo[1]);
+                split_pair(s[2 * k + 1][0], s[2 * k + 1][1], to.hi[2], to.mid[2], to.lo[2]);
+                split_pair(s[2 * k + 1][2], s[2 * k + 1][3], to.hi[3], to.mid[3], to.lo[3]);
+            };
+            // y: C times the state for the tiles of blocks q0 and q0 + 1; then the scores times x, and out with it
+            auto outputs = [&](int q0, float (*y)[4]) {
+                float sum[4][4] = {}, rest[4][4] = {};
+#pragma unroll
+                for (int q = q0; q < q0 + 2; ++q)
+#pragma unroll
+                    for (int j = 0; j < L::XA; ++j)
+                        if (L::takes(pb, ns, q, j))
+                            split_products<1, false>(sum + 2 * (q - q0), rest + 2 * (q - q0), xa[j], Ms + (q * (q + 1) / 2 + L::x_block(pb, ns, j)) * (SPLIT_BLOCK_BYTES / 16), lane);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float2 e = *reinterpret_cast<const float2*>(F + CK_R_E + 16 * q0 + 8 * i + t2);
+                    const float o[4] = {fmaf(e.x, y[i][0], rest[i][0]) + sum[i][0], fmaf(e.y, y[i][1], rest[i][1]) + sum[i][1],
+                                        fmaf(e.x, y[i][2], rest[i][2]) + sum[i][2], fmaf(e.y, y[i][3], rest[i][3]) + sum[i][3]};
+                    constexpr int EACH = 8 / NS;                // a warp adds up and writes EACH tiles
+                    const int tile = 2 * q0 + i, owner = tile / EACH;
+                    if (NS == 1) write(tile, o);
+                    else if (owner != ns) parts[((ns - (ns > owner)) * 8 + tile) * 32] = make_float4(o[0], o[1], o[2], o[3]);
+                    else {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) mine[tile % EACH][e] = o[e];
+                    }
+                }
+            };
+            if constexpr (THREADS <= 256) {                     // registers for all outputs: the state is split as it is used
+                float y[8][4], rest[8][4];
+#pragma unroll
+                for (int k = 0; k < KL; ++k) {
+                    split_state(A, k);
+                    const uint4* block = Cs + k * 4 * (SPLIT_BLOCK_BYTES / 16);
+                    if (k == 0) { split_products<2, true>(y, rest, A, block, lane); split_products<2, true>(y + 4, rest + 4, A, block + 2 * (SPLIT_BLOCK_BYTES / 16), lane); }
+                    else { split_products<2, false>(y, rest, A, block, lane); split_products<2, false>(y + 4, rest + 4, A, block + 2 * (SPLIT_BLOCK_BYTES / 16), lane); }
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) y[i][e] += rest[i][e];
+#pragma unroll
+                for (int j = 0; j < L::XA; ++j) split_x(xa[j], X, L::x_block(pb, ns, j));
+                outputs(0, y);
+                outputs(2, y + 4);
+            } else {
+                SplitA As[KL];
+#pragma unroll
+                for (int k = 0; k < KL; ++k) split_state(As[k], k);
+#pragma unroll
+                for (int j = 0; j < L::XA; ++j) split_x(xa[j], X, L::x_block(pb, ns, j));
+#pragma unroll
+                for (int q0 = 0; q0 < 4; q0 += 2) {
+                    float y[4][4], rest[4][4];
+                    split_products<2, true>(y, rest, As[0], Cs + q0 * (SPLIT_BLOCK_BYTES / 16), lane);
+#pragma unroll
+                    for (int k = 1; k < KL; ++k) split_products<2, false>(y, rest, As[k], Cs + (k * 4 + q0) * (SPLIT_BLOCK_BYTES / 16), lane);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) y[i][e] += rest[i][e];
+                    outputs(q0, y);
+                }
+            }
+        }
+        __syncthreads();                                        // the weighted rows and the parts are there; C and the scores are read
+        fetch_first(chunk + 1);
+        // S^T <- e_63 S^T + (w x)^T B; the larger part is added last: one rounding at the size of the sum
+        in_time = in_time && tc::mbar_wait(bar_b, chunk & 1);
+        const float all = F[CK_R_ALL];
+        const bool long_memory = fabsf(all) > 0.25f;
+        SplitA wa[NS > 1 ? 1 : 4];
+        if (NS == 1)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) split_wx(wa[NS > 1 ? 0 : j], X, F, j);
+#pragma unroll
+        for (int k = 0; k < KL; k += PAIR) {
+            float sum[2 * PAIR][4], rest[2 * PAIR][4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (NS > 1) split_load(wa[0], Ws + j * (SPLIT_BLOCK_BYTES / 16), lane);
+                const uint4* block = Bs + (j * L::KS + k) * (SPLIT_BLOCK_BYTES / 16);
+                if (j == 0) split_products<PAIR, true>(sum, rest, wa[0], block, lane);
+                else split_products<PAIR, false>(sum, rest, wa[NS > 1 ? 0 : j], block, lane);
+            }
+#pragma unroll
+            for (int i = 0; i < 2 * PAIR; ++i)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    float& v = s[2 * k + i][e];
+                    v = long_memory ? fmaf(all, v, sum[i][e] + rest[i][e]) : fmaf(all, v, rest[i][e]) + sum[i][e];
+                }
+        }
+        if (NS > 1) {
+#pragma unroll
+            for (int i = 0; i < 8 / NS; ++i) {
+                const int tile = ns * (8 / NS) + i;
+                float o[4] = {};
+#pragma unroll
+                for (int k = 0; k < NS - 1; ++k) {
+                    const float4 q = parts[(k * 8 + tile) * 32];
+                    o[0] += q.x; o[1] += q.y; o[2] += q.z; o[3] += q.w;
+                }
+#pragma unroll
+                for (int e = 0; e < 4; ++e) o[e] += mine[i][e];
+                write(tile, o);
+            }
+        }
+        if (some_bad) {
+            const int count = min(CK_TOKENS, left);
+            if (bad_from[pb * 16 + gq] < count) load_state(0);
+            if (bad_from[pb * 16 + gq + 8] < count) load_state(1);
+        }
+    }
+    if (!in_time && a.status) atomicOr(a.status, TT_STATUS_WAIT_EXPIRED);
+    store_state();
+}
+
+// on every launch: it holds for the current device alone, and an engine may run on any of the process's
+template <typename Kernel>
+static cudaError_t ck_allow(Kernel kernel, size_t bytes) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); }
+
+template <int NP, int PB, int NS>
+static int scan_chunks_launch(const ScanChunks& a, int max_slots, cudaStream_t stream) {
+    using L = CkWalk<NP, PB, NS>;
+    constexpr size_t prepare_bytes = CkPrepare<NP>::BYTES;
+    cudaError_t code = ck_allow(scan_chunks_prepare_kernel<NP>, prepare_bytes);
+    if (code == cudaSuccess) code = ck_allow(scan_chunks_kernel<NP, PB, NS>, L::BYTES);
+    if (code != cudaSuccess) return (int)code;
+    tt_launch_pdl(scan_chunks_prepare_kernel<NP>, dim3(max_slots, a.groups, (a.heads / a.groups + a.together - 1) / a.together), dim3(CK_THREADS), prepare_bytes, stream, a);
+    tt_launch_pdl(scan_chunks_kernel<NP, PB, NS>, dim3(a.heads, a.sequences, (a.P + L::TP - 1) / L::TP), dim3(L::THREADS), (size_t)L::BYTES, stream, a);
+    TT_LAUNCH_CHECK();
+}
+
+// rows: [tokens][width] with x, B and C from the given columns on (see ScanChunks).  max_slots: n_tokens / 64 + sequences.  scratch: so many
+// times the scores of every group (64 * 64 numbers) and the factors of every head (CK_FACTORS), on a 16-byte boundary: the walk copies
+// it in 16-byte pieces whatever the rows' alignment.  sms: the device's multiprocessors.
+extern "C" int tt_scan_chunks(const float* rows, int width, int x_col, int b_col, int c_col, const float* proj, int splits, long long split_stride,
+                              int cols, int dt_col, const float* dt_bias, const float* a_log, const float* d_skip, const float* fixed_decay, float* state,
+                              float* y, float* scratch, const int* cu, const int* slots, int sequences, int max_slots, int heads,
+                              int groups, int P, int N, int sms, unsigned* status, cudaStream_t stream) {
+    if (sequences <= 0 || max_slots <= 0) return 0;
+    if (N <= 0 || N > 128 || P <= 0 || groups <= 0 || groups > 65535 || heads % groups || sequences > 65535) return (int)cudaErrorInvalidValue;
+    if (!rows || !scratch || ((uintptr_t)scratch & 15) || (!fixed_decay && (!proj || !dt_bias || !a_log))) return (int)cudaErrorInvalidValue;
+    const float *x = rows + x_col, *b = rows + b_col, *c = rows + c_col;
+    const uintptr_t bases = (uintptr_t)x | (uintptr_t)b | (uintptr_t)c | (uintptr_t)y;
+    // heads of a CTA of the first kernel: as few as one wave of two CTAs an SM has room for (a head takes a warp ten blocks of scores, eight heads all of them)
+    int together = 1;
+    while (together < CK_WARPS && (long long)max_slots * groups * ((heads / groups + together - 1) / together) > 2LL * sms) together *= 2;
+    together = together < heads / groups ? together : heads / groups;
+    const ScanChunks a{x, b, c, (size_t)width, proj, splits, cols, dt_col, (size_t)split_stride, dt_bias, a_log, d_skip, fixed_decay, state, y, status,
+                       reinterpret_cast<unsigned char*>(scratch), max_slots, cu, slots, sequences, heads, groups, P, N,
+                       (bases & 15) == 0 && !(width & 3) && !(N & 3) && !(P & 3) ? 1 : 0, together};
+    // Columns of a CTA: rounds of the SMs times what a chunk takes a CTA (hundredths of a microsecond, measured with the GPU to itself: 128 rows 16 columns
+    // 333, 32 453, 64 766, 128 1,363; 64 rows 32 columns 300, 64 500, 128 810, and 16 columns no less than 32).
+    const long long one = (long long)heads * sequences;
+    auto cost = [&](int columns, int chunk) { return (one * ((P + columns - 1) / columns) + sms - 1) / sms * chunk; };
+    const bool small = N <= 64;
+    const long long c16 = cost(16, 333), c32 = cost(32, small ? 300 : 453), c64 = cost(64, small ? 500 : 766), c128 = cost(128, small ? 810 : 1363);
+    if (c128 <= c64 && c128 <= c32 && c128 <= c16) return small ? scan_chunks_launch<64, 8, 1>(a, max_slots, stream) : scan_chunks_launch<128, 8, 1>(a, max_slots, stream);
+    if (c64 <= c32 && c64 <= c16) return small ? scan_chunks_launch<64, 4, 2>(a, max_slots, stream) : scan_chunks_launch<128, 4, 2>(a, max_slots, stream);
+    if (small) return scan_chunks_launch<64, 2, 4>(a, max_slots, stream);
+    return c32 <= c16 ? scan_chunks_launch<128, 2, 4>(a, max_slots, stream) : scan_chunks_launch<128, 1, 8>(a, max_slots, stream);
+}
+
 // The products of a chunk's 64 output rows are shared out over the warps in blocks of rows and, so that a lane can hold four rows of
 // four neighbouring columns (an operand piece read from shared memory then serves four outputs, which is what bounds these
 // products), over slices of k: PL = TP / 4 lanes lie across the columns, RL = 32 / PL across the rows.
@@ -464,189 +1049,6 @@ struct CkLayout {
     static constexpr int B = 0, X = B + CK_TOKENS * NP, M = X + CK_TOKENS * LDX, F = M + CK_TOKENS * CK_MLD, STAGE_FLOATS = F + CK_FACTORS;
     static constexpr size_t BYTES = (size_t)(STAGE + 2 * STAGE_FLOATS) * sizeof(float);
 };
-
-template <int NP, int TP>
-__global__ void __launch_bounds__(CkLayout<NP, TP>::THREADS, 1)
-scan_chunks_kernel(const ScanChunks a) {
-    using L = CkLayout<NP, TP>;
-    constexpr int THREADS = L::THREADS, PL = L::PL, RL = L::RL, ROW_BLOCKS = CK_TOKENS / L::ROWS;
-    constexpr int NL = NP * TP / (THREADS * 4);              // state rows of a lane
-    extern __shared__ __align__(16) float ck_shared[];
-    tt_pdl_launch_dependents();
-    tt_pdl_wait();
-    const int h = blockIdx.x, b = blockIdx.y, p0 = blockIdx.z * TP;
-    const int first = a.cu[b], n = a.cu[b + 1] - first;
-    if (n <= 0) return;
-    const int g = h / (a.heads / a.groups), P = a.P, N = a.N;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int col = 4 * (lane % PL), width = min(TP, P - p0), inner = a.heads * P;
-    // row blocks are dealt to the warps so that the warps of a scheduler (w, w + 4, ..) together have equally long causal sums
-    const int slice = warp / ROW_BLOCKS, block = (warp + (warp >> 2)) % ROW_BLOCKS;
-    const int row = block * L::ROWS + lane / PL;                // first of this lane's four rows, RL apart
-    const int srow = warp * (NP / L::WARPS) + (lane / PL) * NL;        // first of this lane's state rows
-    const float skip = a.d_skip ? __ldg(a.d_skip + h) : 0.0f;
-    float* As = ck_shared + L::A;
-    float* Ss = ck_shared + L::S;
-    float* XW = ck_shared + L::XW;
-    const int chunks = (n + CK_TOKENS - 1) / CK_TOKENS, slot0 = ck_first_slot(a.cu, b);
-    const bool vec_x = a.vec && (width & 3) == 0;
-
-    for (int e = threadIdx.x; e < L::STAGE + 2 * L::STAGE_FLOATS; e += THREADS) ck_shared[e] = 0.0f;     // what no copy writes is zero
-    __syncthreads();
-    auto fetch_a = [&](int chunk) {
-        if (chunk < chunks) {
-            const int c0 = chunk * CK_TOKENS;
-            ck_stage<NP, THREADS>(As, L::LDA, a.c + (size_t)(first + c0) * a.stride + (size_t)g * N, a.stride, min(CK_TOKENS, n - c0), N, a.vec);
-        }
-        ck_commit();
-    };
-    auto fetch_rest = [&](int chunk) {
-        if (chunk < chunks) {
-            const int c0 = chunk * CK_TOKENS, count = min(CK_TOKENS, n - c0);
-            float* stage = ck_shared + L::STAGE + (chunk & 1) * L::STAGE_FLOATS;
-            const size_t at = (size_t)(first + c0) * a.stride;
-            ck_stage<NP, THREADS>(stage + L::B, NP, a.b + at + (size_t)g * N, a.stride, count, N, a.vec);
-            ck_stage<TP, THREADS>(stage + L::X, L::LDX, a.x + at + (size_t)h * P + p0, a.stride, count, width, vec_x);
-            ck_stage<CK_TOKENS, THREADS>(stage + L::M, CK_MLD, a.scores + ((size_t)(slot0 + chunk) * a.groups + g) * CK_TOKENS * CK_TOKENS, CK_TOKENS, CK_TOKENS, CK_TOKENS, true);
-            const float* factors = a.factors + ((size_t)(slot0 + chunk) * a.heads + h) * CK_FACTORS;
-            for (int e = threadIdx.x; e < CK_FACTORS / 4; e += THREADS) ck_copy16(stage + L::F + 4 * e, factors + 4 * e, true);
-        }
-        ck_commit();
-    };
-    fetch_rest(0);
-    fetch_a(0);
-
-    float* S = a.state + (((size_t)a.slots[b] * a.heads + h) * P + p0 + col) * N;
-    unsigned long long s[NL][2];
-#pragma unroll
-    for (int i = 0; i < NL; ++i) {
-        float v[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) v[e] = srow + i < N && p0 + col + e < P ? S[(size_t)e * N + srow + i] : 0.0f;
-        s[i][0] = ck_pair(v[0], v[1]);
-        s[i][1] = ck_pair(v[2], v[3]);
-        *reinterpret_cast<float4*>(Ss + (srow + i) * L::LDX + col) = make_float4(v[0], v[1], v[2], v[3]);
-    }
-
-    for (int chunk = 0; chunk < chunks; ++chunk) {
-        float* stage = ck_shared + L::STAGE + (chunk & 1) * L::STAGE_FLOATS;
-        const float* X = stage + L::X;
-        float* M = stage + L::M;
-        const float* F = stage + L::F;
-        fetch_rest(chunk + 1);
-        ck_wait<1>();
-        __syncthreads();                                        // this chunk's numbers and the state are there
-
-        // the decays into the scores, and the rows the update adds
-        float odd = 0.0f;                                       // no longer zero: an x of the chunk is not finite
-        {
-            const int j = 4 * (threadIdx.x & 15), bj = j >> 3;
-            const float4 v = *reinterpret_cast<const float4*>(F + CK_V + j);
-#pragma unroll
-            for (int k = 0; k < 16 * CK_TOKENS / THREADS; ++k) {
-                const int i = (threadIdx.x >> 4) + THREADS / 16 * k, bi = i >> 3;
-                float4* at = reinterpret_cast<float4*>(M + i * CK_MLD + j);
-                float4 f = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                if (bi > bj) {
-                    const float u = F[CK_U + i] * F[CK_BLOCKS + bi * 8 + bj];
-                    f = make_float4(u * v.x, u * v.y, u * v.z, u * v.w);
-                } else if (bi == bj) {
-                    f = *reinterpret_cast<const float4*>(F + CK_DIAG + bi * 64 + (i & 7) * 8 + (j & 7));
-                }
-                if (bi >= bj) {                                 // what lies above is not read
-                    const float4 m = *at;
-                    *at = make_float4(m.x * f.x, m.y * f.y, m.z * f.z, m.w * f.w);
-                } else {
-                    *at = f;
-                }
-            }
-            for (int e = threadIdx.x; e < CK_TOKENS * PL; e += THREADS) {
-                const int t = e / PL, c = 4 * (e - t * PL);
-                const float4 x = *reinterpret_cast<const float4*>(X + t * L::LDX + c);
-                const float w = F[CK_W + t];
-                odd += ck_not_finite(x);
-                *reinterpret_cast<float4*>(XW + t * L::LDX + c) = make_float4(w * x.x, w * x.y, w * x.z, w * x.w);
-            }
-        }
-        unsigned long long acc[4][2];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) acc[r][0] = acc[r][1] = 0ull;
-        constexpr int K = NP / L::SLICES;
-        ck_state_product<RL, K>(acc, As + row * L::LDA, L::LDA, Ss + col, L::LDX, slice * K);
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const float e = F[CK_E + row + RL * r];
-            acc[r][0] = ck_pair(ck_lo(acc[r][0]) * e, ck_hi(acc[r][0]) * e);
-            acc[r][1] = ck_pair(ck_lo(acc[r][1]) * e, ck_hi(acc[r][1]) * e);
-        }
-        const bool finite = !__syncthreads_or(odd != 0.0f);     // scores and weighted rows are written, C and the old state are read
-        fetch_a(chunk + 1);
-        if (finite) ck_product<RL>(acc, M + row * CK_MLD, CK_MLD, X + col, L::LDX, 4 * slice, 4 * L::SLICES, block * L::ROWS + L::ROWS);
-        else ck_causal_product<RL>(acc, M + row * CK_MLD, CK_MLD, X + col, L::LDX, 4 * slice, 4 * L::SLICES, block * L::ROWS + L::ROWS, row);
-        if (slice > 0) {
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-                *reinterpret_cast<float4*>(ck_shared + L::PARTS + ((slice - 1) * CK_TOKENS + row + RL * r) * L::LDX + col) =
-                    make_float4(ck_lo(acc[r][0]), ck_hi(acc[r][0]), ck_lo(acc[r][1]), ck_hi(acc[r][1]));
-        }
-        float4 own[4];                                          // added last, to the whole sum: one rounding at its size
-#pragma unroll
-        for (int r = 0; r < 4; ++r) own[r] = slice == 0 ? *reinterpret_cast<const float4*>(X + (row + RL * r) * L::LDX + col) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        // S <- e_63 S + B^T (w x)
-        ck_update<NP, NL>(s, F[CK_ALL], stage + L::B + srow, XW + col, L::LDX);
-#pragma unroll
-        for (int i = 0; i < NL; ++i)
-            *reinterpret_cast<float4*>(Ss + (srow + i) * L::LDX + col) = make_float4(ck_lo(s[i][0]), ck_hi(s[i][0]), ck_lo(s[i][1]), ck_hi(s[i][1]));
-        __syncthreads();                                        // this stage may be filled again, the weighted rows be written again
-        if (slice == 0)                                         // the other slices' sums are there: the chunk's outputs
-            ck_outputs<RL, L::SLICES>(acc, ck_shared + L::PARTS, L::LDX, row, col, width, n - chunk * CK_TOKENS, vec_x, skip, own,
-                                      a.y + (size_t)(first + chunk * CK_TOKENS) * inner + (size_t)h * P + p0, inner);
-    }
-    ck_wait<0>();
-#pragma unroll
-    for (int i = 0; i < NL; ++i) {
-        const float v[4] = {ck_lo(s[i][0]), ck_hi(s[i][0]), ck_lo(s[i][1]), ck_hi(s[i][1])};
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-            if (srow + i < N && p0 + col + e < P) S[(size_t)e * N + srow + i] = v[e];
-    }
-}
-
-// on every launch: it holds for the current device alone, and an engine may run on any of the process's
-template <typename Kernel>
-static cudaError_t ck_allow(Kernel kernel, size_t bytes) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); }
-
-template <int NP, int TP>
-static int scan_chunks_launch(const ScanChunks& a, int max_slots, cudaStream_t stream) {
-    constexpr size_t prepare_bytes = (size_t)2 * CK_TOKENS * (NP + 4) * sizeof(float);
-    cudaError_t code = ck_allow(scan_chunks_prepare_kernel<NP>, prepare_bytes);
-    if (code == cudaSuccess) code = ck_allow(scan_chunks_kernel<NP, TP>, CkLayout<NP, TP>::BYTES);
-    if (code != cudaSuccess) return (int)code;
-    tt_launch_pdl(scan_chunks_prepare_kernel<NP>, dim3(max_slots, a.groups, (a.heads / a.groups + CK_WARPS - 1) / CK_WARPS), dim3(CK_THREADS), prepare_bytes, stream, a);
-    tt_launch_pdl(scan_chunks_kernel<NP, TP>, dim3(a.heads, a.sequences, (a.P + TP - 1) / TP), dim3(CkLayout<NP, TP>::THREADS), CkLayout<NP, TP>::BYTES, stream, a);
-    TT_LAUNCH_CHECK();
-}
-
-// rows: [tokens][width] with x, B and C from the given columns on (see ScanChunks).  max_slots: n_tokens / 64 + sequences.  scratch: so many
-// times the scores of every group (64 * 64 numbers) and the factors of every head (CK_FACTORS), on a 16-byte boundary: the walk copies
-// it in 16-byte pieces whatever the rows' alignment.  sms: the device's multiprocessors.
-extern "C" int tt_scan_chunks(const float* rows, int width, int x_col, int b_col, int c_col, const float* proj, int splits, long long split_stride,
-                              int cols, int dt_col, const float* dt_bias, const float* a_log, const float* d_skip, const float* fixed_decay, float* state,
-                              float* y, float* scratch, const int* cu, const int* slots, int sequences, int max_slots, int heads,
-                              int groups, int P, int N, int sms, cudaStream_t stream) {
-    if (sequences <= 0 || max_slots <= 0) return 0;
-    if (N <= 0 || N > 128 || P <= 0 || groups <= 0 || groups > 65535 || heads % groups || sequences > 65535) return (int)cudaErrorInvalidValue;
-    if (!rows || !scratch || ((uintptr_t)scratch & 15) || (!fixed_decay && (!proj || !dt_bias || !a_log))) return (int)cudaErrorInvalidValue;
-    const float *x = rows + x_col, *b = rows + b_col, *c = rows + c_col;
-    float *scores = scratch, *factors = scratch + (size_t)max_slots * groups * CK_TOKENS * CK_TOKENS;
-    const uintptr_t bases = (uintptr_t)x | (uintptr_t)b | (uintptr_t)c | (uintptr_t)y;
-    const ScanChunks a{x, b, c, (size_t)width, proj, splits, cols, dt_col, (size_t)split_stride, dt_bias, a_log, d_skip, fixed_decay, state, y, scores, factors,
-                       cu, slots, sequences, heads, groups, P, N, (bases & 15) == 0 && !(width & 3) && !(N & 3) && !(P & 3) ? 1 : 0};
-    // 32 columns a CTA use a number of C twice; 16 where that grid would leave half of the SMs without one
-    const bool narrow = (long long)heads * sequences * ((P + 31) / 32) * 2 <= sms + sms / 4;
-    if (N <= 64) return narrow ? scan_chunks_launch<64, 16>(a, max_slots, stream) : scan_chunks_launch<64, 32>(a, max_slots, stream);
-    return narrow ? scan_chunks_launch<128, 16>(a, max_slots, stream) : scan_chunks_launch<128, 32>(a, max_slots, stream);
-}
 
 // ------------------------------------------------------------------------------------------------------ the gated delta rule
 //   q = q / |q| * scale, k = k / |k|;  S <- a_t S;  u_t = beta_t (v_t - S^T k_t);  S <- S + k_t u_t^T;  o_t = S^T q_t

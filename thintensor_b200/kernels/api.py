@@ -913,7 +913,7 @@ def mamba2_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_col: int, dt_bias: tor
 
 CHUNK_TOKENS = 64           # tokens of a chunk of the recurrences with a decay per head (CK_TOKENS in csrc/recurrent_chunks.cu)
 CHUNK_MAX_ROWS = 128        # state rows (key size) the chunk kernels take
-_CHUNK_FACTORS = 836
+_CHUNK_HEAD_FLOATS = 10 * 384 + 260         # scores times factors as an operand in three bfloat16 parts, and a record
 _DELTA_CHUNK_FACTORS = 136
 
 
@@ -922,18 +922,21 @@ def chunk_slots(n_tokens: int, sequences: int) -> int:
     return n_tokens // CHUNK_TOKENS + sequences
 
 
-def scan_chunks_scratch(n_tokens: int, sequences: int, heads: int, groups: int) -> tuple[int]:
-    """Shape of the float32 scratch that :func:`scan_chunks` takes: scores for every chunk and group, factors for every chunk and head."""
-    return (chunk_slots(n_tokens, sequences) * (groups * CHUNK_TOKENS * CHUNK_TOKENS + heads * _CHUNK_FACTORS),)
+def scan_chunks_scratch(n_tokens: int, sequences: int, heads: int, groups: int, state_size: int = CHUNK_MAX_ROWS) -> tuple[int]:
+    """Shape of the float32 scratch that :func:`scan_chunks` takes for states of ``state_size`` rows: B and C of every chunk and group and the
+    scores of every chunk and head in three bfloat16 parts, factors for every chunk and head."""
+    padded = 64 if state_size <= 64 else 128
+    return (chunk_slots(n_tokens, sequences) * (groups * 2 * CHUNK_TOKENS * padded * 3 // 2 + heads * _CHUNK_HEAD_FLOATS),)
 
 
 def scan_chunks(rows: torch.Tensor, x_col: int, b_col: int, c_col: int, state: torch.Tensor, y: torch.Tensor, cu: torch.Tensor, slots: torch.Tensor,
                 sequences: int, heads: int, head_dim: int, state_size: int, groups: int, scratch: torch.Tensor,
-                steps: tuple[torch.Tensor, int, torch.Tensor, torch.Tensor, torch.Tensor] | None = None, fixed_decay: torch.Tensor | None = None) -> None:
+                steps: tuple[torch.Tensor, int, torch.Tensor, torch.Tensor, torch.Tensor] | None = None, fixed_decay: torch.Tensor | None = None,
+                status: torch.Tensor | None = None) -> None:
     """The recurrences of :func:`mamba2_scan` and :func:`decay_scan`, a chunk of 64 tokens at a time (for prompts).  ``rows``: float32
     ``[tokens, columns]`` with x (``heads * head_dim`` columns), B and C (``groups * state_size`` columns each) from the given columns on.
     Either ``steps`` = (projection partial sums, first column of the raw step sizes, dt_bias, A_log, D) or ``fixed_decay``
-    (float32 ``[heads]``, step sizes one).  States of up to 128 rows.  ``scratch``, on a 16-byte boundary: see :func:`scan_chunks_scratch`."""
+    (float32 ``[heads]``, step sizes one).  States of up to 128 rows.  ``status``: the device status word.  ``scratch``, on a 16-byte boundary: see :func:`scan_chunks_scratch`."""
     for t, name in ((rows, "x/B/C"), (state, "recurrent state"), (y, "recurrence output"), (scratch, "scratch")):
         _need(t, torch.float32, name)
     _need_aligned(scratch, "scratch")
@@ -942,7 +945,7 @@ def scan_chunks(rows: torch.Tensor, x_col: int, b_col: int, c_col: int, state: t
     tokens, width = rows.shape
     if (state_size > CHUNK_MAX_ROWS or heads % groups or state.shape[1:] != (heads, head_dim, state_size) or y.shape != (tokens, heads * head_dim)
             or min(x_col, b_col, c_col) < 0 or x_col + heads * head_dim > width or max(b_col, c_col) + groups * state_size > width
-            or scratch.numel() < scan_chunks_scratch(tokens, sequences, heads, groups)[0]):
+            or scratch.numel() < scan_chunks_scratch(tokens, sequences, heads, groups, state_size)[0]):
         raise KernelError("scan_chunks: shapes do not fit the sizes")
     p, splits, stride, cols, dt_col, vectors = None, 0, 0, 0, 0, (None, None, None)
     if steps is not None:
@@ -957,10 +960,10 @@ def scan_chunks(rows: torch.Tensor, x_col: int, b_col: int, c_col: int, state: t
                 raise KernelError("scan_chunks: decays, biases and skips have a number per head")
     fn = _fn("recurrent_chunks", "tt_scan_chunks", [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_longlong, c_int, c_int, c_void_p, c_void_p,
                                                     c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
-                                                    c_int, c_int, c_int, c_int, c_void_p])
+                                                    c_int, c_int, c_int, c_int, c_void_p, c_void_p])
     _check(fn(rows.data_ptr(), width, x_col, b_col, c_col, p, splits, stride, cols, dt_col, *(None if t is None else t.data_ptr() for t in vectors),
               None if fixed_decay is None else fixed_decay.data_ptr(), state.data_ptr(), y.data_ptr(), scratch.data_ptr(), _ptr(cu), _ptr(slots), sequences,
-              chunk_slots(tokens, sequences), heads, groups, head_dim, state_size, sm_count(rows.device), _stream()), "scan_chunks", 2)
+              chunk_slots(tokens, sequences), heads, groups, head_dim, state_size, sm_count(rows.device), _ptr(status), _stream()), "scan_chunks", 2)
 
 
 def delta_chunks_scratch(n_tokens: int, sequences: int, heads: int, key_dim: int, value_dim: int) -> tuple[int]:

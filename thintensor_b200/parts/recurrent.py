@@ -111,14 +111,14 @@ def in_blocks(ctx) -> bool:
 
 
 def scan_chunks_pay(n_tokens: int, sequences: int, ctas: int, sms: int) -> bool:
-    """Whether a Mamba-2 or fixed-decay recurrence runs faster in chunks of 64 tokens than token by token.  A CTA of the walk over the
-    chunks (a sequence, head and 32 columns) has an SM to itself, so that every ``sms`` of them cost a round of equal length, while the kernels that go token by
-    token share the SMs evenly from twice as many CTAs on.  Kernel times, chunks against token by token (us, one B200, 148 SMs): 64 CTAs, one
-    sequence of 160 tokens 29 and 55; 256, four of 160 61 and 79; 320, five of 160 83 and 87, five of 800 309 and 423; 512, eight of 160
-    112 and 96, eight of 320 177 and 188 (32 of 320 with 64 x 64 states 140 and 135), eight of 640 330 and 370; 1,024, eight of 640 537 and
-    530, 16 of 700 637 and 579.  640 CTAs of five sequences of 800 tokens took 452 and 621, in rounds that are nearly full; the line stays at four rounds."""
+    """Whether a Mamba-2 or fixed-decay recurrence runs faster in chunks of 64 tokens than token by token.  The kernels that go token by token share
+    the SMs evenly from twice as many CTAs on; a CTA of the walk over the chunks has an SM to itself.  ``ctas``: of 32 columns.  Kernel times, chunks
+    against token by token (us, one B200, 148 SMs): 32 CTAs, 130 tokens 22 and 43; 64, one sequence of 64 tokens 25 and 25, of 130 29 and 47;
+    480, five of 200 104 and 130, of 840 296 and 519; 576, three of 400 141 and 244, of 1,400 405 and 946; 640, five of 400 195 and 322; 960, five of
+    170 132 and 146, of 400 269 and 328, of 840 501 and 696; 1,024, eight of 160 132 and 137.  More CTAs were not measured over the whole range and go
+    token by token, as do shorter prompts on more than three rounds of the SMs, whose gain is small."""
     each = n_tokens // sequences
-    return each >= 160 and (ctas <= 3 * sms or (each >= 400 and ctas <= 4 * sms))
+    return (each >= 128 and ctas <= 3 * sms) or (each >= 350 and 2 * ctas <= 13 * sms)
 
 
 def delta_chunks_pay(n_tokens: int, sequences: int, ctas: int, key_dim: int, sms: int) -> bool:
@@ -210,9 +210,9 @@ class Mamba2(Mixer):
         y = ctx.scratch("mamba2.y", (tokens, self.inner), torch.float32)
         dt_col = self.inner + self.channels
         if in_chunks(ctx, self.heads, self.head_dim, self.state):
-            scratch = ctx.scratch("chunks.scan", api.scan_chunks_scratch(tokens, ctx.sequences, self.heads, self.groups), torch.float32)
+            scratch = ctx.scratch("chunks.scan", api.scan_chunks_scratch(tokens, ctx.sequences, self.heads, self.groups, self.state), torch.float32)
             api.scan_chunks(xbc, 0, self.inner, self.inner + self.groups * self.state, recurrent, y, ctx.cu, ctx.slots, ctx.sequences, self.heads,
-                            self.head_dim, self.state, self.groups, scratch, steps=(proj, dt_col, self.dt_bias, self.a_log, self.d_skip))
+                            self.head_dim, self.state, self.groups, scratch, steps=(proj, dt_col, self.dt_bias, self.a_log, self.d_skip), status=ctx.status)
         else:
             api.mamba2_scan(xbc, proj, dt_col, self.dt_bias, self.a_log, self.d_skip, recurrent, y, ctx.cu, ctx.slots, ctx.sequences, self.heads,
                             self.head_dim, self.state, self.groups)
@@ -448,9 +448,9 @@ class DecayLinearAttention(Mixer):
         elif decay is not None:
             api.row_decay_scan(vkq, decay, recurrent, read, ctx.cu, ctx.slots, ctx.sequences, self.heads, self.key_dim, self.value_dim)
         elif self.chunks and in_chunks(ctx, self.heads, self.value_dim, self.key_dim):
-            scratch = ctx.scratch("chunks.scan", api.scan_chunks_scratch(tokens, ctx.sequences, self.heads, self.heads), torch.float32)
+            scratch = ctx.scratch("chunks.scan", api.scan_chunks_scratch(tokens, ctx.sequences, self.heads, self.heads, self.key_dim), torch.float32)
             api.scan_chunks(vkq, 0, self.v, self.v + self.qk, recurrent, read, ctx.cu, ctx.slots, ctx.sequences, self.heads, self.value_dim, self.key_dim,
-                            self.heads, scratch, fixed_decay=self.decays)
+                            self.heads, scratch, fixed_decay=self.decays, status=ctx.status)
         else:
             api.decay_scan(vkq, self.decays, recurrent, read, ctx.cu, ctx.slots, ctx.sequences, self.heads, self.key_dim, self.value_dim)
         return self.finish(ctx, proj, read)
