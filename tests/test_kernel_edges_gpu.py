@@ -250,6 +250,28 @@ def test_convolution_tiles_inside_and_across_sequences(taps, splits):
         torch.testing.assert_close(state[slot].double(), rows[rows.shape[0] - (taps - 1):], rtol=1e-6, atol=1e-6)
 
 
+@pytest.mark.parametrize("channels,col,extra", [(4, 0, 0), (132, 4, 8), (516, 0, 4), (1032, 8, 0)])
+@pytest.mark.parametrize("news", [[1, 2, 3, 7, 8, 9, 17], [5, 0, 0, 64, 1], [700]])
+def test_convolution_four_channels_a_thread(channels, col, extra, news):
+    """Four taps in 16-byte pieces: sequences shorter than the filter, tiles whole and in part, sequences without tokens; states moved on in the same launch."""
+    from thintensor_b200.kernels import api
+
+    tokens, taps, slot_ids = sum(news), 4, [(3 * i + 1) % 8 for i in range(len(news))]
+    cu = [sum(news[:i]) for i in range(len(news) + 1)]
+    proj, weight, bias = randn(1, tokens, col + channels + extra, seed=33), randn(channels, taps, seed=34), randn(channels, seed=35)
+    state = randn(8, taps - 1, channels, seed=36)
+    before = state.clone()
+    out = torch.full((tokens, channels), 7.0, device=DEV)
+    api.causal_conv(proj, col, channels, weight, bias, False, state, out, i32(cu), i32(slot_ids), len(news), tokens, False)
+    x = proj[0].double()[:, col:col + channels]
+    for s, slot in enumerate(slot_ids):
+        rows = torch.cat((before[slot].double(), x[cu[s]:cu[s + 1]]))
+        want = sum(rows[j:j + news[s]] * weight[:, j].double() for j in range(taps)) + bias.double()
+        torch.testing.assert_close(out[cu[s]:cu[s + 1]].double(), want, rtol=1e-5, atol=1e-5)        # four products in float32
+        assert torch.equal(state[slot].double(), rows[rows.shape[0] - (taps - 1):])
+    assert all(torch.equal(state[i], before[i]) for i in range(8) if i not in slot_ids)
+
+
 @pytest.mark.parametrize("heads,D,V,rotary,tokens", [(3, 128, 256, 128, 5), (2, 64, 20, 24, 1030), (2, 12, 8, 0, 3), (2, 10, 8, 4, 3), (1, 256, 4, 256, 2)])
 @pytest.mark.parametrize("activation", [False, True])
 def test_linear_attention_inputs_by_pieces(heads, D, V, rotary, tokens, activation):

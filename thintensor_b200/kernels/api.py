@@ -882,10 +882,11 @@ def causal_conv(proj: torch.Tensor, col_off: int, channels: int, weight: torch.T
     if col_off < 0 or col_off + channels > cols:
         raise KernelError("convolution: the channels lie outside the projection")
     fn = _fn("recurrent", "tt_causal_conv", [c_void_p, c_int, c_longlong, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p,
-                                             c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p])
+                                             c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p])
+    kernels = c_int(0)
     _check(fn(p, splits, stride, cols, col_off, channels, _ptr(weight), _ptr(bias), taps, 1 if activation else 0, _ptr(state),
               state.stride(0) if state.numel() else 0, _ptr(out), _ptr(cu), _ptr(slots), sequences, n_tokens, 1 if one_token_each else 0,
-              _stream()), "causal_conv", (0 if one_token_each else 1) + (1 if taps > 1 or one_token_each else 0))
+              ctypes.addressof(kernels), _stream()), "causal_conv", kernels.value)
 
 
 SCAN_FORMS = {"auto": 0, "narrow": 1, "wide": 2}
