@@ -8,6 +8,7 @@ another implementation: tensors that are not on a CUDA device are an error.
 from __future__ import annotations
 
 import ctypes
+import functools
 from ctypes import c_float, c_int, c_longlong, c_ulonglong, c_void_p
 from dataclasses import dataclass
 
@@ -37,18 +38,20 @@ def dtype_code(dtype: torch.dtype) -> int:
     raise KernelError(f"kernels take float32 or bfloat16, not {dtype}")
 
 
-def _ptr(t: torch.Tensor | None) -> c_void_p:
+# _ptr, _need and _need_columns, and the calls themselves, are native from the first call of an entry point on (csrc/host_calls.cpp): a
+# step of a small layer is bound by its host's calls (a differential layer of 40 tokens 93 -> 62 us, a latent one 125 -> 88, routed experts 76 -> 49).
+def _ptr(t: torch.Tensor | None) -> int:
     if t is None:
-        return c_void_p(0)
+        return 0
     if not t.is_cuda:
         raise KernelError("thintensor_b200 kernels run on CUDA tensors only; got a tensor on " + str(t.device))
-    return c_void_p(t.data_ptr())
+    return t.data_ptr()
 
 
-def _stream() -> c_void_p:
+def _stream() -> int:
     # the raw handle of torch's current stream on the current device (torch.cuda.current_stream()
     # builds a Stream object around the same number, at ten times the cost)
-    return c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 _launches = 0
@@ -156,13 +159,32 @@ class timed_classes:
         _timer, _label = None, None
 
 
-def _fn(lib: str, name: str, argtypes: list):
-    """The C entry point ``name`` of library ``lib`` (built and loaded at first use), with its prototype set."""
+_host = None               # the native module; False where it cannot be built
+_CTYPES = {"p": c_void_p, "i": c_int, "l": c_longlong, "u": c_ulonglong, "f": c_float}
+
+
+def _bind_host() -> None:
+    """Take the native module's checks and calls; without a C++ compiler or Python's headers ctypes makes the same calls, slower."""
+    global _host, _ptr, _need, _need_columns
+    module = build.host_calls()
+    if module is not None:
+        module.set_error(KernelError)
+        _ptr, _need, _need_columns = module.pointer, module.need, module.need_columns
+    _host = module or False
+
+
+def _fn(lib: str, name: str, signature: str):
+    """The C entry point ``name`` of library ``lib`` (built and loaded at first use).  ``signature``: a letter an argument, p pointer, i int,
+    l long long, u unsigned long long, f float."""
     fn = _functions.get(name)
     if fn is None:
+        if _host is None:
+            _bind_host()
         fn = getattr(build.load(lib), name)
-        fn.argtypes = argtypes
+        fn.argtypes = [_CTYPES[letter] for letter in signature]
         fn.restype = c_int
+        if _host:
+            fn = _host.Function(ctypes.cast(fn, c_void_p).value, signature, name)
         _functions[name] = fn
     if _timer is not None:
         return _timer.wrap(name, fn)
@@ -177,7 +199,7 @@ def embed_gather(table: torch.Tensor, tokens: torch.Tensor, residual: torch.Tens
     if not table.is_contiguous():
         raise KernelError("embedding table must be contiguous")
     n, hidden = tokens.numel(), table.shape[1]
-    fn = _fn("elementwise", "tt_embed_gather", [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_void_p, c_void_p])
+    fn = _fn("elementwise", "tt_embed_gather", "pippiiifpp")
     _check(fn(_ptr(table), dtype_code(table.dtype), _ptr(tokens), _ptr(residual), n, hidden, table.shape[0], scale, _ptr(status), _stream()), "embed_gather")
 
 
@@ -190,8 +212,7 @@ def embed_norm_gather(table: torch.Tensor, tokens: torch.Tensor, weight: torch.T
     n, hidden = tokens.numel(), table.shape[1]
     if not table.is_contiguous() or weight.numel() != hidden or tuple(residual.shape) != (n, hidden):
         raise KernelError("embed_norm_gather: shapes do not fit")
-    fn = _fn("elementwise", "tt_embed_norm_gather", [c_void_p, c_int, c_void_p, c_void_p, c_float, c_void_p, c_int, c_int, c_int, c_float, c_void_p,
-                                                     c_void_p])
+    fn = _fn("elementwise", "tt_embed_norm_gather", "pippfpiiifpp")
     _check(fn(_ptr(table), dtype_code(table.dtype), _ptr(tokens), _ptr(weight), eps, _ptr(residual), n, hidden, table.shape[0], scale, _ptr(status),
               _stream()), "embed_norm_gather")
 
@@ -206,8 +227,7 @@ def embed_position_gather(table: torch.Tensor, positions: torch.Tensor, tokens: 
     if positions.shape[1] != table.shape[1]:
         raise KernelError(f"the position table must have rows of {table.shape[1]} numbers, got {tuple(positions.shape)}")
     n, hidden = tokens.numel(), table.shape[1]
-    fn = _fn("elementwise", "tt_embed_position_gather", [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int,
-                                                         c_int, c_int, c_float, c_void_p, c_void_p])
+    fn = _fn("elementwise", "tt_embed_position_gather", "ppipppipiiiifpp")
     _check(fn(_ptr(table), _ptr(positions), dtype_code(table.dtype), _ptr(tokens), _ptr(cu), _ptr(len_before), sequences, _ptr(residual), n,
               hidden, table.shape[0], positions.shape[0], scale, _ptr(status), _stream()), "embed_position_gather")
 
@@ -226,8 +246,7 @@ def embed_pair_gather(table: torch.Tensor, pair_table: torch.Tensor, tokens: tor
     if pair_table.shape[0] != buckets + 1 or pair_table.shape[1] != table.shape[1]:
         raise KernelError(f"the pair table must be [{buckets + 1}, {table.shape[1]}], got {tuple(pair_table.shape)}")
     n, hidden = tokens.numel(), table.shape[1]
-    fn = _fn("elementwise", "tt_embed_pair_gather", [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
-                                                     c_int, c_int, c_int, c_int, c_longlong, c_longlong, c_float, c_void_p, c_void_p])
+    fn = _fn("elementwise", "tt_embed_pair_gather", "ppipppippiiiillfpp")
     _check(fn(_ptr(table), _ptr(pair_table), dtype_code(table.dtype), _ptr(tokens), _ptr(cu), _ptr(slots), sequences, _ptr(last_token),
               _ptr(residual), n, hidden, table.shape[0], buckets, mul_prev, mul_cur, scale, _ptr(status), _stream()), "embed_pair_gather")
 
@@ -243,7 +262,7 @@ def token_shift(x: torch.Tensor, mix: torch.Tensor, state: torch.Tensor, out: to
     tokens, hidden = x.shape
     if mix.numel() != hidden or state.shape[1] != hidden:
         raise KernelError("token_shift: weights or state do not fit the width")
-    fn = _fn("elementwise", "tt_token_shift", [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p])
+    fn = _fn("elementwise", "tt_token_shift", "pipppppiiip")
     _check(fn(_ptr(x), dtype_code(x.dtype), _ptr(mix), _ptr(state), _ptr(out), _ptr(cu), _ptr(slots), sequences, tokens, hidden, _stream()),
            "token_shift")
 
@@ -264,8 +283,7 @@ def token_shifts(x: torch.Tensor, mix: torch.Tensor, state: torch.Tensor, out: t
         raise KernelError("token_shifts: shapes do not fit")
     if not 1 <= blends <= SHIFT_BLENDS:
         raise KernelError(f"token_shifts makes 1 to {SHIFT_BLENDS} blends, not {blends}")
-    fn = _fn("elementwise", "tt_token_shifts", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int,
-                                                c_int, c_void_p])
+    fn = _fn("elementwise", "tt_token_shifts", "pipipplppiiip")
     _check(fn(_ptr(x), dtype_code(x.dtype), _ptr(mix), blends, _ptr(state), _ptr(out), out.stride(0), _ptr(cu), _ptr(slots), sequences, tokens,
               hidden, _stream()), "token_shifts")
 
@@ -303,8 +321,7 @@ def stream_norm(streams: torch.Tensor, delta: torch.Tensor | None, scale: float,
     n_rows = rows.numel() if rows is not None else tokens
     if tuple(out.shape) != (n_rows, hidden) or not out.is_contiguous():
         raise KernelError("stream_norm: the output does not fit")
-    fn = _fn("streams", "tt_stream_norm", [c_void_p, c_int, c_longlong, c_void_p, c_int, c_longlong, c_float, c_void_p, c_void_p, c_void_p, c_void_p,
-                                           c_int, c_void_p, c_float, c_float, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p])
+    fn = _fn("streams", "tt_stream_norm", "pilpilfppppipffpipiip")
     _check(fn(_ptr(streams), copies, tokens * hidden, _ptr(delta), splits, stride, scale, _ptr(gain), _ptr(mix), _ptr(write), _ptr(read),
               1 if spread else 0, _ptr(weight), weight_offset, eps, _ptr(out), dtype_code(out.dtype), _ptr(rows), n_rows, hidden, _stream()),
            "stream_norm")
@@ -328,7 +345,7 @@ def add_rmsnorm(residual: torch.Tensor, delta: torch.Tensor | None, weight: torc
     n_rows = rows.numel() if rows is not None else residual.shape[0]
     if rows is not None:
         _need(rows, torch.int32, "rows")
-    fn = _fn("elementwise", "tt_add_rmsnorm", [c_void_p, c_void_p, c_int, c_longlong, c_void_p, c_float, c_float, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p])
+    fn = _fn("elementwise", "tt_add_rmsnorm", "ppilpffpipiip")
     _check(fn(_ptr(residual), _ptr(delta), splits, stride, _ptr(weight), weight_offset, eps, _ptr(out), dtype_code(out.dtype), _ptr(rows), n_rows, hidden, _stream()), "add_rmsnorm")
 
 
@@ -366,8 +383,7 @@ def add_rmsnorm_chain(residual: torch.Tensor, delta: torch.Tensor | None, post_w
     n_rows = rows.numel() if rows is not None else residual.shape[0]
     if rows is not None:
         _need(rows, torch.int32, "rows")
-    fn = _fn("elementwise", "tt_add_rmsnorm_chain", [c_void_p, c_void_p, c_int, c_longlong, c_void_p, c_float, c_float, c_void_p, c_longlong, c_int,
-                                                     c_void_p, c_void_p, c_float, c_float, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p])
+    fn = _fn("elementwise", "tt_add_rmsnorm_chain", "ppilpffplippffpipiip")
     _check(fn(_ptr(residual), _ptr(delta), splits, stride, _ptr(post_weight), post_offset, post_eps, _ptr(results), result_stride, index,
               _ptr(depth_weights), _ptr(weight), weight_offset, eps, _ptr(out), dtype_code(out.dtype), _ptr(rows), n_rows, hidden, _stream()),
            "add_rmsnorm_chain")
@@ -391,7 +407,7 @@ def add_layernorm(residual: torch.Tensor, delta: torch.Tensor | None, weight: to
     n_rows = rows.numel() if rows is not None else residual.shape[0]
     if rows is not None:
         _need(rows, torch.int32, "rows")
-    fn = _fn("elementwise", "tt_add_layernorm", [c_void_p, c_void_p, c_int, c_longlong, c_void_p, c_void_p, c_float, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p])
+    fn = _fn("elementwise", "tt_add_layernorm", "ppilppfpipiip")
     _check(fn(_ptr(residual), _ptr(delta), splits, stride, _ptr(weight), _ptr(bias), eps, _ptr(out), dtype_code(out.dtype), _ptr(rows), n_rows, hidden, _stream()), "add_layernorm")
 
 
@@ -425,8 +441,7 @@ def add_norms(residual: torch.Tensor, a: torch.Tensor | None, b: torch.Tensor | 
     n_rows = rows.numel() if rows is not None else residual.shape[0]
     size = lambda t: (_ptr(t), 0 if t is None else t.shape[0], 0 if t is None else t.stride(0))
     w2, b2, o2 = second if second is not None else (None, None, None)
-    fn = _fn("elementwise", "tt_add_norms", [c_void_p, c_void_p, c_int, c_longlong, c_void_p, c_int, c_longlong, c_float, c_void_p, c_void_p, c_void_p,
-                                             c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_float, c_int, c_int, c_void_p, c_int, c_int, c_void_p])
+    fn = _fn("elementwise", "tt_add_norms", "ppilpilfpppppppffiipiip")
     _check(fn(_ptr(residual), *size(a), *size(b), scale, _ptr(addend), _ptr(weight), _ptr(bias), _ptr(out), _ptr(w2), _ptr(b2), _ptr(o2),
               weight_offset, eps, 1 if centered else 0, dtype_code(out.dtype), _ptr(rows), n_rows, hidden, _stream()), "add_norms")
 
@@ -473,10 +488,7 @@ def qk_norm_rope_append(proj: torch.Tensor, q_norm: torch.Tensor | None, k_norm:
         _need(where, torch.int32, "token positions")
         if tuple(cos_sin.shape) != (n_tokens, rotary_dim // 2, 2) or tuple(where.shape) != (n_tokens, 2):
             raise KernelError("the rope table does not fit the step")
-    fn = _fn("elementwise", "tt_qk_norm_rope_append", [c_void_p, c_int, c_longlong, c_int, c_void_p, c_void_p, c_float, c_void_p, c_int, c_int,
-                                                       c_float, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p,
-                                                       c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_float, c_int,
-                                                       c_int, c_void_p, c_void_p])
+    fn = _fn("elementwise", "tt_qk_norm_rope_append", "pilippfpiifpppipiippiiiiiiippifiipp")
     _check(fn(proj_ptr, proj_splits, proj_stride, proj_row, _ptr(q_norm), _ptr(k_norm), norm_eps, _ptr(inv_freq), rotary_dim,
               1 if interleaved else 0, attention_scaling, _ptr(q_out), _ptr(k_pool), _ptr(v_pool), dtype_code(q_out.dtype), _ptr(table),
               table.shape[1], k_pool.shape[0] if write else 0, _ptr(cu), _ptr(len_before), sequences, n_tokens, heads, kv_heads, head_dim,
@@ -499,8 +511,7 @@ def rope_append(qkv: torch.Tensor, inv_freq: torch.Tensor, rotary_dim: int, atte
         raise KernelError(f"qkv has {qkv.shape[-1]} columns, expected {cols}")
     if write and (k_pool.dtype != q_out.dtype or v_pool.dtype != q_out.dtype):
         raise KernelError("cache pools and activations must share a dtype")
-    fn = _fn("elementwise", "tt_rope_append", [c_void_p, c_int, c_longlong, c_void_p, c_int, c_float, c_void_p, c_void_p, c_void_p, c_int,
-                                               c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p])
+    fn = _fn("elementwise", "tt_rope_append", "pilpifpppipiippiiiiiipp")
     _check(fn(_ptr(qkv), qkv.shape[0], qkv.stride(0), _ptr(inv_freq), rotary_dim, attention_scaling, _ptr(q_out), _ptr(k_pool), _ptr(v_pool),
               dtype_code(q_out.dtype), _ptr(table), table.shape[1] if table is not None else 0,
               k_pool.shape[0] if write else 0, _ptr(cu), _ptr(len_before), sequences, n_tokens, heads, kv_heads, head_dim,
@@ -517,7 +528,7 @@ def rope_table(inv_freq: torch.Tensor, rotary_dim: int, cu: torch.Tensor, len_be
     half = rotary_dim // 2
     if tuple(cos_sin.shape) != (n_tokens, half, 2) or tuple(where.shape) != (n_tokens, 2) or inv_freq.numel() < half:
         raise KernelError(f"rope_table: cos_sin must be [{n_tokens}, {half}, 2] and where [{n_tokens}, 2]")
-    fn = _fn("elementwise", "tt_rope_table", [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p])
+    fn = _fn("elementwise", "tt_rope_table", "pippiippp")
     _check(fn(_ptr(inv_freq), half, _ptr(cu), _ptr(len_before), sequences, n_tokens, _ptr(cos_sin), _ptr(where), _stream()), "rope_table")
 
 
@@ -531,7 +542,7 @@ def swiglu(gate_up: torch.Tensor, act: torch.Tensor, activation: str = "silu") -
     if activation not in GATE_ACTIVATIONS:
         raise KernelError(f"gate activation {activation!r} is not one of {sorted(GATE_ACTIVATIONS)}")
     inter = gate_up.shape[-1] // 2
-    fn = _fn("elementwise", "tt_swiglu", [c_void_p, c_int, c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_void_p])
+    fn = _fn("elementwise", "tt_swiglu", "pilpiiiip")
     _check(fn(_ptr(gate_up), gate_up.shape[0], gate_up.stride(0), _ptr(act), dtype_code(act.dtype), gate_up.shape[1], inter,
               GATE_ACTIVATIONS[activation], _stream()), "swiglu")
 
@@ -545,7 +556,7 @@ def activation(x: torch.Tensor, act: torch.Tensor, activation: str = "gelu_tanh"
     _need(x, torch.float32, "the activation's input")
     if x.dim() != 3 or tuple(act.shape) != tuple(x.shape[1:]) or not act.is_contiguous():
         raise KernelError("activation: the output must be contiguous [tokens, inter] for an input [splits, tokens, inter]")
-    fn = _fn("elementwise", "tt_activation", [c_void_p, c_int, c_longlong, c_void_p, c_int, c_longlong, c_int, c_float, c_float, c_void_p])
+    fn = _fn("elementwise", "tt_activation", "pilpiliffp")
     _check(fn(_ptr(x), x.shape[0], x.stride(0), _ptr(act), dtype_code(act.dtype), act.numel(), UNARY_ACTIVATIONS[activation], a, c, _stream()),
            "activation")
 
@@ -560,15 +571,15 @@ def copy_int32(dst: torch.Tensor, src: torch.Tensor, extra: torch.Tensor | None 
         raise KernelError("copy_int32: sizes differ")
     if extra is not None and (extra.dtype != torch.int32 or extra.numel() != 1 or not extra.is_cuda):
         raise KernelError("copy_int32: the extra word must be one int32 on the device")
-    fn = _fn("elementwise", "tt_copy_int32", [c_void_p, c_void_p, c_int, c_void_p, c_void_p])
-    _check(fn(c_void_p(dst.data_ptr()), c_void_p(src.data_ptr()), src.numel(), _ptr(extra), _stream()), "copy_int32")
+    fn = _fn("elementwise", "tt_copy_int32", "ppipp")
+    _check(fn(dst.data_ptr(), src.data_ptr(), src.numel(), _ptr(extra), _stream()), "copy_int32")
 
 
 def advance_lengths(lengths: torch.Tensor, cu: torch.Tensor, sequences: int, counters: torch.Tensor | None = None) -> None:
     """lengths[b] += cu[b + 1] - cu[b] after a step; ``counters`` (int32, one per sequence), if given, go up by one."""
     if counters is not None:
         _need(counters, torch.int32, "step counters")
-    fn = _fn("elementwise", "tt_advance_lengths", [c_void_p, c_void_p, c_void_p, c_int, c_void_p])
+    fn = _fn("elementwise", "tt_advance_lengths", "pppip")
     _check(fn(_ptr(lengths), _ptr(cu), _ptr(counters), sequences, _stream()), "advance_lengths")
 
 
@@ -604,14 +615,12 @@ def attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, table
         _need(slopes, torch.float32, "slopes")
         if slopes.numel() != heads:
             raise KernelError(f"a slope per query head: {heads} numbers, got {slopes.numel()}")
-    g_ptr, g_splits, g_stride, g_row = c_void_p(0), 0, 0, 0
+    g_ptr, g_splits, g_stride, g_row = 0, 0, 0, 0
     if gate is not None:
         g_ptr, g_splits, g_stride, g_row, g_cols = _projection_view(gate)
         if g_cols != (heads if gate_per_head else heads * value_dim) or gate.shape[1] != n_tokens:
             raise KernelError("attention: the gate does not fit the heads")
-    fn = _fn("attention", "tt_attention", [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_int,
-                                           c_int, c_int, c_int, c_int, c_float, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
-                                           c_float, c_void_p, c_void_p, c_int, c_longlong, c_int, c_int, c_void_p])
+    fn = _fn("attention", "tt_attention", "pppipiippiiiiiifpiippppfppiliip")
     _check(fn(_ptr(q), _ptr(k_pool), _ptr(v_pool), dtype_code(q.dtype), _ptr(table), table.shape[1], k_pool.shape[0], _ptr(cu),
               _ptr(len_before), sequences, n_tokens, heads, kv_heads, head_dim, value_dim, scale, _ptr(sinks), window, splits, _ptr(out),
               _ptr(part_acc), _ptr(part_ml), _ptr(status), float(softcap or 0.0), _ptr(slopes), g_ptr, g_splits, g_stride, g_row,
@@ -635,9 +644,7 @@ def differential_attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.
         _need(part_ml, torch.float32, "partial maxima and sums")
         if part_acc.numel() < n_tokens * heads * splits * 2 * value_dim or part_ml.numel() < n_tokens * heads * splits * 4:
             raise KernelError("differential attention: scratch for the slices is too small")
-    fn = _fn("attention_forms", "tt_differential_attention", [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int,
-                                                              c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_float, c_int, c_void_p,
-                                                              c_void_p, c_void_p, c_void_p, c_void_p])
+    fn = _fn("attention_forms", "tt_differential_attention", "pppipiippiiiiiiffffippppp")
     _check(fn(_ptr(q), _ptr(k_pool), _ptr(v_pool), dtype_code(q.dtype), _ptr(table), table.shape[1], k_pool.shape[0], _ptr(cu), _ptr(len_before),
               sequences, n_tokens, heads, kv_heads, dim, value_dim, scale, lam, gain, eps, splits, _ptr(out), _ptr(part_acc), _ptr(part_ml),
               _ptr(status), _stream()), "differential_attention", 2 if splits > 1 else 1)
@@ -649,7 +656,7 @@ def attention_forms_on_tensor_cores(dtype: torch.dtype, differential: bool, head
     (sequence, key/value head) pair and not a (token, query head) row."""
     if dtype != torch.bfloat16:
         return False
-    fn = _fn("attention_forms", "tt_attention_forms_on_tensor_cores", [c_int, c_int, c_int, c_int, c_int])
+    fn = _fn("attention_forms", "tt_attention_forms_on_tensor_cores", "iiiii")
     return bool(fn(1 if differential else 0, heads, kv_heads, dim, value_dim))
 
 
@@ -662,8 +669,7 @@ def pool_blocks(k_pool: torch.Tensor, v_pool: torch.Tensor, table: torch.Tensor,
     ``most_blocks`` bounds the blocks one sequence can complete in the step."""
     if mean_k.dtype != k_pool.dtype or mean_v.dtype != k_pool.dtype:
         raise KernelError("the token cache and the coarser cache must share a dtype")
-    fn = _fn("attention_forms", "tt_pool_blocks", [c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int,
-                                                   c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p])
+    fn = _fn("attention_forms", "tt_pool_blocks", "ppipiipppiippiiiiiipp")
     _check(fn(_ptr(k_pool), _ptr(v_pool), dtype_code(k_pool.dtype), _ptr(table), table.shape[1], k_pool.shape[0], _ptr(mean_k), _ptr(mean_v),
               _ptr(mean_table), mean_table.shape[1], mean_k.shape[0], _ptr(cu), _ptr(len_before), sequences, most_blocks, kv_heads, head_dim,
               value_dim, every, _ptr(status), _stream()), "pool_blocks")
@@ -684,9 +690,7 @@ def pooled_window_attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch
         _need(part_ml, torch.float32, "partial maxima and sums")
         if part_acc.numel() < n_tokens * heads * splits * head_dim or part_ml.numel() < n_tokens * heads * splits * 2:
             raise KernelError("pooled window attention: scratch for the slices is too small")
-    fn = _fn("attention_forms", "tt_pooled_window_attention", [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p,
-                                                               c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
-                                                               c_float, c_float, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p])
+    fn = _fn("attention_forms", "tt_pooled_window_attention", "pppipiipppiiippiiiiiffiippppp")
     _check(fn(_ptr(q), _ptr(k_pool), _ptr(v_pool), dtype_code(q.dtype), _ptr(table), table.shape[1], k_pool.shape[0], _ptr(mean_k), _ptr(mean_v),
               _ptr(mean_table), mean_table.shape[1], mean_k.shape[0], every, _ptr(cu), _ptr(len_before), sequences, n_tokens, heads, kv_heads,
               head_dim, scale, cap, window, splits, _ptr(out), _ptr(part_acc), _ptr(part_ml), _ptr(status), _stream()),
@@ -751,9 +755,7 @@ def attention_mma(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, t
             raise KernelError(f"a slope per query head: {heads} numbers, got {slopes.numel()}")
     if shaped:
         tickets = None                  # the shaped instances combine slices in a cluster or through the merge kernel
-    fn = _fn("attention_mma", "tt_attention_mma", [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_int,
-                                                   c_int, c_int, c_int, c_float, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                                                   c_float, c_void_p, c_void_p])
+    fn = _fn("attention_mma", "tt_attention_mma", "ppppiippiiiiifiiippppppfpp")
     _check(fn(_ptr(q), _ptr(k_pool), _ptr(v_pool), _ptr(table), table.shape[1], k_pool.shape[0], _ptr(cu), _ptr(len_before), sequences,
               n_tokens, heads, kv_heads, head_dim, scale, window, splits, sequences if one_token_each else 0, _ptr(out), _ptr(part_acc),
               _ptr(part_ml), _ptr(tickets), _ptr(status), _ptr(sinks), float(softcap or 0.0), _ptr(slopes),
@@ -798,9 +800,7 @@ def attention_decode_rope(qkv: torch.Tensor, inv_freq: torch.Tensor, rotary_dim:
     if qkv.shape[-1] != cols or qkv.shape[1] != sequences:
         raise KernelError(f"qkv is {tuple(qkv.shape)}, expected [slices, {sequences}, {cols}]")
     _check_tickets(tickets, sequences, kv_heads)
-    fn = _fn("attention_mma", "tt_attention_decode_rope", [c_void_p, c_int, c_longlong, c_void_p, c_int, c_float, c_int, c_void_p, c_void_p,
-                                                           c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_int, c_int, c_float, c_int, c_int,
-                                                           c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p])
+    fn = _fn("attention_mma", "tt_attention_decode_rope", "pilpifipppiipiiiifiipppppp")
     _check(fn(_ptr(qkv), qkv.shape[0], qkv.stride(0), _ptr(inv_freq), rotary_dim, attention_scaling, 1 if write_cache else 0, _ptr(k_pool),
               _ptr(v_pool), _ptr(table), table.shape[1], k_pool.shape[0], _ptr(len_before), sequences, heads, kv_heads, head_dim, scale,
               window, splits, _ptr(out), _ptr(part_acc), _ptr(part_ml), _ptr(tickets), _ptr(status), _stream()), "attention_decode_rope",
@@ -829,7 +829,7 @@ def attention_tcgen05(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tenso
         _need(slopes, torch.float32, "slopes")
         if slopes.numel() != heads:
             raise KernelError(f"a slope per query head: {heads} numbers, got {slopes.numel()}")
-    g_ptr, g_splits, g_stride, g_row = c_void_p(0), 0, 0, 0
+    g_ptr, g_splits, g_stride, g_row = 0, 0, 0, 0
     if gate is not None:
         g_ptr, g_splits, g_stride, g_row, g_cols = _projection_view(gate)
         if g_cols != (heads if gate_per_head else heads * head_dim) or gate.shape[1] != n_tokens:
@@ -838,9 +838,7 @@ def attention_tcgen05(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tenso
         raise KernelError(f"the tcgen05 attention kernel does not take {q.dtype}, {heads}/{kv_heads} heads of size {head_dim}")
     if not (k_pool.dtype == v_pool.dtype == out.dtype == torch.bfloat16) or not q.is_contiguous():
         raise KernelError("queries, cache and output must all be contiguous bfloat16")
-    fn = _fn("attention_tcgen05", "tt_attention_tcgen05", [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int,
-                                                           c_int, c_int, c_int, c_int, c_float, c_void_p, c_int, c_void_p, c_void_p, c_float,
-                                                           c_void_p, c_void_p, c_int, c_longlong, c_int, c_int, c_int, c_void_p])
+    fn = _fn("attention_tcgen05", "tt_attention_tcgen05", "ppppiippiiiiifpippfppiliiip")
     _check(fn(_ptr(q), _ptr(k_pool), _ptr(v_pool), _ptr(table), table.shape[1], k_pool.shape[0], _ptr(cu), _ptr(len_before), sequences,
               n_tokens, heads, kv_heads, head_dim, scale, _ptr(sinks), window, _ptr(out), _ptr(status), float(softcap or 0.0), _ptr(slopes),
               g_ptr, g_splits, g_stride, g_row, 1 if gate_per_head else 0, out_dim, _stream()), "attention_tcgen05")
@@ -881,8 +879,7 @@ def causal_conv(proj: torch.Tensor, col_off: int, channels: int, weight: torch.T
     p, splits, stride, cols = _projection(proj)
     if col_off < 0 or col_off + channels > cols:
         raise KernelError("convolution: the channels lie outside the projection")
-    fn = _fn("recurrent", "tt_causal_conv", [c_void_p, c_int, c_longlong, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p,
-                                             c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p])
+    fn = _fn("recurrent", "tt_causal_conv", "piliiippiiplpppiiipp")
     kernels = c_int(0)
     _check(fn(p, splits, stride, cols, col_off, channels, _ptr(weight), _ptr(bias), taps, 1 if activation else 0, _ptr(state),
               state.stride(0) if state.numel() else 0, _ptr(out), _ptr(cu), _ptr(slots), sequences, n_tokens, 1 if one_token_each else 0,
@@ -906,8 +903,7 @@ def mamba2_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_col: int, dt_bias: tor
     if xbc.shape[1] != inner + 2 * groups * state_size or tuple(state.shape[1:]) != (heads, head_dim, state_size) or y.shape[1] != inner:
         raise KernelError("mamba2_scan: shapes do not fit the sizes")
     p, splits, stride, cols = _projection(proj)
-    fn = _fn("recurrent", "tt_mamba2_scan", [c_void_p, c_int, c_void_p, c_int, c_longlong, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
-                                             c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p])
+    fn = _fn("recurrent", "tt_mamba2_scan", "pipiliipppppppiiiiiip")
     _check(fn(_ptr(xbc), xbc.shape[1], p, splits, stride, cols, dt_col, _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), _ptr(state), _ptr(y),
               _ptr(cu), _ptr(slots), sequences, heads, head_dim, state_size, groups, SCAN_FORMS[form], _stream()), "mamba2_scan")
 
@@ -959,9 +955,7 @@ def scan_chunks(rows: torch.Tensor, x_col: int, b_col: int, c_col: int, state: t
             _need(t, torch.float32, "number per head")
             if t.numel() != heads:
                 raise KernelError("scan_chunks: decays, biases and skips have a number per head")
-    fn = _fn("recurrent_chunks", "tt_scan_chunks", [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_longlong, c_int, c_int, c_void_p, c_void_p,
-                                                    c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
-                                                    c_int, c_int, c_int, c_int, c_void_p, c_void_p])
+    fn = _fn("recurrent_chunks", "tt_scan_chunks", "piiiipiliipppppppppiiiiiiipp")
     _check(fn(rows.data_ptr(), width, x_col, b_col, c_col, p, splits, stride, cols, dt_col, *(None if t is None else t.data_ptr() for t in vectors),
               None if fixed_decay is None else fixed_decay.data_ptr(), state.data_ptr(), y.data_ptr(), scratch.data_ptr(), _ptr(cu), _ptr(slots), sequences,
               chunk_slots(tokens, sequences), heads, groups, head_dim, state_size, sm_count(rows.device), _ptr(status), _stream()), "scan_chunks", 2)
@@ -988,8 +982,7 @@ def delta_chunks(qkv: torch.Tensor, proj: torch.Tensor, b_col: int, a_col: int, 
     p, splits, stride, cols = _projection(proj)
     if min(b_col, a_col) < 0 or max(b_col, a_col) + heads > cols:
         raise KernelError("delta_chunks: write strengths or decays lie outside the projection")
-    fn = _fn("recurrent_chunks", "tt_delta_chunks", [c_void_p, c_int, c_void_p, c_int, c_longlong, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p,
-                                                     c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p])
+    fn = _fn("recurrent_chunks", "tt_delta_chunks", "pipiliiipppppppiiiiiiip")
     _check(fn(qkv.data_ptr(), qkv.shape[1], p, splits, stride, cols, b_col, a_col, dt_bias.data_ptr(), a_log.data_ptr(), state.data_ptr(), out.data_ptr(),
               scratch.data_ptr(), _ptr(cu), _ptr(slots), sequences, chunk_slots(tokens, sequences), heads, qk_heads, key_dim, value_dim, sm_count(qkv.device),
               _stream()), "delta_chunks", 2)
@@ -1015,8 +1008,7 @@ def delta_scan(qkv: torch.Tensor, proj: torch.Tensor, b_col: int, a_col: int, dt
             or out.shape[1] != heads * value_dim):
         raise KernelError("delta_scan: shapes do not fit the sizes")
     p, splits, stride, cols = _projection(proj)
-    fn = _fn("recurrent", "tt_delta_scan", [c_void_p, c_int, c_void_p, c_int, c_longlong, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
-                                            c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p])
+    fn = _fn("recurrent", "tt_delta_scan", "pipiliiipppppppiiiiiip")
     _check(fn(_ptr(qkv), qkv.shape[1], p, splits, stride, cols, b_col, a_col, _ptr(dt_bias), _ptr(a_log), _ptr(row_decay), _ptr(state), _ptr(out),
               _ptr(cu), _ptr(slots), sequences, heads, qk_heads, key_dim, value_dim, SCAN_FORMS[form], _stream()), "delta_scan")
 
@@ -1040,8 +1032,7 @@ def gated_group_norm(y: torch.Tensor, group: int, proj: torch.Tensor, gate_col: 
     p, splits, stride, cols = _projection(proj)
     if gate_col + width > cols:
         raise KernelError("gated_group_norm: the gate lies outside the projection")
-    fn = _fn("recurrent", "tt_gated_group_norm", [c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_longlong, c_int, c_int, c_void_p, c_int,
-                                                  c_float, c_int, c_void_p, c_int, c_int, c_void_p])
+    fn = _fn("recurrent", "tt_gated_group_norm", "piiipiliipifipiip")
     _check(fn(_ptr(y), tokens, width, group, p, splits, stride, cols, gate_col, _ptr(weight), weight.numel(), eps, 1 if gate_first else 0,
               _ptr(out), dtype_code(out.dtype), NORM_GATES[gate], _stream()), "gated_group_norm")
 
@@ -1061,9 +1052,8 @@ def linear_attention_prepare(proj: torch.Tensor, heads: int, key_dim: int, value
         if inv_freq.numel() < rotary_dim // 2:
             raise KernelError("linear_attention_prepare: too few inverse frequencies")
     p, splits, stride, cols = _projection(proj)
-    fn = _fn("recurrent", "tt_linear_attention_prepare", [c_void_p, c_int, c_longlong, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int,
-                                                          c_float, c_float, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p])
-    _check(fn(p, splits, stride, cols, heads, key_dim, value_dim, 1 if activation else 0, _ptr(inv_freq) if rotary_dim else c_void_p(0),
+    fn = _fn("recurrent", "tt_linear_attention_prepare", "piliiiiipiffpppiip")
+    _check(fn(p, splits, stride, cols, heads, key_dim, value_dim, 1 if activation else 0, _ptr(inv_freq) if rotary_dim else 0,
               rotary_dim, q_scale, k_scale, _ptr(vkq), _ptr(cu), _ptr(len_before), sequences, n_tokens, _stream()), "linear_attention_prepare")
 
 
@@ -1078,8 +1068,7 @@ def decay_scan(vkq: torch.Tensor, decay: torch.Tensor, state: torch.Tensor, out:
     if (vkq.shape[1] != heads * value_dim + 2 * heads * key_dim or tuple(state.shape[1:]) != (heads, value_dim, key_dim)
             or out.shape[1] != heads * value_dim or decay.numel() != heads):
         raise KernelError("decay_scan: shapes do not fit the sizes")
-    fn = _fn("recurrent", "tt_decay_scan", [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
-                                            c_int, c_void_p])
+    fn = _fn("recurrent", "tt_decay_scan", "pipppppiiiiip")
     _check(fn(_ptr(vkq), vkq.shape[1], _ptr(decay), _ptr(state), _ptr(out), _ptr(cu), _ptr(slots), sequences, heads, value_dim, key_dim,
               SCAN_FORMS[form], _stream()), "decay_scan")
 
@@ -1098,8 +1087,7 @@ def row_decay_scan(vkq: torch.Tensor, decay: torch.Tensor, state: torch.Tensor, 
     if (vkq.shape[1] != heads * value_dim + 2 * heads * key_dim or tuple(state.shape[1:]) != (heads, value_dim, key_dim)
             or out.shape[1] != heads * value_dim or tuple(decay.shape) != (vkq.shape[0], heads * key_dim)):
         raise KernelError("row_decay_scan: shapes do not fit the sizes")
-    fn = _fn("recurrent", "tt_row_decay_scan", [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
-                                                c_int, c_void_p])
+    fn = _fn("recurrent", "tt_row_decay_scan", "pippppppiiiiip")
     _check(fn(_ptr(vkq), vkq.shape[1], _ptr(decay), _ptr(bonus), _ptr(state), _ptr(out), _ptr(cu), _ptr(slots), sequences, heads, value_dim,
               key_dim, SCAN_FORMS[form], _stream()), "row_decay_scan")
 
@@ -1124,15 +1112,13 @@ def row_decay_blocks(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: t
     if (tuple(decay.shape) != (q.shape[0], heads * key_dim) or tuple(state.shape[1:]) != (heads, value_dim, key_dim)
             or tuple(out.shape) != (q.shape[0], heads * value_dim)):
         raise KernelError("row_decay_blocks: shapes do not fit the sizes")
-    p, splits, stride, cols, b_col = c_void_p(0), 0, 0, 0, 0
+    p, splits, stride, cols, b_col = 0, 0, 0, 0, 0
     if write is not None:
         p, splits, stride, cols = _projection(write[0])
         b_col = int(write[1])
         if b_col < 0 or b_col + heads > cols:
             raise KernelError("row_decay_blocks: the write strengths lie outside the projection")
-    fn = _fn("recurrent", "tt_row_decay_blocks", [c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_int, c_longlong, c_int,
-                                                  c_int, c_float, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
-                                                  c_int, c_void_p])
+    fn = _fn("recurrent", "tt_row_decay_blocks", "ppplpipiliifpppppiiiiip")
     _check(fn(_ptr(q), _ptr(k), _ptr(v), q.stride(0), _ptr(decay), 0 if write is None else 1, p, splits, stride, cols, b_col, q_scale,
               _ptr(bonus), _ptr(state), _ptr(out), _ptr(cu), _ptr(slots), sequences, heads, qk_heads, key_dim, value_dim, _stream()), "row_decay_blocks")
 
@@ -1176,10 +1162,9 @@ def low_rank(proj: torch.Tensor, products: list[LowRank]) -> None:
                 if t.numel() != count:
                     raise KernelError(f"low_rank: {name} has {t.numel()} numbers, needs {count}")
         args += [p.col, rank, n, LOW_RANK_KINDS[p.kind], p.per_head, 1 if p.tanh else 0, _ptr(p.weight), _ptr(p.bias), _ptr(p.a_log), 1.0 / p.tau, _ptr(p.out)]
-    types = [c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_float, c_void_p]
     if len(products) == 1:
-        args += [0, 0, 0, 0, 1, 0, c_void_p(0), c_void_p(0), c_void_p(0), 0.0, c_void_p(0)]
-    fn = _fn("recurrent", "tt_low_rank", [c_void_p, c_int, c_longlong, c_int, c_int, c_int, *types, *types, c_int, c_void_p])
+        args += [0, 0, 0, 0, 1, 0, 0, 0, 0, 0.0, 0]
+    fn = _fn("recurrent", "tt_low_rank", "piliii" + 2 * "iiiiiipppfp" + "ip")
     _check(fn(ptr, splits, stride, cols, len(products), dtype_code(products[0].weight.dtype), *args, tokens, _stream()), "low_rank")
 
 
@@ -1195,9 +1180,8 @@ def low_rank_inputs(proj: torch.Tensor, columns: list[tuple[int, torch.Tensor, b
             raise KernelError("low_rank_inputs: shapes do not fit")
         args += [col, out.shape[1], 1 if tanh else 0, _ptr(out)]
     if len(columns) == 1:
-        args += [0, 0, 0, c_void_p(0)]
-    fn = _fn("recurrent", "tt_low_rank_inputs", [c_void_p, c_int, c_longlong, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_int,
-                                                 c_int, c_void_p])
+        args += [0, 0, 0, 0]
+    fn = _fn("recurrent", "tt_low_rank_inputs", "piliiiipiiipiip")
     _check(fn(ptr, splits, stride, cols, *args, dtype_code(columns[0][1].dtype), proj.shape[1], _stream()), "low_rank_inputs")
 
 
@@ -1211,7 +1195,7 @@ def low_rank_finish(z: torch.Tensor, kind: str, bias: torch.Tensor, out: torch.T
             _need(t, torch.float32, name)
     if kind == "plain" or bias.numel() != n or tuple(out.shape) != (z.shape[1], n) or (a_log is not None and a_log.numel() != -(-n // per_head)):
         raise KernelError("low_rank_finish: shapes do not fit")
-    fn = _fn("recurrent", "tt_low_rank_finish", [c_void_p, c_int, c_longlong, c_int, c_int, c_int, c_void_p, c_void_p, c_float, c_void_p, c_int, c_void_p])
+    fn = _fn("recurrent", "tt_low_rank_finish", "piliiippfpip")
     _check(fn(ptr, splits, stride, n, LOW_RANK_KINDS[kind], per_head, _ptr(bias), _ptr(a_log), 1.0 / tau, _ptr(out), z.shape[1], _stream()),
            "low_rank_finish")
 
@@ -1222,7 +1206,7 @@ def weighted_pair(a: torch.Tensor, wa: float, b: torch.Tensor, wb: float, out: t
         _need(t, torch.float32, name)
     if a.shape[1:] != b.shape[1:] or out.numel() != a[0].numel():
         raise KernelError("weighted_pair: shapes differ")
-    fn = _fn("recurrent", "tt_weighted_pair", [c_void_p, c_int, c_longlong, c_float, c_void_p, c_int, c_longlong, c_float, c_void_p, c_longlong, c_void_p])
+    fn = _fn("recurrent", "tt_weighted_pair", "pilfpilfplp")
     _check(fn(_ptr(a), a.shape[0], a.stride(0), wa, _ptr(b), b.shape[0], b.stride(0), wb, _ptr(out), out.numel(), _stream()), "weighted_pair")
 
 
@@ -1255,9 +1239,7 @@ def latent_prepare(down: torch.Tensor, q_rank: int, rank: int, rot: int, q_weigh
         raise KernelError("latent_prepare: the pool must be [blocks, 1, 64, rank + rot] in the activations' dtype")
     if (cols + 32) * 4 > 48 * 1024:
         raise KernelError(f"latent_prepare: {cols} projected numbers per token are more than the kernel stages")
-    fn = _fn("latent_attention", "tt_latent_prepare", [c_void_p, c_int, c_longlong, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_float,
-                                                       c_void_p, c_int, c_int, c_float, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int,
-                                                       c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p])
+    fn = _fn("latent_attention", "tt_latent_prepare", "piliiiippfpiifpipipiippiipip")
     code = dtype_code(q_latent.dtype if q_rank else pool.dtype)
     _check(fn(p, splits, stride, row_stride, q_rank, rank, rot, _ptr(q_weight), _ptr(kv_weight), eps, _ptr(inv_freq), rotary_dim,
               1 if interleaved else 0, float(rot_scale), _ptr(q_latent), code,
@@ -1292,7 +1274,7 @@ def latent_attention(q: torch.Tensor, w_key: torch.Tensor, w_value: torch.Tensor
         raise KernelError(f"latent attention takes latents of up to {LATENT_MAX_RANK}, rows of up to {LATENT_MAX_ROW} and "
                           f"{LATENT_MAX_DIM} unrotated numbers per head; got {rank}, {rank + rot}, {dim}")
     p, q_splits, q_stride, q_row, q_cols = _projection_view(q)
-    g_ptr, g_splits, g_stride, g_row, g_cols = c_void_p(0), 0, 0, 0, 0
+    g_ptr, g_splits, g_stride, g_row, g_cols = 0, 0, 0, 0, 0
     if gate is not None:
         g_ptr, g_splits, g_stride, g_row, g_cols = _projection_view(gate)
         if g_cols not in (heads, heads * vdim) or gate.shape[1] != n_tokens:
@@ -1309,10 +1291,7 @@ def latent_attention(q: torch.Tensor, w_key: torch.Tensor, w_value: torch.Tensor
     if (absorbed.numel() < n_tokens * heads * (rank + rot) or part_acc.numel() < n_tokens * heads * splits * rank
             or part_ml.numel() < n_tokens * heads * splits * 2):
         raise KernelError("latent_attention: scratch memory is too small")
-    fn = _fn("latent_attention", "tt_latent_attention", [c_void_p, c_int, c_longlong, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p,
-                                                         c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
-                                                         c_void_p, c_int, c_int, c_float, c_float, c_int, c_int, c_void_p, c_void_p, c_void_p,
-                                                         c_void_p, c_int, c_void_p, c_int, c_longlong, c_int, c_int, c_void_p, c_void_p])
+    fn = _fn("latent_attention", "tt_latent_attention", "pilippipipiippiiiiiiipiiffiippppipiliipp")
     _check(fn(p, q_splits, q_stride, q_row, _ptr(w_key), _ptr(w_value), dtype_code(w_key.dtype), _ptr(pool), dtype_code(out.dtype), _ptr(table),
               table.shape[1], pool.shape[0], _ptr(cu), _ptr(len_before), sequences, n_tokens, heads, dim, rot, vdim, rank, _ptr(inv_freq),
               rotary_dim, 1 if interleaved else 0, float(rot_scale), scale, window, splits, _ptr(out), _ptr(absorbed), _ptr(part_acc),
@@ -1351,11 +1330,10 @@ def latent_expand(pool: torch.Tensor, table: torch.Tensor, cu: torch.Tensor, len
             or tuple(keys.shape[:3]) != (bound_blocks, heads, BLOCK_TOKENS) or keys.shape[3] < dim + rot or not (pool.dtype == x.dtype == keys.dtype)
             or tuple(pool.shape[1:]) != (1, BLOCK_TOKENS, rank + rot) or not x.is_contiguous() or not keys.is_contiguous()):
         raise KernelError("latent_expand: shapes do not fit the sizes")
-    fn = _fn("latent_attention", "tt_latent_expand_plan", [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p])
+    fn = _fn("latent_attention", "tt_latent_expand_plan", "ppiiiipppp")
     _check(fn(_ptr(cu), _ptr(len_before), sequences, window, table.shape[1], bound_blocks, _ptr(plan), _ptr(table_tmp), _ptr(status), _stream()),
            "latent_expand_plan")
-    fn = _fn("latent_attention", "tt_latent_gather", [c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int,
-                                                      c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p])
+    fn = _fn("latent_attention", "tt_latent_gather", "pipiippipiiiiiippp")
     _check(fn(_ptr(pool), dtype_code(pool.dtype), _ptr(table), table.shape[1], pool.shape[0], _ptr(cu), _ptr(len_before), sequences, _ptr(plan),
               bound_blocks, heads, dim, rot, rank, keys.shape[3], _ptr(x), _ptr(keys), _stream()), "latent_gather")
 
@@ -1371,8 +1349,7 @@ def latent_scatter(y: torch.Tensor, heads: int, dim: int, rot: int, vdim: int, k
             or keys.shape[3] < max(dim + rot, vdim) or tuple(values.shape) != (blocks, heads, keys.shape[3], BLOCK_TOKENS) or keys.dtype != values.dtype
             or not keys.is_contiguous() or not values.is_contiguous()):
         raise KernelError("latent_scatter: shapes do not fit the sizes")
-    fn = _fn("latent_attention", "tt_latent_scatter", [c_void_p, c_int, c_longlong, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int,
-                                                       c_void_p])
+    fn = _fn("latent_attention", "tt_latent_scatter", "piliiiiippip")
     _check(fn(p, splits, stride, blocks, heads, dim, keys.shape[3], vdim, _ptr(keys), _ptr(values), dtype_code(keys.dtype), _stream()), "latent_scatter")
 
 
@@ -1388,8 +1365,7 @@ def latent_queries(q: torch.Tensor, heads: int, dim: int, rot: int, inv_freq: to
     size = out.shape[1] // heads
     if cols != heads * (dim + rot) or tuple(out.shape) != (n_tokens, heads * size) or size < dim + rot or not out.is_contiguous():
         raise KernelError("latent_queries: shapes do not fit the sizes")
-    fn = _fn("latent_attention", "tt_latent_queries", [c_void_p, c_int, c_longlong, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int, c_float,
-                                                       c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p])
+    fn = _fn("latent_attention", "tt_latent_queries", "piliiiiipiifppiipip")
     _check(fn(p, splits, stride, q_row, heads, dim, rot, size, _ptr(inv_freq), rotary_dim, 1 if interleaved else 0, float(rot_scale), _ptr(cu),
               _ptr(len_before), sequences, n_tokens, _ptr(out), dtype_code(out.dtype), _stream()), "latent_queries")
 
@@ -1401,12 +1377,12 @@ def add_narrow(residual: torch.Tensor, delta: torch.Tensor | None, out: torch.Te
     _need(residual, torch.float32, "residual")
     if tuple(out.shape) != tuple(residual.shape) or not out.is_contiguous():
         raise KernelError("add_narrow: the output has the stream's shape")
-    p, splits, stride = c_void_p(0), 0, 0
+    p, splits, stride = 0, 0, 0
     if delta is not None:
         p, splits, stride, cols = _projection(delta)
         if tuple(delta.shape[1:]) != tuple(residual.shape):
             raise KernelError("add_narrow: the delta does not fit the stream")
-    fn = _fn("elementwise", "tt_add_narrow", [c_void_p, c_void_p, c_int, c_longlong, c_void_p, c_int, c_longlong, c_void_p])
+    fn = _fn("elementwise", "tt_add_narrow", "ppilpilp")
     _check(fn(_ptr(residual), p, splits, stride, _ptr(out), dtype_code(out.dtype), residual.numel(), _stream()), "add_narrow")
 
 
@@ -1419,8 +1395,7 @@ def token_side_gate(x: torch.Tensor, table: torch.Tensor, col_off: int, tokens: 
         raise KernelError("token_side_gate: shapes do not fit")
     if col_off < 0 or col_off + dim > table.shape[1]:
         raise KernelError("token_side_gate: the slice lies outside the table's rows")
-    fn = _fn("elementwise", "tt_token_side_gate", [c_void_p, c_int, c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int,
-                                                   c_void_p, c_int, c_void_p, c_void_p])
+    fn = _fn("elementwise", "tt_token_side_gate", "pilpiiiipiipipp")
     _check(fn(p, splits, stride, _ptr(table), dtype_code(table.dtype), table.shape[0], table.shape[1], col_off, _ptr(tokens), n, dim,
               _ptr(out), dtype_code(out.dtype), _ptr(status), _stream()), "token_side_gate")
 
@@ -1433,7 +1408,7 @@ def sigmoid_gate(y: torch.Tensor, gate: torch.Tensor, head_width: int = 0) -> No
         raise KernelError("sigmoid_gate: shapes do not fit")
     if g_cols != (y.shape[1] // head_width if head_width > 0 else y.shape[1]):
         raise KernelError("sigmoid_gate: the gate does not fit the columns")
-    fn = _fn("elementwise", "tt_sigmoid_gate", [c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_longlong, c_int, c_int, c_void_p])
+    fn = _fn("elementwise", "tt_sigmoid_gate", "piiipiliip")
     _check(fn(_ptr(y), dtype_code(y.dtype), y.shape[0], y.shape[1], g_ptr, g_splits, g_stride, g_row, int(head_width), _stream()), "sigmoid_gate")
 
 
@@ -1481,8 +1456,7 @@ def route_topk(logits: torch.Tensor, top: int, groups: int, keep: int, gates: to
                           f"{experts} experts, {groups} groups of which {keep} stay, top {top}")
     if tuple(gates.shape) != (tokens, experts + extra) or tuple(chosen.shape) != (tokens, top) or tuple(weights.shape) != (tokens, top):
         raise KernelError("route_topk: outputs do not fit the sizes")
-    fn = _fn("routing", "tt_route_topk", [c_void_p, c_int, c_longlong, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p,
-                                          c_int, c_void_p, c_int, c_int, c_int, c_float, c_void_p])
+    fn = _fn("routing", "tt_route_topk", "piliiiiipppipiiifp")
     _check(fn(p, splits, stride, tokens, experts, top, groups, keep, _ptr(gates), _ptr(chosen), _ptr(weights), *options, _stream()),
            "route_topk")
 
@@ -1508,8 +1482,7 @@ def route_rows(x: torch.Tensor, w: torch.Tensor, top: int, groups: int, keep: in
                           f"{experts} experts, {groups} groups of which {keep} stay, top {top}")
     if tuple(gates.shape) != (tokens, experts + extra) or tuple(chosen.shape) != (tokens, top) or tuple(weights.shape) != (tokens, top):
         raise KernelError("route_rows: outputs do not fit the sizes")
-    fn = _fn("routing", "tt_route_rows", [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
-                                          c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_float, c_int, c_void_p])
+    fn = _fn("routing", "tt_route_rows", "pipiiiiiiipppipiiifip")
     _check(fn(_ptr(x), dtype_code(x.dtype), _ptr(w), dtype_code(w.dtype), hidden, tokens, experts, top, groups, keep, _ptr(gates),
               _ptr(chosen), _ptr(weights), *options, sm_count(x.device), _stream()), "route_rows")
 
@@ -1533,7 +1506,7 @@ def scale_expert_columns(act: torch.Tensor, width: int, gates: torch.Tensor, exp
         raise KernelError("scale_expert_columns: the activations do not fit the gates")
     if experts > columns or (shared_width and experts >= columns):
         raise KernelError("scale_expert_columns: too few gates a token")
-    fn = _fn("routing", "tt_scale_expert_columns", [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int, c_void_p])
+    fn = _fn("routing", "tt_scale_expert_columns", "piiiiipiip")
     _check(fn(_ptr(act), dtype_code(act.dtype), tokens, act.stride(0), width, experts, _ptr(gates), columns, int(shared_width), _stream()),
            "scale_expert_columns")
 
@@ -1559,8 +1532,7 @@ def expert_activation(gate_up: torch.Tensor, act: torch.Tensor, experts: int, wi
         raise KernelError("expert_activation: shapes do not fit the sizes")
     if gates is not None and gates.shape[1] < experts + (1 if shared_gated else 0):
         raise KernelError("expert_activation: too few gates a token")
-    fn = _fn("routing", "tt_expert_activation", [c_void_p, c_int, c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_float,
-                                                 c_float, c_void_p, c_int, c_int, c_void_p])
+    fn = _fn("routing", "tt_expert_activation", "pilpiiiiifffpiip")
     _check(fn(p, splits, stride, _ptr(act), dtype_code(act.dtype), tokens, experts, width, shared_width, float(limit or 0.0),
               float(shared_limit or 0.0), float(alpha), _ptr(gates), 0 if gates is None else gates.shape[1], 1 if shared_gated else 0, _stream()),
            "expert_activation")
@@ -1577,8 +1549,7 @@ def expert_unary_activation(up: torch.Tensor, act: torch.Tensor, width: int, act
         raise KernelError("expert_unary_activation: shapes do not fit the sizes")
     if activation not in UNARY_ACTIVATIONS or activation == "xielu":
         raise KernelError(f"expert_unary_activation: {activation!r} is not an activation without parameters")
-    fn = _fn("routing", "tt_expert_unary_activation", [c_void_p, c_int, c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int,
-                                                       c_void_p])
+    fn = _fn("routing", "tt_expert_unary_activation", "pilpiiiiipip")
     _check(fn(p, splits, stride, _ptr(act), dtype_code(act.dtype), tokens, experts, width, UNARY_ACTIVATIONS[activation], _ptr(gates),
               gates.shape[1], _stream()), "expert_unary_activation")
 
@@ -1596,8 +1567,7 @@ def gemm_simt(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None, out: 
         raise KernelError(f"gemm shapes do not fit: x {tuple(x.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}")
     if bias is not None:
         _need(bias, torch.float32, "bias")
-    fn = _fn("gemm_simt", "tt_gemm_simt", [c_void_p, c_int, c_longlong, c_void_p, c_int, c_longlong, c_void_p, c_void_p, c_longlong,
-                                           c_longlong, c_int, c_int, c_int, c_int, c_int, c_void_p])
+    fn = _fn("gemm_simt", "tt_gemm_simt", "pilpilpplliiiiip")
     _check(fn(_ptr(x), dtype_code(x.dtype), x.stride(0), _ptr(w), dtype_code(w.dtype), w.stride(0), _ptr(bias), _ptr(out), out.stride(1),
               out.stride(0), m, n, k, out.shape[0], sm_count(x.device), _stream()), "gemm_simt")
 
@@ -1637,7 +1607,7 @@ def argmax_rows(logits: torch.Tensor, out: torch.Tensor) -> None:
         count = max(rows, 256) * 32
         scratch = (torch.empty(count, dtype=torch.float32, device=logits.device), torch.empty(count, dtype=torch.int32, device=logits.device))
         _argmax_scratch[logits.device] = scratch
-    fn = _fn("sampling", "tt_argmax_rows", [c_void_p, c_longlong, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p])
+    fn = _fn("sampling", "tt_argmax_rows", "pliipppp")
     two_stage = logits.shape[1] >= 8192
     _check(fn(_ptr(logits), logits.stride(0), rows, logits.shape[1], _ptr(out), _ptr(scratch[0]), _ptr(scratch[1]), _stream()),
            "argmax_rows", 2 if two_stage else 1)
@@ -1649,7 +1619,7 @@ def sample_rows(logits: torch.Tensor, temperature: float, top_k: int, top_p: flo
     _need(request, torch.int32, "request ids")
     _need(step, torch.int32, "step ids")
     _need(out, torch.int32, "token output")
-    fn = _fn("sampling", "tt_sample_rows", [c_void_p, c_longlong, c_int, c_int, c_float, c_int, c_float, c_ulonglong, c_void_p, c_void_p, c_void_p, c_void_p])
+    fn = _fn("sampling", "tt_sample_rows", "pliififupppp")
     _check(fn(_ptr(logits), logits.stride(0), logits.shape[0], logits.shape[1], temperature, top_k, top_p, seed & ((1 << 64) - 1),
               _ptr(request), _ptr(step), _ptr(out), _stream()), "sample_rows")
 
@@ -1662,7 +1632,9 @@ def sm_count(device: torch.device | int | None = None) -> int:
     """Streaming multiprocessors of a CUDA device (the current one by default), asked of the device
     once: it sizes the k-slices of few-token products and the key slices of decode attention, which
     the launchers in C++ size from the same attribute."""
-    index = torch.cuda.current_device() if device is None else (device if isinstance(device, int) else (device.index if device.index is not None else torch.cuda.current_device()))
+    index = device if isinstance(device, int) else None if device is None else device.index
+    if index is None:
+        index = torch._C._cuda_getDevice() if torch.cuda.is_initialized() else torch.cuda.current_device()
     count = _sm_counts.get(index)
     if count is None:
         count = _sm_counts[index] = int(torch.cuda.get_device_properties(index).multi_processor_count)
@@ -1675,6 +1647,8 @@ SKINNY_TOKENS = 128         # up to this many tokens the weights go on the 128-r
 def gemm_tcgen05_usable(x: torch.Tensor, w: torch.Tensor) -> bool:
     """TMA needs 16-byte aligned bases and row strides, i.e. k and both leading
     dimensions must be multiples of 8 bfloat16 numbers."""
+    if _host:
+        return _host.tiled_operands(x, w)
     return (x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.shape[1] % 8 == 0 and x.stride(0) % 8 == 0
             and w.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and x.stride(1) == 1 and w.stride(1) == 1)
 
@@ -1691,7 +1665,11 @@ def gemm_tcgen05_splits(tokens: int, features: int, k: int, sms: int | None = No
     one CTA per SM: as many slices as keep its work items within one round of the SMs (a
     512-token prompt has 32 tiles in the 1B shape's output projection), none of them empty.
     ``sms``: the device's multiprocessors (asked of the current device when not given)."""
-    sms = sm_count() if sms is None else sms
+    return _gemm_tcgen05_splits(tokens, features, k, sm_count() if sms is None else sms)
+
+
+@functools.lru_cache(maxsize=4096)
+def _gemm_tcgen05_splits(tokens: int, features: int, k: int, sms: int) -> int:
     k_blocks = -(-k // 64)
     if tokens > SKINNY_TOKENS and -(-tokens // 128) * -(-features // 256) >= PERSISTENT_TILES:
         if tokens >= PAIR_TOKENS:
@@ -1722,7 +1700,11 @@ def gemm_tcgen05_accumulate_pays(tokens: int, features: int, k: int, sms: int | 
     projections, whole prefill: 2,048 tokens 3.98 -> 3.91 ms, 4,096 tokens 8.62 -> 8.51).  Other widths add from
     registers after reading the old values, which pays only where every CTA (or CTA pair) has at least two tiles, so
     that a tile's epilogue runs under the next tile's products."""
-    sms = sm_count() if sms is None else sms
+    return _gemm_tcgen05_accumulate_pays(tokens, features, k, sm_count() if sms is None else sms)
+
+
+@functools.lru_cache(maxsize=4096)
+def _gemm_tcgen05_accumulate_pays(tokens: int, features: int, k: int, sms: int) -> bool:
     if not gemm_tcgen05_accumulates(tokens, features, k, sms):
         return False
     if features % 4 == 0:
@@ -1770,8 +1752,7 @@ def gemm_tcgen05(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None, ou
         _need(bias, torch.float32, "bias")
     if shares is not None and (shares.dtype != torch.int32 or not shares.is_contiguous()):
         raise KernelError("the shares of a tcgen05 gemm must be contiguous int32")
-    fn = _fn("gemm_tcgen05", "tt_gemm_tcgen05", [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_longlong, c_longlong,
-                                                 c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_longlong])
+    fn = _fn("gemm_tcgen05", "tt_gemm_tcgen05", "plplpplliiiiipppl")
     _check(fn(_ptr(x), x.stride(0), _ptr(w), w.stride(0), _ptr(bias), _ptr(out), out.stride(1), out.stride(0), tokens, features, k,
               out.shape[0], 2 if accumulate else 0, _ptr(status), _stream(), _ptr(shares), 0 if shares is None else shares.numel() * 4),
            "gemm_tcgen05")
@@ -1797,8 +1778,7 @@ def gemm_tcgen05_groups(x: torch.Tensor, w: torch.Tensor, group_features: int, o
         raise KernelError(f"grouped tcgen05 gemm cannot take x {tuple(x.shape)} / w {tuple(w.shape)} / out {tuple(out.shape)} in groups of {group_features}")
     if out.shape[0] > -(-k // 64):
         raise KernelError(f"{out.shape[0]} k-slices for k = {k}: a slice needs at least one block of 64")
-    fn = _fn("gemm_tcgen05", "tt_gemm_tcgen05_groups", [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_longlong, c_int, c_int,
-                                                        c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_longlong])
+    fn = _fn("gemm_tcgen05", "tt_gemm_tcgen05_groups", "plplplliiiiipppl")
     _check(fn(_ptr(x), x.stride(1), _ptr(w), w.stride(0), _ptr(out), out.stride(1), out.stride(0), tokens, features, k, out.shape[0],
               group_features, _ptr(status), _stream(), _ptr(shares), 0 if shares is None else shares.numel() * 4), "gemm_tcgen05_groups")
 
@@ -1833,9 +1813,7 @@ def gemm_tcgen05_qkv_rope(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor |
     _need(where, torch.int32, "token positions")
     if tuple(cos_sin.shape) != (tokens, head_dim // 2, 2) or tuple(where.shape) != (tokens, 2):
         raise KernelError("qkv product: the rope table does not fit the step")
-    fn = _fn("gemm_tcgen05", "tt_gemm_tcgen05_qkv_rope", [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_int, c_int, c_void_p, c_void_p,
-                                                          c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float,
-                                                          c_void_p, c_void_p])
+    fn = _fn("gemm_tcgen05", "tt_gemm_tcgen05_qkv_rope", "plplpiippppppiiiiifpp")
     code = fn(_ptr(x), x.stride(0), _ptr(w), w.stride(0), _ptr(bias), tokens, k, _ptr(q_out), _ptr(k_pool), _ptr(v_pool), _ptr(cos_sin),
               _ptr(where), _ptr(table), table.shape[1], k_pool.shape[0], heads, kv_heads, head_dim, attention_scaling, _ptr(status), _stream())
     if code < 0:
@@ -1872,8 +1850,7 @@ def gemm_tcgen05_swiglu(x: torch.Tensor, w: torch.Tensor, act: torch.Tensor, sta
     inter = w.shape[0] // 2
     if not gemm_tcgen05_usable(x, w) or w.shape[1] != k or tuple(act.shape) != (tokens, inter):
         raise KernelError(f"tcgen05 swiglu gemm cannot take x {tuple(x.shape)} / w {tuple(w.shape)} / act {tuple(act.shape)}")
-    fn = _fn("gemm_tcgen05", "tt_gemm_tcgen05", [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_longlong, c_longlong,
-                                                 c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_longlong])
+    fn = _fn("gemm_tcgen05", "tt_gemm_tcgen05", "plplpplliiiiipppl")
     _check(fn(_ptr(x), x.stride(0), _ptr(w), w.stride(0), _ptr(None), _ptr(act), act.stride(0), 0, tokens, inter, k, 1,
               1 + 16 * GATE_ACTIVATIONS[activation], _ptr(status), _stream(), _ptr(None), 0), "gemm_tcgen05_swiglu")
 
@@ -1898,8 +1875,7 @@ def gemm_tcgen05_unary(x: torch.Tensor, w: torch.Tensor, act: torch.Tensor, stat
         _need(scales, torch.float32, "factors")
         if scales.shape[0] != tokens or scales.shape[1] * width < features:
             raise KernelError("gemm_tcgen05_unary: the factors do not fit the product")
-    fn = _fn("gemm_tcgen05", "tt_gemm_tcgen05_unary", [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_int, c_int, c_int,
-                                                       c_void_p, c_int, c_int, c_void_p, c_void_p])
+    fn = _fn("gemm_tcgen05", "tt_gemm_tcgen05_unary", "plplpliiiipiipp")
     _check(fn(_ptr(x), x.stride(0), _ptr(w), w.stride(0), _ptr(act), act.stride(0), tokens, features, k, UNARY_ACTIVATIONS[activation],
               _ptr(scales), 0 if scales is None else scales.shape[1], width, _ptr(status), _stream()), "gemm_tcgen05_unary")
 
@@ -1914,7 +1890,6 @@ def gemm_tcgen05_clamped(x: torch.Tensor, w: torch.Tensor, act: torch.Tensor, st
     inter = w.shape[0] // 2
     if not gemm_tcgen05_usable(x, w) or w.shape[1] != k or tuple(act.shape) != (tokens, inter):
         raise KernelError(f"tcgen05 gated gemm cannot take x {tuple(x.shape)} / w {tuple(w.shape)} / act {tuple(act.shape)}")
-    fn = _fn("gemm_tcgen05", "tt_gemm_tcgen05_clamped", [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_int, c_int,
-                                                         c_float, c_float, c_int, c_float, c_void_p, c_void_p])
+    fn = _fn("gemm_tcgen05", "tt_gemm_tcgen05_clamped", "plplpliiiffifpp")
     _check(fn(_ptr(x), x.stride(0), _ptr(w), w.stride(0), _ptr(act), act.stride(0), tokens, inter, k, float(limit or 0.0),
               float(shared_limit or 0.0), int(split), float(alpha), _ptr(status), _stream()), "gemm_tcgen05_clamped")

@@ -12,11 +12,14 @@ from __future__ import annotations
 
 import ctypes
 import hashlib
+import importlib.machinery
+import importlib.util
 import os
 import shutil
 import stat
 import subprocess
 import sys
+import sysconfig
 import tempfile
 import threading
 import time
@@ -212,6 +215,55 @@ def load(name: str) -> ctypes.CDLL:
         return _loaded[name]
 
 
+_host_calls: list = []
+
+
+def host_calls():
+    """The native module ``csrc/host_calls.cpp`` (calls into the C entry points without ctypes), built with the host's C++ compiler; None where
+    there is none, or no Python headers, or the machine's calling convention is not known to it."""
+    with _lock:
+        if not _host_calls:
+            try:
+                path = _compile_host_calls()
+                loader = importlib.machinery.ExtensionFileLoader("host_calls", str(path))
+                module = importlib.util.module_from_spec(importlib.util.spec_from_loader("host_calls", loader))
+                loader.exec_module(module)
+            except (KernelBuildError, ImportError, OSError) as exc:
+                _log(f"calls go through ctypes: {exc}")
+                module = None
+            _host_calls.append(module)
+        return _host_calls[0]
+
+
+def _compile_host_calls() -> Path:
+    import torch
+
+    source, include, torch_folder = CSRC / "host_calls.cpp", sysconfig.get_paths()["include"], Path(torch.__file__).parent
+    tag = hashlib.sha256(source.read_bytes() + f"{sysconfig.get_config_var('SOABI')} {torch.__version__}".encode()).hexdigest()[:16]
+    file = f"tt_host_calls-{tag}.so"
+    for folder in (build_dir(), CSRC.parent / "_build"):
+        if (folder / file).is_file():
+            return folder / file
+    compiler = next((c for c in (os.environ.get("CXX"), "g++", "c++", "clang++") if c and shutil.which(c)), None)
+    if compiler is None or not (Path(include) / "Python.h").is_file():
+        raise KernelBuildError("no C++ compiler, or no Python headers, for host_calls.cpp")
+    target = build_dir() / file
+    scratch = target.with_suffix(f".{os.getpid()}.tmp")
+    _log("compiling host_calls.cpp ...")
+    done = subprocess.run([compiler, "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-I", include,
+                           "-I", str(torch_folder / "include"), "-I", str(torch_folder / "include/torch/csrc/api/include"), "-o", str(scratch), str(source),
+                           "-L", str(torch_folder / "lib"), "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10"],
+                          stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if done.returncode != 0:
+        scratch.unlink(missing_ok=True)
+        raise KernelBuildError(f"{compiler} failed on host_calls.cpp (exit {done.returncode}):\n{done.stdout}")
+    os.replace(scratch, target)
+    for stale in build_dir().glob("tt_host_calls-*.so"):
+        if stale != target:
+            stale.unlink(missing_ok=True)
+    return target
+
+
 def build_all(names: list[str] | None = None, verbose: bool = True) -> dict[str, Path]:
     """Compile every source (in parallel); used by the build check and before tests."""
     names = list(names or SOURCES)
@@ -231,4 +283,5 @@ def build_all(names: list[str] | None = None, verbose: bool = True) -> dict[str,
         t.join()
     if errors:
         raise errors[0]
+    host_calls()
     return results
