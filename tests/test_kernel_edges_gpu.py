@@ -699,3 +699,87 @@ def test_delta_rule_in_chunks_is_as_close_as_token_by_token(heads, D, V):
     want = torch.stack(want)
     chunked, by_token = (float((out - want).norm() / want.norm()) for out in outs)
     assert chunked <= 1.05 * by_token, (chunked, by_token)
+
+
+# --------------------------------------------------------------------------------- experts' products of sorted tokens
+@pytest.mark.parametrize("tokens,top,experts,hidden,inter", [(1, 1, 1, 64, 128), (300, 2, 3, 72, 128), (513, 4, 16, 256, 256), (1500, 1, 5, 264, 384), (200, 3, 70, 128, 128)])
+def test_experts_of_sorted_tokens(tokens, top, experts, hidden, inter):
+    """Experts without tokens, with one, with whole tiles of 256 and a remainder; choices that a token does not have; widths that end inside a tile."""
+    from thintensor_b200.kernels import api
+
+    g = torch.Generator(device=DEV).manual_seed(tokens + experts)
+    order = torch.rand(tokens, experts, generator=g, device=DEV)
+    order[:, 0] += 0.3                                     # an expert with most tokens
+    if experts > 2:
+        order[:, 1] = -1.0                                 # one that nobody chose
+    chosen = order.topk(top, 1).indices.int()
+    if top > 1:
+        chosen[::7, top - 1] = -1
+    x, w = randn(tokens, hidden, seed=140).bfloat16(), randn(2 * experts * inter, hidden, seed=141, scale=hidden ** -0.5).bfloat16()
+    down, weights = randn(hidden, experts * inter, seed=142, scale=inter ** -0.5).bfloat16(), torch.rand(tokens, top, generator=g, device=DEV)
+    weights[::5] = 0.0
+    tiles = api.expert_tiles(tokens, top, experts)
+    xs = torch.full((256 * tiles, hidden), 7.0, dtype=torch.bfloat16, device=DEV)
+    place, table = torch.full((tokens, top), 99, dtype=torch.int32, device=DEV), torch.full((1 + experts + tiles,), 99, dtype=torch.int32, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    api.sort_tokens(x, chosen, experts, xs, place, table)
+    counts = torch.stack([(chosen == e).sum() for e in range(experts)])
+    padded = (counts + 255) // 256 * 256
+    first = padded.cumsum(0) - padded
+    assert int(table[0]) == int(padded.sum()) // 256 and torch.equal(table[1:1 + experts].long(), counts)
+    assert torch.equal(table[1 + experts:1 + experts + int(table[0])].long(), torch.arange(experts, device=DEV).repeat_interleave(padded // 256))
+    for e in range(experts):
+        mine = chosen == e
+        rows = first[e] + torch.arange(int(counts[e]), device=DEV)
+        assert torch.equal(place[mine].long(), rows)       # in the tokens' order
+        assert torch.equal(xs[rows], x[mine.any(1)])
+    assert bool((place[chosen < 0] == -1).all())
+    act = torch.full((256 * tiles, inter), float("nan"), dtype=torch.bfloat16, device=DEV)
+    api.gemm_tcgen05_experts(xs, w, act, status, hidden, inter, experts, table, "silu", experts * inter)
+    y = torch.full((256 * tiles, hidden), float("nan"), device=DEV)
+    api.gemm_tcgen05_experts(act, down, y, status, inter, hidden, experts, table)
+    out = randn(tokens, hidden, seed=143)
+    want = out.double()
+    api.combine_experts(y, place, weights, out)
+    assert int(status) == 0
+    gate, up = (m.double().view(experts, inter, hidden) for m in w.chunk(2))
+    for t, c in ((t, c) for t in list(range(0, tokens, 61)) + [tokens - 1] for c in range(top)):
+        e = int(chosen[t, c])
+        if e < 0:
+            continue
+        z = gate[e] @ x[t].double()
+        made = z * torch.sigmoid(z) * (up[e] @ x[t].double())
+        got = act[place[t, c]].double()
+        # one rounding to bfloat16 of a float32 sum, and the epilogue's fast exponential
+        torch.testing.assert_close(got, made, rtol=2.0 ** -7, atol=2.0 ** -9 * float(made.abs().max()))
+        product = down.double()[:, e * inter:(e + 1) * inter] @ got
+        torch.testing.assert_close(y[place[t, c]].double(), product, rtol=1e-4, atol=1e-4 * float(product.abs().max()))
+    for c in range(top):
+        has = (chosen[:, c] >= 0) & (weights[:, c] != 0)
+        want[has] += weights[has, c, None].double() * y[place[has, c].long()].double()
+    torch.testing.assert_close(out.double(), want, rtol=1e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("shared,residual", [(0, True), (0, False), (384, True), (384, False)])
+@pytest.mark.parametrize("tokens", [640, 2100])
+def test_mixture_of_sorted_tokens_is_the_mixture_of_columns(shared, residual, tokens, monkeypatch):
+    """The layer both ways: tokens sorted by expert, and every expert's columns for every token with weights of zero."""
+    from thintensor_b200.engine.context import StepContext, Workspace
+    from thintensor_b200.parts import moe
+
+    part = moe.MixtureOfExperts(hidden=256, experts=16, top=3, inter=128, groups=4, keep=2, shared_inter=shared)
+    part.bind({name: (0.06 * randn(*decl.shape, seed=150 + i)).bfloat16() for i, (name, decl) in enumerate(part.weights().items())}, torch.bfloat16, torch.device(DEV))
+    x = randn(tokens, 256, seed=149).bfloat16()
+    outs = []
+    for by_expert in (True, False):
+        stream = randn(tokens, 256, seed=148)
+        ctx = StepContext(n_tokens=tokens, sequences=1, decode=False, max_new=tokens, max_total=tokens, tokens=None, cu=i32([0, tokens]), len_before=i32([0]), slots=i32([0]),
+                          tables=[], act_dtype=torch.bfloat16, workspace=Workspace(torch.device(DEV)), status=torch.zeros(1, dtype=torch.int32, device=DEV))
+        ctx.residual = stream if residual else None
+        part.sorted_takes = lambda rows: by_expert
+        monkeypatch.setattr(moe, "sorted_experts_pay", lambda *sizes: True)
+        delta = part.forward(ctx, x)
+        outs.append((stream if delta.tensor is None else stream + delta.tensor.sum(0)).double() - randn(tokens, 256, seed=148).double())
+        assert int(ctx.status) == 0
+    # activations narrowed before and after the routing weight: two roundings of 2^-9 that the other form does not share
+    assert float((outs[0] - outs[1]).norm() / outs[1].norm()) < 2.0 ** -8

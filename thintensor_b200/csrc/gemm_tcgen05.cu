@@ -108,6 +108,12 @@ struct Args {
     // plain forms: output features in groups of so many, each with activations of its own, the rows of which follow one another (x
     // is [groups][tokens][k]; a tile's features lie in one group).  0: all features read the same activations
     int group_features;
+    // pair kernel, rows sorted by expert (null: one weight matrix for all rows): the expert of every tile of 256 rows and, in device memory, how
+    // many tiles there are.  An expert's weights are expert_rows rows (gated form: gate and up rows each) or expert_k columns of w further than
+    // those of the one before; its rows' tiles are its own (the rows between its last and the tile's end belong to nobody).
+    const int* tile_expert;
+    const int* tile_count;
+    int expert_rows, expert_k;
     unsigned* status;
 };
 
@@ -1025,6 +1031,12 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     const int rank = (int)cluster.block_rank();                 // 0: the CTA that issues
     const int pair = (int)blockIdx.x >> 1, n_pairs = (int)gridDim.x >> 1;
     const int n_kb = (args.k + BK - 1) / BK;
+    if (args.tile_expert) {                                     // the kernel before counted the tiles
+        tt_pdl_wait();
+        const int tiles_f = tiles_total / tiles_m;
+        tiles_m = max(1, min(tiles_m, __ldg(args.tile_count)));
+        tiles_total = tiles_m * tiles_f;
+    }
     // A pair's items: whole tiles pair, pair + n_pairs, ... or, where the launcher gave scratch memory for shares (plain
     // form, fewer whole rounds of tiles than would fill the pairs), its run of the tiles' k-blocks dealt out evenly.
     const bool dealt = FORM == TOKENS_ON_M && args.shares != nullptr;
@@ -1057,8 +1069,9 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                 int tile, kb0, kb1;
                 item(j, tile, kb0, kb1);
                 const int a_row = (tile % tiles_m) * 2 * BM + rank * BM + group_rows((tile / tiles_m) * TILE_N, args);
-                const int b_row = dual ? (rank == 0 ? 0 : args.up_row_offset) + (tile / tiles_m) * TILE_N
-                                       : (tile / tiles_m) * TILE_N + rank * B_ROWS;
+                const int expert = args.tile_expert ? __ldg(args.tile_expert + tile % tiles_m) : 0;
+                const int b_row = (dual ? (rank == 0 ? 0 : args.up_row_offset) + (tile / tiles_m) * TILE_N
+                                        : (tile / tiles_m) * TILE_N + rank * B_ROWS) + expert * args.expert_rows;
                 for (int i = kb0; i < kb1; ++i, ++it) {
                     const int s = (int)(it % PAIR_STAGES);
                     if (!mbar_wait(smem_u32(&empty_bar[s]), (uint32_t)(((it / PAIR_STAGES) & 1) ^ 1))) {
@@ -1069,7 +1082,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                     uint8_t* stage = smem + (size_t)s * PAIR_STAGE_BYTES;
                     const int kx = i * BK;
                     tma_load_2d_pair(smem_u32(stage), &map_a, kx, a_row, bar);
-                    tma_load_2d_pair(smem_u32(stage + BM * BK * 2), &map_b, kx, b_row, bar);
+                    tma_load_2d_pair(smem_u32(stage + BM * BK * 2), &map_b, kx + expert * args.expert_k, b_row, bar);
                 }
             }
             // Every copy issued has landed once the products that read it are done, and the epilogue
@@ -1403,7 +1416,7 @@ static int gemm_dispatch(const void* x, long long ldx, const void* w, long long 
     const int activation = form >> 4;       // the gated form carries its gate's activation in the bits above the form
     form &= 15;
     if (activation < 0 || activation > 4 || (activation && form != 1)) return (int)cudaErrorInvalidValue;
-    Args args;
+    Args args = {};
     args.activation = activation;
     args.clamp_low = clamp.low; args.clamp_high = clamp.high; args.clamp_alpha = clamp.alpha; args.clamp_split = clamp.split;
     args.bias = bias; args.out = out; args.ld_out = ld_out; args.split_stride = split_stride;
@@ -1545,4 +1558,39 @@ extern "C" int tt_gemm_tcgen05_unary(const void* x, long long ldx, const void* w
         return (int)cudaErrorInvalidValue;
     return gemm_dispatch(x, ldx, w, ldw, nullptr, out, ld_out, 0, tokens, features / 2, k, 1, 1 + 16 * 4, status, stream, nullptr, 0,
                          GateClamp{0.0f, 0.0f, 1.0f, 0}, 0, Unary{activation, scales, scale_row, scale_width});
+}
+
+// Products of rows sorted by expert with the expert's own weights: x holds `rows` rows (a multiple of 256) in tiles of 256 that each belong to one
+// expert (tile_expert, of which tile_count[0] count; the rest of the rows is not touched).
+//   gated: out[r][f] = act(x[r] . w[e * features + f]) * (x[r] . w[up_row_offset + e * features + f]) in bfloat16; features a multiple of 128
+//   plain: out[r][f] = sum over i < k of x[r][i] * w[f][e * k + i] in float32; k a multiple of 64
+// tile_expert null: all rows have the weights of expert 0, and rows need not be a multiple of 256 (for a shared expert's rows among others').
+extern "C" int tt_gemm_tcgen05_experts(const void* x, long long ldx, const void* w, long long ldw, long long w_rows, long long w_cols, void* out,
+                                       long long ld_out, int rows, int features, int k, int gated, int activation, long long up_row_offset,
+                                       const int* tile_expert, const int* tile_count, unsigned* status, cudaStream_t stream) {
+    if (rows <= 0 || features <= 0) return 0;
+    if (k <= 0 || (k % 8) || (ldx % 8) || (ldw % 8) || ((uintptr_t)x & 15) || ((uintptr_t)w & 15) || ((uintptr_t)out & 15) || activation < 0 || activation > 2 ||
+        (tile_expert && (!tile_count || rows % 256)) || w_rows > 2147483647LL || w_cols > 2147483647LL || up_row_offset > 2147483647LL)
+        return (int)cudaErrorInvalidValue;
+    if (gated ? (features % 128 || ld_out % 8) : ((tile_expert && k % BK) || ld_out % 4)) return (int)cudaErrorInvalidValue;
+    Args args = {};
+    args.out = out; args.ld_out = ld_out; args.tokens = rows; args.features = features; args.k = k;
+    args.k_blocks_per_split = (k + BK - 1) / BK;
+    args.up_row_offset = (int)up_row_offset; args.status = status; args.activation = activation; args.clamp_alpha = 1.0f;
+    args.bulk_out = 1;
+    args.tile_expert = tile_expert; args.tile_count = tile_count;
+    args.expert_rows = gated ? features : 0;
+    args.expert_k = gated ? 0 : k;
+    CUtensorMap map_a, map_b, map_out;
+    if (!make_map(&map_a, x, rows, k, ldx, BM) || !make_map(&map_b, w, w_rows, w_cols, ldw, 128)) return -1;
+    const int tiles_m = (rows + 2 * BM - 1) / (2 * BM);
+    if (gated) {
+        const cuuint64_t dims[2] = {(cuuint64_t)features, (cuuint64_t)rows};
+        const cuuint64_t strides[1] = {(cuuint64_t)ld_out * 2};
+        const cuuint32_t box[2] = {64, 32};
+        if (!tc::make_map(&map_out, out, 2, dims, strides, box)) return -1;
+        return launch_pair<TOKENS_ON_M_SWIGLU>(map_a, map_b, map_out, args, tiles_m, tiles_m * (features / 128), stream);
+    }
+    if (!make_map_f32_out(&map_out, out, 1, rows, features, ld_out, (long long)rows * ld_out)) return -1;
+    return launch_pair<TOKENS_ON_M>(map_a, map_b, map_out, args, tiles_m, tiles_m * ((features + 255) / 256), stream);
 }

@@ -1495,6 +1495,62 @@ def route_rows_takes(hidden: int, experts: int) -> bool:
     return (hidden + experts + 32) * 4 <= 48 * 1024 and hidden <= ROUTE_MAX_HIDDEN
 
 
+EXPERT_TILE = 256           # rows of a tile of tokens sorted by expert (SORT_TILE in csrc/routing.cu)
+
+
+def expert_tiles(tokens: int, top: int, experts: int) -> int:
+    """Tiles of 256 rows that a step's tokens, sorted by expert, take at most."""
+    items = tokens * top
+    return (items + (EXPERT_TILE - 1) * min(experts, items)) // EXPERT_TILE
+
+
+def sort_tokens(x: torch.Tensor, chosen: torch.Tensor, experts: int, xs: torch.Tensor, place: torch.Tensor, tiles: torch.Tensor) -> None:
+    """The rows of ``x`` (bfloat16) for every choice ``chosen`` [tokens, top], expert after expert in tiles of 256 rows, into ``xs``; ``place``
+    [tokens, top] receives their rows (-1 for no choice), ``tiles`` (int32) the count of tiles, the experts' token counts and the tiles' experts."""
+    tokens, hidden = x.shape
+    top, count = chosen.shape[1], expert_tiles(tokens, chosen.shape[1], experts)
+    for t, dtype, name in ((x, torch.bfloat16, "activations"), (xs, torch.bfloat16, "sorted activations"), (chosen, torch.int32, "choices"),
+                           (place, torch.int32, "places"), (tiles, torch.int32, "tiles")):
+        _need(t, dtype, name)
+    if (chosen.shape[0] != tokens or place.shape != chosen.shape or tuple(xs.shape) != (EXPERT_TILE * count, hidden) or hidden % 8
+            or tiles.numel() < 1 + experts + count):
+        raise KernelError("sort_tokens: shapes do not fit")
+    fn = _fn("routing", "tt_sort_tokens", "pipiiipppppp")
+    at = tiles.data_ptr()
+    _check(fn(_ptr(x), hidden, _ptr(chosen), tokens, top, experts, at + 4, _ptr(place), _ptr(xs), at + 4 * (1 + experts), at, _stream()), "sort_tokens", 2)
+
+
+def gemm_tcgen05_experts(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, status: torch.Tensor, k: int, features: int, experts: int,
+                         tiles: torch.Tensor | None, activation: str | None = None, up_rows: int = 0) -> None:
+    """Products of rows sorted by :func:`sort_tokens` with their expert's weights.  With an ``activation`` (a gate's): ``w`` [rows, k] holds
+    ``features`` gate rows an expert, the up rows ``up_rows`` further, and ``out`` (bfloat16) receives act(gate) * up.  Without: ``w``
+    [features, columns] holds ``k`` columns an expert and ``out`` is the float32 product.  ``tiles`` None: all rows are expert 0's."""
+    gated = activation is not None
+    _need(out, torch.bfloat16 if gated else torch.float32, "expert products")
+    rows = x.shape[0]
+    if (not gemm_tcgen05_usable(x, w) or x.shape[1] != k or tuple(out.shape) != (rows, features)
+            or (w.shape[1] != k or w.shape[0] < up_rows + experts * features or features % 128 if gated
+                else w.shape[0] != features or w.shape[1] < experts * k or features % 4 or (tiles is not None and k % 64))
+            or (tiles is not None and rows % EXPERT_TILE)):
+        raise KernelError(f"expert products cannot take x {tuple(x.shape)} / w {tuple(w.shape)} / out {tuple(out.shape)}")
+    fn = _fn("gemm_tcgen05", "tt_gemm_tcgen05_experts", "plplllpliiiiilpppp")
+    at = 0 if tiles is None else _ptr(tiles)
+    _check(fn(_ptr(x), x.stride(0), _ptr(w), w.stride(0), w.shape[0], w.shape[1], _ptr(out), features, rows, features, k, 1 if gated else 0,
+              GATE_ACTIVATIONS[activation] if gated else 0, up_rows, 0 if tiles is None else at + 4 * (1 + experts), at, _ptr(status), _stream()),
+           "gemm_tcgen05_experts")
+
+
+def combine_experts(y: torch.Tensor, place: torch.Tensor, weights: torch.Tensor, out: torch.Tensor) -> None:
+    """out[t] += sum over choices of weights[t, c] * y[place[t, c]] (float32)."""
+    for t, dtype, name in ((y, torch.float32, "expert products"), (place, torch.int32, "places"), (weights, torch.float32, "weights"), (out, torch.float32, "sum")):
+        _need(t, dtype, name)
+    tokens, top = place.shape
+    if weights.shape != place.shape or out.shape[0] != tokens or out.shape[1] != y.shape[1] or y.shape[1] % 4:
+        raise KernelError("combine_experts: shapes do not fit")
+    fn = _fn("routing", "tt_combine_experts", "pppiipip")
+    _check(fn(_ptr(y), _ptr(place), _ptr(weights), tokens, top, _ptr(out), y.shape[1], _stream()), "combine_experts")
+
+
 def scale_expert_columns(act: torch.Tensor, width: int, gates: torch.Tensor, experts: int | None = None, shared_width: int = 0) -> None:
     """act[t, e * width + j] *= gates[t, e] for the ``experts * width`` leading columns of ``act`` (in place; columns behind
     them stay as they are).  ``experts``: fewer than ``gates`` has columns; with ``shared_width`` the next so many columns of

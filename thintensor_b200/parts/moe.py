@@ -18,8 +18,9 @@ The experts run as ONE gated product over the concatenation of all experts' gate
 behind them) and ONE down product over the concatenated columns: a token's activations are multiplied by its
 routing weight per expert (zero for experts it did not choose) in between, so the down product's sum over its input
 IS the weighted sum over experts.  Every matrix is read once per step whatever the routing, which is what a decode
-step of more than a few sequences does anyway, and prompts keep the tensor-core tiles full; the price is the
-arithmetic of the experts a token did not choose.
+step of more than a few sequences does anyway; the price is the arithmetic of the experts a token did not choose.
+Where that is large (prompts, see :func:`sorted_experts_pay`) the tokens are sorted by the experts they chose, each expert's
+matrices multiply its own rows, and a token's products are weighted and added in float32.
 """
 from __future__ import annotations
 
@@ -28,6 +29,17 @@ import torch
 from ..kernels import api
 from .base import FEED_FORWARDS, Delta, FeedForward, WeightDecl
 from .linear import GatedLinear, Linear
+
+
+def sorted_experts_pay(tokens: int, experts: int, top: int, hidden: int, inter: int) -> bool:
+    """Whether a prompt's tokens are sorted by the experts they chose: where that saves 12 G multiply-adds in each of an expert's matrices (rows of
+    whole tiles of 256 an expert against every token), which is what sorting, gathering and adding up cost.  Layers, every expert's
+    columns for every token against sorted tokens (us, one B200, captured): 16 experts of 1,024 of which 4, 2,048 wide, beside a shared one of 4,096,
+    512 tokens 142 and 148, 700 175 and 156, 1,000 221 and 182, 2,048 391 and 268, 4,096 758 and 452; 1,024 wide, 700 104 and 107, 1,000
+    129 and 121, 2,048 260 and 170; 64 experts of which 6, 300 tokens 309 and 368, 400 387 and 368, 2,048 1,274 and 453; 32 of 512 of
+    which 8, 1,000 135 and 139, 1,500 183 and 169."""
+    rows = max(tokens * top + 128 * experts, 256 * experts)
+    return (tokens * experts - rows) * hidden * inter >= 12_000_000_000
 
 
 @FEED_FORWARDS.register("moe")
@@ -142,11 +154,57 @@ class MixtureOfExperts(FeedForward):
                 api.expert_activation(self.gate_up.fused(ctx, x, "moe.gate_up"), act, self.experts, self.inter, self.shared_inter, self.limit,
                                       self.shared_limit, self.alpha, gates, self.shared_gate)
             return self.down.delta(ctx, act, "moe.down")
+        if self.sorted_takes(x) and sorted_experts_pay(tokens, self.experts, self.top, self.hidden, self.inter):
+            return self.by_expert(ctx, x, chosen, weights)
         act = self.gate_up(ctx, x, "moe.gate_up")
         api.scale_expert_columns(act, self.inter, gates)
         if extra:
             raise NotImplementedError("a gated shared expert goes with the clamped unit")
         return self.down.delta(ctx, act, "moe.down")
+
+    def sorted_takes(self, x) -> bool:
+        """Whether the experts' matrices can be multiplied with the rows that chose them: whole tiles of 128 rows an expert, operands of the
+        tensor-core product."""
+        return (self.gated and self.activation in api.GATE_ACTIVATIONS and not self.shared_gate and self.inter % 128 == 0 and self.shared_inter % 128 == 0
+                and self.hidden % 8 == 0 and api.gemm_tcgen05_usable(x, self.gate_up.fused.weight) and self.down.weight.dtype == torch.bfloat16
+                and self.down.weight.shape[1] % 8 == 0)
+
+    def by_expert(self, ctx, x, chosen, weights) -> Delta:
+        """A prompt's tokens sorted by expert: every expert's matrices multiply the rows that chose it, and a token's products are weighted and
+        added in float32.  The shared expert's product takes all tokens as they are."""
+        tokens, experts, inter, shared, total = ctx.n_tokens, self.experts, self.inter, self.shared_inter, self.experts * self.inter + self.shared_inter
+        tiles = api.expert_tiles(tokens, self.top, experts)
+        xs = ctx.scratch("moe.sorted", (api.EXPERT_TILE * tiles, self.hidden))
+        place = ctx.scratch("moe.place", (tokens, self.top), torch.int32)
+        table = ctx.scratch("moe.tiles", (1 + experts + tiles,), torch.int32)
+        gate_up, down = self.gate_up.fused.weight, self.down.weight
+        api.sort_tokens(x, chosen, experts, xs, place, table)
+        act = ctx.scratch("moe.sorted.act", (xs.shape[0], inter))
+        api.set_label("moe.gate_up")
+        api.gemm_tcgen05_experts(xs, gate_up, act, ctx.status, self.hidden, inter, experts, table, self.activation, total)
+        y = ctx.scratch("moe.sorted.out", (xs.shape[0], self.hidden), torch.float32)
+        api.set_label("moe.down")
+        api.gemm_tcgen05_experts(act, down, y, ctx.status, inter, self.hidden, experts, table)
+        residual, out = getattr(ctx, "residual", None), None
+        if residual is None or tuple(residual.shape) != (tokens, self.hidden):
+            residual, out = None, ctx.scratch("moe.out", (1, tokens, self.hidden), torch.float32)
+        if shared:
+            act = ctx.scratch("moe.shared.act", (tokens, shared))
+            api.set_label("moe.shared.gate_up")
+            api.gemm_tcgen05_experts(x, gate_up[experts * inter:], act, ctx.status, self.hidden, shared, 1, None, self.activation, total)
+            columns = down[:, experts * inter:]
+            accumulate = residual is not None and api.gemm_tcgen05_accumulates(tokens, self.hidden, shared)
+            if residual is not None and not accumulate:
+                residual, out = None, ctx.scratch("moe.out", (api.gemm_tcgen05_splits(tokens, self.hidden, shared), tokens, self.hidden), torch.float32)
+            elif residual is None:
+                out = ctx.scratch("moe.out", (api.gemm_tcgen05_splits(tokens, self.hidden, shared), tokens, self.hidden), torch.float32)
+            api.set_label("moe.shared.down")
+            api.gemm_tcgen05(act, columns, None, residual.unsqueeze(0) if accumulate else out, ctx.status, accumulate=accumulate,
+                             shares=Linear.shares(ctx, tokens))
+        elif out is not None:
+            out.zero_()
+        api.combine_experts(y, place, weights, residual if residual is not None else out[0])
+        return Delta(out)
 
     def ungated(self, ctx, x, gates) -> torch.Tensor:
         """``f(up x)`` of every expert's columns times the token's weight for the expert."""
