@@ -783,3 +783,47 @@ def test_mixture_of_sorted_tokens_is_the_mixture_of_columns(shared, residual, to
         assert int(ctx.status) == 0
     # activations narrowed before and after the routing weight: two roundings of 2^-9 that the other form does not share
     assert float((outs[0] - outs[1]).norm() / outs[1].norm()) < 2.0 ** -8
+
+
+# --------------------------------------------------------------------------------- differential attention of prompts
+@pytest.mark.parametrize("heads,kv_heads", [(16, 4), (3, 3), (6, 2), (16, 1), (2, 1)])
+@pytest.mark.parametrize("news,before", [([1, 63, 64, 65, 130], [0, 0, 5, 64, 127]), ([300], [0]), ([0, 40, 0, 129], [3, 200, 0, 1])])
+def test_differential_attention_in_tiles(heads, kv_heads, news, before):
+    """Tiles of 128 rows whole and in part, groups that do not divide 128, contexts from earlier steps, sequences without tokens; a map with scores of one size
+    and one with a few large ones."""
+    from thintensor_b200.kernels import api
+
+    tokens, sequences, width = sum(news), len(news), 8
+    g = torch.Generator(device=DEV).manual_seed(heads)
+    table = torch.randperm(sequences * width, generator=g, device=DEV).int().view(sequences, width).contiguous()
+    k_pool = torch.randn(sequences * width, kv_heads, 64, 128, generator=g, device=DEV).bfloat16()
+    v_pool = torch.randn(sequences * width, kv_heads, 128, 64, generator=g, device=DEV).bfloat16()
+    q = torch.randn(tokens, heads, 2, 64, generator=g, device=DEV)
+    q[:, :, 1] *= 4.0
+    q = q.bfloat16().view(tokens, heads * 128)
+    cu = [sum(news[:i]) for i in range(sequences + 1)]
+    out, maps = torch.full((tokens, heads * 128), 7.0, dtype=torch.bfloat16, device=DEV), torch.full((2, tokens, heads, 128), float("nan"), device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    scale, lam, gain, eps = 0.125, 0.3, 0.8, 1e-5
+    api.differential_attention_tcgen05(q, k_pool, v_pool, table, i32(cu), i32(before), sequences, tokens, heads, kv_heads, scale, lam, gain, eps, maps, out, status)
+    assert int(status) == 0
+    group = heads // kv_heads
+    for s in range(sequences):
+        if not news[s]:
+            continue
+        span, seen = slice(cu[s], cu[s + 1]), before[s] + news[s]
+        keys = k_pool[table[s].long()].double().permute(1, 0, 2, 3).reshape(kv_heads, -1, 128)[:, :seen].repeat_interleave(group, 0)
+        values = v_pool[table[s].long()].double().permute(1, 0, 3, 2).reshape(kv_heads, -1, 128)[:, :seen].repeat_interleave(group, 0)
+        hidden = torch.arange(seen, device=DEV)[None] > before[s] + torch.arange(news[s], device=DEV)[:, None]
+        made = []
+        for m in range(2):
+            score = torch.einsum("ihd,hjd->hij", q[span].double().view(-1, heads, 128)[:, :, 64 * m:64 * m + 64], keys[:, :, 64 * m:64 * m + 64]) * scale
+            made.append(torch.einsum("hij,hjd->ihd", torch.softmax(score.masked_fill(hidden, -float("inf")), -1), values))
+            # probabilities narrowed to bfloat16 (2^-9 each) and summed in float32 over values of size one
+            assert float((maps[m, span].double() - made[m]).abs().max()) <= 2.0 ** -8 * float(values.abs().max())
+        o = made[0] - lam * made[1]
+        # the errors of both maps, carried by the division by the root mean square, and one more rounding
+        norm = o.square().mean(-1, keepdim=True).add(eps).sqrt()
+        want = o / norm * gain
+        error = (out[span].double().view(-1, heads, 128) - want).abs()
+        assert bool((error <= gain * (2.0 ** -7 * float(values.abs().max()) / norm + 2.0 ** -8 * want.abs())).all())

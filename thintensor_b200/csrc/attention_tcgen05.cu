@@ -68,7 +68,10 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
     return d;
 }
 
-template <int HD> struct Layout {
+// MAPS (head size 64 only): two attention maps a head over the same values, of twice a map's size (differential attention): a CTA makes one of them,
+// float32, and differential_combine_kernel the heads' outputs.  P lies over the score accumulator that it was made from, which its thread has read and
+// which is not written again before the products of P are done, so that O's 128 columns leave room for a second CTA on the SM.
+template <int HD, bool MAPS = false> struct Layout {
     // Threads per query row in the softmax.  Head size 128 leaves room for one CTA per SM only, and
     // four softmax warps cannot hide their own latencies: two threads per row (8 warps) are 10 %
     // faster there.  Head size 64 runs two CTAs per SM and is bound elsewhere: one thread per row.
@@ -76,11 +79,13 @@ template <int HD> struct Layout {
     static constexpr int THREADS = 64 + SPLIT * ROWS;
     static constexpr int CHUNKS = HD / 64;                      // 64-wide slices of the head dimension
     static constexpr int Q_BYTES = ROWS * HD * 2;
-    static constexpr int K_BYTES = KEYS * HD * 2;               // = V tile
-    static constexpr int STAGE_BYTES = 2 * K_BYTES;
+    static constexpr int VD = MAPS ? 2 * HD : HD;               // numbers of a value
+    static constexpr int K_BYTES = KEYS * HD * 2;
+    static constexpr int STAGE_BYTES = K_BYTES + KEYS * VD * 2;
     static constexpr int SMEM = Q_BYTES + KV_STAGES * STAGE_BYTES + 1024;
     static constexpr int O_COL = 128;                           // S: 2 x 64 columns, then O: HD, then P: 2 x 32 (bfloat16 pairs)
-    static constexpr int P_COL = O_COL + HD;
+    static constexpr int P_COL = MAPS ? 0 : O_COL + HD, P_STEP = MAPS ? 64 : 32;
+    static_assert(!MAPS || HD == 64, "two maps a head: of 64 numbers each");
     static constexpr int TMEM_COLS = HD == 64 ? 256 : 512;
 };
 
@@ -104,13 +109,16 @@ struct Args {
     const float* gate;
     int gate_splits, gate_row, gate_per_head;
     long long gate_split_stride;
+    float* maps;            // the MAPS instance's output: [2][tokens][heads][128]
+    int n_tokens;
 };
 
-template <int HD, bool SHAPED>
-__global__ void __launch_bounds__(Layout<HD>::THREADS, HD == 64 ? 2 : 1)
+template <int HD, bool SHAPED, bool MAPS = false>
+__global__ void __launch_bounds__(Layout<HD, MAPS>::THREADS, HD == 64 ? 2 : 1)
 attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                          const __grid_constant__ CUtensorMap map_v, const Args args) {
-    using L = Layout<HD>;
+    using L = Layout<HD, MAPS>;
+    constexpr int VD = L::VD;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* q_smem = smem;
@@ -125,7 +133,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     // The grid is (kv heads, tiles) and blocks are handed out with x running fastest: the heaviest tile of every
     // head comes first, then the next heaviest of every head, so the CTAs that start last are the lightest ones
     // (with the heads on y, whole heads, heavy tiles included, started behind others' light tiles).
-    const int kh = blockIdx.x;
+    const int kh = MAPS ? blockIdx.x >> 1 : blockIdx.x, map_col = MAPS ? (blockIdx.x & 1) * HD : 0;      // the map's first number in a row of q or k
 
     if (warp == 0) {
         // which sequence and which of its tiles (late tiles, which see most keys, first)
@@ -188,7 +196,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             mbar_expect_tx(qbar, (uint32_t)(L::CHUNKS * args.group * args.tokens_per_tile * 128));
 #pragma unroll
             for (int c = 0; c < L::CHUNKS; ++c)
-                tma_load_3d(smem_u32(q_smem + c * ROWS * 128), &map_q, c * 64, kh * args.group, seq_begin + tok0, qbar);
+                tma_load_3d(smem_u32(q_smem + c * ROWS * 128), &map_q, map_col + c * 64, kh * args.group, seq_begin + tok0, qbar);
             const int* table_row = args.table + (size_t)b * args.table_width;
             int issued = 0;
             for (int i = 0; i < n_blocks; ++i) {
@@ -201,9 +209,9 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 const uint32_t bar = smem_u32(&kv_full[s]);
                 mbar_expect_tx(bar, L::STAGE_BYTES);
                 uint8_t* stage = kv_smem + (size_t)s * L::STAGE_BYTES;
-                const int k_row = (block * args.kv_heads + kh) * KEYS, v_row = (block * args.kv_heads + kh) * HD;
+                const int k_row = (block * args.kv_heads + kh) * KEYS, v_row = (block * args.kv_heads + kh) * VD;
 #pragma unroll
-                for (int c = 0; c < L::CHUNKS; ++c) tma_load_2d(smem_u32(stage + c * KEYS * 128), &map_k, c * 64, k_row, bar);
+                for (int c = 0; c < L::CHUNKS; ++c) tma_load_2d(smem_u32(stage + c * KEYS * 128), &map_k, map_col + c * 64, k_row, bar);
                 tma_load_2d(smem_u32(stage + L::K_BYTES), &map_v, 0, v_row, bar);
                 ++issued;
             }
@@ -213,7 +221,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
         if (lane == 0) {
-            constexpr uint32_t idesc_s = instr_desc(ROWS, KEYS), idesc_o = instr_desc(ROWS, HD);
+            constexpr uint32_t idesc_s = instr_desc(ROWS, KEYS), idesc_o = instr_desc(ROWS, VD);
             bool ok = mbar_wait(smem_u32(&q_full), 0);
             if (!ok) atomicOr(args.status, TT_STATUS_WAIT_EXPIRED);
             auto issue_s = [&](int i) {                           // S_i = Q K_i^T into S accumulator i & 1
@@ -235,13 +243,15 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 if (!mbar_wait(smem_u32(&p_ready[i & 1]), (uint32_t)((i >> 1) & 1))) { atomicOr(args.status, TT_STATUS_WAIT_EXPIRED); ok = false; break; }
                 fence_after_sync();
                 const int s = i % KV_STAGES;
-                const uint32_t p_tmem = tmem_base + L::P_COL + (i & 1) * 32;
+                const uint32_t p_tmem = tmem_base + L::P_COL + (i & 1) * L::P_STEP;
                 const uint32_t v_addr = smem_u32(kv_smem + (size_t)s * L::STAGE_BYTES + L::K_BYTES);
 #pragma unroll
                 for (int kk = 0; kk < KEYS / 16; ++kk)
                     umma_bf16_a_in_tmem(tmem_base + L::O_COL, p_tmem + kk * 8, smem_desc(v_addr + kk * 32), idesc_o, (i > 0 || kk > 0) ? 1u : 0u);
                 umma_commit(smem_u32(&kv_empty[s]));              // K_i and V_i are free once these products are done
                 umma_commit(smem_u32(&pv_done[i & 1]));
+                // P_i lies in the next but one block's score accumulator: the products that read it must be done
+                if (MAPS && i + 2 < n_blocks && !mbar_wait(smem_u32(&pv_done[i & 1]), (uint32_t)((i >> 1) & 1))) { atomicOr(args.status, TT_STATUS_WAIT_EXPIRED); ok = false; break; }
                 if (i + 2 < n_blocks) issue_s(i + 2);             // its S accumulator was read before P_i was announced
             }
         }
@@ -260,7 +270,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         const int pos = row_ok ? before + tok0 + local : -1;
         const int first = tt_first_key(pos, args.window);
         const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16);
-        constexpr int SPLIT = L::SPLIT, HALF_KEYS = KEYS / SPLIT, O_COLS = HD / SPLIT;   // what one thread of a row handles
+        constexpr int SPLIT = L::SPLIT, HALF_KEYS = KEYS / SPLIT, O_COLS = VD / SPLIT;   // what one thread of a row handles
         float m_used = -INFINITY, l = 0.0f;                       // the scale in use (log2 units) and this thread's part of the sum
         bool ok = true;
         // shaped scores are brought to log2 units key by key, so the scale that follows is one
@@ -406,7 +416,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             // issuing thread asked for them before it asked for S_i, its products complete in the order it issues them, and
             // this thread has seen S_i complete.  (A wait of its own on pv_done here cost 160 cycles of 1,500 a block.)
             if (SPLIT == 2) tmem_store16(lane_base + L::P_COL + (i & 1) * 32 + half * 16, packed);
-            else tmem_store32(lane_base + L::P_COL + (i & 1) * 32, reinterpret_cast<const float*>(packed));
+            else tmem_store32(lane_base + L::P_COL + (i & 1) * L::P_STEP, reinterpret_cast<const float*>(packed));
             fence_before_sync();
             __syncwarp();
             if (lane == 0 && ok) mbar_arrive(smem_u32(&p_ready[i & 1]));
@@ -429,6 +439,17 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             fence_after_sync();
             const float inv = l > 0.0f ? 1.0f / l : 0.0f;
             const int token = seq_begin + tok0 + local, head = kh * args.group + (r - local * args.group);
+            if constexpr (MAPS) {
+                float* dst = args.maps + (((size_t)(blockIdx.x & 1) * args.n_tokens + token) * args.heads + head) * VD;
+#pragma unroll
+                for (int c = 0; c < VD; c += 32) {
+                    float o[32];
+                    tmem_load32(lane_base + L::O_COL + c, o);
+                    if (row_ok)
+#pragma unroll
+                        for (int e = 0; e < 32; e += 4) *reinterpret_cast<float4*>(dst + c + e) = make_float4(o[e] * inv, o[e + 1] * inv, o[e + 2] * inv, o[e + 3] * inv);
+                }
+            } else {
             __nv_bfloat16* dst = args.out + ((size_t)token * args.heads + head) * args.out_dim + half * O_COLS;
             const bool gated = SHAPED && args.gate != nullptr && row_ok;
             float head_gate = 1.0f;
@@ -474,6 +495,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                     }
                 }
             }
+            }
         }
     }
     fence_before_sync();
@@ -481,36 +503,53 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     if (warp == 1) tmem_dealloc(tmem_base, L::TMEM_COLS);
 }
 
-template <int HD, bool SHAPED>
+// A head's output from its two maps' (see differential_write in attention_forms.cu): o = a1 - lambda a2 divided by its root mean square, times
+// gain.  A warp a head of 128 numbers.
+__global__ void __launch_bounds__(256)
+differential_combine_kernel(const float* __restrict__ maps, long long rows, float lambda, float gain, float eps, __nv_bfloat16* __restrict__ out) {
+    tt_pdl_launch_dependents();
+    tt_pdl_wait();
+    const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (row >= rows) return;
+    const int c = 4 * (threadIdx.x & 31);
+    const float4 a = __ldg(reinterpret_cast<const float4*>(maps + row * 128 + c)), b = __ldg(reinterpret_cast<const float4*>(maps + (rows + row) * 128 + c));
+    const float4 o = make_float4(a.x - lambda * b.x, a.y - lambda * b.y, a.z - lambda * b.z, a.w - lambda * b.w);
+    const float r = rsqrtf(tt_warp_sum(fmaf(o.x, o.x, fmaf(o.y, o.y, fmaf(o.z, o.z, o.w * o.w)))) / 128.0f + eps) * gain;
+    __nv_bfloat162 v[2] = {__floats2bfloat162_rn(o.x * r, o.y * r), __floats2bfloat162_rn(o.z * r, o.w * r)};
+    *reinterpret_cast<uint2*>(out + row * 128 + c) = *reinterpret_cast<uint2*>(v);
+}
+
+template <int HD, bool SHAPED, bool MAPS = false>
 int launch(const void* q, const void* k_pool, const void* v_pool, const Args& args, int n_tokens, cudaStream_t stream) {
-    using L = Layout<HD>;
+    using L = Layout<HD, MAPS>;
+    constexpr int ROW = MAPS ? 2 * HD : HD;                      // numbers of a row of q or k
     CUtensorMap map_q, map_k, map_v;
     {   // q [token][head][dim]: a box of 64 dims x group heads x tokens_per_tile tokens = up to 128 rows of 128 bytes
-        const cuuint64_t dims[3] = {(cuuint64_t)HD, (cuuint64_t)args.heads, (cuuint64_t)n_tokens};
-        const cuuint64_t strides[2] = {(cuuint64_t)HD * 2, (cuuint64_t)args.heads * HD * 2};
+        const cuuint64_t dims[3] = {(cuuint64_t)ROW, (cuuint64_t)args.heads, (cuuint64_t)n_tokens};
+        const cuuint64_t strides[2] = {(cuuint64_t)ROW * 2, (cuuint64_t)args.heads * ROW * 2};
         const cuuint32_t box[3] = {64, (cuuint32_t)args.group, (cuuint32_t)args.tokens_per_tile};
         if (!tc::make_map(&map_q, q, 3, dims, strides, box)) return -1;
     }
     {   // keys [block * kv_head * 64 tokens][dim]
-        const cuuint64_t dims[2] = {(cuuint64_t)HD, (cuuint64_t)args.pool_blocks * args.kv_heads * KEYS};
-        const cuuint64_t strides[1] = {(cuuint64_t)HD * 2};
+        const cuuint64_t dims[2] = {(cuuint64_t)ROW, (cuuint64_t)args.pool_blocks * args.kv_heads * KEYS};
+        const cuuint64_t strides[1] = {(cuuint64_t)ROW * 2};
         const cuuint32_t box[2] = {64, KEYS};
         if (!tc::make_map(&map_k, k_pool, 2, dims, strides, box)) return -1;
     }
     {   // values [block * kv_head * dim][64 tokens]
-        const cuuint64_t dims[2] = {(cuuint64_t)KEYS, (cuuint64_t)args.pool_blocks * args.kv_heads * HD};
+        const cuuint64_t dims[2] = {(cuuint64_t)KEYS, (cuuint64_t)args.pool_blocks * args.kv_heads * L::VD};
         const cuuint64_t strides[1] = {(cuuint64_t)KEYS * 2};
-        const cuuint32_t box[2] = {KEYS, (cuuint32_t)HD};
+        const cuuint32_t box[2] = {KEYS, (cuuint32_t)L::VD};
         if (!tc::make_map(&map_v, v_pool, 2, dims, strides, box)) return -1;
     }
     static bool configured = false;
-    auto kernel = attention_tcgen05_kernel<HD, SHAPED>;
+    auto kernel = attention_tcgen05_kernel<HD, SHAPED, MAPS>;
     if (!configured) {
         const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM);
         if (err != cudaSuccess) return (int)err;
         configured = true;
     }
-    tt_launch_pdl(kernel, dim3(args.kv_heads, args.cta_tiles), dim3(L::THREADS), (size_t)L::SMEM, stream, map_q, map_k, map_v, args);
+    tt_launch_pdl(kernel, dim3(args.kv_heads * (MAPS ? 2 : 1), args.cta_tiles), dim3(L::THREADS), (size_t)L::SMEM, stream, map_q, map_k, map_v, args);
     return (int)cudaGetLastError();
 }
 
@@ -534,7 +573,7 @@ extern "C" int tt_attention_tcgen05(const void* q, const void* k_pool, const voi
     if (!tt_attention_tcgen05_supports(heads, kv_heads, head_dim) || ((uintptr_t)q & 15) || ((uintptr_t)k_pool & 15) || ((uintptr_t)v_pool & 15))
         return (int)cudaErrorInvalidValue;
     if (out_dim < 1 || out_dim > head_dim || (gate && out_dim != head_dim)) return (int)cudaErrorInvalidValue;
-    Args args;
+    Args args = {};
     args.out_dim = out_dim;
     args.table = table; args.table_width = table_width; args.pool_blocks = pool_blocks; args.cu = cu; args.len_before = len_before;
     args.sequences = sequences; args.heads = heads; args.kv_heads = kv_heads; args.group = heads / kv_heads;
@@ -550,4 +589,26 @@ extern "C" int tt_attention_tcgen05(const void* q, const void* k_pool, const voi
     }
     if (head_dim == 64) return launch<64, false>(q, k_pool, v_pool, args, n_tokens, stream);
     return launch<128, false>(q, k_pool, v_pool, args, n_tokens, stream);
+}
+
+// Differential attention of packed prompts, bfloat16, two maps of 64 numbers over values of 128: q [tokens][heads][2 x 64], key rows of 2 x 64 numbers.
+// maps: float32 scratch [2][tokens][heads][128].  out = norm(a1 - lambda a2) * gain as in tt_differential_attention.
+extern "C" int tt_differential_attention_tcgen05(const void* q, const void* k_pool, const void* v_pool, const int* table, int table_width, int pool_blocks,
+                                                 const int* cu, const int* len_before, int sequences, int n_tokens, int heads, int kv_heads, float scale,
+                                                 float lambda, float gain, float eps, float* maps, void* out, unsigned* status, cudaStream_t stream) {
+    if (n_tokens <= 0) return 0;
+    if (!tt_attention_tcgen05_supports(heads, kv_heads, 64) || (((uintptr_t)q | (uintptr_t)k_pool | (uintptr_t)v_pool | (uintptr_t)maps | (uintptr_t)out) & 15))
+        return (int)cudaErrorInvalidValue;
+    Args args = {};
+    args.table = table; args.table_width = table_width; args.pool_blocks = pool_blocks; args.cu = cu; args.len_before = len_before;
+    args.sequences = sequences; args.heads = heads; args.kv_heads = kv_heads; args.group = heads / kv_heads;
+    args.tokens_per_tile = ROWS / args.group;
+    args.cta_tiles = (n_tokens + args.tokens_per_tile - 1) / args.tokens_per_tile + sequences;
+    const long long rows = (long long)n_tokens * heads;
+    if (args.cta_tiles > 65535 || (rows + 7) / 8 > 2147483647LL) return (int)cudaErrorInvalidValue;
+    args.scale_log2 = scale * 1.4426950408889634f; args.status = status; args.maps = maps; args.n_tokens = n_tokens;
+    const int code = launch<64, false, true>(q, k_pool, v_pool, args, n_tokens, stream);
+    if (code != 0) return code;
+    tt_launch_pdl(differential_combine_kernel, dim3((unsigned)((rows + 7) / 8)), dim3(256), 0, stream, (const float*)maps, rows, lambda, gain, eps, (__nv_bfloat16*)out);
+    TT_LAUNCH_CHECK();
 }

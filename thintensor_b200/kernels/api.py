@@ -650,6 +650,30 @@ def differential_attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.
               _ptr(status), _stream()), "differential_attention", 2 if splits > 1 else 1)
 
 
+def differential_attention_tcgen05_takes(q: torch.Tensor, heads: int, kv_heads: int, dim: int, value_dim: int) -> bool:
+    """Whether :func:`differential_attention_tcgen05` takes these sizes."""
+    return q.dtype == torch.bfloat16 and dim == 64 and value_dim == 128 and heads % kv_heads == 0 and heads // kv_heads <= 16
+
+
+def differential_attention_tcgen05(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, table: torch.Tensor, cu: torch.Tensor,
+                                   len_before: torch.Tensor, sequences: int, n_tokens: int, heads: int, kv_heads: int, scale: float, lam: float,
+                                   gain: float, eps: float, maps: torch.Tensor, out: torch.Tensor, status: torch.Tensor) -> None:
+    """:func:`differential_attention` for prompts, two maps of 64 numbers over values of 128 in bfloat16, both products of a map on the
+    5th-generation tensor cores.  ``maps``: float32 scratch ``[2, tokens, heads, 128]``."""
+    for t, dtype, name in ((q, torch.bfloat16, "queries"), (k_pool, torch.bfloat16, "key pool"), (v_pool, torch.bfloat16, "value pool"),
+                           (out, torch.bfloat16, "output"), (maps, torch.float32, "maps")):
+        _need(t, dtype, name)
+    if (not differential_attention_tcgen05_takes(q, heads, kv_heads, k_pool.shape[-1] // 2, v_pool.shape[-2]) or tuple(q.shape) != (n_tokens, heads * 128)
+            or out.shape != q.shape or maps.numel() < 2 * n_tokens * heads * 128):
+        raise KernelError("differential attention on tcgen05: shapes do not fit")
+    fn = _fn("attention_tcgen05", "tt_differential_attention_tcgen05", "ppppiippiiiiffffpppp")
+    code = fn(_ptr(q), _ptr(k_pool), _ptr(v_pool), _ptr(table), table.shape[1], k_pool.shape[0], _ptr(cu), _ptr(len_before), sequences, n_tokens,
+              heads, kv_heads, scale, lam, gain, eps, _ptr(maps), _ptr(out), _ptr(status), _stream())
+    if code == -1:
+        raise KernelError("differential attention on tcgen05: a tensor map could not be made")
+    _check(code, "differential_attention_tcgen05", 2)
+
+
 def attention_forms_on_tensor_cores(dtype: torch.dtype, differential: bool, heads: int, kv_heads: int, dim: int, value_dim: int) -> bool:
     """Whether differential attention (``dim`` numbers a map) or window attention with pooled blocks (``value_dim == dim``)
     runs on tensor cores at these sizes: bfloat16, and a size the kernels are built for; its parallel unit is then a

@@ -35,6 +35,13 @@ def _slice_scratch(ctx, name: str, rows: int, splits: int, per_row: int, maps: i
             ctx.scratch(name + ".part_ml", (rows * splits * maps * 2,), torch.float32))
 
 
+def tiled_maps_pay(n_tokens: int, sequences: int) -> bool:
+    """Whether a prompt's maps are made in tiles of 128 rows on the 5th-generation tensor cores, one map a CTA, and not both maps of a few rows by
+    ``mma.sync``.  16 heads, 4 of keys (us, one B200, ``mma.sync`` and tiles): 128 tokens 9.2 and 9.6, 200 12.2 and 9.6, 500 21.5 and 16.8, 2,048 133 and
+    49, 4,200 511 and 142, five of 100 9.2 and 12.3, of 200 19.7 and 15.6; 8 heads, 2 of keys, five of 200 12.0 and 12.7, 300 15.2 and 11.5."""
+    return n_tokens >= 224 * sequences
+
+
 @MIXERS.register("differential_attention")
 class DifferentialAttention(Mixer):
     NAMES = {"q": "q_proj.weight", "k": "k_proj.weight", "v": "v_proj.weight", "o": "o_proj.weight", "q_bias": "q_proj.bias",
@@ -108,6 +115,11 @@ class DifferentialAttention(Mixer):
                                 cache.v_pool if cache.writes else None, table, ctx.cu, ctx.len_before, ctx.sequences, ctx.n_tokens,
                                 self.heads, self.kv_heads, row, self.value_dim, ctx.status, q_gain=self.q_gain)
         mixed = ctx.scratch("attention.mixed", (ctx.n_tokens, self.heads * self.value_dim))
+        if not ctx.decode and api.differential_attention_tcgen05_takes(q, self.heads, self.kv_heads, self.dim, self.value_dim) and tiled_maps_pay(ctx.n_tokens, ctx.sequences):
+            maps = ctx.scratch("differential.maps", (2, ctx.n_tokens, self.heads, 128), torch.float32)
+            api.differential_attention_tcgen05(q, cache.k_pool, cache.v_pool, table, ctx.cu, ctx.len_before, ctx.sequences, ctx.n_tokens, self.heads,
+                                               self.kv_heads, self.scale, self.lam, 1.0 - self.diff, self.eps, maps, mixed, ctx.status)
+            return self.out.delta(ctx, mixed, "attention.out")
         if self.on_tensor_cores is None:        # asked once: the answer depends on the sizes and the activations' type only
             self.on_tensor_cores = api.attention_forms_on_tensor_cores(q.dtype, True, self.heads, self.kv_heads, self.dim, self.value_dim)
         if self.on_tensor_cores:
