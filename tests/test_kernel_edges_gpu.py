@@ -827,3 +827,38 @@ def test_differential_attention_in_tiles(heads, kv_heads, news, before):
         want = o / norm * gain
         error = (out[span].double().view(-1, heads, 128) - want).abs()
         assert bool((error <= gain * (2.0 ** -7 * float(values.abs().max()) / norm + 2.0 ** -8 * want.abs())).all())
+
+
+@pytest.mark.parametrize("news,before", [([1, 15, 16, 17, 100], [0, 3, 16, 40, 60]), ([600], [127]), ([300, 0, 212], [0, 5, 64])])
+@pytest.mark.parametrize("kv_heads,head_dim,value_dim,from_keys", [(1, 64, 64, False), (3, 40, 72, False), (2, 96, 96, True)])
+def test_heads_and_values_of_prompts(news, before, kv_heads, head_dim, value_dim, from_keys):
+    """The plain copy (from 256 tokens in one slice on) and the general form: queries, keys and values where they belong, nothing else written."""
+    from thintensor_b200.kernels import api
+
+    tokens, sequences, heads, width = sum(news), len(news), 7, 12
+    cols = (heads + kv_heads) * head_dim + (0 if from_keys else kv_heads * value_dim)
+    proj = randn(1, tokens, cols, seed=160)
+    table = torch.randperm(sequences * width, device=DEV).int().view(sequences, width).contiguous()
+    k_pool = torch.full((sequences * width, kv_heads, 64, head_dim), 7.0, dtype=torch.bfloat16, device=DEV)
+    v_pool = torch.full((sequences * width, kv_heads, value_dim, 64), 7.0, dtype=torch.bfloat16, device=DEV)
+    q, status = torch.empty(tokens, heads * head_dim, dtype=torch.bfloat16, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    cu = [sum(news[:i]) for i in range(sequences + 1)]
+    api.qk_norm_rope_append(proj, None, None, 0.0, torch.zeros(1, device=DEV), 0, False, 1.0, q, k_pool, v_pool, table, i32(cu), i32(before), sequences, tokens, heads,
+                            kv_heads, head_dim, value_dim, status, **({"value_from_keys": True} if from_keys else {}))
+    assert int(status) == 0
+    want = torch.full_like(v_pool, 7.0)
+    at = heads * head_dim + (0 if from_keys else kv_heads * head_dim)
+    values = proj.sum(0)[:, at:at + kv_heads * value_dim].bfloat16().view(tokens, kv_heads, value_dim)
+    for s in range(sequences):
+        for i in range(news[s]):
+            place = before[s] + i
+            want[int(table[s, place // 64]), :, :, place % 64] = values[cu[s] + i]
+    assert torch.equal(v_pool, want)
+    keys = torch.full_like(k_pool, 7.0)
+    made = proj.sum(0).bfloat16()
+    assert torch.equal(q, made[:, :heads * head_dim])
+    for s in range(sequences):
+        for i in range(news[s]):
+            place = before[s] + i
+            keys[int(table[s, place // 64]), :, place % 64] = made[cu[s] + i, heads * head_dim:(heads + kv_heads) * head_dim].view(kv_heads, head_dim)
+    assert torch.equal(k_pool, keys)

@@ -824,6 +824,70 @@ __global__ void qk_norm_rope_append_kernel(const float* __restrict__ proj, int s
     for (int d = rotary_dim + lane; d < head_dim; d += 32) dst[d] = tt_from_float<TAct>(x[d]);
 }
 
+// The same where nothing is normed or rotated (differential layers): what is left is a copy, four numbers a lane, QK_PLAIN heads of a token by a warp
+// with their loads in flight together, the token's place found once.  Bound by its latency and the values' 2-byte writes: 2,048 tokens of 16
+// heads of 128 and 4 of keys and values 43 -> 16 us (38 MB; several heads a warp of the general form one after another took 51).
+constexpr int QK_PLAIN = 3;
+template <typename TAct>
+__global__ void __launch_bounds__(QK_WARPS * 32)
+qk_append_plain_kernel(const float* __restrict__ proj, int cols, TAct* __restrict__ q_out, TAct* __restrict__ k_pool, TAct* __restrict__ v_pool,
+                       const int* __restrict__ table, int table_width, int pool_blocks, const int* __restrict__ cu, const int* __restrict__ len_before,
+                       int sequences, int heads, int kv_heads, int head_dim, int value_dim, int write_cache, float q_gain_coef, int q_gain_every,
+                       unsigned* status) {
+    tt_pdl_launch_dependents();
+    const int t = blockIdx.x, items = heads + (write_cache ? 2 * kv_heads : 0), c = 4 * (threadIdx.x & 31);
+    const int item0 = (blockIdx.y * QK_WARPS + (threadIdx.x >> 5)) * QK_PLAIN;
+    if (item0 >= items) return;
+    const int b = tt_find_sequence(cu, sequences, t), pos = len_before[b] + (t - cu[b]);        // written before the step's first kernel
+    const int* table_row = table + (size_t)b * table_width;
+    tt_pdl_wait();
+    const int q_cols = heads * head_dim, k_cols = kv_heads * head_dim;
+    const float* row = proj + (size_t)t * cols;
+    float gain = 1.0f;
+    if (q_gain_every > 0) gain += q_gain_coef * logf((float)((pos + 1) / q_gain_every + 1));
+    for (int c0 = c; c0 < max(head_dim, value_dim); c0 += 128) {
+        float4 v[QK_PLAIN];
+#pragma unroll
+        for (int k = 0; k < QK_PLAIN; ++k) {
+            const int item = item0 + k, value = item - heads - kv_heads;
+            v[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (item < items && c0 < (value >= 0 ? value_dim : head_dim))
+                v[k] = __ldg(reinterpret_cast<const float4*>(row + (value >= 0 ? q_cols + k_cols + value * value_dim : item * head_dim) + c0));
+        }
+#pragma unroll
+        for (int k = 0; k < QK_PLAIN; ++k) {
+            const int item = item0 + k, value = item - heads - kv_heads;
+            if (item >= items || c0 >= (value >= 0 ? value_dim : head_dim)) continue;
+            if (value >= 0) {
+                const long long off = tt_value_offset(table_row, pos, value, kv_heads, value_dim, pool_blocks, status);
+                if (off < 0) continue;
+                TAct* to = v_pool + off + (long long)c0 * TT_BLOCK_TOKENS;
+                to[0] = tt_from_float<TAct>(v[k].x);
+                to[TT_BLOCK_TOKENS] = tt_from_float<TAct>(v[k].y);
+                to[2 * TT_BLOCK_TOKENS] = tt_from_float<TAct>(v[k].z);
+                to[3 * TT_BLOCK_TOKENS] = tt_from_float<TAct>(v[k].w);
+                continue;
+            }
+            TAct* to;
+            float r = 1.0f;
+            if (item < heads) {
+                to = q_out + (size_t)t * q_cols + item * head_dim;
+                r = gain;
+            } else {
+                const long long off = tt_cache_offset(table_row, pos, item - heads, kv_heads, head_dim, pool_blocks, status);
+                if (off < 0) continue;
+                to = k_pool + off;
+            }
+            if constexpr (sizeof(TAct) == 2) {
+                __nv_bfloat162 two[2] = {__floats2bfloat162_rn(v[k].x * r, v[k].y * r), __floats2bfloat162_rn(v[k].z * r, v[k].w * r)};
+                *reinterpret_cast<uint2*>(to + c0) = *reinterpret_cast<uint2*>(two);
+            } else {
+                *reinterpret_cast<float4*>(to + c0) = make_float4(v[k].x * r, v[k].y * r, v[k].z * r, v[k].w * r);
+            }
+        }
+    }
+}
+
 extern "C" int tt_qk_norm_rope_append(const float* proj, int splits, long long split_stride, int cols, const float* q_norm,
                                       const float* k_norm, float norm_eps, const float* inv_freq, int rotary_dim, int interleaved,
                                       float attention_scaling, void* q_out, void* k_pool, void* v_pool, int act_dtype,
@@ -838,6 +902,17 @@ extern "C" int tt_qk_norm_rope_append(const float* proj, int splits, long long s
     if ((cos_sin == nullptr) != (where == nullptr)) return (int)cudaErrorInvalidValue;
     if (rotary_dim < 0 || rotary_dim % 2 || rotary_dim > head_dim || head_dim <= 0 || value_dim <= 0) return (int)cudaErrorInvalidValue;
     if (value_from_keys && value_dim != head_dim) return (int)cudaErrorInvalidValue;
+    const int plain_items = heads + (write_cache ? 2 * kv_heads : 0), plain_rows = (plain_items + QK_WARPS * QK_PLAIN - 1) / (QK_WARPS * QK_PLAIN);
+    // (few tokens leave the warps of the general form, a head each, room)
+    if (n_tokens >= 256 && splits == 1 && rotary_dim == 0 && !q_norm && !k_norm && !unit_norm && !value_from_keys && head_dim % 4 == 0 && value_dim % 4 == 0 && cols % 4 == 0
+        && plain_rows <= 65535 && (((uintptr_t)proj | (uintptr_t)q_out | (uintptr_t)k_pool | (uintptr_t)v_pool) & 15) == 0) {
+        const dim3 grid(n_tokens, plain_rows);
+        if (act_dtype == TT_F32)
+            tt_launch_pdl(qk_append_plain_kernel<float>, grid, dim3(QK_WARPS * 32), 0, stream, proj, cols, (float*)q_out, (float*)k_pool, (float*)v_pool, table, table_width, pool_blocks, cu, len_before, sequences, heads, kv_heads, head_dim, value_dim, write_cache, q_gain_coef, q_gain_every, status);
+        else
+            tt_launch_pdl(qk_append_plain_kernel<__nv_bfloat16>, grid, dim3(QK_WARPS * 32), 0, stream, proj, cols, (__nv_bfloat16*)q_out, (__nv_bfloat16*)k_pool, (__nv_bfloat16*)v_pool, table, table_width, pool_blocks, cu, len_before, sequences, heads, kv_heads, head_dim, value_dim, write_cache, q_gain_coef, q_gain_every, status);
+        TT_LAUNCH_CHECK();
+    }
     const long long warps = (long long)n_tokens * (heads + (write_cache ? 2 * kv_heads : 0));
     const unsigned blocks = (unsigned)((warps + QK_WARPS - 1) / QK_WARPS);
     const size_t shared = (size_t)QK_WARPS * (head_dim > value_dim ? head_dim : value_dim) * sizeof(float);
