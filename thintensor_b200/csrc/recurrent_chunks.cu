@@ -67,15 +67,6 @@ __device__ __forceinline__ void ck_stage(float* to, int to_stride, const float* 
     }
 }
 
-__device__ __forceinline__ void ck_fma2(unsigned long long& d, unsigned long long a, unsigned long long b) {
-    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
-}
-__device__ __forceinline__ unsigned long long ck_pair(float lo, float hi) {
-    return ((unsigned long long)__float_as_uint(hi) << 32) | __float_as_uint(lo);
-}
-__device__ __forceinline__ float ck_lo(unsigned long long v) { return __uint_as_float((unsigned)v); }
-__device__ __forceinline__ float ck_hi(unsigned long long v) { return __uint_as_float((unsigned)(v >> 32)); }
-
 // Where a sequence's chunks lie among the slots of scratch memory: sequence b's first is cu[b] / 64 + b, which leaves room for
 // every chunk before the next sequence's first, whatever the lengths are.  n_tokens / 64 + sequences slots are enough.
 __device__ __forceinline__ int ck_first_slot(const int* __restrict__ cu, int b) { return cu[b] / CK_TOKENS + b; }
@@ -854,202 +845,6 @@ extern "C" int tt_scan_chunks(const float* rows, int width, int x_col, int b_col
     return c32 <= c16 ? scan_chunks_launch<128, 2, 4>(a, max_slots, stream) : scan_chunks_launch<128, 1, 8>(a, max_slots, stream);
 }
 
-// The products of a chunk's 64 output rows are shared out over the warps in blocks of rows and, so that a lane can hold four rows of
-// four neighbouring columns (an operand piece read from shared memory then serves four outputs, which is what bounds these
-// products), over slices of k: PL = TP / 4 lanes lie across the columns, RL = 32 / PL across the rows.
-// acc[r] += sum over k of A[row r][k] * B[k][columns], four k a step, k = k0, k0 + stride, ..; the next step's numbers are
-// on their way while this one's are multiplied.
-template <int RL>
-__device__ __forceinline__ void ck_product(unsigned long long (&acc)[4][2], const float* __restrict__ A, int lda, const float* __restrict__ B, int ldb, int k0, int stride, int k_end) {
-    float4 av[4], an[4];
-    ulonglong2 bv[4], bn[4];
-    auto load = [&](float4 (&x)[4], ulonglong2 (&y)[4], int k) {
-#pragma unroll
-        for (int r = 0; r < 4; ++r) x[r] = *reinterpret_cast<const float4*>(A + r * RL * lda + k);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) y[e] = *reinterpret_cast<const ulonglong2*>(B + (k + e) * ldb);
-    };
-    auto multiply = [&](const float4 (&x)[4], const ulonglong2 (&y)[4]) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const float v = e == 0 ? x[r].x : e == 1 ? x[r].y : e == 2 ? x[r].z : x[r].w;
-                const unsigned long long twice = ck_pair(v, v);
-                ck_fma2(acc[r][0], twice, y[e].x);
-                ck_fma2(acc[r][1], twice, y[e].y);
-            }
-    };
-    if (k0 >= k_end) return;
-    load(av, bv, k0);
-    for (int k = k0; k < k_end; k += 2 * stride) {
-        if (k + stride < k_end) load(an, bn, k + stride);
-        multiply(av, bv);
-        if (k + stride >= k_end) break;
-        if (k + 2 * stride < k_end) load(av, bv, k + 2 * stride);
-        multiply(an, bn);
-    }
-}
-
-// The same with what lies behind a row left out instead of multiplied by the zeros that stand there: for a chunk with numbers in B
-// that are not finite, which must not reach the tokens before them (0 * inf is no number).  row: this lane's first.
-template <int RL>
-__device__ __forceinline__ void ck_causal_product(unsigned long long (&acc)[4][2], const float* __restrict__ A, int lda, const float* __restrict__ B, int ldb, int k0, int stride, int k_end, int row) {
-#pragma unroll 1
-    for (int k = k0; k < k_end; k += stride)
-#pragma unroll 1
-        for (int e = 0; e < 4; ++e) {
-            const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(B + (k + e) * ldb);
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                if (k + e > row + RL * r) continue;
-                const float v = A[r * RL * lda + k + e];
-                const unsigned long long twice = ck_pair(v, v);
-                ck_fma2(acc[r][0], twice, y.x);
-                ck_fma2(acc[r][1], twice, y.y);
-            }
-        }
-}
-// zero for finite numbers, no number otherwise
-__device__ __forceinline__ float ck_not_finite(const float4& x) { return fmaf(x.x, 0.0f, fmaf(x.y, 0.0f, fmaf(x.z, 0.0f, x.w * 0.0f))); }
-
-// Two such products with the same B (k0 .. k0 + K - 1 in sums of 32, which are added up: a long chain of additions loses more)
-template <int RL, int K>
-__device__ __forceinline__ void ck_two_products(unsigned long long (&acc0)[4][2], const float* __restrict__ A0, unsigned long long (&acc1)[4][2],
-                                                const float* __restrict__ A1, int lda, const float* __restrict__ B, int ldb, int k0) {
-    constexpr int SUM = K < 32 ? K : 32;
-    float4 x0[2][4], x1[2][4];
-    ulonglong2 y[2][4];
-    auto load = [&](int at, int k) {
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            x0[at][r] = *reinterpret_cast<const float4*>(A0 + r * RL * lda + k);
-            x1[at][r] = *reinterpret_cast<const float4*>(A1 + r * RL * lda + k);
-        }
-#pragma unroll
-        for (int e = 0; e < 4; ++e) y[at][e] = *reinterpret_cast<const ulonglong2*>(B + (k + e) * ldb);
-    };
-    load(0, k0);
-#pragma unroll 1
-    for (int ks = 0; ks < K; ks += SUM) {
-        unsigned long long p0[4][2], p1[4][2];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) p0[r][0] = p0[r][1] = p1[r][0] = p1[r][1] = 0ull;
-#pragma unroll
-        for (int step = 0; step < SUM / 4; ++step) {
-            const int at = step & 1, next = ks + 4 * (step + 1);
-            if (next < K) load(at ^ 1, k0 + next);
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-#pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    const float v0 = e == 0 ? x0[at][r].x : e == 1 ? x0[at][r].y : e == 2 ? x0[at][r].z : x0[at][r].w;
-                    const float v1 = e == 0 ? x1[at][r].x : e == 1 ? x1[at][r].y : e == 2 ? x1[at][r].z : x1[at][r].w;
-                    const unsigned long long t0 = ck_pair(v0, v0), t1 = ck_pair(v1, v1);
-                    ck_fma2(p0[r][0], t0, y[at][e].x);
-                    ck_fma2(p0[r][1], t0, y[at][e].y);
-                    ck_fma2(p1[r][0], t1, y[at][e].x);
-                    ck_fma2(p1[r][1], t1, y[at][e].y);
-                }
-        }
-#pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-            for (int c = 0; c < 2; ++c) {
-                acc0[r][c] = ck_pair(ck_lo(acc0[r][c]) + ck_lo(p0[r][c]), ck_hi(acc0[r][c]) + ck_hi(p0[r][c]));
-                acc1[r][c] = ck_pair(ck_lo(acc1[r][c]) + ck_lo(p1[r][c]), ck_hi(acc1[r][c]) + ck_hi(p1[r][c]));
-            }
-    }
-}
-
-// acc += A * B over K numbers of k from k0 on, in sums of 32 (a long chain of additions loses more)
-template <int RL, int K>
-__device__ __forceinline__ void ck_state_product(unsigned long long (&acc)[4][2], const float* __restrict__ A, int lda, const float* __restrict__ B, int ldb, int k0) {
-    constexpr int SUM = K < 32 ? K : 32;
-#pragma unroll 1
-    for (int k = k0; k < k0 + K; k += SUM) {
-        unsigned long long part[4][2];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) part[r][0] = part[r][1] = 0ull;
-        ck_product<RL>(part, A, lda, B, ldb, k, 4, k + SUM);
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            acc[r][0] = ck_pair(ck_lo(acc[r][0]) + ck_lo(part[r][0]), ck_hi(acc[r][0]) + ck_hi(part[r][0]));
-            acc[r][1] = ck_pair(ck_lo(acc[r][1]) + ck_lo(part[r][1]), ck_hi(acc[r][1]) + ck_hi(part[r][1]));
-        }
-    }
-}
-
-// S <- all S + sum over the chunk's tokens of B[j] (w x)[j]^T: NL state rows and four columns of a lane; B: row j at j * NP
-template <int NP, int NL>
-__device__ __forceinline__ void ck_update(unsigned long long (&s)[NL][2], float all, const float* __restrict__ B, const float* __restrict__ XW, int ldx) {
-#pragma unroll
-    for (int i = 0; i < NL; ++i) {
-        s[i][0] = ck_pair(ck_lo(s[i][0]) * all, ck_hi(s[i][0]) * all);
-        s[i][1] = ck_pair(ck_lo(s[i][1]) * all, ck_hi(s[i][1]) * all);
-    }
-#pragma unroll 8
-    for (int j = 0; j < CK_TOKENS; ++j) {
-        float bv[NL];
-        if constexpr (NL == 4) {
-            const float4 q = *reinterpret_cast<const float4*>(B + j * NP);
-            bv[0] = q.x; bv[1] = q.y; bv[2] = q.z; bv[3] = q.w;
-        } else if constexpr (NL == 2) {
-            const float2 q = *reinterpret_cast<const float2*>(B + j * NP);
-            bv[0] = q.x; bv[1] = q.y;
-        } else {
-            bv[0] = B[j * NP];
-        }
-        const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(XW + j * ldx);
-#pragma unroll
-        for (int i = 0; i < NL; ++i) {
-            const unsigned long long twice = ck_pair(bv[i], bv[i]);
-            ck_fma2(s[i][0], twice, x.x);
-            ck_fma2(s[i][1], twice, x.y);
-        }
-    }
-}
-
-// A chunk's outputs: this lane's sums and the other slices', then skip times own (if there is one); rows from `left` on do not exist
-template <int RL, int SLICES>
-__device__ __forceinline__ void ck_outputs(const unsigned long long (&acc)[4][2], const float* __restrict__ parts, int ldx, int row, int col, int width, int left,
-                                           bool vec, float skip, const float4* own, float* __restrict__ out, int stride) {
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        const int i = row + RL * r;
-        float o[4] = {ck_lo(acc[r][0]), ck_hi(acc[r][0]), ck_lo(acc[r][1]), ck_hi(acc[r][1])};
-#pragma unroll
-        for (int k = 0; k < SLICES - 1; ++k) {
-            const float4 q = *reinterpret_cast<const float4*>(parts + (k * CK_TOKENS + i) * ldx + col);
-            o[0] += q.x; o[1] += q.y; o[2] += q.z; o[3] += q.w;
-        }
-        if (own) {
-            o[0] = fmaf(skip, own[r].x, o[0]); o[1] = fmaf(skip, own[r].y, o[1]);
-            o[2] = fmaf(skip, own[r].z, o[2]); o[3] = fmaf(skip, own[r].w, o[3]);
-        }
-        if (i >= left || col >= width) continue;
-        float* to = out + (size_t)i * stride + col;
-        if (vec) {
-            *reinterpret_cast<float4*>(to) = make_float4(o[0], o[1], o[2], o[3]);
-        } else {
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-                if (col + e < width) to[e] = o[e];
-        }
-    }
-}
-
-template <int NP, int TP>
-struct CkLayout {
-    static constexpr int LDA = NP + 4, LDX = TP + 4;
-    static constexpr int PL = TP / 4, RL = 32 / PL, ROWS = 4 * RL;          // lanes across columns and rows; output rows of a warp
-    static constexpr int THREADS = CK_THREADS, WARPS = THREADS / 32;
-    static constexpr int SLICES = WARPS * ROWS / CK_TOKENS;                 // of k
-    static constexpr int A = 0, S = A + CK_TOKENS * LDA, XW = S + NP * LDX, PARTS = XW + CK_TOKENS * LDX, STAGE = PARTS + (SLICES - 1) * CK_TOKENS * LDX;
-    static constexpr int B = 0, X = B + CK_TOKENS * NP, M = X + CK_TOKENS * LDX, F = M + CK_TOKENS * CK_MLD, STAGE_FLOATS = F + CK_FACTORS;
-    static constexpr size_t BYTES = (size_t)(STAGE + 2 * STAGE_FLOATS) * sizeof(float);
-};
-
 // ------------------------------------------------------------------------------------------------------ the gated delta rule
 //   q = q / |q| * scale, k = k / |k|;  S <- a_t S;  u_t = beta_t (v_t - S^T k_t);  S <- S + k_t u_t^T;  o_t = S^T q_t
 // (lengths with 1e-6 under the root, scale = D^-1/2).  Inside a chunk that starts from state S
@@ -1057,13 +852,13 @@ struct CkLayout {
 // is a unit lower triangular system, (I + A) U = beta V - (beta e K) S, whose solution is U = U0 - W S with (I + A) U0 = beta V and
 // (I + A) W = beta e K: neither needs the state, so the first kernel solves for both, parallel over chunks and heads, and the second
 // walks the chunks with   U = U0 - W S,   o = e Q S + P U (P_ij = f(i, j) q_i . k_j, j <= i),   S <- e_63 S + (w K)^T U.
-// Products and sums are float32 multiply-adds (lengths, and products of factors with scores, float64 rounded once: in float32 throughout the
-// outputs were 14 % further from 64 bits than token by token, now 15 % closer, for 2 % of the time); the systems are solved by forward
-// substitution, a column a thread.  16 heads of 128 x 128 on 4,097 tokens: 1,900 us token by token, now 486: the first kernel 130 (bound by issue and shared memory; two columns a thread and half the
-// threads 229, the whole substitution unrolled 278), the second 345 (bound like the one above; the two products with the state,
-// W S and Q S, take an operand of S from shared memory once for both: one after the other 408).
+// All products are the split products of split_mma.cuh, in the systems too (what the rows before a block of 16 take off it; the triangle of the 16
+// is float32 multiply-adds, a column a thread); lengths, and products of factors with scores, are formed in float64 and rounded once.  Against 64
+// bits, 24 runs, the outputs' error is 0.85 and the states' 0.94 of token by token in the mean (float32 multiply-adds in chunks: 0.91 and 0.94).
+// 16 heads of 128 x 128 on 4,097 tokens, us: token by token 1,900, chunks of float32 multiply-adds 485, now 379, of which the first kernel takes 150
+// (issue around splitting its operands, at two CTAs an SM; with scores and systems of multiply-adds 172) and the walk 246 (three barriers a
+// chunk and the latency of what lies between them; half of a chunk's time is its products).
 constexpr int CD_THREADS = 256;
-constexpr int CD_E = 0, CD_W = 64, CD_ALL = 128, CD_FACTORS = 136;        // of a chunk and head, for the second kernel
 
 struct DeltaChunks {
     const float* qkv;           // float32 rows [q | k | v]: query/key head g at g * D, value head h at 2 * qk_heads * D + h * V
@@ -1075,12 +870,25 @@ struct DeltaChunks {
     const float* a_log;
     float* state;               // [slots][heads][V][D]
     float* out;                 // [tokens][heads * V]
-    float* scratch;             // [slots][heads]: W [64][D], U0 [64][V], P [64][64], factors [CD_FACTORS]
+    unsigned* status;           // or null
+    unsigned char* scratch;     // [slots][qk_heads]: q as an operand of the walk; [slots][heads]: W, w K and the scores P as operands, the record, U0 [64][V]
     const int* cu;
     const int* slots;
-    int sequences, heads, qk_heads, D, V, vec, vec_v;
-    __host__ __device__ size_t chunk_floats() const { return (size_t)CK_TOKENS * (D + V + CK_TOKENS) + CD_FACTORS; }
-    __device__ float* chunk_scratch(int slot, int h) const { return scratch + ((size_t)slot * heads + h) * chunk_floats(); }
+    int sequences, max_slots, heads, qk_heads, D, V, vec;
+    static __host__ __device__ constexpr size_t matrix_bytes(int padded) { return (size_t)padded / 16 * 4 * SPLIT_BLOCK_BYTES; }
+    static __host__ __device__ constexpr size_t operand_bytes(int padded) { return 2 * matrix_bytes(padded) + CK_MBLOCKS * SPLIT_BLOCK_BYTES + CK_RECORD * sizeof(float); }
+    __host__ __device__ size_t head_bytes(int padded) const { return operand_bytes(padded) + (size_t)CK_TOKENS * V * sizeof(float); }
+    template <int NP> __device__ uint4* group_scratch(int slot, int g) const { return reinterpret_cast<uint4*>(scratch + ((size_t)slot * qk_heads + g) * matrix_bytes(NP)); }
+    template <int NP> __device__ uint4* head_scratch(int slot, int h) const {
+        return reinterpret_cast<uint4*>(scratch + (size_t)max_slots * qk_heads * matrix_bytes(NP) + ((size_t)slot * heads + h) * head_bytes(NP));
+    }
+    template <int NP> __device__ float* values(int slot, int h) const { return reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(head_scratch<NP>(slot, h)) + operand_bytes(NP)); }
+};
+
+template <int NP>
+struct CdPrepare {
+    static constexpr int LD = NP + 4;
+    static constexpr size_t BYTES = (size_t)(2 * CK_TOKENS * LD + 2 * CK_TOKENS * CK_MLD + CK_FACTORS + 7 * CK_TOKENS) * sizeof(float);
 };
 
 template <int NP>
@@ -1093,11 +901,13 @@ delta_chunks_prepare_kernel(const DeltaChunks a) {
     float* ks = ck_shared;                                      // [64][LD]
     float* qs = ks + CK_TOKENS * LD;                            // [64][LD]
     float* As = qs + CK_TOKENS * LD;                            // [64][CK_MLD]
-    float* f = As + CK_TOKENS * CK_MLD;                         // [CK_FACTORS]
+    float* Ps = As + CK_TOKENS * CK_MLD;                        // [64][CK_MLD]
+    float* f = Ps + CK_TOKENS * CK_MLD;                         // [CK_FACTORS]
     double* nq = reinterpret_cast<double*>(f + CK_FACTORS);     // [64] each: D^-1/2 / |q|, 1 / |k|; then beta
     double* nk = nq + CK_TOKENS;
     float* beta = reinterpret_cast<float*>(nk + CK_TOKENS);
     float* scalars = beta + CK_TOKENS;                          // [2][64]; then the rows' factors of W's right-hand side
+    __shared__ int bad;                                         // the first token with a number that is not finite
     const int slot = blockIdx.x, h = blockIdx.y, D = a.D, V = a.V;
     int lo = 0, hi = a.sequences;
     while (hi - lo > 1) {
@@ -1108,136 +918,191 @@ delta_chunks_prepare_kernel(const DeltaChunks a) {
     if (c0 >= n) return;
     const int count = min(CK_TOKENS, n - c0), g = h / (a.heads / a.qk_heads);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (D < NP) {
+    if (threadIdx.x == 0) bad = CK_TOKENS;
+    if (D < NP)
         for (int e = threadIdx.x; e < 2 * CK_TOKENS * LD; e += CD_THREADS) ck_shared[e] = 0.0f;
-        __syncthreads();
-    }
+    __syncthreads();
+    uint4* head = a.head_scratch<NP>(slot, h);
+    float* record = reinterpret_cast<float*>(head) + (2 * DeltaChunks::matrix_bytes(NP) + CK_MBLOCKS * SPLIT_BLOCK_BYTES) / 4;
     const float* rows = a.qkv + (size_t)(first + c0) * a.stride;
     ck_stage<NP, CD_THREADS>(qs, LD, rows + (size_t)g * D, a.stride, count, D, a.vec);
     ck_stage<NP, CD_THREADS>(ks, LD, rows + (size_t)(a.qk_heads + g) * D, a.stride, count, D, a.vec);
     ck_commit();
+    float raw_a[2] = {}, raw_b[2] = {};                         // the first warp's: what the chunk's decays and write strengths are made of
+    if (warp == 0)
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            const float* row = a.proj + (size_t)(first + c0 + lane + 32 * half) * a.cols + h;
+            if (lane + 32 * half < count) {
+                raw_a[half] = ck_sum_slices(row + a.a_col, a.splits, a.split_stride);
+                raw_b[half] = ck_sum_slices(row + a.b_col, a.splits, a.split_stride);
+            }
+        }
+    ck_wait<0>();
+    __syncthreads();
+    // numbers that are not finite are left out here: the walk takes such a token and what follows it in the chunk one by one
+    for (int e = threadIdx.x; e < 2 * CK_TOKENS * (NP / 4); e += CD_THREADS) {
+        const int row = e / (NP / 4);
+        float* at = ck_shared + row * LD + 4 * (e % (NP / 4));
+        const float4 v = *reinterpret_cast<const float4*>(at);
+        if (!(ck_usable(v.x) && ck_usable(v.y) && ck_usable(v.z) && ck_usable(v.w))) {
+            atomicMin(&bad, row & (CK_TOKENS - 1));
+            *reinterpret_cast<float4*>(at) = make_float4(ck_usable(v.x) ? v.x : 0.0f, ck_usable(v.y) ? v.y : 0.0f, ck_usable(v.z) ? v.z : 0.0f, ck_usable(v.w) ? v.w : 0.0f);
+        }
+    }
+    __syncthreads();
+    // lengths: four lanes a row
+    for (int item = threadIdx.x >> 2; item < 2 * CK_TOKENS; item += CD_THREADS / 4) {
+        const float* row = (item < CK_TOKENS ? qs : ks) + (item & (CK_TOKENS - 1)) * LD;
+        double sum = 0.0, more = 0.0;                           // (zeros behind D)
+        for (int c = threadIdx.x & 3; c < NP; c += 8) {
+            sum = fma((double)row[c], (double)row[c], sum);
+            more = fma((double)row[c + 4], (double)row[c + 4], more);
+        }
+        sum += more;
+        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+        if (!(threadIdx.x & 3)) (item < CK_TOKENS ? nq : nk)[item & (CK_TOKENS - 1)] = 1.0 / sqrt((sum + 1e-6) * (item < CK_TOKENS ? (double)D : 1.0));
+    }
+    // k . k and q . k on and below the diagonal, a warp 16 rows of the one or the other; the first, whose rows are the shortest, makes the factors too
+    const int t2 = 2 * (lane & 3), gq = lane >> 2;
     if (warp == 0) {
         float decay[2];
         const float neg_a = -expf(__ldg(a.a_log + h)), bias = __ldg(a.dt_bias + h);
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
             const int i = lane + 32 * half;
-            const float* row = a.proj + (size_t)(first + c0 + i) * a.cols + h;
             decay[half] = 1.0f;
             float write = 0.0f;
             if (i < count) {
-                const float raw = ck_sum_slices(row + a.a_col, a.splits, a.split_stride) + bias;
+                const float raw = raw_a[half] + bias;
                 decay[half] = expf(neg_a * (raw > 20.0f ? raw : log1pf(expf(raw))));
-                write = 1.0f / (1.0f + expf(-ck_sum_slices(row + a.b_col, a.splits, a.split_stride)));
+                write = 1.0f / (1.0f + expf(-raw_b[half]));
             }
-            beta[i] = write;
+            if (!ck_usable(decay[half]) || !ck_usable(write)) atomicMin(&bad, i);
+            beta[i] = ck_usable(write) ? write : 0.0f;
+            record[CK_R_DECAY + i] = decay[half];
+            record[CK_R_DT + i] = write;
         }
         ck_factors(f, decay[0], decay[1], 1.0f, 1.0f, lane, scalars, scalars + CK_TOKENS);
     }
-    ck_wait<0>();
-    __syncthreads();
-    // lengths: four lanes a row
-    for (int item = threadIdx.x >> 2; item < 2 * CK_TOKENS; item += CD_THREADS / 4) {
-        const float* row = (item < CK_TOKENS ? qs : ks) + (item & (CK_TOKENS - 1)) * LD;
-        double sum = 0.0;
-        for (int c = threadIdx.x & 3; c < D; c += 4) sum = fma((double)row[c], (double)row[c], sum);
-        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-        if (!(threadIdx.x & 3)) (item < CK_TOKENS ? nq : nk)[item & (CK_TOKENS - 1)] = 1.0 / sqrt((sum + 1e-6) * (item < CK_TOKENS ? (double)D : 1.0));
-    }
-    __syncthreads();
-    float* scratch = a.chunk_scratch(slot, h);
-    float* P = scratch + (size_t)CK_TOKENS * (D + V);
-    // k . k and q . k: 16 x 16 threads, rows and columns 16 apart
     {
-        const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-        float kk[4][4], qk[4][4];
-#pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) kk[r][c] = qk[r][c] = 0.0f;
+        const int q = warp >> 1;
+        float sums[4][2][4] = {}, rest[4][2][4] = {};
+        auto rows_of = [&](const float* m, int row, int k, float2 (&v)[2]) {
+            const float* at = m + row * LD + 16 * k + t2;
+            v[0] = *reinterpret_cast<const float2*>(at);
+            v[1] = *reinterpret_cast<const float2*>(at + 8);
+        };
 #pragma unroll 1
-        for (int k0 = 0; k0 < NP; k0 += 32) {                   // sums of 8, added up to 32, added up: long chains lose more
-            float hk[4][4], hq[4][4];
+        for (int k = 0; k < NP / 16; ++k) {
+            SplitA A;
+            float2 v[2];
 #pragma unroll
-            for (int r = 0; r < 4; ++r)
-#pragma unroll
-                for (int c = 0; c < 4; ++c) hk[r][c] = hq[r][c] = 0.0f;
-#pragma unroll 1
-            for (int k1 = k0; k1 < k0 + 32; k1 += 8) {
-                float pk[4][4], pq[4][4];
-#pragma unroll
-                for (int r = 0; r < 4; ++r)
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) pk[r][c] = pq[r][c] = 0.0f;
-#pragma unroll
-                for (int k = k1; k < k1 + 8; k += 4) {
-                    float4 b[4];
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) b[c] = *reinterpret_cast<const float4*>(ks + (tx + 16 * c) * LD + k);
-#pragma unroll
-                    for (int r = 0; r < 4; ++r) {
-                        const float4 x = *reinterpret_cast<const float4*>(ks + (ty + 16 * r) * LD + k), y = *reinterpret_cast<const float4*>(qs + (ty + 16 * r) * LD + k);
-#pragma unroll
-                        for (int c = 0; c <= r; ++c) {              // the others lie above the diagonal
-                            pk[r][c] = fmaf(x.x, b[c].x, pk[r][c]); pk[r][c] = fmaf(x.y, b[c].y, pk[r][c]);
-                            pk[r][c] = fmaf(x.z, b[c].z, pk[r][c]); pk[r][c] = fmaf(x.w, b[c].w, pk[r][c]);
-                            pq[r][c] = fmaf(y.x, b[c].x, pq[r][c]); pq[r][c] = fmaf(y.y, b[c].y, pq[r][c]);
-                            pq[r][c] = fmaf(y.z, b[c].z, pq[r][c]); pq[r][c] = fmaf(y.w, b[c].w, pq[r][c]);
-                        }
-                    }
-                }
-#pragma unroll
-                for (int r = 0; r < 4; ++r)
-#pragma unroll
-                    for (int c = 0; c <= r; ++c) { hk[r][c] += pk[r][c]; hq[r][c] += pq[r][c]; }
+            for (int e = 0; e < 2; ++e) {
+                rows_of(warp & 1 ? qs : ks, 16 * q + gq + 8 * e, k, v);
+                split_pair(v[0].x, v[0].y, A.hi[e], A.mid[e], A.lo[e]);
+                split_pair(v[1].x, v[1].y, A.hi[2 + e], A.mid[2 + e], A.lo[2 + e]);
             }
 #pragma unroll
-            for (int r = 0; r < 4; ++r)
+            for (int s = 0; s < 4; ++s) {
+                if (s > q) continue;
+                uint32_t hi[2][2], mid[2][2], lo[2][2];
 #pragma unroll
-                for (int c = 0; c <= r; ++c) { kk[r][c] += hk[r][c]; qk[r][c] += hq[r][c]; }
+                for (int tile = 0; tile < 2; ++tile) {
+                    rows_of(ks, 16 * s + 8 * tile + gq, k, v);
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) split_pair(v[e].x, v[e].y, hi[tile][e], mid[tile][e], lo[tile][e]);
+                }
+#pragma unroll
+                for (int tile = 0; tile < 2; ++tile) split_mma(rest[s][tile], A.lo, hi[tile][0], hi[tile][1]);
+#pragma unroll
+                for (int tile = 0; tile < 2; ++tile) split_mma_add(sums[s][tile], A.hi, hi[tile][0], hi[tile][1]);
+#pragma unroll
+                for (int tile = 0; tile < 2; ++tile) split_mma(rest[s][tile], A.hi, lo[tile][0], lo[tile][1]);
+#pragma unroll
+                for (int tile = 0; tile < 2; ++tile) split_mma(rest[s][tile], A.mid, mid[tile][0], mid[tile][1]);
+#pragma unroll
+                for (int tile = 0; tile < 2; ++tile) split_mma(rest[s][tile], A.mid, hi[tile][0], hi[tile][1]);
+#pragma unroll
+                for (int tile = 0; tile < 2; ++tile) split_mma(rest[s][tile], A.hi, mid[tile][0], mid[tile][1]);
+            }
         }
+        __syncthreads();                                        // lengths, factors and write strengths are there
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const int i = ty + 16 * r, bi = i >> 3;
+        for (int s = 0; s < 4; ++s) {
+            if (s > q) continue;
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const int j = tx + 16 * c, bj = j >> 3;
-                if (c > r) {
-                    As[i * CK_MLD + j] = P[i * CK_TOKENS + j] = 0.0f;
-                    continue;
+            for (int tile = 0; tile < 2; ++tile)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int i = 16 * q + gq + 8 * (e >> 1), j = 16 * s + 8 * tile + t2 + (e & 1), bi = 2 * q + (e >> 1), bj = 2 * s + tile;
+                    // products of the factors in float64, rounded once
+                    const double fij = bi > bj ? (double)f[CK_U + i] * (double)f[CK_BLOCKS + bi * 8 + bj] * (double)f[CK_V + j]
+                                     : bi == bj ? (double)f[CK_DIAG + bi * 64 + (i & 7) * 8 + (j & 7)] : 0.0;
+                    const double product = fij * nk[j] * ((double)sums[s][tile][e] + (double)rest[s][tile][e]);
+                    float m = warp & 1 ? (j <= i ? (float)(nq[i] * product) : 0.0f) : (j < i ? -(float)((double)beta[i] * nk[i] * product) : 0.0f);        // P, -A
+                    if (!ck_usable(m)) {
+                        atomicMin(&bad, i);
+                        m = 0.0f;
+                    }
+                    (warp & 1 ? Ps : As)[i * CK_MLD + j] = m;
                 }
-                // products of the factors in float64, rounded once
-                const double fij = bi > bj ? (double)f[CK_U + i] * (double)f[CK_BLOCKS + bi * 8 + bj] * (double)f[CK_V + j] : bi == bj ? (double)f[CK_DIAG + bi * 64 + (i & 7) * 8 + (j & 7)] : 0.0;
-                const double fk = fij * nk[j];
-                As[i * CK_MLD + j] = j < i ? -(float)((double)beta[i] * nk[i] * fk * (double)kk[r][c]) : 0.0f;         // -A
-                P[i * CK_TOKENS + j] = j <= i ? (float)(nq[i] * fk * (double)qk[r][c]) : 0.0f;
-            }
         }
     }
     if (threadIdx.x < CK_TOKENS) {
-        float* factors = P + CK_TOKENS * CK_TOKENS;
-        factors[CD_E + threadIdx.x] = (float)((double)f[CK_E + threadIdx.x] * nq[threadIdx.x]);
-        factors[CD_W + threadIdx.x] = (float)((double)f[CK_W + threadIdx.x] * nk[threadIdx.x]);
-        scalars[threadIdx.x] = (float)((double)beta[threadIdx.x] * (double)f[CK_E + threadIdx.x] * nk[threadIdx.x]);
-        if (threadIdx.x == 0) factors[CD_ALL] = f[CK_ALL];
+        const int i = threadIdx.x;
+        const float start = (float)((double)beta[i] * (double)f[CK_E + i] * nk[i]), w = (float)((double)f[CK_W + i] * nk[i]);
+        record[CK_R_E + i] = (float)((double)f[CK_E + i] * nq[i]);
+        scalars[i] = ck_usable(start) ? start : 0.0f;
+        scalars[CK_TOKENS + i] = ck_usable(w) ? w : 0.0f;       // (not so: no column's state comes from these products)
+        if (i == 0) record[CK_R_ALL] = f[CK_ALL];
     }
     __syncthreads();
-    // (I + A) x = r for the columns of beta e K (made W) and of beta V (made U0), one a thread, 16 rows at a time: what the rows
-    // before contribute as a product (sums of 16 added up), then the triangle of the 16.  Half of the CTA takes the keys'
+    // the operands that do not need the systems: w K (k = tokens, columns = state rows), and by the first head of a group q (k = state rows, columns = tokens)
+    constexpr int KS = NP / 16, BLOCK = SPLIT_BLOCK_BYTES / 16;
+    auto by_token = [&](const float* m, int item, float (&v)[2][4]) {           // k = the matrix' columns, columns = its rows
+        const int ks = item >> 2, q = item & 3;
+#pragma unroll
+        for (int tile = 0; tile < 2; ++tile) {
+            const float* at = m + (16 * q + 8 * tile + gq) * LD + 16 * ks + t2;
+            const float2 x = *reinterpret_cast<const float2*>(at), y = *reinterpret_cast<const float2*>(at + 8);
+            v[tile][0] = x.x; v[tile][1] = x.y; v[tile][2] = y.x; v[tile][3] = y.y;
+        }
+    };
+    for (int item = warp; item < KS * 4; item += CD_THREADS / 32) {
+        float v[2][4];
+        const int j = item / KS, q = item % KS;
+#pragma unroll
+        for (int tile = 0; tile < 2; ++tile)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int token = 16 * j + t2 + (e & 1) + 8 * (e >> 1);
+                v[tile][e] = scalars[CK_TOKENS + token] * ks[token * LD + 16 * q + 8 * tile + gq];
+            }
+        split_store(head + DeltaChunks::matrix_bytes(NP) / 16 + item * BLOCK, lane, v);
+        if (h % (a.heads / a.qk_heads) == 0) {
+            by_token(qs, item, v);
+            split_store(a.group_scratch<NP>(slot, g) + item * BLOCK, lane, v);
+        }
+    }
+    __syncthreads();                                            // keys and queries are read
+    // (I + A) x = r for the columns of beta e K (made W) and of beta V (made U0), 16 rows at a time: what the rows before contribute as a product on the
+    // tensor cores, a warp its 32 columns, then the triangle of the 16, a column a thread.  Half of the CTA takes the keys'
     // columns, in place, and every second tile of NP value columns; the other half the other tiles, where the queries lay.
     const int half = threadIdx.x / (CD_THREADS / 2), col = threadIdx.x % (CD_THREADS / 2);
     float* xs = (half ? qs : ks) + col;
     const float* values = rows + (size_t)2 * a.qk_heads * D + (size_t)h * V;
-    for (int job = half; (job - 1) * NP < V; job += 2) {       // job 0: the keys; job t: value columns from (t - 1) * NP on
+    auto solve = [&](int job) {                                 // job 0: the keys; job t: value columns from (t - 1) * NP on
         const int c = (job ? (job - 1) * NP : 0) + col, width = job ? V : D;
-        if (col >= NP || c >= width) continue;
-        float* to = scratch + (job ? (size_t)CK_TOKENS * D : 0) + c;
+        if (col - lane >= NP || c - lane >= width) return;      // the same for the whole warp
+        const bool live = c < width;
+        float* to = a.values<NP>(slot, h) + c;
         float raw[16];                                          // the next 16 rows' values, fetched ahead
         auto fetch = [&](int i0) {
             if (!job) return;
 #pragma unroll
-            for (int r = 0; r < 16; ++r) raw[r] = i0 + r < count ? __ldg(values + (size_t)(i0 + r) * a.stride + c) : 0.0f;
+            for (int r = 0; r < 16; ++r) raw[r] = live && i0 + r < count ? __ldg(values + (size_t)(i0 + r) * a.stride + c) : 0.0f;
         };
         fetch(0);
 #pragma unroll 1
@@ -1245,33 +1110,48 @@ delta_chunks_prepare_kernel(const DeltaChunks a) {
             // the right-hand side, and what the rows before take off it, summed apart: many small terms added to x one by one would each round it
             float x[16], before[16];
 #pragma unroll
-            for (int r = 0; r < 16; ++r) {
-                const int i = i0 + r;
-                before[r] = 0.0f;
-                x[r] = job ? beta[i] * raw[r] : scalars[i] * xs[i * LD];
-            }
+            for (int r = 0; r < 16; ++r) x[r] = job ? beta[i0 + r] * raw[r] : scalars[i0 + r] * xs[(i0 + r) * LD];
             if (i0 + 16 < CK_TOKENS) fetch(i0 + 16);
+            if (i0) {
+                float sums[4][4] = {}, rest[4][4] = {};
+                const float* mine = xs - lane;
 #pragma unroll 1
-            for (int j0 = 0; j0 < i0; j0 += 16) {
-                float sum[16];
+                for (int j0 = 0; j0 < i0; j0 += 16) {
+                    SplitA A;
 #pragma unroll
-                for (int r = 0; r < 16; ++r) sum[r] = 0.0f;
+                    for (int e = 0; e < 4; ++e) {
+                        const float2 v = *reinterpret_cast<const float2*>(As + (i0 + gq + 8 * (e & 1)) * CK_MLD + j0 + t2 + 8 * (e >> 1));
+                        split_pair(v.x, v.y, A.hi[e], A.mid[e], A.lo[e]);
+                    }
 #pragma unroll
-                for (int j = j0; j < j0 + 16; j += 4) {
-                    float y[4];
+                    for (int tile = 0; tile < 4; ++tile) {
+                        uint32_t hi[2], mid[2], lo[2];
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) y[e] = xs[(j + e) * LD];
-#pragma unroll
-                    for (int r = 0; r < 16; ++r) {
-                        const float4 m = *reinterpret_cast<const float4*>(As + (i0 + r) * CK_MLD + j);
-                        sum[r] = fmaf(m.x, y[0], sum[r]);
-                        sum[r] = fmaf(m.y, y[1], sum[r]);
-                        sum[r] = fmaf(m.z, y[2], sum[r]);
-                        sum[r] = fmaf(m.w, y[3], sum[r]);
+                        for (int e = 0; e < 2; ++e) {
+                            const float* at = mine + (j0 + t2 + 8 * e) * LD + 8 * tile + gq;
+                            split_pair(at[0], at[LD], hi[e], mid[e], lo[e]);
+                        }
+                        split_mma(rest[tile], A.lo, hi[0], hi[1]);
+                        split_mma_add(sums[tile], A.hi, hi[0], hi[1]);
+                        split_mma(rest[tile], A.hi, lo[0], lo[1]);
+                        split_mma(rest[tile], A.mid, mid[0], mid[1]);
+                        split_mma(rest[tile], A.mid, hi[0], hi[1]);
+                        split_mma(rest[tile], A.hi, mid[0], mid[1]);
                     }
                 }
+                __syncwarp();                                   // the right-hand sides are read: the sums take their place on the way to their columns' threads
+                float* out = xs - lane + (i0 + gq) * LD + t2;
 #pragma unroll
-                for (int r = 0; r < 16; ++r) before[r] += sum[r];
+                for (int tile = 0; tile < 4; ++tile)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e)
+                        *reinterpret_cast<float2*>(out + 8 * e * LD + 8 * tile) = make_float2(sums[tile][2 * e] + rest[tile][2 * e], sums[tile][2 * e + 1] + rest[tile][2 * e + 1]);
+                __syncwarp();
+#pragma unroll
+                for (int r = 0; r < 16; ++r) before[r] = xs[(i0 + r) * LD];
+            } else {
+#pragma unroll
+                for (int r = 0; r < 16; ++r) before[r] = 0.0f;
             }
             x[0] += before[0];
 #pragma unroll
@@ -1289,179 +1169,358 @@ delta_chunks_prepare_kernel(const DeltaChunks a) {
 #pragma unroll
             for (int r = 0; r < 16; ++r) {
                 xs[(i0 + r) * LD] = x[r];
-                to[(size_t)(i0 + r) * width] = x[r];
+                if (job && live) to[(size_t)(i0 + r) * width] = x[r];
             }
+            __syncwarp();
+        }
+    };
+    for (int job = half; (job - 1) * NP < V; job += 2) {
+        solve(job);
+        if (job == 0) {                                         // W lies where the keys were: as an operand, before value columns take its place
+            asm volatile("bar.sync 1, %0;" ::"n"(CD_THREADS / 2) : "memory");
+            for (int item = warp; item < KS * 4 + CK_MBLOCKS; item += CD_THREADS / 64) {
+                float v[2][4];
+                if (item < KS * 4) {
+                    by_token(ks, item, v);
+#pragma unroll
+                    for (int tile = 0; tile < 2; ++tile)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e)
+                            if (!ck_usable(v[tile][e])) {
+                                atomicMin(&bad, 16 * (item & 3) + 8 * tile + gq);
+                                v[tile][e] = 0.0f;
+                            }
+                    split_store(head + item * BLOCK, lane, v);
+                } else {
+                    const int block = item - KS * 4, q = ck_block_row(block), s = block - q * (q + 1) / 2;
+#pragma unroll
+                    for (int tile = 0; tile < 2; ++tile) {
+                        const float* at = Ps + (16 * q + 8 * tile + gq) * CK_MLD + 16 * s + t2;
+                        const float2 x = *reinterpret_cast<const float2*>(at), y = *reinterpret_cast<const float2*>(at + 8);
+                        v[tile][0] = x.x; v[tile][1] = x.y; v[tile][2] = y.x; v[tile][3] = y.y;
+                    }
+                    split_store(head + 2 * DeltaChunks::matrix_bytes(NP) / 16 + block * BLOCK, lane, v);
+                }
+            }
+            if (V > NP) asm volatile("bar.sync 1, %0;" ::"n"(CD_THREADS / 2) : "memory");
         }
     }
+    __syncthreads();
+    if (threadIdx.x == 0) reinterpret_cast<int*>(record)[CK_R_BAD] = bad;
 }
 
-template <int NP, int TP>
-struct CdLayout {
-    using L = CkLayout<NP, TP>;                                 // lanes, rows and slices as above
-    static constexpr int LDA = L::LDA, LDX = L::LDX;
-    static constexpr int Q = 0, W = Q + CK_TOKENS * LDA, S = W + CK_TOKENS * LDA, XW = S + NP * LDX, PARTS = XW + CK_TOKENS * LDX;
-    static constexpr int STAGE = PARTS + (L::SLICES - 1) * CK_TOKENS * LDX;
-    static constexpr int K = 0, X = K + CK_TOKENS * NP, M = X + CK_TOKENS * LDX, F = M + CK_TOKENS * CK_MLD, STAGE_FLOATS = F + CD_FACTORS;
-    static constexpr size_t BYTES = (size_t)(STAGE + 2 * STAGE_FLOATS) * sizeof(float);
+// One column's chunk token by token, by one warp: for chunks with numbers that are not finite.  Outputs from token `from` on.
+__device__ __noinline__ void ck_delta_column(const DeltaChunks& a, const float* record, int token, int count, int h, int g, int p, float* S, int from) {
+    const int lane = threadIdx.x & 31, D = a.D;
+    float s[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) s[r] = lane + 32 * r < D ? S[lane + 32 * r] : 0.0f;
+    for (int i = 0; i < count; ++i) {
+        const float* row = a.qkv + (size_t)(token + i) * a.stride;
+        float q[4], k[4], qq = 0.0f, kk = 0.0f, sk = 0.0f, o = 0.0f;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int n = lane + 32 * r;
+            q[r] = n < D ? row[(size_t)g * D + n] : 0.0f;
+            k[r] = n < D ? row[(size_t)(a.qk_heads + g) * D + n] : 0.0f;
+            qq = fmaf(q[r], q[r], qq);
+            kk = fmaf(k[r], k[r], kk);
+        }
+        const float nq = rsqrtf(tt_warp_sum(qq) + 1e-6f) * rsqrtf((float)D), nk = rsqrtf(tt_warp_sum(kk) + 1e-6f), decay = record[CK_R_DECAY + i];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            k[r] *= nk;
+            s[r] *= decay;
+            if (lane + 32 * r < D) sk = fmaf(s[r], k[r], sk);
+        }
+        const float u = record[CK_R_DT + i] * (row[(size_t)2 * a.qk_heads * D + (size_t)h * a.V + p] - tt_warp_sum(sk));
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+            if (lane + 32 * r < D) {
+                s[r] = fmaf(k[r], u, s[r]);
+                o = fmaf(s[r], q[r] * nq, o);
+            }
+        o = tt_warp_sum(o);
+        if (lane == 0 && i >= from) a.out[(size_t)(token + i) * a.heads * a.V + (size_t)h * a.V + p] = o;
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+        if (lane + 32 * r < D) S[lane + 32 * r] = s[r];
+}
+
+// The walk, transposed and split like the scan's: a warp holds 16 value columns and a slice of the state's rows.  W S and Q S of a chunk are added up over
+// the slices through shared memory, and of what comes of it U^T goes back as the operand of both products that need it; a warp that adds up a tile
+// of 8 tokens also makes its outputs.  w is in K already, which the first kernel wrote.
+template <int NP, int PB, int NS>
+struct CdWalk {
+    static constexpr int THREADS = 32 * PB * NS, TP = 16 * PB, KS = NP / 16, KL = KS / NS, EACH = 8 / NS;
+    static constexpr int MATRIX = KS * 4 * SPLIT_BLOCK_BYTES;
+    static constexpr int W = 0, Q = W + MATRIX, K = Q + MATRIX, M = K + MATRIX, R = M + CK_MBLOCKS * SPLIT_BLOCK_BYTES, PARTS = R + 2 * CK_RECORD * 4;
+    static constexpr int U = PARTS + 2 * PB * (NS - 1) * 8 * 512, BAD = U + PB * 4 * SPLIT_BLOCK_BYTES, BAR = BAD + TP * 4, BYTES = BAR + 16;
+    static constexpr int REST_BYTES = CK_MBLOCKS * SPLIT_BLOCK_BYTES + MATRIX;
 };
 
-template <int NP, int TP>
-__global__ void __launch_bounds__(CK_THREADS, 1)
+template <int NP, int PB, int NS>
+__global__ void __launch_bounds__(32 * PB * NS, 1)
 delta_chunks_kernel(const DeltaChunks a) {
-    using D_ = CdLayout<NP, TP>;
-    using L = CkLayout<NP, TP>;
-    constexpr int PL = L::PL, RL = L::RL, ROW_BLOCKS = CK_TOKENS / L::ROWS, SLICE_K = NP / L::SLICES;
-    constexpr int NL = NP * TP / (CK_THREADS * 4);              // state rows of a lane
-    extern __shared__ __align__(16) float ck_shared[];
+    using L = CdWalk<NP, PB, NS>;
+    constexpr int THREADS = L::THREADS, TP = L::TP, KL = L::KL, EACH = L::EACH, BLOCK = SPLIT_BLOCK_BYTES / 16, PAIR = KL > 1 ? 2 : 1;
+    extern __shared__ __align__(16) unsigned char ck_bytes[];
     tt_pdl_launch_dependents();
     tt_pdl_wait();
     const int h = blockIdx.x, b = blockIdx.y, p0 = blockIdx.z * TP;
     const int first = a.cu[b], n = a.cu[b + 1] - first;
     if (n <= 0) return;
-    const int g = h / (a.heads / a.qk_heads), V = a.V, D = a.D;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int col = 4 * (lane % PL), width = min(TP, V - p0);
-    const int slice = warp / ROW_BLOCKS, block = (warp + (warp >> 2)) % ROW_BLOCKS;
-    const int row = block * L::ROWS + lane / PL;
-    const int srow = warp * (NP / CK_WARPS) + (lane / PL) * NL;
-    float* Qs = ck_shared + D_::Q;
-    float* Ws = ck_shared + D_::W;
-    float* Ss = ck_shared + D_::S;
-    float* XW = ck_shared + D_::XW;
+    const int g = h / (a.heads / a.qk_heads), V = a.V, D = a.D, width = min(TP, V - p0);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, pb = warp / NS, ns = warp % NS;
+    const int t2 = 2 * (lane & 3), gq = lane >> 2;
     const int chunks = (n + CK_TOKENS - 1) / CK_TOKENS, slot0 = ck_first_slot(a.cu, b);
-    const bool vec_x = a.vec_v && (width & 3) == 0;
-
-    for (int e = threadIdx.x; e < D_::STAGE + 2 * D_::STAGE_FLOATS; e += CK_THREADS) ck_shared[e] = 0.0f;
-    __syncthreads();
-    auto fetch_first = [&](int chunk) {                         // what meets the state: q and W
-        if (chunk < chunks) {
-            const int c0 = chunk * CK_TOKENS;
-            ck_stage<NP>(Qs, D_::LDA, a.qkv + (size_t)(first + c0) * a.stride + (size_t)g * D, a.stride, min(CK_TOKENS, n - c0), D, a.vec);
-            ck_stage<NP>(Ws, D_::LDA, a.chunk_scratch(slot0 + chunk, h), D, CK_TOKENS, D, !(D & 3));
-        }
-        ck_commit();
-    };
-    auto fetch_rest = [&](int chunk) {
-        if (chunk < chunks) {
-            const int c0 = chunk * CK_TOKENS;
-            float* stage = ck_shared + D_::STAGE + (chunk & 1) * D_::STAGE_FLOATS;
-            const float* scratch = a.chunk_scratch(slot0 + chunk, h);
-            ck_stage<NP>(stage + D_::K, NP, a.qkv + (size_t)(first + c0) * a.stride + (size_t)(a.qk_heads + g) * D, a.stride, min(CK_TOKENS, n - c0), D, a.vec);
-            ck_stage<TP>(stage + D_::X, D_::LDX, scratch + (size_t)CK_TOKENS * D + p0, V, CK_TOKENS, width, vec_x);
-            const float* P = scratch + (size_t)CK_TOKENS * (D + V);
-            ck_stage<CK_TOKENS>(stage + D_::M, CK_MLD, P, CK_TOKENS, CK_TOKENS, CK_TOKENS, true);
-            for (int e = threadIdx.x; e < CD_FACTORS / 4; e += CK_THREADS) ck_copy16(stage + D_::F + 4 * e, P + CK_TOKENS * CK_TOKENS + 4 * e, true);
-        }
-        ck_commit();
-    };
-    fetch_rest(0);
-    fetch_first(0);
-
-    float* S = a.state + (((size_t)a.slots[b] * a.heads + h) * V + p0 + col) * D;
-    unsigned long long s[NL][2];
-#pragma unroll
-    for (int i = 0; i < NL; ++i) {
-        float v[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) v[e] = srow + i < D && p0 + col + e < V ? S[(size_t)e * D + srow + i] : 0.0f;
-        s[i][0] = ck_pair(v[0], v[1]);
-        s[i][1] = ck_pair(v[2], v[3]);
-        *reinterpret_cast<float4*>(Ss + (srow + i) * D_::LDX + col) = make_float4(v[0], v[1], v[2], v[3]);
+    const uint4* Ws = reinterpret_cast<const uint4*>(ck_bytes + L::W) + ns * KL * 4 * BLOCK;
+    const uint4* Qs = reinterpret_cast<const uint4*>(ck_bytes + L::Q) + ns * KL * 4 * BLOCK;
+    const uint4* Ks = reinterpret_cast<const uint4*>(ck_bytes + L::K) + ns * KL * BLOCK;
+    const uint4* Ms = reinterpret_cast<const uint4*>(ck_bytes + L::M);
+    uint4* Us = reinterpret_cast<uint4*>(ck_bytes + L::U) + pb * 4 * BLOCK;
+    float4* parts_w = reinterpret_cast<float4*>(ck_bytes + L::PARTS) + pb * (NS - 1) * 8 * 32 + lane;          // [another warp][tile of 8 tokens][lane]
+    float4* parts_q = parts_w + PB * (NS - 1) * 8 * 32;
+    int* bad_from = reinterpret_cast<int*>(ck_bytes + L::BAD);
+    const uint32_t bar = tc::smem_u32(ck_bytes + L::BAR), bar_rest = bar + 8;
+    if (threadIdx.x == 0) {
+        tc::mbar_init(bar, 1);
+        tc::mbar_init(bar_rest, 1);
+        tc::fence_barrier_init();
     }
+    __syncthreads();
+    bool in_time = true;                                        // no wait has run out
+
+    auto records = [&](int chunk) { return reinterpret_cast<float*>(ck_bytes + L::R) + (chunk & 1) * CK_RECORD; };
+    auto fetch_first = [&](int chunk) {                         // what meets the state, and the record
+        if (threadIdx.x || chunk >= chunks) return;
+        const uint4* head = a.head_scratch<NP>(slot0 + chunk, h);
+        tc::mbar_expect_tx(bar, 2 * L::MATRIX + CK_RECORD * 4);
+        ck_fetch(ck_bytes + L::W, head, L::MATRIX, bar);
+        ck_fetch(ck_bytes + L::Q, a.group_scratch<NP>(slot0 + chunk, g), L::MATRIX, bar);
+        ck_fetch(records(chunk), head + (2 * L::MATRIX + CK_MBLOCKS * SPLIT_BLOCK_BYTES) / 16, CK_RECORD * 4, bar);
+    };
+    auto fetch_rest = [&](int chunk) {                          // K and the scores
+        if (threadIdx.x || chunk >= chunks) return;
+        const uint4* head = a.head_scratch<NP>(slot0 + chunk, h);
+        tc::mbar_expect_tx(bar_rest, L::REST_BYTES);
+        ck_fetch(ck_bytes + L::K, head + L::MATRIX / 16, L::MATRIX, bar_rest);
+        ck_fetch(ck_bytes + L::M, head + 2 * L::MATRIX / 16, CK_MBLOCKS * SPLIT_BLOCK_BYTES, bar_rest);
+    };
+    fetch_first(0);
+    fetch_rest(0);
+
+    // this warp's state: tile k: columns pb * 16 + gq (and 8 further), rows row0 + 8 k + t2 and the next
+    const int row0 = ns * (NP / NS);
+    float* S = a.state + (((size_t)a.slots[b] * a.heads + h) * V + p0) * D;
+    float s[2 * KL][4];
+    auto load_state = [&](int half) {
+        const int p = pb * 16 + gq + 8 * half;
+#pragma unroll
+        for (int k = 0; k < 2 * KL; ++k)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int r = row0 + 8 * k + t2 + e;
+                s[k][2 * half + e] = p < width && r < D ? S[(size_t)p * D + r] : 0.0f;
+            }
+    };
+    auto store_state = [&]() {
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            const int p = pb * 16 + gq + 8 * half;
+#pragma unroll
+            for (int k = 0; k < 2 * KL; ++k)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int r = row0 + 8 * k + t2 + e;
+                    if (p < width && r < D) S[(size_t)p * D + r] = s[k][2 * half + e];
+                }
+        }
+    };
+    load_state(0);
+    load_state(1);
 
     for (int chunk = 0; chunk < chunks; ++chunk) {
-        float* stage = ck_shared + D_::STAGE + (chunk & 1) * D_::STAGE_FLOATS;
-        float* X = stage + D_::X;
-        const float* M = stage + D_::M;
-        const float* F = stage + D_::F;
-        fetch_rest(chunk + 1);
-        ck_wait<1>();
-        __syncthreads();                                        // this chunk's numbers and the state are there
-        unsigned long long acc[4][2], ws[4][2];
+        const float* F = records(chunk);
+        const int left = n - chunk * CK_TOKENS;
+        // this warp's tiles of U0, on their way while the products run
+        float u[EACH][4];
+        const float* from = a.values<NP>(slot0 + chunk, h) + p0 + pb * 16 + gq;
 #pragma unroll
-        for (int r = 0; r < 4; ++r) acc[r][0] = acc[r][1] = ws[r][0] = ws[r][1] = 0ull;
-        ck_two_products<RL, SLICE_K>(ws, Ws + row * D_::LDA, acc, Qs + row * D_::LDA, D_::LDA, Ss + col, D_::LDX, slice * SLICE_K);
-        {                                                       // W S: the first slice's sums lie where the weighted rows will
-            float* to = slice == 0 ? XW : ck_shared + D_::PARTS + (slice - 1) * CK_TOKENS * D_::LDX;
+        for (int i = 0; i < EACH; ++i)
 #pragma unroll
-            for (int r = 0; r < 4; ++r)
-                *reinterpret_cast<float4*>(to + (row + RL * r) * D_::LDX + col) = make_float4(ck_lo(ws[r][0]), ck_hi(ws[r][0]), ck_lo(ws[r][1]), ck_hi(ws[r][1]));
-        }
-        __syncthreads();                                        // W S is whole; q, W and the old state are read
-        fetch_first(chunk + 1);
-        float odd = 0.0f;                                       // no longer zero: a number of U is not finite
-        for (int e = threadIdx.x; e < CK_TOKENS * PL; e += CK_THREADS) {           // U = U0 - W S, and the rows the update adds
-            const int t = e / PL, c = 4 * (e % PL);
-            float4 u = *reinterpret_cast<const float4*>(X + t * D_::LDX + c);
-            float4 ws = *reinterpret_cast<const float4*>(XW + t * D_::LDX + c);
-#pragma unroll
-            for (int k = 0; k < L::SLICES - 1; ++k) {
-                const float4 q = *reinterpret_cast<const float4*>(ck_shared + D_::PARTS + (k * CK_TOKENS + t) * D_::LDX + c);
-                ws.x += q.x; ws.y += q.y; ws.z += q.z; ws.w += q.w;
+            for (int e = 0; e < 4; ++e) {
+                const int token = 8 * (ns * EACH + i) + t2 + (e & 1), p = 8 * (e >> 1);
+                u[i][e] = pb * 16 + gq + p < width ? __ldg(from + (size_t)token * V + p) : 0.0f;
             }
-            u.x -= ws.x; u.y -= ws.y; u.z -= ws.z; u.w -= ws.w;
-            const float w = F[CD_W + t];
-            odd += ck_not_finite(u);
-            *reinterpret_cast<float4*>(X + t * D_::LDX + c) = u;
-            *reinterpret_cast<float4*>(XW + t * D_::LDX + c) = make_float4(w * u.x, w * u.y, w * u.z, w * u.w);
-        }
+        in_time = in_time && tc::mbar_wait(bar, chunk & 1);
+        for (int p = threadIdx.x; p < TP; p += THREADS) bad_from[p] = __float_as_int(F[CK_R_BAD]);
+        float qs[EACH][4], ws[EACH][4];                         // this warp's tiles
+        {
+            SplitA A[KL];
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const float e = F[CD_E + row + RL * r];
-            acc[r][0] = ck_pair(ck_lo(acc[r][0]) * e, ck_hi(acc[r][0]) * e);
-            acc[r][1] = ck_pair(ck_lo(acc[r][1]) * e, ck_hi(acc[r][1]) * e);
-        }
-        const bool finite = !__syncthreads_or(odd != 0.0f);     // U is there
-        if (finite) ck_product<RL>(acc, M + row * CK_MLD, CK_MLD, X + col, D_::LDX, 4 * slice, 4 * L::SLICES, block * L::ROWS + L::ROWS);
-        else ck_causal_product<RL>(acc, M + row * CK_MLD, CK_MLD, X + col, D_::LDX, 4 * slice, 4 * L::SLICES, block * L::ROWS + L::ROWS, row);
-        if (slice > 0) {
+            for (int k = 0; k < KL; ++k) {
+                split_pair(s[2 * k][0], s[2 * k][1], A[k].hi[0], A[k].mid[0], A[k].lo[0]);
+                split_pair(s[2 * k][2], s[2 * k][3], A[k].hi[1], A[k].mid[1], A[k].lo[1]);
+                split_pair(s[2 * k + 1][0], s[2 * k + 1][1], A[k].hi[2], A[k].mid[2], A[k].lo[2]);
+                split_pair(s[2 * k + 1][2], s[2 * k + 1][3], A[k].hi[3], A[k].mid[3], A[k].lo[3]);
+            }
 #pragma unroll
-            for (int r = 0; r < 4; ++r)
-                *reinterpret_cast<float4*>(ck_shared + D_::PARTS + ((slice - 1) * CK_TOKENS + row + RL * r) * D_::LDX + col) =
-                    make_float4(ck_lo(acc[r][0]), ck_hi(acc[r][0]), ck_lo(acc[r][1]), ck_hi(acc[r][1]));
-        }
-        const float all = F[CD_ALL];
-        ck_update<NP, NL>(s, all, stage + D_::K + srow, XW + col, D_::LDX);
+            for (int which = 0; which < 2; ++which) {
+                const uint4* operand = which ? Qs : Ws;
+                float4* parts = which ? parts_q : parts_w;
+                float (&own)[EACH][4] = which ? qs : ws;
 #pragma unroll
-        for (int i = 0; i < NL; ++i)
-            *reinterpret_cast<float4*>(Ss + (srow + i) * D_::LDX + col) = make_float4(ck_lo(s[i][0]), ck_hi(s[i][0]), ck_lo(s[i][1]), ck_hi(s[i][1]));
-        __syncthreads();
-        if (slice == 0)
-            ck_outputs<RL, L::SLICES>(acc, ck_shared + D_::PARTS, D_::LDX, row, col, width, n - chunk * CK_TOKENS, vec_x, 0.0f, nullptr,
-                                      a.out + (size_t)(first + chunk * CK_TOKENS) * (a.heads * V) + (size_t)h * V + p0, a.heads * V);
+                for (int q0 = 0; q0 < 4; q0 += 2) {
+                    float y[4][4], rest[4][4];
+                    split_products<2, true>(y, rest, A[0], operand + q0 * BLOCK, lane);
+#pragma unroll
+                    for (int k = 1; k < KL; ++k) split_products<2, false>(y, rest, A[k], operand + (k * 4 + q0) * BLOCK, lane);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int tile = 2 * q0 + i, owner = tile / EACH;
+                        const float4 v = make_float4(y[i][0] + rest[i][0], y[i][1] + rest[i][1], y[i][2] + rest[i][2], y[i][3] + rest[i][3]);
+                        if (owner == ns) { own[tile % EACH][0] = v.x; own[tile % EACH][1] = v.y; own[tile % EACH][2] = v.z; own[tile % EACH][3] = v.w; }
+                        else parts[((ns - (ns > owner)) * 8 + tile) * 32] = v;
+                    }
+                }
+            }
+        }
+        __syncthreads();                                        // the parts are there; W and Q are read
+        fetch_first(chunk + 1);
+        bool odd = false;
+#pragma unroll
+        for (int i = 0; i < EACH; ++i) {
+            const int tile = ns * EACH + i;
+            float sum[4] = {};
+            float more[4] = {};
+#pragma unroll
+            for (int k = 0; k < NS - 1; ++k) {
+                const float4 v = parts_w[(k * 8 + tile) * 32], w = parts_q[(k * 8 + tile) * 32];
+                sum[0] += v.x; sum[1] += v.y; sum[2] += v.z; sum[3] += v.w;
+                more[0] += w.x; more[1] += w.y; more[2] += w.z; more[3] += w.w;
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                u[i][e] -= ws[i][e] + sum[e];
+                qs[i][e] += more[e];
+                if (!ck_usable(u[i][e])) {
+                    odd = true;
+                    atomicMin(bad_from + pb * 16 + gq + 8 * (e >> 1), 8 * tile + t2 + (e & 1));
+                    u[i][e] = 0.0f;
+                }
+            }
+            uint32_t part[3][2];
+            split_pair(u[i][0], u[i][1], part[0][0], part[1][0], part[2][0]);
+            split_pair(u[i][2], u[i][3], part[0][1], part[1][1], part[2][1]);
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                reinterpret_cast<uint2*>(Us + (tile >> 1) * BLOCK + 32 * k + lane)[tile & 1] = make_uint2(part[k][0], part[k][1]);
+        }
+        bool some_bad = __syncthreads_or(odd);                  // U is there
+        some_bad |= __float_as_int(F[CK_R_BAD]) < CK_TOKENS;
+        if (some_bad) {                                         // as in the scan: columns from their first such token on go token by token
+            store_state();
+            __syncthreads();
+            const int count = min(CK_TOKENS, left);
+            for (int p = warp; p < width; p += THREADS / 32)
+                if (bad_from[p] < count) ck_delta_column(a, F, first + chunk * CK_TOKENS, count, h, g, p0 + p, S + (size_t)p * D, bad_from[p]);
+            __syncthreads();
+        }
+        in_time = in_time && tc::mbar_wait(bar_rest, chunk & 1);
+        // S^T <- e_63 S^T + U^T (w K); the larger part is added last
+        const float all = F[CK_R_ALL];
+        const bool long_memory = fabsf(all) > 0.25f;
+        SplitA A;
+#pragma unroll
+        for (int k = 0; k < KL; k += PAIR) {
+            float sum[2 * PAIR][4], rest[2 * PAIR][4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                split_load(A, Us + j * BLOCK, lane);
+                if (j == 0) split_products<PAIR, true>(sum, rest, A, Ks + (j * L::KS + k) * BLOCK, lane);
+                else split_products<PAIR, false>(sum, rest, A, Ks + (j * L::KS + k) * BLOCK, lane);
+            }
+#pragma unroll
+            for (int i = 0; i < 2 * PAIR; ++i)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    float& v = s[2 * k + i][e];
+                    v = long_memory ? fmaf(all, v, sum[i][e] + rest[i][e]) : fmaf(all, v, rest[i][e]) + sum[i][e];
+                }
+        }
+        // outputs: Q S times its factor and the scores times U, for this warp's tiles
+        float* out = a.out + (size_t)(first + chunk * CK_TOKENS) * a.heads * V + (size_t)h * V + p0 + pb * 16 + gq;
+        const int limit[2] = {pb * 16 + gq < width ? min(left, some_bad ? bad_from[pb * 16 + gq] : CK_TOKENS) : 0,
+                              pb * 16 + gq + 8 < width ? min(left, some_bad ? bad_from[pb * 16 + gq + 8] : CK_TOKENS) : 0};
+#pragma unroll
+        for (int i = 0; i < EACH; ++i) {
+            const int tile = ns * EACH + i, q = tile >> 1;
+            float sum[4] = {}, rest[4] = {}, more[4] = {};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (j > q) continue;
+                split_load(A, Us + j * BLOCK, lane);
+                const uint2* block = reinterpret_cast<const uint2*>(Ms + (q * (q + 1) / 2 + j) * BLOCK + lane) + (tile & 1);
+                const uint2 hi = block[0], mid = block[64], lo = block[128];
+                split_mma(rest, A.lo, hi.x, hi.y);
+                split_mma(more, A.mid, mid.x, mid.y);
+                split_mma_add(sum, A.hi, hi.x, hi.y);
+                split_mma(rest, A.hi, lo.x, lo.y);
+                split_mma(more, A.mid, hi.x, hi.y);
+                split_mma(rest, A.hi, mid.x, mid.y);
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) rest[k] += more[k];
+            const float2 e = *reinterpret_cast<const float2*>(F + CK_R_E + 8 * tile + t2);
+            float* to = out + (size_t)(8 * tile + t2) * a.heads * V;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const float o = fmaf(k & 1 ? e.y : e.x, qs[i][k], rest[k]) + sum[k];
+                if (8 * tile + t2 + (k & 1) < limit[k >> 1]) to[(k & 1 ? (size_t)a.heads * V : 0) + 8 * (k >> 1)] = o;
+            }
+        }
+        if (some_bad) {
+            const int count = min(CK_TOKENS, left);
+            if (bad_from[pb * 16 + gq] < count) load_state(0);
+            if (bad_from[pb * 16 + gq + 8] < count) load_state(1);
+        }
+        __syncthreads();                                        // K, the scores and U are read
+        fetch_rest(chunk + 1);
     }
-    ck_wait<0>();
-#pragma unroll
-    for (int i = 0; i < NL; ++i) {
-        const float v[4] = {ck_lo(s[i][0]), ck_hi(s[i][0]), ck_lo(s[i][1]), ck_hi(s[i][1])};
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-            if (srow + i < D && p0 + col + e < V) S[(size_t)e * D + srow + i] = v[e];
-    }
+    if (!in_time && a.status) atomicOr(a.status, TT_STATUS_WAIT_EXPIRED);
+    store_state();
 }
 
-template <int NP, int TP>
+template <int NP, int PB, int NS>
 static int delta_chunks_launch(const DeltaChunks& a, int max_slots, cudaStream_t stream) {
-    constexpr size_t prepare_bytes = (size_t)(2 * CK_TOKENS * (NP + 4) + CK_TOKENS * CK_MLD + CK_FACTORS + 7 * CK_TOKENS) * sizeof(float);
+    using L = CdWalk<NP, PB, NS>;
+    constexpr size_t prepare_bytes = CdPrepare<NP>::BYTES;
     cudaError_t code = ck_allow(delta_chunks_prepare_kernel<NP>, prepare_bytes);
-    if (code == cudaSuccess) code = ck_allow(delta_chunks_kernel<NP, TP>, CdLayout<NP, TP>::BYTES);
+    if (code == cudaSuccess) code = ck_allow(delta_chunks_kernel<NP, PB, NS>, L::BYTES);
     if (code != cudaSuccess) return (int)code;
     tt_launch_pdl(delta_chunks_prepare_kernel<NP>, dim3(max_slots, a.heads), dim3(CD_THREADS), prepare_bytes, stream, a);
-    tt_launch_pdl(delta_chunks_kernel<NP, TP>, dim3(a.heads, a.sequences, (a.V + TP - 1) / TP), dim3(CK_THREADS), CdLayout<NP, TP>::BYTES, stream, a);
+    tt_launch_pdl(delta_chunks_kernel<NP, PB, NS>, dim3(a.heads, a.sequences, (a.V + L::TP - 1) / L::TP), dim3(L::THREADS), (size_t)L::BYTES, stream, a);
     TT_LAUNCH_CHECK();
 }
 
-// scratch: max_slots * heads * (64 * (D + V + 64) + CD_FACTORS) floats on a 16-byte boundary; max_slots as for tt_scan_chunks
+// scratch: max_slots times the operands of every query/key head and of every head (see DeltaChunks), on a 16-byte boundary; max_slots as for tt_scan_chunks
 extern "C" int tt_delta_chunks(const float* qkv, int qkv_cols, const float* proj, int splits, long long split_stride, int cols, int b_col, int a_col,
                                const float* dt_bias, const float* a_log, float* state, float* out, float* scratch, const int* cu, const int* slots,
-                               int sequences, int max_slots, int heads, int qk_heads, int D, int V, int sms, cudaStream_t stream) {
+                               int sequences, int max_slots, int heads, int qk_heads, int D, int V, int sms, unsigned* status, cudaStream_t stream) {
     if (sequences <= 0 || max_slots <= 0) return 0;
     if (D <= 0 || D > 128 || V <= 0 || qk_heads <= 0 || heads % qk_heads || heads > 65535 || sequences > 65535) return (int)cudaErrorInvalidValue;
     if (!qkv || !proj || !dt_bias || !a_log || !scratch || ((uintptr_t)scratch & 15)) return (int)cudaErrorInvalidValue;
     const int vec = ((uintptr_t)qkv & 15) == 0 && !(qkv_cols & 3) && !(D & 3);
-    const DeltaChunks a{qkv, (size_t)qkv_cols, proj, splits, cols, b_col, a_col, (size_t)split_stride, dt_bias, a_log, state, out, scratch, cu, slots,
-                        sequences, heads, qk_heads, D, V, vec, ((uintptr_t)out & 15) == 0 && !(V & 3) ? 1 : 0};
-    const bool narrow = (long long)heads * sequences * ((V + 31) / 32) * 2 <= sms + sms / 4;        // as for tt_scan_chunks
-    if (D <= 64) return narrow ? delta_chunks_launch<64, 16>(a, max_slots, stream) : delta_chunks_launch<64, 32>(a, max_slots, stream);
-    return narrow ? delta_chunks_launch<128, 16>(a, max_slots, stream) : delta_chunks_launch<128, 32>(a, max_slots, stream);
+    const DeltaChunks a{qkv, (size_t)qkv_cols, proj, splits, cols, b_col, a_col, (size_t)split_stride, dt_bias, a_log, state, out, status,
+                        reinterpret_cast<unsigned char*>(scratch), cu, slots, sequences, max_slots, heads, qk_heads, D, V, vec};
+    // columns of a CTA, as for tt_scan_chunks: a chunk takes a CTA of 16, 32 and 64 columns 3.5, 5.5 and 10.7 us with keys of 128, 3.7, 5.4 and 8.4 with keys of 64
+    const long long one = (long long)heads * sequences;
+    auto cost = [&](int columns, int chunk) { return (one * ((V + columns - 1) / columns) + sms - 1) / sms * chunk; };
+    const bool small = D <= 64;
+    const long long c16 = cost(16, small ? 370 : 352), c32 = cost(32, small ? 540 : 550), c64 = cost(64, small ? 840 : 1070);
+    if (c64 <= c32 && c64 <= c16) return small ? delta_chunks_launch<64, 4, 2>(a, max_slots, stream) : delta_chunks_launch<128, 4, 2>(a, max_slots, stream);
+    if (c32 <= c16) return small ? delta_chunks_launch<64, 2, 4>(a, max_slots, stream) : delta_chunks_launch<128, 2, 4>(a, max_slots, stream);
+    return small ? delta_chunks_launch<64, 1, 4>(a, max_slots, stream) : delta_chunks_launch<128, 1, 8>(a, max_slots, stream);
 }

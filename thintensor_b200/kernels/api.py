@@ -935,7 +935,6 @@ def mamba2_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_col: int, dt_bias: tor
 CHUNK_TOKENS = 64           # tokens of a chunk of the recurrences with a decay per head (CK_TOKENS in csrc/recurrent_chunks.cu)
 CHUNK_MAX_ROWS = 128        # state rows (key size) the chunk kernels take
 _CHUNK_HEAD_FLOATS = 10 * 384 + 260         # scores times factors as an operand in three bfloat16 parts, and a record
-_DELTA_CHUNK_FACTORS = 136
 
 
 def chunk_slots(n_tokens: int, sequences: int) -> int:
@@ -985,31 +984,33 @@ def scan_chunks(rows: torch.Tensor, x_col: int, b_col: int, c_col: int, state: t
               chunk_slots(tokens, sequences), heads, groups, head_dim, state_size, sm_count(rows.device), _ptr(status), _stream()), "scan_chunks", 2)
 
 
-def delta_chunks_scratch(n_tokens: int, sequences: int, heads: int, key_dim: int, value_dim: int) -> tuple[int]:
-    """Shape of the float32 scratch that :func:`delta_chunks` takes."""
-    return (chunk_slots(n_tokens, sequences) * heads * (CHUNK_TOKENS * (key_dim + value_dim + CHUNK_TOKENS) + _DELTA_CHUNK_FACTORS),)
+def delta_chunks_scratch(n_tokens: int, sequences: int, heads: int, key_dim: int, value_dim: int, qk_heads: int | None = None) -> tuple[int]:
+    """Shape of the float32 scratch that :func:`delta_chunks` takes: of every chunk and query/key head (``qk_heads`` None: as many as heads) q, of every
+    chunk and head W, the keys and the scores in three bfloat16 parts, factors and U0."""
+    matrix = CHUNK_TOKENS * (64 if key_dim <= 64 else 128) * 3 // 2
+    return (chunk_slots(n_tokens, sequences) * ((heads if qk_heads is None else qk_heads) * matrix + heads * (2 * matrix + _CHUNK_HEAD_FLOATS + CHUNK_TOKENS * value_dim)),)
 
 
 def delta_chunks(qkv: torch.Tensor, proj: torch.Tensor, b_col: int, a_col: int, dt_bias: torch.Tensor, a_log: torch.Tensor, state: torch.Tensor,
                  out: torch.Tensor, cu: torch.Tensor, slots: torch.Tensor, sequences: int, heads: int, qk_heads: int, key_dim: int, value_dim: int,
-                 scratch: torch.Tensor) -> None:
+                 scratch: torch.Tensor, status: torch.Tensor | None = None) -> None:
     """:func:`delta_scan` with a decay per head, a chunk of 64 tokens at a time (for prompts; key sizes of up to 128).  ``scratch``, on
-    a 16-byte boundary: see :func:`delta_chunks_scratch`."""
+    a 16-byte boundary: see :func:`delta_chunks_scratch`.  ``status``: the device status word."""
     for t, name in ((qkv, "q/k/v"), (dt_bias, "dt_bias"), (a_log, "A_log"), (state, "recurrent state"), (out, "recurrence output"), (scratch, "scratch")):
         _need(t, torch.float32, name)
     _need_aligned(scratch, "scratch")
     tokens = qkv.shape[0]
     if (qkv.shape[1] != 2 * qk_heads * key_dim + heads * value_dim or state.shape[1:] != (heads, value_dim, key_dim) or heads % qk_heads
             or out.shape != (tokens, heads * value_dim) or key_dim > CHUNK_MAX_ROWS or dt_bias.numel() != heads or a_log.numel() != heads
-            or scratch.numel() < delta_chunks_scratch(tokens, sequences, heads, key_dim, value_dim)[0]):
+            or scratch.numel() < delta_chunks_scratch(tokens, sequences, heads, key_dim, value_dim, qk_heads)[0]):
         raise KernelError("delta_chunks: shapes do not fit the sizes")
     p, splits, stride, cols = _projection(proj)
     if min(b_col, a_col) < 0 or max(b_col, a_col) + heads > cols:
         raise KernelError("delta_chunks: write strengths or decays lie outside the projection")
-    fn = _fn("recurrent_chunks", "tt_delta_chunks", "pipiliiipppppppiiiiiiip")
+    fn = _fn("recurrent_chunks", "tt_delta_chunks", "pipiliiipppppppiiiiiiipp")
     _check(fn(qkv.data_ptr(), qkv.shape[1], p, splits, stride, cols, b_col, a_col, dt_bias.data_ptr(), a_log.data_ptr(), state.data_ptr(), out.data_ptr(),
               scratch.data_ptr(), _ptr(cu), _ptr(slots), sequences, chunk_slots(tokens, sequences), heads, qk_heads, key_dim, value_dim, sm_count(qkv.device),
-              _stream()), "delta_chunks", 2)
+              _ptr(status), _stream()), "delta_chunks", 2)
 
 
 def delta_scan(qkv: torch.Tensor, proj: torch.Tensor, b_col: int, a_col: int, dt_bias: torch.Tensor | None, a_log: torch.Tensor | None,

@@ -319,9 +319,9 @@ class GatedDelta(Mixer):
             api.row_decay_blocks(qkv[:, :self.qk], qkv[:, self.qk: 2 * self.qk], qkv[:, 2 * self.qk:], decay, recurrent, read, ctx.cu, ctx.slots,
                                  ctx.sequences, self.heads, self.qk_heads, self.key_dim, self.value_dim, self.key_dim ** -0.5, (proj, self.b_col))
         elif decay is None and in_chunks(ctx, self.heads, self.value_dim, self.key_dim, delta=True):
-            shape = api.delta_chunks_scratch(tokens, ctx.sequences, self.heads, self.key_dim, self.value_dim)
+            shape = api.delta_chunks_scratch(tokens, ctx.sequences, self.heads, self.key_dim, self.value_dim, self.qk_heads)
             api.delta_chunks(qkv, proj, self.b_col, self.a_col, self.dt_bias, self.a_log, recurrent, read, ctx.cu, ctx.slots, ctx.sequences, self.heads,
-                             self.qk_heads, self.key_dim, self.value_dim, ctx.scratch("chunks.delta", shape, torch.float32))
+                             self.qk_heads, self.key_dim, self.value_dim, ctx.scratch("chunks.delta", shape, torch.float32), ctx.status)
         else:
             api.delta_scan(qkv, proj, self.b_col, self.a_col, self.dt_bias, self.a_log, recurrent, read, ctx.cu,
                            ctx.slots, ctx.sequences, self.heads, self.qk_heads, self.key_dim, self.value_dim, row_decay=decay)
