@@ -43,6 +43,65 @@ def test_exact_product_slices_follow_the_sizes():
         assert 1 <= splits <= 8 and k >= 256 * splits
 
 
+@pytest.mark.parametrize("m,n,k,pad,splits", [
+    (1, 1, 1, 0, 1), (17, 255, 63, 1, 1), (32, 256, 64, 4, 1), (33, 257, 65, 2, 2), (100, 40, 1000, 0, 4), (193, 600, 520, 4, 3),
+    (224, 512, 128, 0, 9), (256, 300, 192, 3, 1), (257, 130, 320, 0, 2), (600, 270, 72, 4, 1),
+])
+def test_product_in_parts_at_tile_edges(m, n, k, pad, splits):
+    """As above, the operands in three bfloat16 parts; more slices than blocks of 64 k leave slices of zeros."""
+    from thintensor_b200.kernels import api
+
+    x, w, bias = randn(m, k + pad, seed=1)[:, pad:], randn(n, k + pad, seed=2)[:, pad:], randn(n, seed=3)
+    wide = torch.full((splits, m, n + pad), 7.0, device=DEV)
+    parts = torch.empty(api.gemm_split_parts(m, k), dtype=torch.bfloat16, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    api.gemm_split(x, w, bias, wide[:, :, :n], parts, status)
+    want = x.double() @ w.double().T + bias.double()
+    # what three parts leave off a product is at most 2^-25 of it; the sum of 64 k takes 24 additions that lose up to 2^-23 each, then come the blocks and slices
+    size = x.double().abs() @ w.double().abs().T + bias.double().abs()
+    error = (wide[:, :, :n].double().sum(0) - want).abs()
+    assert bool((error <= (2.0 ** -25 + 24 * 2.0 ** -23 + (k // 64 + splits + 2) * 2.0 ** -24) * size).all())
+    # and no further from 64 bits than the multiply-adds, which round k times
+    plain = torch.empty(1, m, n, device=DEV)
+    api.gemm_simt(x, w, bias, plain)
+    if m * n * k >= 1 << 20:
+        assert float(error.square().mean()) <= float((plain[0].double() - want).square().mean())
+    assert bool((wide[:, :, n:] == 7.0).all()) and int(status) == 0
+
+
+def test_product_in_parts_of_what_is_not_finite():
+    """Infinities, NaN and numbers whose first part would round up to infinity: what the multiply-adds make of them, and nothing
+    else is touched."""
+    from thintensor_b200.kernels import api
+
+    m, n, k = 70, 300, 200
+    x, w = randn(m, k, seed=4), randn(n, k, seed=5)
+    clean = torch.empty(1, m, n, device=DEV)
+    parts = torch.empty(api.gemm_split_parts(m, k), dtype=torch.bfloat16, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    api.gemm_split(x, w, None, clean, parts, status)
+    x[3, 7], x[40, 199], x[69, 0] = float("inf"), float("nan"), 3.4028e38
+    w[299, 100], w[0, 0] = float("-inf"), 1e-30
+    w[5, 0] = 0.0
+    got, want = torch.empty(1, m, n, device=DEV), torch.empty(1, m, n, device=DEV)
+    api.gemm_split(x, w, None, got, parts, status)
+    api.gemm_simt(x, w, None, want)
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf()) and int(status) == 0
+    torch.testing.assert_close(got, want, rtol=2.0 ** -24 * k, atol=2.0 ** -24 * k * k ** 0.5, equal_nan=True)
+    rows = torch.ones(m, dtype=torch.bool)
+    rows[[3, 40, 69]] = False
+    assert torch.equal(got[0][rows][:, 6:299], clean[0][rows][:, 6:299])
+
+
+def test_slices_of_products_in_parts_follow_the_sizes():
+    from thintensor_b200.kernels import api
+
+    assert api.gemm_split_splits(193, 2048, 255, 148) == 1              # slices hold at least 128
+    assert api.gemm_split_splits(193, 16384, 2048, 148) == 1            # enough tiles
+    assert api.gemm_split_splits(193, 2048, 8192, 148) == 9             # 8 pairs of 74
+    assert not api.gemm_split_pays(16, 2048, 8192) and api.gemm_split_pays(17, 2048, 2048) and not api.gemm_split_pays(300, 64, 64)
+
+
 # ----------------------------------------------------------- recurrences with a decay per head, a chunk of 64 tokens at a time
 def i32(values):
     return torch.tensor(values, dtype=torch.int32, device=DEV)

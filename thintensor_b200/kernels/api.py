@@ -1673,6 +1673,59 @@ def gemm_simt_splits(tokens: int, features: int, k: int, sms: int | None = None)
     return best
 
 
+def gemm_split_pays(tokens: int, features: int, k: int) -> bool:
+    """Whether :func:`gemm_split` (two launches, scratch memory) takes the place of :func:`gemm_simt`: behind the rows that the kernel for few takes,
+    from weights of a million numbers on.  Smaller ones gain at most 6 us (17 to 300 rows: 256 features of 2,048 20 to 26 us against 15 to 17, 64 of 512 20 to 22
+    against 13 to 15, the smallest nothing: a launch more), and keep one kernel and its rounding; 1,024 of 1,024 21 to 35 us against 15 to 20."""
+    return tokens > 16 and features * k >= 1 << 20
+
+
+def gemm_split_splits(tokens: int, features: int, k: int, sms: int | None = None) -> int:
+    """Into how many slices :func:`gemm_split` cuts k: every CTA pair has 256 features and up to 256 tokens of a slice of at least 128, and
+    the pairs come in rounds.  In us: a pair's start and end, a block of 64 k (its products, however few the tokens at least the weights'
+    way through the kernel), and 8 bytes of every partial sum, which the consumer reads again.  Measured (us in 1, 2, 4, 6, 9, 16 slices): 193 tokens,
+    2,048 features of 8,192 204, 114, 68, 54, 44, 52; 16,384 of 2,048 69, 77, 91, 99, 112, 151; 256 of 2,048 60, 38, 26, 24, 20, 17."""
+    sms = sm_count() if sms is None else sms
+    tiles = -(-tokens // 256)
+    rows = -(-(-(-tokens // tiles)) // 32) * 32
+    pairs, blocks = -(-features // 256) * tiles, -(-k // 64)
+    block = max(0.9, 0.0065 * rows)
+    best, cost = 1, None
+    for splits in range(1, 17):
+        if splits > 1 and k < 128 * splits:
+            break
+        now = -(-pairs * splits // (sms // 2)) * (4.0 + block * -(-blocks // splits)) + splits * tokens * features * 8 / 5e6
+        if cost is None or now < cost:
+            best, cost = splits, now
+    return best
+
+
+def gemm_split_parts(tokens: int, k: int) -> tuple[int, int, int]:
+    """Shape of the bfloat16 scratch memory in which :func:`gemm_split` lays the parts of its activations."""
+    return (3, tokens, -(-k // 8) * 8)
+
+
+def gemm_split(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None, out: torch.Tensor, parts: torch.Tensor, status: torch.Tensor) -> None:
+    """:func:`gemm_simt` of float32 operands on the tensor cores, its errors no larger: the operands as three bfloat16 parts each.
+    ``parts``: scratch memory (:func:`gemm_split_parts`)."""
+    _need_columns(out, torch.float32, "gemm output")
+    if x.dtype != torch.float32 or w.dtype != torch.float32 or x.stride(-1) != 1 or w.stride(-1) != 1:
+        raise KernelError("gemm operands must be float32 and contiguous along k")
+    m, k = x.shape
+    n = w.shape[0]
+    if w.shape[1] != k or out.shape[1:] != (m, n):
+        raise KernelError(f"gemm shapes do not fit: x {tuple(x.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}")
+    if bias is not None:
+        _need(bias, torch.float32, "bias")
+    _need(parts, torch.bfloat16, "gemm parts")
+    _need(status, torch.int32, "status")
+    if tuple(parts.shape) != gemm_split_parts(m, k) or parts.data_ptr() % 16:
+        raise KernelError(f"gemm parts must be {gemm_split_parts(m, k)} on a 16-byte boundary, got {tuple(parts.shape)}")
+    fn = _fn("gemm_split", "tt_gemm_split", "plplppllppiiiiip")
+    _check(fn(_ptr(x), x.stride(0), _ptr(w), w.stride(0), _ptr(bias), _ptr(out), out.stride(1), out.stride(0), _ptr(parts), _ptr(status), m, n, k,
+              out.shape[0], sm_count(x.device), _stream()), "gemm_split", 2)
+
+
 # ---------------------------------------------------------------------------- sampling
 _argmax_scratch: dict[torch.device, tuple[torch.Tensor, torch.Tensor]] = {}
 

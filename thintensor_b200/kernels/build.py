@@ -34,6 +34,7 @@ SOURCES: dict[str, list[str]] = {
     "elementwise": [],
     "attention": [],
     "gemm_simt": [],
+    "gemm_split": [],
     "sampling": [],
     "attention_static_scratch": [],
     "gemm_tcgen05": [],

@@ -8,8 +8,9 @@ without a reduction kernel of its own.
 
 Which kernel runs is decided by the operands alone: bfloat16 activations with a
 bfloat16 weight whose rows TMA can address (k a multiple of 8) use the tcgen05
-tensor-core kernel; everything else (the true 32-bit path, a weight that the checkpoint
-stores in float32, an odd k) uses the exact FMA kernel.
+tensor-core kernel; prompts of the true 32-bit path use the tensor cores too, with float32
+operands in three bfloat16 parts each; everything else (few tokens in 32 bits, a weight that the
+checkpoint stores in float32 beside bfloat16 activations, an odd k) uses the exact FMA kernel.
 """
 from __future__ import annotations
 
@@ -49,10 +50,17 @@ class Linear:
                 out = ctx.scratch(name, (splits, tokens, self.out_features), torch.float32)
             api.gemm_tcgen05(x, self.weight, self.bias, out, ctx.status, operands_checked=True, shares=self.shares(ctx, tokens))
             return out
+        split = (x.dtype == self.weight.dtype == torch.float32 and x.stride(1) == 1
+                 and api.gemm_split_pays(tokens, self.out_features, self.in_features))
+        slices = api.gemm_split_splits if split else api.gemm_simt_splits
         # a caller that brings an output wants the product itself: no slices that it would have to add up
         out = into.unsqueeze(0) if into is not None else ctx.scratch(
-            name, (api.gemm_simt_splits(tokens, self.out_features, self.in_features), tokens, self.out_features), torch.float32)
-        api.gemm_simt(x, self.weight, self.bias, out)
+            name, (slices(tokens, self.out_features, self.in_features), tokens, self.out_features), torch.float32)
+        if split:
+            parts = ctx.scratch("gemm.parts", api.gemm_split_parts(tokens, self.in_features), torch.bfloat16)
+            api.gemm_split(x, self.weight, self.bias, out, parts, ctx.status)
+        else:
+            api.gemm_simt(x, self.weight, self.bias, out)
         return out
 
 
