@@ -15,8 +15,9 @@
 //
 // What bounds it: the six products (a block of 64 k of 224 tokens is 24 of them, 2,690 of the 3,000 cycles a block takes); below about 100
 // tokens the way of a block through the kernel, 2,700 cycles; few features the pairs' start and end.  The rows of weights go behind the arrival
-// of the block before, and the arrival carries no release to the cluster: with loads ahead of it and with that release the fences took 1,500 cycles more
-// a block.  us with a cold L2 (about 8 of them the events'), multiply-adds of gemm_simt.cu and now: 193 rows, 16,384 features of 2,048 349 -> 69, 2,048 of 8,192
+// of the block before: with loads ahead of it the fence took 750 cycles more a block.  What the odd CTA's warps wrote has to be released to the
+// cluster, which took every warp 1,700 cycles when each did it (its fence waits for the warp's loads): they arrive at a barrier of their own CTA, and one thread
+// without loads passes that on.  us with a cold L2 (about 8 of them the events'), multiply-adds of gemm_simt.cu and now: 193 rows, 16,384 features of 2,048 349 -> 69, 2,048 of 8,192
 // 215 -> 44, 3,072 of 2,048 78 -> 28, 256 of 2,048 21.5 -> 17.4; 17 rows, 16,384 of 2,048 79 -> 60, 64 of 512 19.5 -> 13.3; 2,048 rows, 16,384 of 2,048 2,660 -> 546.  Relative error
 // against 64 bits, normal numbers: 193 rows, 2,048 of 8,192 6.6e-7 -> 1.1e-7, 17 rows, 40 of 72 1.6e-7 -> 0.8e-7.
 //
@@ -98,7 +99,7 @@ struct Args {
 __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_constant__ CUtensorMap map_x, const Args args) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    __shared__ uint64_t full_bar[2], done_bar[2];
+    __shared__ uint64_t full_bar[2], done_bar[2], cut_bar[2];
     __shared__ uint32_t tmem_base_shared;
 
     tt_pdl_launch_dependents();
@@ -111,8 +112,13 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
     const int steps = max(0, min((args.k + BK - 1) / BK - kb0, args.k_blocks_per_split));
 
     if (threadIdx.x == 0) {
-        // full: the announced copies and the workers' warps of both CTAs; done: the products of a stage
-        for (int s = 0; s < 2; ++s) { mbar_init(smem_u32(&full_bar[s]), 1 + 2 * WARPS); mbar_init(smem_u32(&done_bar[s]), 1); }
+        // full (the even CTA's): the announced copies, its workers' warps, and one arrival for all of the odd CTA's; cut (the odd CTA's): its workers'
+        // warps; done: the products of a stage
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(smem_u32(&full_bar[s]), 2 + WARPS);
+            mbar_init(smem_u32(&cut_bar[s]), WARPS);
+            mbar_init(smem_u32(&done_bar[s]), 1);
+        }
         fence_barrier_init();
     }
     cluster.sync();
@@ -143,7 +149,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
             const uint32_t idesc = instr_desc(2 * BM, args.tokens);
             for (int i = 0; i < steps; ++i) {
                 const int s = i & 1;
-                if (!mbar_wait(smem_u32(&full_bar[s]), (i >> 1) & 1)) { atomicOr(args.status, TT_STATUS_WAIT_EXPIRED); break; }
+                if (!mbar_wait<true>(smem_u32(&full_bar[s]), (i >> 1) & 1)) { atomicOr(args.status, TT_STATUS_WAIT_EXPIRED); break; }
                 fence_after_sync();
                 const uint32_t a = smem_u32(smem + (size_t)s * STAGE_BYTES), b = a + PARTS * A_BYTES, acc = tmem_base + s * 256;
                 // parts of (weights, activations), the smallest products first
@@ -155,6 +161,16 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
                         umma_bf16_pair(acc, smem_desc(a + PA[p] * A_BYTES + kk * UMMA_K * 2), smem_desc(b + PB[p] * half * BK * 2 + kk * UMMA_K * 2), idesc,
                                        (p > 0 || kk > 0) ? 1u : 0u);
                 umma_commit_pair(smem_u32(&done_bar[s]), 3);
+            }
+        }
+        if (warp == WARPS + 1 && lane == 0 && rank == 1) {
+            // the odd CTA's rows of weights, and its reading of the accumulator two blocks ago, handed to the issuer
+            for (int i = 0; i < steps; ++i) {
+                const int s = i & 1;
+                if (!mbar_wait(smem_u32(&cut_bar[s]), (i >> 1) & 1)) { atomicOr(args.status, TT_STATUS_WAIT_EXPIRED); break; }
+                fence_after_sync();
+                fence_before_sync();
+                mbar_release_even_cta(smem_u32(&full_bar[s]));
             }
         }
     } else {
@@ -221,7 +237,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
             }
             fence_async_shared();
             __syncwarp();
-            if (lane == 0) mbar_arrive_even_cta(smem_u32(&full_bar[i & 1]));
+            if (lane == 0) mbar_arrive(smem_u32(rank ? &cut_bar[i & 1] : &full_bar[i & 1]));
             __syncwarp();
 #pragma unroll
             for (int j = 0; j < 4; ++j)

@@ -34,23 +34,33 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+// CLUSTER: arrivals with release from the cluster's other CTA count too (mbar_release_even_cta)
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
     uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+    if (CLUSTER)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done) : "r"(bar), "r"(parity) : "memory");
     return done != 0;
 }
 // Wait for the phase of the given parity to complete; false when WAIT_LIMIT_NS ran out.
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
     for (int i = 0; i < 64; ++i)
-        if (mbar_try(bar, parity)) return true;
+        if (mbar_try<CLUSTER>(bar, parity)) return true;
     const unsigned long long start = global_time_ns();
     for (;;) {
         for (int i = 0; i < 64; ++i)
-            if (mbar_try(bar, parity)) return true;
+            if (mbar_try<CLUSTER>(bar, parity)) return true;
         if (global_time_ns() - start > wait_limit_ns) return false;
     }
 }
@@ -232,9 +242,15 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
         "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
         ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar & PEER_MASK) : "memory");
 }
-// An arrival on the even CTA's barrier from either CTA.
+// An arrival on the even CTA's barrier from either CTA, for an accumulator that was read: the reading is done when tcgen05.wait::ld is, so there is
+// nothing to release (a release at the cluster's scope would wait for the thread's stores: prompts of 2,048 tokens 0.6 % slower).
 __device__ __forceinline__ void mbar_arrive_even_cta(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar & PEER_MASK) : "memory");
+}
+// The same for memory that was written: what this thread wrote, or saw written on a barrier of its own CTA, is there for who waits with acquire at the
+// cluster's scope (mbar_wait<true>).  Without a scope an arrival releases to its own CTA only.
+__device__ __forceinline__ void mbar_release_even_cta(uint32_t bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar & PEER_MASK) : "memory");
 }
 
 __device__ __forceinline__ void tmem_store16(uint32_t addr, const uint32_t* v) {
