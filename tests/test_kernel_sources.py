@@ -38,3 +38,12 @@ def test_rows_cut_by_the_odd_cta_are_released_by_a_thread_that_has_seen_them():
     assert text.count("mbar_release_even_cta(") == 1 and "mbar_arrive_even_cta(" not in text
     workers = text[text.index("fence_async_shared();"):]
     assert re.match(r"fence_async_shared\(\);\s*__syncwarp\(\);\s*if \(lane == 0\) mbar_arrive\(smem_u32\(rank \? &cut_bar\[i & 1\] : &full_bar\[i & 1\]\)\);", workers)
+
+
+@pytest.mark.parametrize("path", SOURCES, ids=lambda p: p.name)
+def test_shared_memory_is_asked_for_on_every_launch(path):
+    """What a kernel may have beyond 48 KB holds for the device that was current when it was asked for: nothing remembers for the whole process that it was."""
+    text = code(path)
+    for ask in re.finditer(r"cudaFuncSetAttribute|tt_allow_shared\(", text):
+        function = text[text.rfind("\n}", 0, ask.start()) + 2:ask.start()]
+        assert not re.search(r"\bstatic\s+(?:bool|int|size_t)\s+\w+\s*=", function), function[-400:]

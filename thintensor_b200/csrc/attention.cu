@@ -224,8 +224,7 @@ template <typename T, int SIZE>
 static int attention_tiles_launch(const void* q, const void* k_pool, const void* v_pool, const int* table, int table_width, int pool_blocks, const int* cu,
                                   const int* len_before, int sequences, int n_tokens, int heads, int kv_heads, int head_dim, int value_dim, float scale,
                                   const float* sinks, int window, void* out, unsigned* status, const AttnExtra& extra, cudaStream_t stream) {
-    // on every launch: it holds for the current device alone, and an engine may run on any of the process's
-    const cudaError_t code = cudaFuncSetAttribute(attention_tiles_kernel<T, SIZE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)at_shared<SIZE>());
+    const cudaError_t code = tt_allow_shared(attention_tiles_kernel<T, SIZE>, at_shared<SIZE>());
     if (code != cudaSuccess) return (int)code;
     tt_launch_pdl(attention_tiles_kernel<T, SIZE>, dim3((unsigned)(n_tokens / AT_QUERIES + sequences), (unsigned)heads), dim3(AT_THREADS), at_shared<SIZE>(), stream,
                   (const T*)q, (const T*)k_pool, (const T*)v_pool, table, table_width, pool_blocks, cu, len_before, sequences, heads, kv_heads, head_dim, value_dim,

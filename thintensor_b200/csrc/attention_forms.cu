@@ -769,12 +769,8 @@ template <int KD, int VD, int MAPS, bool POOLED, int TILES>
 int form_launch_tiles(FormArgs a, int n_tokens, cudaStream_t stream) {
     using S = FormShape<KD, VD, MAPS, TILES>;
     auto kernel = form_kernel<KD, VD, MAPS, POOLED, TILES>;
-    static bool configured = false;
-    if (!configured) {
-        const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SHARED);
-        if (err != cudaSuccess) return (int)err;
-        configured = true;
-    }
+    const cudaError_t err = tt_allow_shared(kernel, S::SHARED);
+    if (err != cudaSuccess) return (int)err;
     a.tokens_per_tile = 16 / (a.heads / a.kv_heads);
     const int tokens_per_cta = a.tokens_per_tile * TILES;
     a.cta_tiles = (n_tokens + tokens_per_cta - 1) / tokens_per_cta + a.sequences;       // upper bound; spare CTAs leave at once

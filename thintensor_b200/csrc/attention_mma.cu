@@ -915,25 +915,17 @@ cudaError_t launch_decode_tiles(const void* q, const DecodeRope& rope, void* k_p
     static_assert(shared >= D::WARPS * 16 * (HD + 6) * 4 + 16 * (HD + 2) * 4, "the slots must also hold the warps' and the CTA's partial results");
     if constexpr (SHAPE == ONE_PER_SM && !SHAPED) {
         if (tickets && splits > 1 && !slices_form_cluster(splits)) {
-            static bool configured_tickets = false;
             auto with_tickets = attention_decode_kernel<HD, ROPE, SHAPE, true, NQ>;
-            if (!configured_tickets) {
-                const cudaError_t err = cudaFuncSetAttribute(with_tickets, cudaFuncAttributeMaxDynamicSharedMemorySize, shared);
-                if (err != cudaSuccess) return err;
-                configured_tickets = true;
-            }
+            const cudaError_t err = tt_allow_shared(with_tickets, shared);
+            if (err != cudaSuccess) return err;
             return tt_launch_pdl(with_tickets, dim3(sequences, kv_heads, splits), dim3(D::WARPS * 32), shared, stream,
                 (const __nv_bfloat16*)q, rope, (__nv_bfloat16*)k_pool, (__nv_bfloat16*)v_pool, table, table_width, pool_blocks,
                 len_before, heads, kv_heads, scale_log2, window, splits, 0, (__nv_bfloat16*)out, part_acc, part_ml, tickets, decode_undelivered_bytes_for_tests, status, sinks, shaping);
         }
     }
-    static bool configured = false;
     auto kernel = attention_decode_kernel<HD, ROPE, SHAPE, false, NQ, SHAPED>;
-    if (!configured) {
-        const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, shared);
-        if (err != cudaSuccess) return err;
-        configured = true;
-    }
+    const cudaError_t err = tt_allow_shared(kernel, shared);
+    if (err != cudaSuccess) return err;
     if (slices_form_cluster(splits))
         return tt_launch_pdl_cluster(kernel, dim3(sequences, kv_heads, splits), dim3(D::WARPS * 32), shared, stream, (unsigned)splits,
             (const __nv_bfloat16*)q, rope, (__nv_bfloat16*)k_pool, (__nv_bfloat16*)v_pool, table, table_width, pool_blocks,
@@ -991,12 +983,8 @@ int launch(const void* q, const void* k_pool, const void* v_pool, const int* tab
         return merge_slices<HD>(n_tokens, heads, splits, out, part_acc, part_ml, stream, slices_form_cluster(splits));
     }
     if (one_token_each) {
-        static int sm_count = 0;
-        if (sm_count == 0) {
-            int device = 0;
-            if ((err = cudaGetDevice(&device)) != cudaSuccess) return (int)err;
-            if ((err = cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess) return (int)err;
-        }
+        int sm_count = 0;
+        if ((err = tt_sm_count(&sm_count)) != cudaSuccess) return (int)err;
         const long long ctas = (long long)sequences * kv_heads * splits;
         if (ctas > sm_count) tickets = nullptr;         // several CTAs per SM: the variants without tickets, and the merge kernel
         bool done = false;
@@ -1022,13 +1010,9 @@ int launch(const void* q, const void* k_pool, const void* v_pool, const int* tab
         if (splits != 1) return (int)cudaErrorInvalidValue;
         using P = PromptShape<HD>;
         constexpr int shared = P::STAGES * 2 * P::TILE_BYTES;
-        static bool configured = false;
         auto kernel = attention_mma_kernel<HD>;
-        if (!configured) {
-            err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, shared);
-            if (err != cudaSuccess) return (int)err;
-            configured = true;
-        }
+        err = tt_allow_shared(kernel, shared);
+        if (err != cudaSuccess) return (int)err;
         const int tokens_per_tile = 16 / group;
         const int tokens_per_cta = tokens_per_tile * MMA_WARPS;
         const int cta_tiles = (n_tokens + tokens_per_cta - 1) / tokens_per_cta + sequences;   // upper bound; spare CTAs leave at once

@@ -542,13 +542,9 @@ int launch(const void* q, const void* k_pool, const void* v_pool, const Args& ar
         const cuuint32_t box[2] = {KEYS, (cuuint32_t)L::VD};
         if (!tc::make_map(&map_v, v_pool, 2, dims, strides, box)) return -1;
     }
-    static bool configured = false;
     auto kernel = attention_tcgen05_kernel<HD, SHAPED, MAPS>;
-    if (!configured) {
-        const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM);
-        if (err != cudaSuccess) return (int)err;
-        configured = true;
-    }
+    const cudaError_t err = tt_allow_shared(kernel, L::SMEM);
+    if (err != cudaSuccess) return (int)err;
     tt_launch_pdl(kernel, dim3(args.kv_heads * (MAPS ? 2 : 1), args.cta_tiles), dim3(L::THREADS), (size_t)L::SMEM, stream, map_q, map_k, map_v, args);
     return (int)cudaGetLastError();
 }

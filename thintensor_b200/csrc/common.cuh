@@ -48,6 +48,19 @@ static inline cudaError_t tt_launch_pdl(Kernel kernel, dim3 grid, dim3 block, si
     return cudaLaunchKernelEx(&config, kernel, args...);
 }
 
+// Dynamic shared memory beyond 48 KB, asked for on every launch: what was allowed holds for the device that was current alone, and an engine may run on any
+// of the process's.
+template <typename Kernel>
+static inline cudaError_t tt_allow_shared(Kernel kernel, size_t bytes) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+// The current device's multiprocessors.
+static inline cudaError_t tt_sm_count(int* count) {
+    int device = 0;
+    const cudaError_t code = cudaGetDevice(&device);
+    return code != cudaSuccess ? code : cudaDeviceGetAttribute(count, cudaDevAttrMultiProcessorCount, device);
+}
+
 // The same with the grid's z dimension grouped into thread-block clusters of cluster_z CTAs.
 template <typename Kernel, typename... Args>
 static inline cudaError_t tt_launch_pdl_cluster(Kernel kernel, dim3 grid, dim3 block, size_t shared, cudaStream_t stream,

@@ -296,12 +296,8 @@ extern "C" int tt_gemm_split(const float* x, long long ldx, const float* w, long
     const int kp = (k + 7) / 8 * 8;
     const int tiles = (m + 255) / 256, tokens = ((m + tiles - 1) / tiles + 31) / 32 * 32;
     if (tiles > 65535) return (int)cudaErrorInvalidValue;
-    static bool configured = false;
-    if (!configured) {
-        const cudaError_t err = cudaFuncSetAttribute(gemm_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SHARED);
-        if (err != cudaSuccess) return (int)err;
-        configured = true;
-    }
+    cudaError_t err = tt_allow_shared(gemm_split_kernel, SHARED);
+    if (err != cudaSuccess) return (int)err;
     CUtensorMap map;
     const cuuint64_t dims[3] = {(cuuint64_t)k, (cuuint64_t)m, PARTS};
     const cuuint64_t strides[2] = {(cuuint64_t)kp * 2, (cuuint64_t)m * kp * 2};
@@ -309,7 +305,7 @@ extern "C" int tt_gemm_split(const float* x, long long ldx, const float* w, long
     if (!tc::make_map(&map, parts, 3, dims, strides, box)) return (int)cudaErrorInvalidValue;
     const long long quads = (long long)m * (kp / 4);
     const int blocks = (int)std::min((quads + 255) / 256, (long long)sms * 8);
-    cudaError_t err = tt_launch_pdl(cut_kernel, dim3(blocks), dim3(256), 0, stream, x, ldx, (__nv_bfloat16*)parts, m, k, kp,
+    err = tt_launch_pdl(cut_kernel, dim3(blocks), dim3(256), 0, stream, x, ldx, (__nv_bfloat16*)parts, m, k, kp,
                                     (int)((uintptr_t)x % 16 == 0 && ldx % 4 == 0));
     if (err != cudaSuccess) return (int)err;
     Args args = {x, w, bias, out, status, ldx, ldw, ldo, split_stride, m, n, k, ((k + BK - 1) / BK + splits - 1) / splits, tokens,

@@ -1215,13 +1215,9 @@ bool make_map(CUtensorMap* map, const void* base, long long rows, long long k, l
 template <int FORM, int BN, int STAGES, int GROUP = 1>
 int launch(const CUtensorMap& map_a, const CUtensorMap& map_b, const Args& args, dim3 grid, cudaStream_t stream) {
     constexpr int shared = Shape<FORM, BN>::stage_bytes * STAGES + 1024;
-    static bool configured = false;
     auto kernel = gemm_tcgen05_kernel<FORM, BN, STAGES, GROUP>;
-    if (!configured) {
-        const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, shared);
-        if (err != cudaSuccess) return (int)err;
-        configured = true;
-    }
+    const cudaError_t err = tt_allow_shared(kernel, shared);
+    if (err != cudaSuccess) return (int)err;
     tt_launch_pdl(kernel, grid, dim3(THREADS), shared, stream, map_a, map_b, args);
     return (int)cudaGetLastError();
 }
@@ -1230,17 +1226,11 @@ template <int FORM, int WIDE = 256>
 int launch_persistent(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensorMap& map_out, const Args& args, int tiles_m, int tiles_total,
                       int splits, cudaStream_t stream) {
     constexpr int shared = P_STAGE_BYTES * P_STAGES + 1024 + (FORM == TOKENS_ON_M || FORM == TOKENS_ON_M_SWIGLU ? OUT_SLAB_BYTES : 0);
-    static bool configured = false;
-    static int sm_count = 0;
+    int sm_count = 0;
     auto kernel = gemm_tcgen05_persistent_kernel<FORM, WIDE>;
-    if (!configured) {
-        cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, shared);
-        if (err != cudaSuccess) return (int)err;
-        int device = 0;
-        if ((err = cudaGetDevice(&device)) != cudaSuccess) return (int)err;
-        if ((err = cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess) return (int)err;
-        configured = true;
-    }
+    cudaError_t err = tt_allow_shared(kernel, shared);
+    if (err == cudaSuccess) err = tt_sm_count(&sm_count);
+    if (err != cudaSuccess) return (int)err;
     const int items = tiles_total * splits;
     const int ctas = items < sm_count ? items : sm_count;
     tt_launch_pdl(kernel, dim3(ctas), dim3(THREADS), shared, stream, map_a, map_b, map_out, args, tiles_m, tiles_total, splits);
@@ -1251,17 +1241,11 @@ template <int FORM, int WIDE = 256>
 int launch_pair(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensorMap& map_out, const Args& args, int tiles_m, int tiles_total,
                 cudaStream_t stream) {
     constexpr int shared = PAIR_STAGE_BYTES * PAIR_STAGES + 1024 + (FORM == TOKENS_ON_M || FORM == TOKENS_ON_M_SWIGLU ? OUT_SLAB_BYTES : 0);
-    static bool configured = false;
-    static int sm_count = 0;
+    int sm_count = 0;
     auto kernel = gemm_tcgen05_pair_kernel<FORM, WIDE>;
-    if (!configured) {
-        cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, shared);
-        if (err != cudaSuccess) return (int)err;
-        int device = 0;
-        if ((err = cudaGetDevice(&device)) != cudaSuccess) return (int)err;
-        if ((err = cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess) return (int)err;
-        configured = true;
-    }
+    cudaError_t err = tt_allow_shared(kernel, shared);
+    if (err == cudaSuccess) err = tt_sm_count(&sm_count);
+    if (err != cudaSuccess) return (int)err;
     // with the tiles' k-blocks dealt out (args.shares) every pair has work even where the tiles are fewer than the pairs
     const int pairs = (tiles_total < sm_count / 2 && !args.shares) ? tiles_total : sm_count / 2;
     cudaLaunchConfig_t config = {};
@@ -1278,7 +1262,7 @@ int launch_pair(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtens
     attribute[1].val.clusterDim.z = 1;
     config.attrs = attribute;
     config.numAttrs = 2;
-    const cudaError_t err = cudaLaunchKernelEx(&config, kernel, map_a, map_b, map_out, args, tiles_m, tiles_total);
+    err = cudaLaunchKernelEx(&config, kernel, map_a, map_b, map_out, args, tiles_m, tiles_total);
     return err != cudaSuccess ? (int)err : (int)cudaGetLastError();
 }
 

@@ -429,6 +429,7 @@ __global__ void latent_attention_rows_kernel(const float* __restrict__ absorbed,
 // 16 heads: 59 -> 37 us with a cold L2 (four warps, the queries in float32 and narrowed here, an integer division for every 16 bytes copied).
 constexpr int LT_KEYS = 64, LT_HEADS = 16, LT_S_LD = LT_KEYS + 4, LT_P_LD = LT_KEYS + 8, LT_WARPS = 8;
 
+constexpr size_t LT_MOST_SHARED = 200 * 1024;
 static size_t latent_decode_shared(int row_len) {
     return (size_t)(LT_HEADS + LT_KEYS) * (row_len + 8) * sizeof(__nv_bfloat16) + (size_t)2 * LT_HEADS * LT_S_LD * sizeof(float) +
            (size_t)LT_HEADS * LT_P_LD * sizeof(__nv_bfloat16);
@@ -745,13 +746,9 @@ extern "C" int tt_latent_attention(const float* q, int q_splits, long long q_str
 #define TT_ATT_ROWS(TA) tt_launch_pdl(latent_attention_rows_kernel<TA>, grid, block, 0, stream, (const float*)absorbed, (const TA*)pool, table, table_width, pool_blocks, cu, len_before, sequences, n_tokens, heads, rot, rank, window, splits, part_acc, part_ml, status)
     const int piece = act_dtype == TT_F32 ? 4 : 8;              // numbers in 16 bytes of a cache row
     if (one_token_each == 2) {                                  // the caller has checked tt_latent_decode_mma_takes and set splits for slices of LT_KEYS
-        static size_t allowed = 0;
         const size_t need = latent_decode_shared(rank + rot);
-        if (need > allowed) {
-            const cudaError_t e = cudaFuncSetAttribute(latent_decode_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need);
-            if (e != cudaSuccess) return (int)e;
-            allowed = need;
-        }
+        const cudaError_t e = tt_allow_shared(latent_decode_mma_kernel, LT_MOST_SHARED);    // (not what this launch needs: a captured one may need more)
+        if (e != cudaSuccess) return (int)e;
         tt_launch_pdl(latent_decode_mma_kernel, dim3(n_tokens, splits, (heads + LT_HEADS - 1) / LT_HEADS), dim3(32 * LT_WARPS), need, stream,
                       (const __nv_bfloat16*)(const void*)absorbed, (const __nv_bfloat16*)pool, table, table_width, pool_blocks, len_before, heads, rot, rank, window,
                       splits, part_acc, part_ml, status);
@@ -948,6 +945,6 @@ extern "C" int tt_latent_queries(const float* q, int splits, long long split_str
 // Whether the tensor-core decode kernel takes these sizes (bfloat16 cache, latent and rotated part multiples of 16, shared memory), and
 // the keys of one of its slices.
 extern "C" int tt_latent_decode_mma_takes(int act_dtype, int rank, int rot) {
-    return act_dtype == TT_BF16 && rank % 16 == 0 && rot % 16 == 0 && rank + rot <= LAT_MAX_ROW && latent_decode_shared(rank + rot) <= 200 * 1024;
+    return act_dtype == TT_BF16 && rank % 16 == 0 && rot % 16 == 0 && rank + rot <= LAT_MAX_ROW && latent_decode_shared(rank + rot) <= LT_MOST_SHARED;
 }
 extern "C" int tt_latent_decode_slice_keys() { return LT_KEYS; }

@@ -522,12 +522,8 @@ constexpr int REC_WIDE_GROUPS = 16, REC_WIDE_COLS = 4;      // the form for grid
 static bool rec_wide(int mode, long long ctas, int rows) {
     if (rows > 16 * REC_LANES) return false;
     if (mode) return mode == 2;
-    static int sms = 0;
-    if (!sms) {
-        int device = 0;
-        cudaGetDevice(&device);
-        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms <= 0) sms = 148;
-    }
+    int sms = 0;
+    if (tt_sm_count(&sms) != cudaSuccess || sms <= 0) sms = 148;
     return ctas >= 2LL * sms;
 }
 static bool rec_aligned(const void* p, int a, int b, int c, int d) { return (((uintptr_t)p & 15) == 0) && !((a | b | c | d) & 3); }
@@ -1230,12 +1226,8 @@ row_decay_blocks_kernel(const RowScan a) {
 template <int K, bool DELTA, bool BONUS>
 static int row_decay_blocks_launch(const RowScan& scan, int sequences, cudaStream_t stream) {
     constexpr size_t shared = (size_t)2 * RB_BLOCKS * (((DELTA ? 3 : 2) * RB_BLOCK + 1) * K * RB_LANES + RB_SCALARS) * sizeof(float);
-    static bool allowed = false;
-    if (!allowed) {
-        const cudaError_t code = cudaFuncSetAttribute(row_decay_blocks_kernel<K, DELTA, BONUS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
-        if (code != cudaSuccess) return (int)code;
-        allowed = true;
-    }
+    const cudaError_t code = tt_allow_shared(row_decay_blocks_kernel<K, DELTA, BONUS>, shared);
+    if (code != cudaSuccess) return (int)code;
     tt_launch_pdl(row_decay_blocks_kernel<K, DELTA, BONUS>, dim3(scan.heads, sequences, (scan.V + RB_TILE - 1) / RB_TILE), dim3(RB_THREADS), shared, stream, scan);
     TT_LAUNCH_CHECK();
 }

@@ -798,16 +798,12 @@ scan_chunks_kernel(const ScanChunks a) {
     store_state();
 }
 
-// on every launch: it holds for the current device alone, and an engine may run on any of the process's
-template <typename Kernel>
-static cudaError_t ck_allow(Kernel kernel, size_t bytes) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); }
-
 template <int NP, int PB, int NS>
 static int scan_chunks_launch(const ScanChunks& a, int max_slots, cudaStream_t stream) {
     using L = CkWalk<NP, PB, NS>;
     constexpr size_t prepare_bytes = CkPrepare<NP>::BYTES;
-    cudaError_t code = ck_allow(scan_chunks_prepare_kernel<NP>, prepare_bytes);
-    if (code == cudaSuccess) code = ck_allow(scan_chunks_kernel<NP, PB, NS>, L::BYTES);
+    cudaError_t code = tt_allow_shared(scan_chunks_prepare_kernel<NP>, prepare_bytes);
+    if (code == cudaSuccess) code = tt_allow_shared(scan_chunks_kernel<NP, PB, NS>, L::BYTES);
     if (code != cudaSuccess) return (int)code;
     tt_launch_pdl(scan_chunks_prepare_kernel<NP>, dim3(max_slots, a.groups, (a.heads / a.groups + a.together - 1) / a.together), dim3(CK_THREADS), prepare_bytes, stream, a);
     tt_launch_pdl(scan_chunks_kernel<NP, PB, NS>, dim3(a.heads, a.sequences, (a.P + L::TP - 1) / L::TP), dim3(L::THREADS), (size_t)L::BYTES, stream, a);
@@ -1497,8 +1493,8 @@ template <int NP, int PB, int NS>
 static int delta_chunks_launch(const DeltaChunks& a, int max_slots, cudaStream_t stream) {
     using L = CdWalk<NP, PB, NS>;
     constexpr size_t prepare_bytes = CdPrepare<NP>::BYTES;
-    cudaError_t code = ck_allow(delta_chunks_prepare_kernel<NP>, prepare_bytes);
-    if (code == cudaSuccess) code = ck_allow(delta_chunks_kernel<NP, PB, NS>, L::BYTES);
+    cudaError_t code = tt_allow_shared(delta_chunks_prepare_kernel<NP>, prepare_bytes);
+    if (code == cudaSuccess) code = tt_allow_shared(delta_chunks_kernel<NP, PB, NS>, L::BYTES);
     if (code != cudaSuccess) return (int)code;
     tt_launch_pdl(delta_chunks_prepare_kernel<NP>, dim3(max_slots, a.heads), dim3(CD_THREADS), prepare_bytes, stream, a);
     tt_launch_pdl(delta_chunks_kernel<NP, PB, NS>, dim3(a.heads, a.sequences, (a.V + L::TP - 1) / L::TP), dim3(L::THREADS), (size_t)L::BYTES, stream, a);
