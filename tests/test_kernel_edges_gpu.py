@@ -93,6 +93,24 @@ def test_product_in_parts_of_what_is_not_finite():
     assert torch.equal(got[0][rows][:, 6:299], clean[0][rows][:, 6:299])
 
 
+@pytest.mark.parametrize("small_x,small_w", [(2.0 ** -100, 1.0), (2.0 ** -110, 1.0), (2.0 ** -120, 1.0), (2.0 ** -70, 2.0 ** -50), (1.0, 2.0 ** -118)])
+def test_product_in_parts_of_tiny_numbers(small_x, small_w):
+    """Numbers whose third part is below what bfloat16 holds keep the bits of float32; rows of zeros beside them stay zeros."""
+    from thintensor_b200.kernels import api
+
+    m, n, k = 40, 130, 192
+    x, w = randn(m, k, seed=6) * small_x, randn(n, k, seed=7) * small_w
+    x[5], w[9] = 0.0, 0.0
+    out, plain = torch.empty(2, m, n, device=DEV), torch.empty(1, m, n, device=DEV)
+    parts, status = torch.empty(api.gemm_split_parts(m, k), dtype=torch.bfloat16, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    api.gemm_split(x, w, None, out, parts, status)
+    api.gemm_simt(x, w, None, plain)
+    want = x.double() @ w.double().T
+    in_parts, multiplied = (float((got.double().sum(0) - want).norm() / want.norm()) for got in (out, plain))
+    assert in_parts <= multiplied, (in_parts, multiplied)
+    assert bool((out[:, 5] == 0.0).all()) and bool((out[:, :, 9] == 0.0).all()) and int(status) == 0
+
+
 def test_slices_of_products_in_parts_follow_the_sizes():
     from thintensor_b200.kernels import api
 

@@ -22,7 +22,9 @@
 // against 64 bits, normal numbers: 193 rows, 2,048 of 8,192 6.6e-7 -> 1.1e-7, 17 rows, 40 of 72 1.6e-7 -> 0.8e-7.
 //
 // A sum that comes out infinite or NaN (an operand that is, one that rounds up to infinity, parts of infinite products of opposite
-// signs) is formed again by multiply-adds, by the thread that has it: such outputs are what gemm_simt.cu makes of them.
+// signs) is formed again by multiply-adds, by the thread that has it: such outputs are what gemm_simt.cu makes of them.  So is a sum below 2^-90: the third
+// part of a number below 2^-109 falls under the smallest bfloat16 number, 2^-133, and is lost (x of 1e-36: errors of 2.6e-5 instead of 1.5e-7).  Sums of
+// such numbers times others that reach 2^-90 all the same (others above 2^18 / k) keep the bits that two parts have.
 #include <algorithm>
 
 #include <cooperative_groups.h>
@@ -82,6 +84,13 @@ __global__ void __launch_bounds__(256) cut_kernel(const float* __restrict__ x, l
         *reinterpret_cast<uint2*>(to + plane) = mid;
         *reinterpret_cast<uint2*>(to + 2 * plane) = lo;
     }
+}
+
+// not finite, or neither zero nor as large as 2^-90
+__device__ __forceinline__ bool form_again(float sum) {
+    constexpr uint32_t LEAST = (127u - 90u) << 23, INF = 255u << 23;
+    const uint32_t bits = __float_as_uint(sum) & 0x7fffffffu;
+    return bits - LEAST >= INF - LEAST && bits != 0u;
 }
 
 struct Args {
@@ -262,7 +271,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
                 for (int e = 0; e < 16; ++e) {
                     if (b * 16 + e < count) {
                         to[0] = acc[b][e] + bias;
-                        again[b] |= (unsigned)!(fabsf(acc[b][e]) <= 3.402823466e38f) << e;
+                        again[b] |= (unsigned)form_again(acc[b][e]) << e;
                     }
                     to += args.ldo;
                 }
