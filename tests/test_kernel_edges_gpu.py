@@ -778,6 +778,88 @@ def test_delta_rule_in_chunks_is_as_close_as_token_by_token(heads, D, V):
     assert chunked <= 1.05 * by_token, (chunked, by_token)
 
 
+DECAYS = [0.9999, 0.999, 0.99, 0.95, 0.9, 0.8, 0.7, 0.5, 0.3, 0.1, 0.05]
+
+
+def closeness(outs, want, heads):
+    """Relative errors [outputs, states] of every decay's heads, in chunks and token by token."""
+    result = []
+    for got, exact in zip(zip(*outs), want):
+        exact = exact.reshape(-1, len(DECAYS), heads // len(DECAYS), exact[0, 0].numel())
+        result.append([((o.reshape(exact.shape) - exact).square().sum((0, 2, 3)) / exact.square().sum((0, 2, 3))).sqrt().cpu() for o in got])
+    return result
+
+
+@pytest.mark.parametrize("tokens", [357, 130, 80])
+@pytest.mark.parametrize("P,N", [(16, 128), (32, 100), (64, 128), (50, 70), (128, 128), (100, 128), (32, 64), (64, 64), (128, 40)])
+def test_recurrence_in_chunks_of_every_decay(P, N, tokens):
+    """Outputs and states of slow and of fast decays, each decay's heads by themselves, against 64 bits: no further off than token by token but for a twentieth.
+    (States that hold only the last few tokens were up to 2.3 times as far off: the tensor cores truncate their sums.)"""
+    from thintensor_b200.kernels import api
+
+    copies = 12
+    heads = copies * len(DECAYS)
+    inner = heads * P
+    rows, decays = randn(tokens, inner + 2 * heads * N, seed=170), torch.tensor(DECAYS, device=DEV).repeat_interleave(copies).contiguous()
+    cu, slots, outs = i32([0, tokens]), i32([0]), []
+    for chunks in (True, False):
+        state, y = torch.zeros(1, heads, P, N, device=DEV), torch.empty(tokens, inner, device=DEV)
+        if chunks:
+            scratch = torch.full(api.scan_chunks_scratch(tokens, 1, heads, heads, N), float("nan"), device=DEV)
+            api.scan_chunks(rows, 0, inner, inner + heads * N, state, y, cu, slots, 1, heads, P, N, heads, scratch, fixed_decay=decays)
+        else:
+            api.decay_scan(rows, decays, state, y, cu, slots, 1, heads, N, P)
+        outs.append((y.double().reshape(tokens, heads, P), state[0].double().reshape(1, heads, P * N)))
+    x, b, c = (z.double().reshape(tokens, heads, -1) for z in rows.split((inner, heads * N, heads * N), 1))
+    S, want = torch.zeros(heads, P, N, dtype=torch.float64, device=DEV), torch.empty(tokens, heads, P, dtype=torch.float64, device=DEV)
+    for t in range(tokens):
+        S = torch.baddbmm(decays.double()[:, None, None] * S, x[t][:, :, None], b[t][:, None, :])
+        want[t] = torch.bmm(S, c[t][:, :, None])[..., 0]
+    for name, (chunked, by_token) in zip(("outputs", "states"), closeness(outs, (want, S.reshape(1, heads, P * N)), heads)):
+        assert bool((chunked <= 1.05 * by_token).all()), (name, chunked / by_token)
+
+
+@pytest.mark.parametrize("D,V", [(128, 16), (100, 32), (128, 64), (64, 16), (64, 32), (40, 50)])
+def test_delta_rule_in_chunks_of_every_decay(D, V):
+    """As above.  A state's error is mostly that of the last rows that went into it, a few numbers a head, so states of fast decays are compared in the mean over
+    lengths and decays (0.83 to 1.02 at a length; 1.04 to 1.23 with their sums on the tensor cores)."""
+    from thintensor_b200.kernels import api
+
+    copies, fast = 12, []
+    heads = copies * len(DECAYS)
+    qk = heads * D
+    decays = torch.tensor(DECAYS, dtype=torch.float64, device=DEV).repeat_interleave(copies)
+    a_log, dt_bias = torch.log(-torch.log(decays)).float(), torch.full((heads,), 0.5413248546, device=DEV)
+    for tokens in (357, 130, 80):
+        qkv, raw = randn(tokens, 2 * qk + heads * V, seed=175), randn(1, tokens, 2 * heads, seed=176)
+        raw[:, :, heads:] = 0.0                            # softplus(0 + 0.5413) = 1: a decay is exp(-exp(a_log))
+        cu, slots, outs = i32([0, tokens]), i32([0]), []
+        for chunks in (True, False):
+            state, out = torch.zeros(1, heads, V, D, device=DEV), torch.empty(tokens, heads * V, device=DEV)
+            if chunks:
+                scratch = torch.full(api.delta_chunks_scratch(tokens, 1, heads, D, V), float("nan"), device=DEV)
+                api.delta_chunks(qkv, raw, 0, heads, dt_bias, a_log, state, out, cu, slots, 1, heads, heads, D, V, scratch)
+            else:
+                api.delta_scan(qkv, raw, 0, heads, dt_bias, a_log, state, out, cu, slots, 1, heads, heads, D, V)
+            outs.append((out.double().reshape(tokens, heads, V), state[0].double().reshape(1, heads, V * D)))
+        z = raw[0].double()
+        beta, decay = torch.sigmoid(z[:, :heads]), torch.exp(-torch.exp(a_log.double()) * torch.nn.functional.softplus(z[:, heads:] + dt_bias.double()))
+        unit = lambda y: y / (y.square().sum(-1, keepdim=True) + 1e-6).sqrt()
+        q, k = (unit(part.double().reshape(tokens, heads, D)) for part in qkv[:, :2 * qk].split(qk, 1))
+        v, S = qkv[:, 2 * qk:].double().reshape(tokens, heads, V), torch.zeros(heads, V, D, dtype=torch.float64, device=DEV)
+        want = torch.empty(tokens, heads, V, dtype=torch.float64, device=DEV)
+        for t in range(tokens):
+            S = decay[t][:, None, None] * S
+            S = torch.baddbmm(S, (beta[t][:, None] * (v[t] - torch.bmm(S, k[t][:, :, None])[..., 0]))[:, :, None], k[t][:, None, :])
+            want[t] = torch.bmm(S, q[t][:, :, None])[..., 0] * D ** -0.5
+        (chunked, by_token), (state_chunked, state_by_token) = closeness(outs, (want, S.reshape(1, heads, V * D)), heads)
+        assert bool((chunked <= 1.1 * by_token).all()), (tokens, chunked / by_token)
+        slow = [i for i, d in enumerate(DECAYS) if d >= 0.95]
+        assert bool((state_chunked <= 1.1 * state_by_token)[slow].all()), (tokens, state_chunked / state_by_token)
+        fast.append((state_chunked / state_by_token)[[i for i, d in enumerate(DECAYS) if d <= 0.7]])
+    assert float(torch.stack(fast).mean()) <= 1.03, fast
+
+
 # --------------------------------------------------------------------------------- experts' products of sorted tokens
 @pytest.mark.parametrize("tokens,top,experts,hidden,inter", [(1, 1, 1, 64, 128), (300, 2, 3, 72, 128), (513, 4, 16, 256, 256), (1500, 1, 5, 264, 384), (200, 3, 70, 128, 128)])
 def test_experts_of_sorted_tokens(tokens, top, experts, hidden, inter):

@@ -6,10 +6,10 @@
 // With f(i, j) = a_(j+1) * .. * a_i, e_i = a_0 * .. * a_i and w_j = f(63, j) dt_j, a chunk that starts from state S gives
 //   y_i = e_i (S^T C_i) + sum_(j<=i) f(i, j) dt_j (C_i . B_j) x_j + D x_i,     S <- e_63 S + sum_j w_j B_j x_j^T
 // so the token-by-token chain of row products becomes four matrix products a chunk.  They run on the tensor cores with every operand in three
-// bfloat16 parts (split_mma.cuh), which keeps them float32 products: against 64 bits, 30 runs, the outputs' error is 0.75 and the states' 0.81 of
-// token by token in the mean (float32 multiply-adds in chunks: 0.93 and 0.94; states that hold only the last few tokens are up to a third
-// further off).  The decays only ever enter as products of decays (never as quotients, never as differences of sums of logarithms): nothing cancels,
-// and a constant decay may have any sign.  Up to 64 of them are multiplied before they meet a state, so none may exceed one (callers see to
+// bfloat16 parts (split_mma.cuh); the rows that a state of fast decays is made of are added by multiply-adds (ck_tail).  Error against 64 bits by decay, relative to
+// token by token (and of float32 multiply-adds in chunks): outputs 0.999 a token 0.25 (0.73), 0.9 0.77 (0.92), 0.5 0.93 (1.05), 0.1 0.89 (1.01); states 0.23 (0.75),
+// 0.67 (0.83), 1.00 (1.00), 1.00 (1.00).  The decays only ever enter as products of decays (never as quotients, never as differences of sums of logarithms): nothing
+// cancels, and a constant decay may have any sign.  Up to 64 of them are multiplied before they meet a state, so none may exceed one (callers see to
 // it).  Products of decays are formed in float64 from the float32 decays and rounded once inside an 8-token block and in e, w and e_63; across
 // blocks f(i, j) dt_j is the product of three such numbers (in float32 here: five roundings; in float64, rounded once, for the delta rule below).
 // Numbers that are not finite reach the tokens they reach in the recurrence and no others: the first kernel leaves them out and says which
@@ -23,7 +23,8 @@
 // adding up outputs and waiting for one another).  16 warps with half the registers were slower at every size (64 heads of 64 x 128, 2,048
 // tokens: 222 against 169 us), as was fetching the operands with 16-byte copies by all threads instead of the copy engine (198).
 // Token by token, in chunks of float32 multiply-adds, and now (us, one B200, back to back): 64 heads of 64 x 128, one sequence of 2,048 tokens
-// 748, 227, 170, four of 731 423, 340, 236; 16 heads of 256 x 128, four of 1,024 590, 476, 311.
+// 748, 227, 171 (180 where every chunk has a tail), four of 731 423, 340, 236; 16 heads of 256 x 128, four of
+// 1,024 590, 476, 313 (334).
 #include "common.cuh"
 #include "split_mma.cuh"
 #include "tcgen05.cuh"
@@ -79,10 +80,42 @@ __device__ __forceinline__ float ck_sum_slices(const float* __restrict__ p, int 
 }
 
 constexpr int CK_MBLOCKS = 10;                                  // blocks of 16 x 16 on and below the diagonal of 64 x 64
-// a chunk's record for one head: e [64], w [64] (times dt), decay [64], dt [64], then e_63 and the first token with a number that is not finite
-constexpr int CK_R_E = 0, CK_R_W = 64, CK_R_DECAY = 128, CK_R_DT = 192, CK_R_ALL = 256, CK_R_BAD = 257, CK_RECORD = 260;
+// a chunk's record for one head: e [64], w [64] (times dt; zero for the tail's tokens), e_63, the first token with a number that is not finite, the first
+// token of the tail, the tail's w [8] (so far in shared memory in the walk), then decay [64] and dt [64]
+constexpr int CK_R_E = 0, CK_R_W = 64, CK_R_ALL = 128, CK_R_BAD = 129, CK_R_TAIL = 130, CK_R_TAIL_W = 132, CK_NEAR = 140, CK_R_DECAY = 140, CK_R_DT = 204, CK_RECORD = 268;
 
-
+// The rows of a chunk's last 8 tokens (its tail) are added to the state by multiply-adds, token after token, instead of by products on the tensor
+// cores, where their decays multiply to less than CK_SHORT (0.77 a token).  Those rows are most of the state then, and a sum that a few products
+// dominate is right to half a unit as a chain of multiply-adds, while the tensor cores truncate it.  The first kernel writes the 8 rows of B, or of w K.  Error of a state against 64 bits relative to token by
+// token, without tails and with them: 0.8 a token 0.89 and 0.89, 0.7 1.03 and 0.93, 0.5 1.41 and 1.00, 0.1 2.28 and 1.00.  So are all rows of a chunk of up to 8
+// tokens.  CK_TOKENS: no tail.
+constexpr int CK_TAIL_ROWS = 8;
+constexpr float CK_SHORT = 1.0f / 8.0f;
+__device__ __forceinline__ int ck_tail(const float* decay, int count, int lane) {       // by a whole warp
+    if (count <= CK_TAIL_ROWS) return 0;
+    float last = fabsf(decay[count - CK_TAIL_ROWS + (lane & 7)]);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) last *= __shfl_xor_sync(0xffffffffu, last, o);
+    return last < CK_SHORT ? count - CK_TAIL_ROWS : CK_TOKENS;
+}
+// where a state row's number lies in a row of the tail: a lane's rows of two tiles of 8 (2 q, 2 q + 1, 2 q + 8, 2 q + 9) side by side
+__device__ __forceinline__ int ck_tail_place(int row) { return (row & ~15) + 4 * ((row & 7) >> 1) + 2 * ((row >> 3) & 1) + (row & 1); }
+// s += x times the tail's row for this lane's two columns; at: the row at the warp's first state row and the lane's four numbers
+template <int TILES>
+__device__ __forceinline__ void ck_add_row(float (&s)[TILES][4], float x0, float x1, const float* at) {
+#pragma unroll
+    for (int k = 0; k < TILES; k += 2) {
+        const float4 v = *reinterpret_cast<const float4*>(at + 8 * k);
+        s[k][0] = fmaf(x0, v.x, s[k][0]);
+        s[k][1] = fmaf(x0, v.y, s[k][1]);
+        s[k][2] = fmaf(x1, v.x, s[k][2]);
+        s[k][3] = fmaf(x1, v.y, s[k][3]);
+        s[k + 1][0] = fmaf(x0, v.z, s[k + 1][0]);
+        s[k + 1][1] = fmaf(x0, v.w, s[k + 1][1]);
+        s[k + 1][2] = fmaf(x1, v.z, s[k + 1][2]);
+        s[k + 1][3] = fmaf(x1, v.w, s[k + 1][3]);
+    }
+}
 struct ScanChunks {
     const float* x;             // float32 rows of `stride` numbers: x of head h at + h * P, B and C of group g at + g * N
     const float* b;
@@ -98,12 +131,12 @@ struct ScanChunks {
     float* state;               // [slots][heads][P][N]
     float* y;                   // [tokens][heads * P]
     unsigned* status;           // or null
-    unsigned char* scratch;     // [slots][groups]: C and B as operands of the walk; [slots][heads]: scores times factors as an operand, the record
+    unsigned char* scratch;     // [slots][groups]: C and B as operands of the walk, B's rows of the tail; [slots][heads]: scores times factors as an operand, the record
     int max_slots;
     const int* cu;
     const int* slots;
     int sequences, heads, groups, P, N, vec, together;
-    static __host__ __device__ constexpr size_t group_bytes(int padded) { return (size_t)2 * padded / 16 * 4 * SPLIT_BLOCK_BYTES; }
+    static __host__ __device__ constexpr size_t group_bytes(int padded) { return (size_t)2 * padded / 16 * 4 * SPLIT_BLOCK_BYTES + CK_TAIL_ROWS * padded * sizeof(float); }
     static __host__ __device__ constexpr size_t head_bytes() { return (size_t)CK_MBLOCKS * SPLIT_BLOCK_BYTES + CK_RECORD * sizeof(float); }
     template <int NP> __device__ uint4* group_scratch(int slot, int g) const {
         return reinterpret_cast<uint4*>(scratch + ((size_t)slot * groups + g) * group_bytes(NP));
@@ -261,6 +294,11 @@ scan_chunks_prepare_kernel(const ScanChunks a) {
                     atomicMin(&bad, r);
                     x = make_float4(ck_usable(x.x) ? x.x : 0.0f, ck_usable(x.y) ? x.y : 0.0f, ck_usable(x.z) ? x.z : 0.0f, ck_usable(x.w) ? x.w : 0.0f);
                 }
+                if (const int tail = r - max(count - CK_TAIL_ROWS, 0); matrix && blockIdx.z == 0 && tail >= 0 && tail < CK_TAIL_ROWS) {
+                    float* to = reinterpret_cast<float*>(a.group_scratch<NP>(slot, g) + 2 * KS * 4 * (SPLIT_BLOCK_BYTES / 16)) + tail * NP;
+                    *reinterpret_cast<float2*>(to + ck_tail_place(c)) = make_float2(x.x, x.y);
+                    *reinterpret_cast<float2*>(to + ck_tail_place(c + 2)) = make_float2(x.z, x.w);
+                }
                 uint2 hi, mid, lo;
                 split_pair(x.x, x.y, hi.x, mid.x, lo.x);
                 split_pair(x.z, x.w, hi.y, mid.y, lo.y);
@@ -368,16 +406,19 @@ scan_chunks_prepare_kernel(const ScanChunks a) {
             if (!ck_usable(decay[half]) || !ck_usable(step[half])) first_bad = min(first_bad, lane + 32 * half);
         first_bad = __reduce_min_sync(0xffffffffu, first_bad);
         float* record = reinterpret_cast<float*>(a.head_scratch<NP>(slot, h) + CK_MBLOCKS * (SPLIT_BLOCK_BYTES / 16));
+        const int tail = ck_tail(scalars[own][0], count, lane);
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
             const int i = lane + 32 * half;
             record[CK_R_E + i] = f[CK_E + i];
-            record[CK_R_W + i] = f[CK_W + i];
+            record[CK_R_W + i] = i < tail ? f[CK_W + i] : 0.0f;
+            if (i >= tail && i < tail + CK_TAIL_ROWS) record[CK_R_TAIL_W + i - tail] = f[CK_W + i];
             record[CK_R_DECAY + i] = decay[half];
             record[CK_R_DT + i] = step[half];
         }
         if (lane == 0) {
             record[CK_R_ALL] = f[CK_ALL];
+            record[CK_R_TAIL] = __int_as_float(tail);
             bad_head[own] = first_bad;
         }
     }
@@ -443,10 +484,11 @@ scan_chunks_prepare_kernel(const ScanChunks a) {
 template <int NP, int PB, int NS>
 struct CkWalk {
     static constexpr int THREADS = 32 * PB * NS, TP = 16 * PB, LDX = TP + 4, KS = NP / 16, KL = KS / NS;
-    static constexpr int C = 0, B = C + KS * 4 * SPLIT_BLOCK_BYTES, M = B + KS * 4 * SPLIT_BLOCK_BYTES, X = M + CK_MBLOCKS * SPLIT_BLOCK_BYTES;
-    static constexpr int X_BYTES = CK_TOKENS * LDX * 4, R = X + 2 * X_BYTES, PARTS = R + 2 * CK_RECORD * 4;
+    static constexpr int C = 0, B = C + KS * 4 * SPLIT_BLOCK_BYTES, TAIL = B + KS * 4 * SPLIT_BLOCK_BYTES, M = TAIL + CK_TAIL_ROWS * NP * 4, X = M + CK_MBLOCKS * SPLIT_BLOCK_BYTES;
+    static constexpr int X_BYTES = CK_TOKENS * LDX * 4, R = X + 2 * X_BYTES, PARTS = R + 2 * CK_NEAR * 4;
     static constexpr int W = PARTS + (NS > 1 ? PB * (NS - 1) * 8 * 512 : 0), BAD = W + (NS > 1 ? PB * 4 * SPLIT_BLOCK_BYTES : 0), BAR = BAD + TP * 4, BYTES = BAR + 16;
-    static constexpr int FIRST_BYTES = CK_RECORD * 4 + CK_MBLOCKS * SPLIT_BLOCK_BYTES + KS * 4 * SPLIT_BLOCK_BYTES, B_BYTES = KS * 4 * SPLIT_BLOCK_BYTES;
+    static_assert(BYTES <= 227 * 1024, "a CTA's shared memory");
+    static constexpr int FIRST_BYTES = CK_NEAR * 4 + CK_MBLOCKS * SPLIT_BLOCK_BYTES + KS * 4 * SPLIT_BLOCK_BYTES, B_BYTES = KS * 4 * SPLIT_BLOCK_BYTES;
     // Which 16 tokens' x (j) a warp multiplies with the scores of which outputs (q >= j): a block each, about as many for the warps of
     // every scheduler
     static constexpr int XA = NS >= 4 ? 1 : 4 / NS;
@@ -540,6 +582,7 @@ scan_chunks_kernel(const ScanChunks a) {
     uint4* Ws = reinterpret_cast<uint4*>(ck_bytes + L::W) + pb * 4 * (SPLIT_BLOCK_BYTES / 16);
     float4* parts = reinterpret_cast<float4*>(ck_bytes + L::PARTS) + pb * (NS - 1) * 8 * 32 + lane;          // [another warp][tile of 8 tokens][lane]
     int* bad_from = reinterpret_cast<int*>(ck_bytes + L::BAD);
+    const float* tail = reinterpret_cast<const float*>(ck_bytes + L::TAIL) + ns * (NP / NS) + 4 * (lane & 3);
     for (int e = threadIdx.x; e < 2 * CK_TOKENS * LDX; e += THREADS) reinterpret_cast<float*>(ck_bytes + L::X)[e] = 0.0f;      // what no copy writes is zero
     const uint32_t bar = tc::smem_u32(ck_bytes + L::BAR), bar_b = bar + 8;
     if (threadIdx.x == 0) {
@@ -551,7 +594,7 @@ scan_chunks_kernel(const ScanChunks a) {
     bool in_time = true;                                        // no wait has run out
 
     auto xs = [&](int chunk) { return reinterpret_cast<float*>(ck_bytes + L::X + (chunk & 1) * L::X_BYTES); };
-    auto records = [&](int chunk) { return reinterpret_cast<float*>(ck_bytes + L::R) + (chunk & 1) * CK_RECORD; };
+    auto records = [&](int chunk) { return reinterpret_cast<float*>(ck_bytes + L::R) + (chunk & 1) * CK_NEAR; };
     auto fetch_first = [&](int chunk) {                         // x, C, scores and factors
         if (chunk >= chunks) return;
         const int c0 = chunk * CK_TOKENS;
@@ -562,7 +605,7 @@ scan_chunks_kernel(const ScanChunks a) {
             tc::mbar_expect_tx(bar, L::FIRST_BYTES);
             ck_fetch(ck_bytes + L::C, a.group_scratch<NP>(slot0 + chunk, g), L::B_BYTES, bar);
             ck_fetch(ck_bytes + L::M, head, CK_MBLOCKS * SPLIT_BLOCK_BYTES, bar);
-            ck_fetch(records(chunk), head + CK_MBLOCKS * (SPLIT_BLOCK_BYTES / 16), CK_RECORD * 4, bar);
+            ck_fetch(records(chunk), head + CK_MBLOCKS * (SPLIT_BLOCK_BYTES / 16), CK_NEAR * 4, bar);
         }
     };
     fetch_first(0);
@@ -627,9 +670,11 @@ scan_chunks_kernel(const ScanChunks a) {
         // x, C, scores and factors are there; B, the weighted rows and the parts of the chunk before are read
         bool some_bad = __syncthreads_or(odd);
         some_bad |= __float_as_int(F[CK_R_BAD]) < CK_TOKENS;
+        const int count = min(CK_TOKENS, left), tail0 = __float_as_int(F[CK_R_TAIL]);
         if (threadIdx.x == 0) {
-            tc::mbar_expect_tx(bar_b, L::B_BYTES);
-            ck_fetch(ck_bytes + L::B, a.group_scratch<NP>(slot0 + chunk, g) + L::KS * 4 * (SPLIT_BLOCK_BYTES / 16), L::B_BYTES, bar_b);
+            const uint32_t bytes = L::B_BYTES + (tail0 < CK_TOKENS ? CK_TAIL_ROWS * NP * 4 : 0);
+            tc::mbar_expect_tx(bar_b, bytes);
+            ck_fetch(ck_bytes + L::B, a.group_scratch<NP>(slot0 + chunk, g) + L::KS * 4 * (SPLIT_BLOCK_BYTES / 16), bytes, bar_b);
         }
         if (some_bad) {
             // columns from their first token on that is, or meets, a number that is not finite go token by token; the others as ever
@@ -649,9 +694,9 @@ scan_chunks_kernel(const ScanChunks a) {
                 }
             store_state();
             __syncthreads();
-            const int count = min(CK_TOKENS, left);
+            const float* record = reinterpret_cast<const float*>(a.head_scratch<NP>(slot0 + chunk, h) + CK_MBLOCKS * (SPLIT_BLOCK_BYTES / 16));
             for (int p = warp; p < width; p += THREADS / 32)
-                if (bad_from[p] < count) ck_scan_column(a, F, first + chunk * CK_TOKENS, count, h, g, p0 + p, S + (size_t)p * N, bad_from[p]);
+                if (bad_from[p] < count) ck_scan_column(a, record, first + chunk * CK_TOKENS, count, h, g, p0 + p, S + (size_t)p * N, bad_from[p]);
             __syncthreads();
         }
         float* out = a.y + (size_t)(first + chunk * CK_TOKENS) * inner + (size_t)h * P + p0 + pb * 16 + gq;
@@ -773,6 +818,15 @@ scan_chunks_kernel(const ScanChunks a) {
                     v = long_memory ? fmaf(all, v, sum[i][e] + rest[i][e]) : fmaf(all, v, rest[i][e]) + sum[i][e];
                 }
         }
+        if (tail0 < CK_TOKENS) {
+            const float* x = own + tail0 * LDX;
+            const float4 w[2] = {reinterpret_cast<const float4*>(F + CK_R_TAIL_W)[0], reinterpret_cast<const float4*>(F + CK_R_TAIL_W)[1]};
+#pragma unroll
+            for (int i = 0; i < CK_TAIL_ROWS; ++i) {            // (zeros behind the last token)
+                const float wi = i & 2 ? (i & 1 ? w[i >> 2].w : w[i >> 2].z) : (i & 1 ? w[i >> 2].y : w[i >> 2].x);
+                ck_add_row(s, wi * x[i * LDX], wi * x[i * LDX + 8], tail + i * NP);
+            }
+        }
         if (NS > 1) {
 #pragma unroll
             for (int i = 0; i < 8 / NS; ++i) {
@@ -789,7 +843,6 @@ scan_chunks_kernel(const ScanChunks a) {
             }
         }
         if (some_bad) {
-            const int count = min(CK_TOKENS, left);
             if (bad_from[pb * 16 + gq] < count) load_state(0);
             if (bad_from[pb * 16 + gq + 8] < count) load_state(1);
         }
@@ -849,9 +902,10 @@ extern "C" int tt_scan_chunks(const float* rows, int width, int x_col, int b_col
 // (I + A) W = beta e K: neither needs the state, so the first kernel solves for both, parallel over chunks and heads, and the second
 // walks the chunks with   U = U0 - W S,   o = e Q S + P U (P_ij = f(i, j) q_i . k_j, j <= i),   S <- e_63 S + (w K)^T U.
 // All products are the split products of split_mma.cuh, in the systems too (what the rows before a block of 16 take off it; the triangle of the 16
-// is float32 multiply-adds, a column a thread); lengths, and products of factors with scores, are formed in float64 and rounded once.  Against 64
-// bits, 24 runs, the outputs' error is 0.85 and the states' 0.94 of token by token in the mean (float32 multiply-adds in chunks: 0.91 and 0.94).
-// 16 heads of 128 x 128 on 4,097 tokens, us: token by token 1,900, chunks of float32 multiply-adds 485, now 379, of which the first kernel takes 150
+// is float32 multiply-adds, a column a thread); lengths, and products of factors with scores, are formed in float64 and rounded once; a chunk's tail is
+// added to the state as in the scan.  Error against 64 bits by decay, relative to token by token (and of float32 multiply-adds in chunks), 22 heads of 128 x 128: outputs
+// 0.999 a token 1.00 (1.00), 0.9 0.79 (0.77), 0.5 0.61 (0.69), 0.1 0.62 (0.66); states 1.01 (1.01), 1.03 (1.01), 0.92 (0.92), 0.87 (0.87).
+// 16 heads of 128 x 128 on 4,097 tokens, us: token by token 1,900, chunks of float32 multiply-adds 485, now 385 (392 where every chunk has a tail), of which the first kernel takes 150
 // (issue around splitting its operands, at two CTAs an SM; with scores and systems of multiply-adds 172) and the walk 246 (three barriers a
 // chunk and the latency of what lies between them; half of a chunk's time is its products).
 constexpr int CD_THREADS = 256;
@@ -867,12 +921,13 @@ struct DeltaChunks {
     float* state;               // [slots][heads][V][D]
     float* out;                 // [tokens][heads * V]
     unsigned* status;           // or null
-    unsigned char* scratch;     // [slots][qk_heads]: q as an operand of the walk; [slots][heads]: W, w K and the scores P as operands, the record, U0 [64][V]
+    unsigned char* scratch;     // [slots][qk_heads]: q as an operand of the walk; [slots][heads]: W, w K and the scores P as operands, w K's rows of the tail, the record, U0 [64][V]
     const int* cu;
     const int* slots;
     int sequences, max_slots, heads, qk_heads, D, V, vec;
     static __host__ __device__ constexpr size_t matrix_bytes(int padded) { return (size_t)padded / 16 * 4 * SPLIT_BLOCK_BYTES; }
-    static __host__ __device__ constexpr size_t operand_bytes(int padded) { return 2 * matrix_bytes(padded) + CK_MBLOCKS * SPLIT_BLOCK_BYTES + CK_RECORD * sizeof(float); }
+    static __host__ __device__ constexpr size_t record_at(int padded) { return 2 * matrix_bytes(padded) + CK_MBLOCKS * SPLIT_BLOCK_BYTES + CK_TAIL_ROWS * padded * sizeof(float); }
+    static __host__ __device__ constexpr size_t operand_bytes(int padded) { return record_at(padded) + CK_RECORD * sizeof(float); }
     __host__ __device__ size_t head_bytes(int padded) const { return operand_bytes(padded) + (size_t)CK_TOKENS * V * sizeof(float); }
     template <int NP> __device__ uint4* group_scratch(int slot, int g) const { return reinterpret_cast<uint4*>(scratch + ((size_t)slot * qk_heads + g) * matrix_bytes(NP)); }
     template <int NP> __device__ uint4* head_scratch(int slot, int h) const {
@@ -903,7 +958,8 @@ delta_chunks_prepare_kernel(const DeltaChunks a) {
     double* nk = nq + CK_TOKENS;
     float* beta = reinterpret_cast<float*>(nk + CK_TOKENS);
     float* scalars = beta + CK_TOKENS;                          // [2][64]; then the rows' factors of W's right-hand side
-    __shared__ int bad;                                         // the first token with a number that is not finite
+    __shared__ int bad, tail;                                   // the first token with a number that is not finite, the tail's first
+    __shared__ float tail_w[CK_TAIL_ROWS];
     const int slot = blockIdx.x, h = blockIdx.y, D = a.D, V = a.V;
     int lo = 0, hi = a.sequences;
     while (hi - lo > 1) {
@@ -919,7 +975,7 @@ delta_chunks_prepare_kernel(const DeltaChunks a) {
         for (int e = threadIdx.x; e < 2 * CK_TOKENS * LD; e += CD_THREADS) ck_shared[e] = 0.0f;
     __syncthreads();
     uint4* head = a.head_scratch<NP>(slot, h);
-    float* record = reinterpret_cast<float*>(head) + (2 * DeltaChunks::matrix_bytes(NP) + CK_MBLOCKS * SPLIT_BLOCK_BYTES) / 4;
+    float* record = reinterpret_cast<float*>(head) + DeltaChunks::record_at(NP) / 4;
     const float* rows = a.qkv + (size_t)(first + c0) * a.stride;
     ck_stage<NP, CD_THREADS>(qs, LD, rows + (size_t)g * D, a.stride, count, D, a.vec);
     ck_stage<NP, CD_THREADS>(ks, LD, rows + (size_t)(a.qk_heads + g) * D, a.stride, count, D, a.vec);
@@ -981,6 +1037,8 @@ delta_chunks_prepare_kernel(const DeltaChunks a) {
             record[CK_R_DT + i] = write;
         }
         ck_factors(f, decay[0], decay[1], 1.0f, 1.0f, lane, scalars, scalars + CK_TOKENS);
+        const int first_of_tail = ck_tail(scalars, count, lane);
+        if (lane == 0) record[CK_R_TAIL] = __int_as_float(tail = first_of_tail);
     }
     {
         const int q = warp >> 1;
@@ -1051,10 +1109,16 @@ delta_chunks_prepare_kernel(const DeltaChunks a) {
         const float start = (float)((double)beta[i] * (double)f[CK_E + i] * nk[i]), w = (float)((double)f[CK_W + i] * nk[i]);
         record[CK_R_E + i] = (float)((double)f[CK_E + i] * nq[i]);
         scalars[i] = ck_usable(start) ? start : 0.0f;
-        scalars[CK_TOKENS + i] = ck_usable(w) ? w : 0.0f;       // (not so: no column's state comes from these products)
+        scalars[CK_TOKENS + i] = ck_usable(w) && i < tail ? w : 0.0f;       // (not usable: no column's state comes from these products)
+        if (i >= tail && i < tail + CK_TAIL_ROWS) tail_w[i - tail] = w;
         if (i == 0) record[CK_R_ALL] = f[CK_ALL];
     }
     __syncthreads();
+    if (tail < CK_TOKENS)
+        for (int e = threadIdx.x; e < CK_TAIL_ROWS * NP; e += CD_THREADS) {     // (zeros behind the last token)
+            const int r = e / NP, c = e % NP;
+            (record - CK_TAIL_ROWS * NP)[r * NP + ck_tail_place(c)] = tail_w[r] * ks[(tail + r) * LD + c];
+        }
     // the operands that do not need the systems: w K (k = tokens, columns = state rows), and by the first head of a group q (k = state rows, columns = tokens)
     constexpr int KS = NP / 16, BLOCK = SPLIT_BLOCK_BYTES / 16;
     auto by_token = [&](const float* m, int item, float (&v)[2][4]) {           // k = the matrix' columns, columns = its rows
@@ -1251,9 +1315,10 @@ template <int NP, int PB, int NS>
 struct CdWalk {
     static constexpr int THREADS = 32 * PB * NS, TP = 16 * PB, KS = NP / 16, KL = KS / NS, EACH = 8 / NS;
     static constexpr int MATRIX = KS * 4 * SPLIT_BLOCK_BYTES;
-    static constexpr int W = 0, Q = W + MATRIX, K = Q + MATRIX, M = K + MATRIX, R = M + CK_MBLOCKS * SPLIT_BLOCK_BYTES, PARTS = R + 2 * CK_RECORD * 4;
-    static constexpr int U = PARTS + 2 * PB * (NS - 1) * 8 * 512, BAD = U + PB * 4 * SPLIT_BLOCK_BYTES, BAR = BAD + TP * 4, BYTES = BAR + 16;
-    static constexpr int REST_BYTES = CK_MBLOCKS * SPLIT_BLOCK_BYTES + MATRIX;
+    static constexpr int W = 0, Q = W + MATRIX, K = Q + MATRIX, M = K + MATRIX, TAIL = M + CK_MBLOCKS * SPLIT_BLOCK_BYTES, R = TAIL + CK_TAIL_ROWS * NP * 4, PARTS = R + 2 * CK_NEAR * 4;
+    static constexpr int U = PARTS + 2 * PB * (NS - 1) * 8 * 512, BAD = U + PB * 4 * SPLIT_BLOCK_BYTES, BAR = BAD + TP * 4, TAIL_U = BAR + 16;
+    static constexpr int BYTES = TAIL_U + CK_TAIL_ROWS * TP * 4, REST_BYTES = R - K;
+    static_assert(BYTES <= 227 * 1024, "a CTA's shared memory");
 };
 
 template <int NP, int PB, int NS>
@@ -1279,6 +1344,8 @@ delta_chunks_kernel(const DeltaChunks a) {
     float4* parts_w = reinterpret_cast<float4*>(ck_bytes + L::PARTS) + pb * (NS - 1) * 8 * 32 + lane;          // [another warp][tile of 8 tokens][lane]
     float4* parts_q = parts_w + PB * (NS - 1) * 8 * 32;
     int* bad_from = reinterpret_cast<int*>(ck_bytes + L::BAD);
+    const float* tail = reinterpret_cast<const float*>(ck_bytes + L::TAIL) + ns * (NP / NS) + 4 * (lane & 3);
+    float* tail_u = reinterpret_cast<float*>(ck_bytes + L::TAIL_U) + pb * 16 + 2 * gq;                                                             // [token][columns c and c + 8 side by side]
     const uint32_t bar = tc::smem_u32(ck_bytes + L::BAR), bar_rest = bar + 8;
     if (threadIdx.x == 0) {
         tc::mbar_init(bar, 1);
@@ -1288,21 +1355,19 @@ delta_chunks_kernel(const DeltaChunks a) {
     __syncthreads();
     bool in_time = true;                                        // no wait has run out
 
-    auto records = [&](int chunk) { return reinterpret_cast<float*>(ck_bytes + L::R) + (chunk & 1) * CK_RECORD; };
+    auto records = [&](int chunk) { return reinterpret_cast<float*>(ck_bytes + L::R) + (chunk & 1) * CK_NEAR; };
     auto fetch_first = [&](int chunk) {                         // what meets the state, and the record
         if (threadIdx.x || chunk >= chunks) return;
         const uint4* head = a.head_scratch<NP>(slot0 + chunk, h);
-        tc::mbar_expect_tx(bar, 2 * L::MATRIX + CK_RECORD * 4);
+        tc::mbar_expect_tx(bar, 2 * L::MATRIX + CK_NEAR * 4);
         ck_fetch(ck_bytes + L::W, head, L::MATRIX, bar);
         ck_fetch(ck_bytes + L::Q, a.group_scratch<NP>(slot0 + chunk, g), L::MATRIX, bar);
-        ck_fetch(records(chunk), head + (2 * L::MATRIX + CK_MBLOCKS * SPLIT_BLOCK_BYTES) / 16, CK_RECORD * 4, bar);
+        ck_fetch(records(chunk), head + DeltaChunks::record_at(NP) / 16, CK_NEAR * 4, bar);
     };
-    auto fetch_rest = [&](int chunk) {                          // K and the scores
+    auto fetch_rest = [&](int chunk) {                          // K, the scores and the tail
         if (threadIdx.x || chunk >= chunks) return;
-        const uint4* head = a.head_scratch<NP>(slot0 + chunk, h);
         tc::mbar_expect_tx(bar_rest, L::REST_BYTES);
-        ck_fetch(ck_bytes + L::K, head + L::MATRIX / 16, L::MATRIX, bar_rest);
-        ck_fetch(ck_bytes + L::M, head + 2 * L::MATRIX / 16, CK_MBLOCKS * SPLIT_BLOCK_BYTES, bar_rest);
+        ck_fetch(ck_bytes + L::K, a.head_scratch<NP>(slot0 + chunk, h) + L::MATRIX / 16, L::REST_BYTES, bar_rest);
     };
     fetch_first(0);
     fetch_rest(0);
@@ -1351,6 +1416,7 @@ delta_chunks_kernel(const DeltaChunks a) {
                 u[i][e] = pb * 16 + gq + p < width ? __ldg(from + (size_t)token * V + p) : 0.0f;
             }
         in_time = in_time && tc::mbar_wait(bar, chunk & 1);
+        const int count = min(CK_TOKENS, left), tail0 = __float_as_int(F[CK_R_TAIL]);
         for (int p = threadIdx.x; p < TP; p += THREADS) bad_from[p] = __float_as_int(F[CK_R_BAD]);
         float qs[EACH][4], ws[EACH][4];                         // this warp's tiles
         {
@@ -1407,6 +1473,11 @@ delta_chunks_kernel(const DeltaChunks a) {
                     u[i][e] = 0.0f;
                 }
             }
+            if (8 * tile + 8 > tail0) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (const int r = 8 * tile + t2 + (e & 1) - tail0; r >= 0 && r < CK_TAIL_ROWS) tail_u[r * TP + (e >> 1)] = u[i][e];
+            }
             uint32_t part[3][2];
             split_pair(u[i][0], u[i][1], part[0][0], part[1][0], part[2][0]);
             split_pair(u[i][2], u[i][3], part[0][1], part[1][1], part[2][1]);
@@ -1419,9 +1490,9 @@ delta_chunks_kernel(const DeltaChunks a) {
         if (some_bad) {                                         // as in the scan: columns from their first such token on go token by token
             store_state();
             __syncthreads();
-            const int count = min(CK_TOKENS, left);
+            const float* record = reinterpret_cast<const float*>(a.head_scratch<NP>(slot0 + chunk, h) + DeltaChunks::record_at(NP) / 16);
             for (int p = warp; p < width; p += THREADS / 32)
-                if (bad_from[p] < count) ck_delta_column(a, F, first + chunk * CK_TOKENS, count, h, g, p0 + p, S + (size_t)p * D, bad_from[p]);
+                if (bad_from[p] < count) ck_delta_column(a, record, first + chunk * CK_TOKENS, count, h, g, p0 + p, S + (size_t)p * D, bad_from[p]);
             __syncthreads();
         }
         in_time = in_time && tc::mbar_wait(bar_rest, chunk & 1);
@@ -1445,6 +1516,13 @@ delta_chunks_kernel(const DeltaChunks a) {
                     float& v = s[2 * k + i][e];
                     v = long_memory ? fmaf(all, v, sum[i][e] + rest[i][e]) : fmaf(all, v, rest[i][e]) + sum[i][e];
                 }
+        }
+        if (tail0 < CK_TOKENS) {
+#pragma unroll
+            for (int i = 0; i < CK_TAIL_ROWS; ++i) {
+                const float2 u = *reinterpret_cast<const float2*>(tail_u + i * TP);
+                ck_add_row(s, u.x, u.y, tail + i * NP);
+            }
         }
         // outputs: Q S times its factor and the scores times U, for this warp's tiles
         float* out = a.out + (size_t)(first + chunk * CK_TOKENS) * a.heads * V + (size_t)h * V + p0 + pb * 16 + gq;
@@ -1478,7 +1556,6 @@ delta_chunks_kernel(const DeltaChunks a) {
             }
         }
         if (some_bad) {
-            const int count = min(CK_TOKENS, left);
             if (bad_from[pb * 16 + gq] < count) load_state(0);
             if (bad_from[pb * 16 + gq + 8] < count) load_state(1);
         }

@@ -934,7 +934,8 @@ def mamba2_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_col: int, dt_bias: tor
 
 CHUNK_TOKENS = 64           # tokens of a chunk of the recurrences with a decay per head (CK_TOKENS in csrc/recurrent_chunks.cu)
 CHUNK_MAX_ROWS = 128        # state rows (key size) the chunk kernels take
-_CHUNK_HEAD_FLOATS = 10 * 384 + 260         # scores times factors as an operand in three bfloat16 parts, and a record
+_CHUNK_TAIL = 8             # rows of a chunk that are handed on as they are too (CK_TAIL_ROWS)
+_CHUNK_HEAD_FLOATS = 10 * 384 + 268         # scores times factors as an operand in three bfloat16 parts, and a record
 
 
 def chunk_slots(n_tokens: int, sequences: int) -> int:
@@ -946,7 +947,7 @@ def scan_chunks_scratch(n_tokens: int, sequences: int, heads: int, groups: int, 
     """Shape of the float32 scratch that :func:`scan_chunks` takes for states of ``state_size`` rows: B and C of every chunk and group and the
     scores of every chunk and head in three bfloat16 parts, factors for every chunk and head."""
     padded = 64 if state_size <= 64 else 128
-    return (chunk_slots(n_tokens, sequences) * (groups * 2 * CHUNK_TOKENS * padded * 3 // 2 + heads * _CHUNK_HEAD_FLOATS),)
+    return (chunk_slots(n_tokens, sequences) * (groups * (2 * CHUNK_TOKENS * padded * 3 // 2 + _CHUNK_TAIL * padded) + heads * _CHUNK_HEAD_FLOATS),)
 
 
 def scan_chunks(rows: torch.Tensor, x_col: int, b_col: int, c_col: int, state: torch.Tensor, y: torch.Tensor, cu: torch.Tensor, slots: torch.Tensor,
@@ -987,8 +988,9 @@ def scan_chunks(rows: torch.Tensor, x_col: int, b_col: int, c_col: int, state: t
 def delta_chunks_scratch(n_tokens: int, sequences: int, heads: int, key_dim: int, value_dim: int, qk_heads: int | None = None) -> tuple[int]:
     """Shape of the float32 scratch that :func:`delta_chunks` takes: of every chunk and query/key head (``qk_heads`` None: as many as heads) q, of every
     chunk and head W, the keys and the scores in three bfloat16 parts, factors and U0."""
-    matrix = CHUNK_TOKENS * (64 if key_dim <= 64 else 128) * 3 // 2
-    return (chunk_slots(n_tokens, sequences) * ((heads if qk_heads is None else qk_heads) * matrix + heads * (2 * matrix + _CHUNK_HEAD_FLOATS + CHUNK_TOKENS * value_dim)),)
+    padded = 64 if key_dim <= 64 else 128
+    matrix, q_heads = CHUNK_TOKENS * padded * 3 // 2, heads if qk_heads is None else qk_heads
+    return (chunk_slots(n_tokens, sequences) * (q_heads * matrix + heads * (2 * matrix + _CHUNK_TAIL * padded + _CHUNK_HEAD_FLOATS + CHUNK_TOKENS * value_dim)),)
 
 
 def delta_chunks(qkv: torch.Tensor, proj: torch.Tensor, b_col: int, a_col: int, dt_bias: torch.Tensor, a_log: torch.Tensor, state: torch.Tensor,
