@@ -47,3 +47,20 @@ def test_shared_memory_is_asked_for_on_every_launch(path):
     for ask in re.finditer(r"cudaFuncSetAttribute|tt_allow_shared\(", text):
         function = text[text.rfind("\n}", 0, ask.start()) + 2:ask.start()]
         assert not re.search(r"\bstatic\s+(?:bool|int|size_t)\s+\w+\s*=", function), function[-400:]
+
+
+def test_no_copy_is_left_on_its_way_when_a_wait_runs_out():
+    """A CTA whose wait ran out ends, and its shared memory is the next one's: it fetches nothing more and waits for what it has fetched."""
+    text = code(CSRC / "recurrent_chunks.cu")
+    for name in ("scan_chunks_kernel", "delta_chunks_kernel"):
+        kernel = text[text.index(f"\n{name}(const"):]
+        kernel = kernel[:kernel.index("\n}\n")]
+        for expect in re.finditer(r"mbar_expect_tx\(", kernel):
+            condition = kernel[:expect.start()]
+            condition = condition[condition.rindex("if (threadIdx.x"):]
+            assert "in_time" in condition, condition
+        # every wait that may run out sets the flag, and every barrier is waited for again at the end
+        waits = set(re.findall(r"if \(in_time && !tc::mbar_wait\((\w+), chunk & 1\)\) \{ in_time = false; late = ", kernel))
+        end = kernel[kernel.rindex("if (!in_time && threadIdx.x == 0)"):]
+        assert len(waits) == 2 and all(f"tc::mbar_wait({bar}, " in end for bar in waits)
+        assert kernel[:-len(end)].count("tc::mbar_wait(") == len(re.findall(r"in_time && !?tc::mbar_wait\(", kernel))

@@ -152,7 +152,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
                         "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
                         ::"r"(to + p * half * BK * 2), "l"(&map_x), "r"((kb0 + i) * BK), "r"(token0 + rank * half), "r"(p), "r"(bar & PEER_MASK) : "memory");
             }
-            // every copy has landed once the products that read it are done, for which the workers wait
+            // every copy has landed once the products that read it are done, for which the workers wait; where a wait ran out, theirs or this one, the
+            // copies before it were asked for a limit ago
         }
         if (warp == WARPS + 1 && lane == 0 && rank == 0) {
             const uint32_t idesc = instr_desc(2 * BM, args.tokens);

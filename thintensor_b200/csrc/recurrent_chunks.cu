@@ -487,7 +487,7 @@ struct CkWalk {
     static constexpr int C = 0, B = C + KS * 4 * SPLIT_BLOCK_BYTES, TAIL = B + KS * 4 * SPLIT_BLOCK_BYTES, M = TAIL + CK_TAIL_ROWS * NP * 4, X = M + CK_MBLOCKS * SPLIT_BLOCK_BYTES;
     static constexpr int X_BYTES = CK_TOKENS * LDX * 4, R = X + 2 * X_BYTES, PARTS = R + 2 * CK_NEAR * 4;
     static constexpr int W = PARTS + (NS > 1 ? PB * (NS - 1) * 8 * 512 : 0), BAD = W + (NS > 1 ? PB * 4 * SPLIT_BLOCK_BYTES : 0), BAR = BAD + TP * 4, BYTES = BAR + 16;
-    static_assert(BYTES <= 227 * 1024, "a CTA's shared memory");
+    static_assert(BYTES + 16 <= 227 * 1024, "a CTA's shared memory");
     static constexpr int FIRST_BYTES = CK_NEAR * 4 + CK_MBLOCKS * SPLIT_BLOCK_BYTES + KS * 4 * SPLIT_BLOCK_BYTES, B_BYTES = KS * 4 * SPLIT_BLOCK_BYTES;
     // Which 16 tokens' x (j) a warp multiplies with the scores of which outputs (q >= j): a block each, about as many for the warps of
     // every scheduler
@@ -565,6 +565,7 @@ scan_chunks_kernel(const ScanChunks a) {
     using L = CkWalk<NP, PB, NS>;
     constexpr int THREADS = L::THREADS, TP = L::TP, LDX = L::LDX, KL = L::KL, PAIR = KL > 1 ? 2 : 1;
     extern __shared__ __align__(16) unsigned char ck_bytes[];
+    __shared__ int late;                                        // twice the chunk whose wait ran out, and one for its second wait
     tt_pdl_launch_dependents();
     tt_pdl_wait();
     const int h = blockIdx.x, b = blockIdx.y, p0 = blockIdx.z * TP;
@@ -591,7 +592,7 @@ scan_chunks_kernel(const ScanChunks a) {
         tc::fence_barrier_init();
     }
     __syncthreads();
-    bool in_time = true;                                        // no wait has run out
+    bool in_time = true;                                        // no wait has run out; else nothing more is fetched
 
     auto xs = [&](int chunk) { return reinterpret_cast<float*>(ck_bytes + L::X + (chunk & 1) * L::X_BYTES); };
     auto records = [&](int chunk) { return reinterpret_cast<float*>(ck_bytes + L::R) + (chunk & 1) * CK_NEAR; };
@@ -601,7 +602,7 @@ scan_chunks_kernel(const ScanChunks a) {
         const uint4* head = a.head_scratch<NP>(slot0 + chunk, h);
         ck_stage<TP, THREADS>(xs(chunk), LDX, a.x + (size_t)(first + c0) * a.stride + (size_t)h * P + p0, a.stride, min(CK_TOKENS, n - c0), width, vec_x);
         ck_commit();
-        if (threadIdx.x == 0) {
+        if (threadIdx.x == 0 && in_time) {
             tc::mbar_expect_tx(bar, L::FIRST_BYTES);
             ck_fetch(ck_bytes + L::C, a.group_scratch<NP>(slot0 + chunk, g), L::B_BYTES, bar);
             ck_fetch(ck_bytes + L::M, head, CK_MBLOCKS * SPLIT_BLOCK_BYTES, bar);
@@ -661,7 +662,9 @@ scan_chunks_kernel(const ScanChunks a) {
         const float* F = records(chunk);
         const int left = n - chunk * CK_TOKENS;
         ck_wait<0>();
-        in_time = in_time && tc::mbar_wait(bar, chunk & 1);
+        // (the same in two forms: with the branch the compiler's schedule of 128 columns is 3 % slower, without it that of the others 1 to 4 %)
+        if constexpr (NS == 1) in_time = in_time && tc::mbar_wait(bar, chunk & 1);
+        else if (in_time && !tc::mbar_wait(bar, chunk & 1)) { in_time = false; late = 2 * chunk; }
         bool odd = ck_staged_odd<TP, THREADS>(X, LDX, width, vec_x);
 #pragma unroll
         for (int k = 0; k < 2 * KL; ++k)
@@ -671,7 +674,7 @@ scan_chunks_kernel(const ScanChunks a) {
         bool some_bad = __syncthreads_or(odd);
         some_bad |= __float_as_int(F[CK_R_BAD]) < CK_TOKENS;
         const int count = min(CK_TOKENS, left), tail0 = __float_as_int(F[CK_R_TAIL]);
-        if (threadIdx.x == 0) {
+        if (threadIdx.x == 0 && in_time) {
             const uint32_t bytes = L::B_BYTES + (tail0 < CK_TOKENS ? CK_TAIL_ROWS * NP * 4 : 0);
             tc::mbar_expect_tx(bar_b, bytes);
             ck_fetch(ck_bytes + L::B, a.group_scratch<NP>(slot0 + chunk, g) + L::KS * 4 * (SPLIT_BLOCK_BYTES / 16), bytes, bar_b);
@@ -793,7 +796,8 @@ scan_chunks_kernel(const ScanChunks a) {
         __syncthreads();                                        // the weighted rows and the parts are there; C and the scores are read
         fetch_first(chunk + 1);
         // S^T <- e_63 S^T + (w x)^T B; the larger part is added last: one rounding at the size of the sum
-        in_time = in_time && tc::mbar_wait(bar_b, chunk & 1);
+        if constexpr (NS == 1) in_time = in_time && tc::mbar_wait(bar_b, chunk & 1);
+        else if (in_time && !tc::mbar_wait(bar_b, chunk & 1)) { in_time = false; late = 2 * chunk + 1; }
         const float all = F[CK_R_ALL];
         const bool long_memory = fabsf(all) > 0.25f;
         SplitA wa[NS > 1 ? 1 : 4];
@@ -848,6 +852,14 @@ scan_chunks_kernel(const ScanChunks a) {
         }
     }
     if (!in_time && a.status) atomicOr(a.status, TT_STATUS_WAIT_EXPIRED);
+    if (!in_time && threadIdx.x == 0) {                         // its copies that may still be on their way to this shared memory
+        if (NS == 1)
+            for (int phase = 0; phase < 2; ++phase) { tc::mbar_wait(bar, phase); tc::mbar_wait(bar_b, phase); }
+        else {
+            if (late & 1) tc::mbar_wait(bar_b, (late >> 1) & 1);
+            if (const int chunk = (late + 1) >> 1; chunk < chunks) tc::mbar_wait(bar, chunk & 1);
+        }
+    }
     store_state();
 }
 
@@ -1318,7 +1330,7 @@ struct CdWalk {
     static constexpr int W = 0, Q = W + MATRIX, K = Q + MATRIX, M = K + MATRIX, TAIL = M + CK_MBLOCKS * SPLIT_BLOCK_BYTES, R = TAIL + CK_TAIL_ROWS * NP * 4, PARTS = R + 2 * CK_NEAR * 4;
     static constexpr int U = PARTS + 2 * PB * (NS - 1) * 8 * 512, BAD = U + PB * 4 * SPLIT_BLOCK_BYTES, BAR = BAD + TP * 4, TAIL_U = BAR + 16;
     static constexpr int BYTES = TAIL_U + CK_TAIL_ROWS * TP * 4, REST_BYTES = R - K;
-    static_assert(BYTES <= 227 * 1024, "a CTA's shared memory");
+    static_assert(BYTES + 16 <= 227 * 1024, "a CTA's shared memory");
 };
 
 template <int NP, int PB, int NS>
@@ -1327,6 +1339,7 @@ delta_chunks_kernel(const DeltaChunks a) {
     using L = CdWalk<NP, PB, NS>;
     constexpr int THREADS = L::THREADS, TP = L::TP, KL = L::KL, EACH = L::EACH, BLOCK = SPLIT_BLOCK_BYTES / 16, PAIR = KL > 1 ? 2 : 1;
     extern __shared__ __align__(16) unsigned char ck_bytes[];
+    __shared__ int late;                                        // twice the chunk whose wait ran out, and one for its second wait
     tt_pdl_launch_dependents();
     tt_pdl_wait();
     const int h = blockIdx.x, b = blockIdx.y, p0 = blockIdx.z * TP;
@@ -1353,11 +1366,11 @@ delta_chunks_kernel(const DeltaChunks a) {
         tc::fence_barrier_init();
     }
     __syncthreads();
-    bool in_time = true;                                        // no wait has run out
+    bool in_time = true;                                        // no wait has run out; else nothing more is fetched
 
     auto records = [&](int chunk) { return reinterpret_cast<float*>(ck_bytes + L::R) + (chunk & 1) * CK_NEAR; };
     auto fetch_first = [&](int chunk) {                         // what meets the state, and the record
-        if (threadIdx.x || chunk >= chunks) return;
+        if (threadIdx.x || chunk >= chunks || !in_time) return;
         const uint4* head = a.head_scratch<NP>(slot0 + chunk, h);
         tc::mbar_expect_tx(bar, 2 * L::MATRIX + CK_NEAR * 4);
         ck_fetch(ck_bytes + L::W, head, L::MATRIX, bar);
@@ -1365,7 +1378,7 @@ delta_chunks_kernel(const DeltaChunks a) {
         ck_fetch(records(chunk), head + DeltaChunks::record_at(NP) / 16, CK_NEAR * 4, bar);
     };
     auto fetch_rest = [&](int chunk) {                          // K, the scores and the tail
-        if (threadIdx.x || chunk >= chunks) return;
+        if (threadIdx.x || chunk >= chunks || !in_time) return;
         tc::mbar_expect_tx(bar_rest, L::REST_BYTES);
         ck_fetch(ck_bytes + L::K, a.head_scratch<NP>(slot0 + chunk, h) + L::MATRIX / 16, L::REST_BYTES, bar_rest);
     };
@@ -1415,7 +1428,7 @@ delta_chunks_kernel(const DeltaChunks a) {
                 const int token = 8 * (ns * EACH + i) + t2 + (e & 1), p = 8 * (e >> 1);
                 u[i][e] = pb * 16 + gq + p < width ? __ldg(from + (size_t)token * V + p) : 0.0f;
             }
-        in_time = in_time && tc::mbar_wait(bar, chunk & 1);
+        if (in_time && !tc::mbar_wait(bar, chunk & 1)) { in_time = false; late = 2 * chunk; }
         const int count = min(CK_TOKENS, left), tail0 = __float_as_int(F[CK_R_TAIL]);
         for (int p = threadIdx.x; p < TP; p += THREADS) bad_from[p] = __float_as_int(F[CK_R_BAD]);
         float qs[EACH][4], ws[EACH][4];                         // this warp's tiles
@@ -1495,7 +1508,7 @@ delta_chunks_kernel(const DeltaChunks a) {
                 if (bad_from[p] < count) ck_delta_column(a, record, first + chunk * CK_TOKENS, count, h, g, p0 + p, S + (size_t)p * D, bad_from[p]);
             __syncthreads();
         }
-        in_time = in_time && tc::mbar_wait(bar_rest, chunk & 1);
+        if (in_time && !tc::mbar_wait(bar_rest, chunk & 1)) { in_time = false; late = 2 * chunk + 1; }
         // S^T <- e_63 S^T + U^T (w K); the larger part is added last
         const float all = F[CK_R_ALL];
         const bool long_memory = fabsf(all) > 0.25f;
@@ -1563,6 +1576,10 @@ delta_chunks_kernel(const DeltaChunks a) {
         fetch_rest(chunk + 1);
     }
     if (!in_time && a.status) atomicOr(a.status, TT_STATUS_WAIT_EXPIRED);
+    if (!in_time && threadIdx.x == 0) {                         // its copies that may still be on their way to this shared memory
+        tc::mbar_wait(bar_rest, (late >> 1) & 1);
+        if (const int chunk = (late + 1) >> 1; chunk < chunks) tc::mbar_wait(bar, chunk & 1);
+    }
     store_state();
 }
 
