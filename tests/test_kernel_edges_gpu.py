@@ -919,6 +919,26 @@ def test_experts_of_sorted_tokens(tokens, top, experts, hidden, inter):
     torch.testing.assert_close(out.double(), want, rtol=1e-5, atol=1e-5)
 
 
+def test_sorted_tokens_without_choices():
+    """Nobody chose: no tiles, and the products' look at the first tile's expert finds one; the sums stay as they are."""
+    from thintensor_b200.kernels import api
+
+    tokens, top, experts, hidden, inter = 300, 2, 3, 128, 128
+    x, chosen = randn(tokens, hidden, seed=145).bfloat16(), torch.full((tokens, top), -1, dtype=torch.int32, device=DEV)
+    tiles = api.expert_tiles(tokens, top, experts)
+    xs, place = torch.zeros(256 * tiles, hidden, dtype=torch.bfloat16, device=DEV), torch.full((tokens, top), 99, dtype=torch.int32, device=DEV)
+    table, status = torch.full((1 + experts + tiles,), 99, dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    api.sort_tokens(x, chosen, experts, xs, place, table)
+    assert table[:2 + experts].tolist() == [0] * (2 + experts) and bool((place == -1).all())
+    act, y = torch.zeros(256 * tiles, inter, dtype=torch.bfloat16, device=DEV), torch.zeros(256 * tiles, hidden, device=DEV)
+    w, down = randn(2 * experts * inter, hidden, seed=146).bfloat16(), randn(hidden, experts * inter, seed=147).bfloat16()
+    api.gemm_tcgen05_experts(xs, w, act, status, hidden, inter, experts, table, "silu", experts * inter)
+    api.gemm_tcgen05_experts(act, down, y, status, inter, hidden, experts, table)
+    out = randn(tokens, hidden, seed=148)
+    api.combine_experts(y, place, torch.rand(tokens, top, device=DEV), out)
+    assert torch.equal(out, randn(tokens, hidden, seed=148)) and int(status) == 0
+
+
 @pytest.mark.parametrize("shared,residual", [(0, True), (0, False), (384, True), (384, False)])
 @pytest.mark.parametrize("tokens", [640, 2100])
 def test_mixture_of_sorted_tokens_is_the_mixture_of_columns(shared, residual, tokens, monkeypatch):

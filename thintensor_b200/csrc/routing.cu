@@ -563,7 +563,10 @@ gather_tokens_kernel(const __nv_bfloat16* __restrict__ x, int hidden, const int*
         for (int e = warp; e < experts; e += SORT_ROWS) {
             const int first = sort_first_row(counts, e, lane) / SORT_TILE, n = (__ldg(counts + e) + SORT_TILE - 1) / SORT_TILE;
             for (int i = lane; i < n; i += 32) tile_expert[first + i] = e;
-            if (e == experts - 1 && lane == 0) *tile_count = first + n;
+            if (e == experts - 1 && lane == 0) {
+                *tile_count = first + n;
+                if (first + n == 0) tile_expert[0] = 0;         // nobody has a choice: the products still look at their first tile's expert
+            }
         }
         return;
     }
