@@ -939,6 +939,33 @@ def test_sorted_tokens_without_choices():
     assert torch.equal(out, randn(tokens, hidden, seed=148)) and int(status) == 0
 
 
+@pytest.mark.parametrize("which", range(4))
+def test_sorted_tokens_refuse_tensors_elsewhere(which):
+    from thintensor_b200.kernels import api
+
+    tokens, top, experts, hidden = 40, 2, 3, 64
+    tiles = api.expert_tiles(tokens, top, experts)
+    operands = [randn(tokens, hidden, seed=149).bfloat16(), torch.zeros(tokens, top, dtype=torch.int32, device=DEV), torch.zeros(256 * tiles, hidden, dtype=torch.bfloat16, device=DEV),
+                torch.zeros(tokens, top, dtype=torch.int32, device=DEV), torch.zeros(1 + experts + tiles, dtype=torch.int32, device=DEV)]
+    at = (0, 1, 2, 4)[which]
+    operands[at] = operands[at].cpu()
+    x, chosen, xs, place, table = operands
+    with pytest.raises(api.KernelError, match="CUDA tensors only"):
+        api.sort_tokens(x, chosen, experts, xs, place, table)
+
+
+@pytest.mark.parametrize("which", ["rows", "state", "y", "scratch", "decays"])
+def test_recurrences_in_chunks_refuse_tensors_elsewhere(which):
+    from thintensor_b200.kernels import api
+
+    heads, P, N, tokens = 2, 16, 32, 70
+    t = {"rows": randn(tokens, heads * (P + 2 * N), seed=150), "state": torch.zeros(1, heads, P, N, device=DEV), "y": torch.zeros(tokens, heads * P, device=DEV),
+         "scratch": torch.zeros(api.scan_chunks_scratch(tokens, 1, heads, heads), device=DEV), "decays": torch.full((heads,), 0.9, device=DEV)}
+    t[which] = t[which].cpu()
+    with pytest.raises(api.KernelError, match="CUDA tensors only"):
+        api.scan_chunks(t["rows"], 0, heads * P, heads * (P + N), t["state"], t["y"], i32([0, tokens]), i32([0]), 1, heads, P, N, heads, t["scratch"], fixed_decay=t["decays"])
+
+
 @pytest.mark.parametrize("shared,residual", [(0, True), (0, False), (384, True), (384, False)])
 @pytest.mark.parametrize("tokens", [640, 2100])
 def test_mixture_of_sorted_tokens_is_the_mixture_of_columns(shared, residual, tokens, monkeypatch):

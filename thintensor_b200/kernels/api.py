@@ -980,8 +980,8 @@ def scan_chunks(rows: torch.Tensor, x_col: int, b_col: int, c_col: int, state: t
             if t.numel() != heads:
                 raise KernelError("scan_chunks: decays, biases and skips have a number per head")
     fn = _fn("recurrent_chunks", "tt_scan_chunks", "piiiipiliipppppppppiiiiiiipp")
-    _check(fn(rows.data_ptr(), width, x_col, b_col, c_col, p, splits, stride, cols, dt_col, *(None if t is None else t.data_ptr() for t in vectors),
-              None if fixed_decay is None else fixed_decay.data_ptr(), state.data_ptr(), y.data_ptr(), scratch.data_ptr(), _ptr(cu), _ptr(slots), sequences,
+    _check(fn(_ptr(rows), width, x_col, b_col, c_col, p, splits, stride, cols, dt_col, *(_ptr(t) for t in vectors),
+              _ptr(fixed_decay), _ptr(state), _ptr(y), _ptr(scratch), _ptr(cu), _ptr(slots), sequences,
               chunk_slots(tokens, sequences), heads, groups, head_dim, state_size, sm_count(rows.device), _ptr(status), _stream()), "scan_chunks", 2)
 
 
@@ -1010,8 +1010,8 @@ def delta_chunks(qkv: torch.Tensor, proj: torch.Tensor, b_col: int, a_col: int, 
     if min(b_col, a_col) < 0 or max(b_col, a_col) + heads > cols:
         raise KernelError("delta_chunks: write strengths or decays lie outside the projection")
     fn = _fn("recurrent_chunks", "tt_delta_chunks", "pipiliiipppppppiiiiiiipp")
-    _check(fn(qkv.data_ptr(), qkv.shape[1], p, splits, stride, cols, b_col, a_col, dt_bias.data_ptr(), a_log.data_ptr(), state.data_ptr(), out.data_ptr(),
-              scratch.data_ptr(), _ptr(cu), _ptr(slots), sequences, chunk_slots(tokens, sequences), heads, qk_heads, key_dim, value_dim, sm_count(qkv.device),
+    _check(fn(_ptr(qkv), qkv.shape[1], p, splits, stride, cols, b_col, a_col, _ptr(dt_bias), _ptr(a_log), _ptr(state), _ptr(out),
+              _ptr(scratch), _ptr(cu), _ptr(slots), sequences, chunk_slots(tokens, sequences), heads, qk_heads, key_dim, value_dim, sm_count(qkv.device),
               _ptr(status), _stream()), "delta_chunks", 2)
 
 
@@ -1543,7 +1543,7 @@ def sort_tokens(x: torch.Tensor, chosen: torch.Tensor, experts: int, xs: torch.T
             or tiles.numel() < 1 + experts + count):
         raise KernelError("sort_tokens: shapes do not fit")
     fn = _fn("routing", "tt_sort_tokens", "pipiiipppppp")
-    at = tiles.data_ptr()
+    at = _ptr(tiles)
     _check(fn(_ptr(x), hidden, _ptr(chosen), tokens, top, experts, at + 4, _ptr(place), _ptr(xs), at + 4 * (1 + experts), at, _stream()), "sort_tokens", 2)
 
 
