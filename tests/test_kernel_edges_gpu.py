@@ -1,4 +1,6 @@
 """Kernels at the sizes where their tiles, slices and vector accesses change: against the same arithmetic in float64."""
+import ctypes
+
 import pytest
 import torch
 
@@ -57,16 +59,48 @@ def test_product_in_parts_at_tile_edges(m, n, k, pad, splits):
     status = torch.zeros(1, dtype=torch.int32, device=DEV)
     api.gemm_split(x, w, bias, wide[:, :, :n], parts, status)
     want = x.double() @ w.double().T + bias.double()
-    # what three parts leave off a product is at most 2^-25 of it; the sum of 64 k takes 24 additions that lose up to 2^-23 each, then come the blocks and slices
+    # the products of parts that are left out are at most 2^-23 of a product; the sum of 64 k takes 24 additions that lose up to 2^-23 each, then come the blocks and slices
     size = x.double().abs() @ w.double().abs().T + bias.double().abs()
     error = (wide[:, :, :n].double().sum(0) - want).abs()
-    assert bool((error <= (2.0 ** -25 + 24 * 2.0 ** -23 + (k // 64 + splits + 2) * 2.0 ** -24) * size).all())
+    assert bool((error <= (2.0 ** -23 + 24 * 2.0 ** -23 + (k // 64 + splits + 2) * 2.0 ** -24) * size).all())
     # and no further from 64 bits than the multiply-adds, which round k times
     plain = torch.empty(1, m, n, device=DEV)
     api.gemm_simt(x, w, bias, plain)
     if m * n * k >= 1 << 20:
         assert float(error.square().mean()) <= float((plain[0].double() - want).square().mean())
     assert bool((wide[:, :, n:] == 7.0).all()) and int(status) == 0
+
+
+@pytest.mark.parametrize("m,n,k", [(17, 4096, 64), (100, 1000, 100), (193, 2048, 512), (40, 1024, 2048)])
+@pytest.mark.parametrize("kind", ["one sign", "cancelling", "few large", "one alone"])
+def test_product_in_parts_of_other_sums(m, n, k, kind):
+    """Sums of one sign (the tensor cores truncate), sums that cancel to a thousandth, sums that one product in a few dozen dominates: no further from 64 bits than the
+    multiply-adds.  A product that stands alone is right to a unit or two in the last place."""
+    from thintensor_b200.kernels import api
+
+    x, w = randn(m, k, seed=190), randn(n, k, seed=191)
+    if kind == "one sign":
+        x, w = x.abs(), w.abs()
+    elif kind == "cancelling":
+        half = k // 2
+        x[:, half:2 * half] = x[:, :half]
+        w[:, half:2 * half] = 1e-3 * randn(n, half, seed=192) - w[:, :half]
+    elif kind == "few large":
+        x[:, ::40] *= 1e5
+    else:
+        x[:, 1:] = 0.0
+    out, plain = torch.empty(1, m, n, device=DEV), torch.empty(1, m, n, device=DEV)
+    parts, status = torch.empty(api.gemm_split_parts(m, k), dtype=torch.bfloat16, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    api.gemm_split(x, w, None, out, parts, status)
+    api.gemm_simt(x, w, None, plain)
+    want = x.double() @ w.double().T
+    assert int(status) == 0
+    if kind == "one alone":
+        # two products of parts left out, 2^-24 of it at most each, and a truncation to the 24 bits of the largest term (two units of a sum just below a power of two)
+        assert bool(((out[0].double() - want).abs() <= (2.0 ** -23 + 2.0 ** -22) * want.abs()).all())
+    else:
+        in_parts, multiplied = (float((got[0].double() - want).norm() / want.norm()) for got in (out, plain))
+        assert in_parts <= multiplied, (in_parts, multiplied)
 
 
 def test_product_in_parts_of_what_is_not_finite():
@@ -703,19 +737,50 @@ def test_recurrence_in_chunks_is_as_close_as_token_by_token(heads, groups, P, N)
         assert chunked <= 1.05 * by_token, (i, chunked, by_token)
 
 
-@pytest.mark.parametrize("heads,groups,P,N", [(40, 40, 130, 128), (40, 20, 130, 64), (40, 8, 70, 128), (40, 40, 70, 40), (3, 3, 50, 128), (5, 1, 90, 64)])
+def scan_columns(heads, sequences, P, N):
+    """Columns of a CTA of the walk over the chunks, as the launcher chooses them."""
+    from thintensor_b200.kernels import api, build
+
+    return build.load("recurrent_chunks").tt_scan_chunks_columns(heads, sequences, P, N, api.sm_count())
+
+
+def delta_columns(heads, sequences, D, V):
+    from thintensor_b200.kernels import api, build
+
+    return build.load("recurrent_chunks").tt_delta_chunks_columns(heads, sequences, D, V, api.sm_count())
+
+
+CHUNKED = 6         # sequences of test_recurrence_in_chunks
+
+
+@pytest.mark.parametrize("heads,groups,P,N,columns", [(24, 24, 128, 128, 128), (22, 22, 100, 128, 128), (24, 24, 130, 128, 32), (24, 24, 256, 128, 128), (24, 24, 120, 64, 128), (24, 4, 110, 50, 128),
+                                                      (24, 4, 64, 128, 64), (24, 24, 50, 128, 64), (40, 40, 130, 128, 64), (24, 24, 50, 40, 64), (40, 8, 70, 128, 32), (3, 3, 50, 128, 16),
+                                                      (5, 1, 90, 128, 32), (5, 1, 90, 64, 32)])
 @pytest.mark.parametrize("fixed", [False, True])
-def test_recurrence_in_chunks_in_wide_tiles(heads, groups, P, N, fixed):
-    """Grids whose CTAs hold 64 and 128 columns, whole and in part, and 16 and 32 columns with several tiles."""
+def test_recurrence_in_chunks_in_wide_tiles(heads, groups, P, N, columns, fixed):
+    """Grids whose CTAs hold 16 to 128 columns, whole and in part, with one tile and several."""
+    assert scan_columns(heads, CHUNKED, P, N) == columns
     test_recurrence_in_chunks(heads, groups, P, N, 0, fixed)
 
 
-@pytest.mark.parametrize("heads,P,N", [(100, 130, 128), (100, 130, 64), (100, 70, 128), (1, 20, 128)])
+@pytest.mark.parametrize("n_tokens,sequences,heads,groups,N", [(1, 1, 1, 1, 1), (200, 3, 8, 4, 64), (4097, 1, 64, 1, 65), (700, 16, 3, 3, 128)])
+def test_chunks_scratch_is_what_the_kernels_lay_out(n_tokens, sequences, heads, groups, N):
+    from thintensor_b200.kernels import api, build
+
+    lib, slots = build.load("recurrent_chunks"), api.chunk_slots(n_tokens, sequences)
+    lib.tt_scan_chunks_scratch_bytes.restype = lib.tt_delta_chunks_scratch_bytes.restype = ctypes.c_longlong
+    assert 4 * api.scan_chunks_scratch(n_tokens, sequences, heads, groups, N)[0] == lib.tt_scan_chunks_scratch_bytes(slots, heads, groups, N)
+    for V in (1, 20, 128):
+        assert 4 * api.delta_chunks_scratch(n_tokens, sequences, heads, N, V, groups)[0] == lib.tt_delta_chunks_scratch_bytes(slots, heads, groups, N, V)
+
+
+@pytest.mark.parametrize("heads,P,N,columns", [(70, 128, 128, 128), (70, 100, 64, 128), (70, 64, 128, 64), (70, 130, 64, 64), (100, 130, 64, 32), (100, 130, 128, 32), (1, 20, 128, 16)])
 @pytest.mark.parametrize("what", ["x", "c", "state"])
-def test_recurrence_in_chunks_keeps_other_columns(heads, P, N, what):
+def test_recurrence_in_chunks_keeps_other_columns(heads, P, N, columns, what):
     """A number that is not finite, in the widths of a CTA's columns: what it does not reach keeps its bits, what it reaches is what it is token by token."""
     from thintensor_b200.kernels import api
 
+    assert scan_columns(heads, 2, P, N) == columns
     news, inner = [150, 70], heads * P
     tokens = sum(news)
     cu, slots, decays = i32([0, news[0], tokens]), i32([1, 0]), torch.full((heads,), 0.9, device=DEV)
@@ -800,6 +865,7 @@ def test_recurrence_in_chunks_of_every_decay(P, N, tokens):
     copies = 12
     heads = copies * len(DECAYS)
     inner = heads * P
+    assert scan_columns(heads, 1, P, N) == {(16, 128): 16, (32, 100): 32, (64, 128): 64, (50, 70): 64, (128, 128): 128, (100, 128): 128, (32, 64): 32, (64, 64): 64, (128, 40): 128}[P, N]
     rows, decays = randn(tokens, inner + 2 * heads * N, seed=170), torch.tensor(DECAYS, device=DEV).repeat_interleave(copies).contiguous()
     cu, slots, outs = i32([0, tokens]), i32([0]), []
     for chunks in (True, False):
@@ -827,6 +893,7 @@ def test_delta_rule_in_chunks_of_every_decay(D, V):
 
     copies, fast = 12, []
     heads = copies * len(DECAYS)
+    assert delta_columns(heads, 1, D, V) == {(128, 16): 16, (100, 32): 32, (128, 64): 64, (64, 16): 16, (64, 32): 32, (40, 50): 64}[D, V]
     qk = heads * D
     decays = torch.tensor(DECAYS, dtype=torch.float64, device=DEV).repeat_interleave(copies)
     a_log, dt_bias = torch.log(-torch.log(decays)).float(), torch.full((heads,), 0.5413248546, device=DEV)
@@ -1037,32 +1104,41 @@ def test_differential_attention_in_tiles(heads, kv_heads, news, before):
 
 @pytest.mark.parametrize("news,before", [([1, 15, 16, 17, 100], [0, 3, 16, 40, 60]), ([600], [127]), ([300, 0, 212], [0, 5, 64])])
 @pytest.mark.parametrize("kv_heads,head_dim,value_dim,from_keys", [(1, 64, 64, False), (3, 40, 72, False), (2, 96, 96, True)])
-def test_heads_and_values_of_prompts(news, before, kv_heads, head_dim, value_dim, from_keys):
-    """The plain copy (from 256 tokens in one slice on) and the general form: queries, keys and values where they belong, nothing else written."""
+@pytest.mark.parametrize("dtype,gain", [(torch.bfloat16, None), (torch.float32, None), (torch.bfloat16, (0.3, 100)), (torch.float32, (0.2, 64))])
+def test_heads_and_values_of_prompts(news, before, kv_heads, head_dim, value_dim, from_keys, dtype, gain):
+    """The plain copy (from 256 tokens in one slice on) and the general form: queries, keys and values where they belong, nothing else written; queries times
+    1 + c ln(floor((position + 1) / every) + 1) where they have a gain, whose steps the positions straddle."""
     from thintensor_b200.kernels import api
 
     tokens, sequences, heads, width = sum(news), len(news), 7, 12
     cols = (heads + kv_heads) * head_dim + (0 if from_keys else kv_heads * value_dim)
     proj = randn(1, tokens, cols, seed=160)
     table = torch.randperm(sequences * width, device=DEV).int().view(sequences, width).contiguous()
-    k_pool = torch.full((sequences * width, kv_heads, 64, head_dim), 7.0, dtype=torch.bfloat16, device=DEV)
-    v_pool = torch.full((sequences * width, kv_heads, value_dim, 64), 7.0, dtype=torch.bfloat16, device=DEV)
-    q, status = torch.empty(tokens, heads * head_dim, dtype=torch.bfloat16, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    k_pool = torch.full((sequences * width, kv_heads, 64, head_dim), 7.0, dtype=dtype, device=DEV)
+    v_pool = torch.full((sequences * width, kv_heads, value_dim, 64), 7.0, dtype=dtype, device=DEV)
+    q, status = torch.empty(tokens, heads * head_dim, dtype=dtype, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
     cu = [sum(news[:i]) for i in range(sequences + 1)]
     api.qk_norm_rope_append(proj, None, None, 0.0, torch.zeros(1, device=DEV), 0, False, 1.0, q, k_pool, v_pool, table, i32(cu), i32(before), sequences, tokens, heads,
-                            kv_heads, head_dim, value_dim, status, **({"value_from_keys": True} if from_keys else {}))
+                            kv_heads, head_dim, value_dim, status, q_gain=gain, **({"value_from_keys": True} if from_keys else {}))
     assert int(status) == 0
     want = torch.full_like(v_pool, 7.0)
     at = heads * head_dim + (0 if from_keys else kv_heads * head_dim)
-    values = proj.sum(0)[:, at:at + kv_heads * value_dim].bfloat16().view(tokens, kv_heads, value_dim)
+    values = proj.sum(0)[:, at:at + kv_heads * value_dim].to(dtype).view(tokens, kv_heads, value_dim)
     for s in range(sequences):
         for i in range(news[s]):
             place = before[s] + i
             want[int(table[s, place // 64]), :, :, place % 64] = values[cu[s] + i]
     assert torch.equal(v_pool, want)
     keys = torch.full_like(k_pool, 7.0)
-    made = proj.sum(0).bfloat16()
-    assert torch.equal(q, made[:, :heads * head_dim])
+    made = proj.sum(0).to(dtype)
+    if gain is None:
+        assert torch.equal(q, made[:, :heads * head_dim])
+    else:
+        at = torch.cat([torch.arange(news[s], device=DEV) + before[s] for s in range(sequences)]).double()
+        factor = 1.0 + gain[0] * torch.log(torch.floor((at + 1) / gain[1]) + 1)
+        # the factor in float32 (a logarithm's error, a product and a sum), one product, and where queries are narrow one more rounding: half a unit of 8 bits, 2^-8
+        want_q = proj[0][:, :heads * head_dim].double() * factor[:, None]
+        assert bool(((q.double() - want_q).abs() <= (4 * 2.0 ** -24 + (2.0 ** -8 if dtype == torch.bfloat16 else 0.0)) * want_q.abs()).all())
     for s in range(sequences):
         for i in range(news[s]):
             place = before[s] + i

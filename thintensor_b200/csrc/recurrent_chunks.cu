@@ -875,9 +875,25 @@ static int scan_chunks_launch(const ScanChunks& a, int max_slots, cudaStream_t s
     TT_LAUNCH_CHECK();
 }
 
-// rows: [tokens][width] with x, B and C from the given columns on (see ScanChunks).  max_slots: n_tokens / 64 + sequences.  scratch: so many
-// times the scores of every group (64 * 64 numbers) and the factors of every head (CK_FACTORS), on a 16-byte boundary: the walk copies
-// it in 16-byte pieces whatever the rows' alignment.  sms: the device's multiprocessors.
+// Columns of a CTA of the walk: rounds of the SMs times what a chunk takes a CTA (hundredths of a microsecond, measured with the GPU to itself: 128 rows 16 columns
+// 333, 32 453, 64 766, 128 1,363; 64 rows 32 columns 300, 64 500, 128 810, and 16 columns no less than 32).
+extern "C" int tt_scan_chunks_columns(int heads, int sequences, int P, int N, int sms) {
+    const long long one = (long long)heads * sequences;
+    auto cost = [&](int columns, int chunk) { return (one * ((P + columns - 1) / columns) + sms - 1) / sms * chunk; };
+    const bool small = N <= 64;
+    const long long c16 = cost(16, 333), c32 = cost(32, small ? 300 : 453), c64 = cost(64, small ? 500 : 766), c128 = cost(128, small ? 810 : 1363);
+    if (c128 <= c64 && c128 <= c32 && c128 <= c16) return 128;
+    if (c64 <= c32 && c64 <= c16) return 64;
+    return small || c32 <= c16 ? 32 : 16;
+}
+
+// Bytes of scratch memory for max_slots chunks.
+extern "C" long long tt_scan_chunks_scratch_bytes(int max_slots, int heads, int groups, int N) {
+    return (long long)max_slots * ((long long)groups * ScanChunks::group_bytes(N <= 64 ? 64 : 128) + (long long)heads * ScanChunks::head_bytes());
+}
+
+// rows: [tokens][width] with x, B and C from the given columns on (see ScanChunks).  max_slots: n_tokens / 64 + sequences.  scratch:
+// tt_scan_chunks_scratch_bytes, on a 16-byte boundary (the walk copies it in 16-byte pieces whatever the rows' alignment).  sms: the device's multiprocessors.
 extern "C" int tt_scan_chunks(const float* rows, int width, int x_col, int b_col, int c_col, const float* proj, int splits, long long split_stride,
                               int cols, int dt_col, const float* dt_bias, const float* a_log, const float* d_skip, const float* fixed_decay, float* state,
                               float* y, float* scratch, const int* cu, const int* slots, int sequences, int max_slots, int heads,
@@ -894,16 +910,13 @@ extern "C" int tt_scan_chunks(const float* rows, int width, int x_col, int b_col
     const ScanChunks a{x, b, c, (size_t)width, proj, splits, cols, dt_col, (size_t)split_stride, dt_bias, a_log, d_skip, fixed_decay, state, y, status,
                        reinterpret_cast<unsigned char*>(scratch), max_slots, cu, slots, sequences, heads, groups, P, N,
                        (bases & 15) == 0 && !(width & 3) && !(N & 3) && !(P & 3) ? 1 : 0, together};
-    // Columns of a CTA: rounds of the SMs times what a chunk takes a CTA (hundredths of a microsecond, measured with the GPU to itself: 128 rows 16 columns
-    // 333, 32 453, 64 766, 128 1,363; 64 rows 32 columns 300, 64 500, 128 810, and 16 columns no less than 32).
-    const long long one = (long long)heads * sequences;
-    auto cost = [&](int columns, int chunk) { return (one * ((P + columns - 1) / columns) + sms - 1) / sms * chunk; };
     const bool small = N <= 64;
-    const long long c16 = cost(16, 333), c32 = cost(32, small ? 300 : 453), c64 = cost(64, small ? 500 : 766), c128 = cost(128, small ? 810 : 1363);
-    if (c128 <= c64 && c128 <= c32 && c128 <= c16) return small ? scan_chunks_launch<64, 8, 1>(a, max_slots, stream) : scan_chunks_launch<128, 8, 1>(a, max_slots, stream);
-    if (c64 <= c32 && c64 <= c16) return small ? scan_chunks_launch<64, 4, 2>(a, max_slots, stream) : scan_chunks_launch<128, 4, 2>(a, max_slots, stream);
-    if (small) return scan_chunks_launch<64, 2, 4>(a, max_slots, stream);
-    return c32 <= c16 ? scan_chunks_launch<128, 2, 4>(a, max_slots, stream) : scan_chunks_launch<128, 1, 8>(a, max_slots, stream);
+    switch (tt_scan_chunks_columns(heads, sequences, P, N, sms)) {
+        case 128: return small ? scan_chunks_launch<64, 8, 1>(a, max_slots, stream) : scan_chunks_launch<128, 8, 1>(a, max_slots, stream);
+        case 64: return small ? scan_chunks_launch<64, 4, 2>(a, max_slots, stream) : scan_chunks_launch<128, 4, 2>(a, max_slots, stream);
+        case 32: return small ? scan_chunks_launch<64, 2, 4>(a, max_slots, stream) : scan_chunks_launch<128, 2, 4>(a, max_slots, stream);
+    }
+    return scan_chunks_launch<128, 1, 8>(a, max_slots, stream);
 }
 
 // ------------------------------------------------------------------------------------------------------ the gated delta rule
@@ -1595,7 +1608,21 @@ static int delta_chunks_launch(const DeltaChunks& a, int max_slots, cudaStream_t
     TT_LAUNCH_CHECK();
 }
 
-// scratch: max_slots times the operands of every query/key head and of every head (see DeltaChunks), on a 16-byte boundary; max_slots as for tt_scan_chunks
+// columns of a CTA, as for the scan: a chunk takes a CTA of 16, 32 and 64 columns 3.5, 5.5 and 10.7 us with keys of 128, 3.7, 5.4 and 8.4 with keys of 64
+extern "C" int tt_delta_chunks_columns(int heads, int sequences, int D, int V, int sms) {
+    const long long one = (long long)heads * sequences;
+    auto cost = [&](int columns, int chunk) { return (one * ((V + columns - 1) / columns) + sms - 1) / sms * chunk; };
+    const bool small = D <= 64;
+    const long long c16 = cost(16, small ? 370 : 352), c32 = cost(32, small ? 540 : 550), c64 = cost(64, small ? 840 : 1070);
+    return c64 <= c32 && c64 <= c16 ? 64 : c32 <= c16 ? 32 : 16;
+}
+
+extern "C" long long tt_delta_chunks_scratch_bytes(int max_slots, int heads, int qk_heads, int D, int V) {
+    const int padded = D <= 64 ? 64 : 128;
+    return (long long)max_slots * ((long long)qk_heads * DeltaChunks::matrix_bytes(padded) + (long long)heads * (DeltaChunks::operand_bytes(padded) + (long long)CK_TOKENS * V * sizeof(float)));
+}
+
+// scratch: tt_delta_chunks_scratch_bytes, on a 16-byte boundary; max_slots as for tt_scan_chunks
 extern "C" int tt_delta_chunks(const float* qkv, int qkv_cols, const float* proj, int splits, long long split_stride, int cols, int b_col, int a_col,
                                const float* dt_bias, const float* a_log, float* state, float* out, float* scratch, const int* cu, const int* slots,
                                int sequences, int max_slots, int heads, int qk_heads, int D, int V, int sms, unsigned* status, cudaStream_t stream) {
@@ -1605,12 +1632,10 @@ extern "C" int tt_delta_chunks(const float* qkv, int qkv_cols, const float* proj
     const int vec = ((uintptr_t)qkv & 15) == 0 && !(qkv_cols & 3) && !(D & 3);
     const DeltaChunks a{qkv, (size_t)qkv_cols, proj, splits, cols, b_col, a_col, (size_t)split_stride, dt_bias, a_log, state, out, status,
                         reinterpret_cast<unsigned char*>(scratch), cu, slots, sequences, max_slots, heads, qk_heads, D, V, vec};
-    // columns of a CTA, as for tt_scan_chunks: a chunk takes a CTA of 16, 32 and 64 columns 3.5, 5.5 and 10.7 us with keys of 128, 3.7, 5.4 and 8.4 with keys of 64
-    const long long one = (long long)heads * sequences;
-    auto cost = [&](int columns, int chunk) { return (one * ((V + columns - 1) / columns) + sms - 1) / sms * chunk; };
     const bool small = D <= 64;
-    const long long c16 = cost(16, small ? 370 : 352), c32 = cost(32, small ? 540 : 550), c64 = cost(64, small ? 840 : 1070);
-    if (c64 <= c32 && c64 <= c16) return small ? delta_chunks_launch<64, 4, 2>(a, max_slots, stream) : delta_chunks_launch<128, 4, 2>(a, max_slots, stream);
-    if (c32 <= c16) return small ? delta_chunks_launch<64, 2, 4>(a, max_slots, stream) : delta_chunks_launch<128, 2, 4>(a, max_slots, stream);
+    switch (tt_delta_chunks_columns(heads, sequences, D, V, sms)) {
+        case 64: return small ? delta_chunks_launch<64, 4, 2>(a, max_slots, stream) : delta_chunks_launch<128, 4, 2>(a, max_slots, stream);
+        case 32: return small ? delta_chunks_launch<64, 2, 4>(a, max_slots, stream) : delta_chunks_launch<128, 2, 4>(a, max_slots, stream);
+    }
     return small ? delta_chunks_launch<64, 1, 4>(a, max_slots, stream) : delta_chunks_launch<128, 1, 8>(a, max_slots, stream);
 }
