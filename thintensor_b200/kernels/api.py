@@ -159,6 +159,7 @@ class timed_classes:
         _timer, _label = None, None
 
 
+_ptr_in_python, _need_in_python, _need_columns_in_python = _ptr, _need, _need_columns
 _host = None               # the native module; False where it cannot be built
 _CTYPES = {"p": c_void_p, "i": c_int, "l": c_longlong, "u": c_ulonglong, "f": c_float}
 
