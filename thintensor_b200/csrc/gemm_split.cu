@@ -1,11 +1,13 @@
 // out[s][m][n] = sum over the s-th slice of k of x[m][k] * w[n][k]  (+ bias[n] in s = 0), float32 operands, on the tensor cores
 //
 // The 32-bit product of prompts.  Every operand is cut into three bfloat16 numbers (x = hi + mid + lo, each what the parts before leave,
-// rounded to nearest: 24 bits and more), and six of the nine products of parts (all but mid lo, lo mid and lo lo, at most 2^-26 of the
-// product each) go through tcgen05.mma, whose products of bfloat16 are exact.  What the tensor cores do to a sum is the other
+// rounded to nearest: see split_mma.cuh), and six of the nine products of parts (all but mid lo, lo mid and lo lo: together 2^-23
+// of the product at most, 2^-27 rms) go through tcgen05.mma, whose products of bfloat16 are exact.  What the tensor cores do to a sum is the other
 // half: they truncate, so that a sum that runs through all of k in tensor memory drifts.  So tensor memory only ever holds
 // the sum over 64 k, the small products of them first and the large ones behind; it is then read and added to float32 sums in
-// registers.  The result is nearer to 64 bits than the sum of float32 multiply-adds of gemm_simt.cu (see there for the reference's entry points).
+// registers.  Sums of many terms are nearer to 64 bits than those of the float32 multiply-adds of gemm_simt.cu (see there for the reference's entry
+// points): 0.16 to 0.52 of their error for normal numbers, 0.36 to 0.87 for numbers of one sign (the truncation takes 0.6e-7 to 0.8e-7 of a sum), 0.12 to 0.42 where
+// sums cancel; a product that stands alone is right to a unit or two in the last place instead of half of one (4.7e-8 against 2.7e-8).
 //
 // A CTA pair (cta_group::2) has 256 output features and up to 256 tokens: the weights are the 256-row operand, so they are read and cut
 // up once for all those tokens.  Sixteen warps of each CTA cut the pair's weights up as they come from memory (straight into the
@@ -13,7 +15,7 @@
 // fetches the activations' parts, which a small kernel before wrote; one more, of the even CTA, issues.  Two stages of 64 k, two accumulators: while the
 // products of a block of 64 k run, the warps add up the block before and cut up the one behind.
 //
-// What bounds it: the six products (a block of 64 k of 224 tokens is 24 of them, 2,690 of the 3,000 cycles a block takes); below about 100
+// What bounds it: the six products (a block of 64 k of 224 tokens is 24 of them, 2,690 of the 3,000 cycles a block takes; tensor pipe 76 % busy over a whole launch); below about 100
 // tokens the way of a block through the kernel, 2,700 cycles; few features the pairs' start and end.  The rows of weights go behind the arrival
 // of the block before: with loads ahead of it the fence took 750 cycles more a block.  What the odd CTA's warps wrote has to be released to the
 // cluster, which took every warp 1,700 cycles when each did it (its fence waits for the warp's loads): they arrive at a barrier of their own CTA, and one thread
@@ -29,6 +31,7 @@
 
 #include <cooperative_groups.h>
 
+#include "split_mma.cuh"
 #include "tcgen05.cuh"
 
 namespace cg = cooperative_groups;
@@ -46,17 +49,6 @@ constexpr int MAX_HALF = 128;                                   // rows of activ
 constexpr int STAGE_BYTES = PARTS * A_BYTES + PARTS * MAX_HALF * BK * 2;
 constexpr int AHEAD = 4;                                        // blocks of 64 k that are asked for into the L2
 constexpr int SHARED = 2 * STAGE_BYTES + 1024;
-
-// the three parts of two neighbouring numbers, packed
-__device__ __forceinline__ void cut2(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(hi) : "f"(b), "f"(a));
-    a -= __uint_as_float(hi << 16);
-    b -= __uint_as_float(hi & 0xffff0000u);
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(mid) : "f"(b), "f"(a));
-    a -= __uint_as_float(mid << 16);
-    b -= __uint_as_float(mid & 0xffff0000u);
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(lo) : "f"(b), "f"(a));
-}
 
 // The activations' parts [3][m][kp] (kp: k rounded up to 8, the padding never read), four numbers a thread.  A product is preceded by one
 // such launch; cutting them up with the weights, in every CTA that reads them, would double that work there.
@@ -77,8 +69,8 @@ __global__ void __launch_bounds__(256) cut_kernel(const float* __restrict__ x, l
             for (int e = 0; e < 4; ++e) v[e] = at + e < k ? p[e] : 0.0f;
         }
         uint2 hi, mid, lo;
-        cut2(v[0], v[1], hi.x, mid.x, lo.x);
-        cut2(v[2], v[3], hi.y, mid.y, lo.y);
+        split_pair(v[0], v[1], hi.x, mid.x, lo.x);
+        split_pair(v[2], v[3], hi.y, mid.y, lo.y);
         __nv_bfloat16* to = parts + (size_t)row * kp + at;
         *reinterpret_cast<uint2*>(to) = hi;
         *reinterpret_cast<uint2*>(to + plane) = mid;
@@ -86,12 +78,7 @@ __global__ void __launch_bounds__(256) cut_kernel(const float* __restrict__ x, l
     }
 }
 
-// not finite, or neither zero nor as large as 2^-90
-__device__ __forceinline__ bool form_again(float sum) {
-    constexpr uint32_t LEAST = (127u - 90u) << 23, INF = 255u << 23;
-    const uint32_t bits = __float_as_uint(sum) & 0x7fffffffu;
-    return bits - LEAST >= INF - LEAST && bits != 0u;
-}
+constexpr float LEAST = 8.077935669463161e-28f;                 // 2^-90: smaller sums, but zeros, are formed again
 
 struct Args {
     const float* x;
@@ -239,8 +226,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
                 const int row = load_row + 2 * j;
                 const uint32_t at = to + row * 128 + ((((lane & 15) >> 1) ^ (row & 7)) << 4) + (lane & 1) * 8;
                 uint2 hi, mid, lo;
-                cut2(raw[j].x, raw[j].y, hi.x, mid.x, lo.x);
-                cut2(raw[j].z, raw[j].w, hi.y, mid.y, lo.y);
+                split_pair(raw[j].x, raw[j].y, hi.x, mid.x, lo.x);
+                split_pair(raw[j].z, raw[j].w, hi.y, mid.y, lo.y);
                 asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at), "r"(hi.x), "r"(hi.y) : "memory");
                 asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at + A_BYTES), "r"(mid.x), "r"(mid.y) : "memory");
                 asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at + 2 * A_BYTES), "r"(lo.x), "r"(lo.y) : "memory");
@@ -263,29 +250,39 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_split_kernel(const __grid_con
             const float bias = args.bias && blockIdx.z == 0 ? args.bias[feature] : 0.0f;
             float* out = args.out + (size_t)blockIdx.z * args.split_stride + feature;
             const int first = token0 + column0, count = min(width, args.m - first);
-            unsigned again[4];
+            float least = INFINITY, odd = 0.0f;                 // the smallest sum's size; NaN once a sum is not finite
 #pragma unroll
             for (int b = 0; b < 4; ++b) {
-                again[b] = 0;
                 float* to = out + (size_t)(first + b * 16) * args.ldo;
 #pragma unroll
                 for (int e = 0; e < 16; ++e) {
                     if (b * 16 + e < count) {
                         to[0] = acc[b][e] + bias;
-                        again[b] |= (unsigned)form_again(acc[b][e]) << e;
+                        least = fminf(least, fabsf(acc[b][e]));
+                        odd = fmaf(acc[b][e], 0.0f, odd);
                     }
                     to += args.ldo;
                 }
             }
+            if (!(least >= LEAST) || odd != 0.0f) {             // (asked once for all sums: asked for each, the 32-bit prompt took 1 % more)
+                unsigned again[4];
+#pragma unroll
+                for (int b = 0; b < 4; ++b) {
+                    again[b] = 0;
+#pragma unroll
+                    for (int e = 0; e < 16; ++e)
+                        if (b * 16 + e < count && acc[b][e] != 0.0f && !(fabsf(acc[b][e]) >= LEAST && fabsf(acc[b][e]) <= 3.402823466e38f)) again[b] |= 1u << e;
+                }
 #pragma unroll 1
-            for (int b = 0; b < 4; ++b) {
-                unsigned left = b == 0 ? again[0] : b == 1 ? again[1] : b == 2 ? again[2] : again[3];
-                for (; left; left &= left - 1) {
-                    const int token = first + b * 16 + __ffs(left) - 1;
-                    const float *xr = args.x + (size_t)token * args.ldx, *wr = args.w + (size_t)feature * args.ldw;
-                    float v = 0.0f;
-                    for (int kk = kb0 * BK; kk < min(args.k, (kb0 + steps) * BK); ++kk) v = fmaf(xr[kk], wr[kk], v);
-                    out[(size_t)token * args.ldo] = v + bias;
+                for (int b = 0; b < 4; ++b) {
+                    unsigned left = b == 0 ? again[0] : b == 1 ? again[1] : b == 2 ? again[2] : again[3];
+                    for (; left; left &= left - 1) {
+                        const int token = first + b * 16 + __ffs(left) - 1;
+                        const float *xr = args.x + (size_t)token * args.ldx, *wr = args.w + (size_t)feature * args.ldw;
+                        float v = 0.0f;
+                        for (int kk = kb0 * BK; kk < min(args.k, (kb0 + steps) * BK); ++kk) v = fmaf(xr[kk], wr[kk], v);
+                        out[(size_t)token * args.ldo] = v + bias;
+                    }
                 }
             }
         }
