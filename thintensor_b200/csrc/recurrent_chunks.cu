@@ -19,8 +19,9 @@
 // the factors f(i, j) dt_j of every chunk and head, in parts and in the order in which the walk's lanes take them, and e, w, e_63.  The second
 // walks a sequence's chunks with the state of 16 to 128 columns of one head in its warps' accumulators.
 //
-// What bounds it: issue around the tensor cores (two warps a scheduler; half of a chunk's time is their products, the rest splitting states and x,
-// adding up outputs and waiting for one another).  16 warps with half the registers were slower at every size (64 heads of 64 x 128, 2,048
+// What bounds it: latency, with two warps a scheduler for want of registers (64 heads of 64 x 128: tensor pipe 45 % busy, issue slots 31 %, shared memory 34 %; a warp
+// waits for fixed latencies, then for the pipe, then for shared memory): half of a chunk's time is its products, the rest splitting states and x, adding up outputs and
+// waiting for one another.  16 warps with half the registers were slower at every size (64 heads of 64 x 128, 2,048
 // tokens: 222 against 169 us), as was fetching the operands with 16-byte copies by all threads instead of the copy engine (198).
 // Token by token, in chunks of float32 multiply-adds, and now (us, one B200, back to back): 64 heads of 64 x 128, one sequence of 2,048 tokens
 // 748, 227, 171 (180 where every chunk has a tail), four of 731 423, 340, 236; 16 heads of 256 x 128, four of
@@ -931,8 +932,8 @@ extern "C" int tt_scan_chunks(const float* rows, int width, int x_col, int b_col
 // added to the state as in the scan.  Error against 64 bits by decay, relative to token by token (and of float32 multiply-adds in chunks), 22 heads of 128 x 128: outputs
 // 0.999 a token 1.00 (1.00), 0.9 0.79 (0.77), 0.5 0.61 (0.69), 0.1 0.62 (0.66); states 1.01 (1.01), 1.03 (1.01), 0.92 (0.92), 0.87 (0.87).
 // 16 heads of 128 x 128 on 4,097 tokens, us: token by token 1,900, chunks of float32 multiply-adds 485, now 385 (392 where every chunk has a tail), of which the first kernel takes 150
-// (issue around splitting its operands, at two CTAs an SM; with scores and systems of multiply-adds 172) and the walk 246 (three barriers a
-// chunk and the latency of what lies between them; half of a chunk's time is its products).
+// (issue around splitting its operands, 44 % of the slots at two CTAs an SM, and barriers; with scores and systems of multiply-adds 172) and the walk 246 (three barriers a
+// chunk and the latency of what lies between them; tensor pipe 38 % busy, issue slots 26 %).
 constexpr int CD_THREADS = 256;
 
 struct DeltaChunks {

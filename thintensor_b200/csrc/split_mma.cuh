@@ -1,6 +1,8 @@
-// Float32 matrix products on the tensor cores: every operand in three bfloat16 parts whose sum is the float32 number to within
-// 2^-26 of it (x = hi + mid + lo, each part the rounding of what the parts before leave), six of the nine part products
-// (hi hi, hi mid, mid hi, mid mid, hi lo, lo hi; what is left out is below 2^-25 of the product).
+// Float32 matrix products on the tensor cores: every operand in three bfloat16 parts whose sum is the float32 number
+// (x = hi + mid + lo, each part the rounding of what the parts before leave: 3 x 8 bits), six of the nine part products
+// (hi hi, hi mid, mid hi, mid mid, hi lo, lo hi; what is left out is 2^-23 of the product at most, 2^-27 rms).  The method is that of Henry, Tang and Heinecke, "Leveraging the bfloat16
+// artificial intelligence datatype for higher-precision computations" (2019).  The third part of a number below 2^-109 falls under the smallest bfloat16 number,
+// 2^-133: such a number is kept to 2^-134, which shows only in sums that are as small.
 //
 // The tensor cores add with truncation at 2^-25 of the largest term, and truncate every accumulation again, so a long chain of
 // accumulations drifts towards zero.  Therefore hi hi is taken from zero for every 16 k and added up in registers with
@@ -8,8 +10,8 @@
 // the five others, 2^-8 of it at most, have an accumulator of their own.
 //
 // Rate: an SM issues 1,020 bfloat16 multiply-adds a cycle through mma.sync (measured), 170 of these products; its FMA units 128 at best and
-// 50 to 70 in the loops this replaces.  tcgen05.mma would multiply four times as fast but accumulates in tensor memory: an accumulator for
-// every 16 k and a trip through registers for every state.
+// 50 to 70 in the loops this replaces.  tcgen05.mma multiplies four times as fast, and sums of 64 k in tensor memory are close enough (gemm_split.cu);
+// here it would take the state's parts through shared memory for every chunk, which is not built.
 #pragma once
 #include <stdint.h>
 

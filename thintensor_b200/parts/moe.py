@@ -19,7 +19,7 @@ behind them) and ONE down product over the concatenated columns: a token's activ
 routing weight per expert (zero for experts it did not choose) in between, so the down product's sum over its input
 IS the weighted sum over experts.  Every matrix is read once per step whatever the routing, which is what a decode
 step of more than a few sequences does anyway; the price is the arithmetic of the experts a token did not choose.
-Where that is large (prompts, see :func:`sorted_experts_pay`) the tokens are sorted by the experts they chose, each expert's
+Where that is large (prompts, see :func:`sorted_experts_pay`) and the experts are plainly gated, the tokens are sorted by the experts they chose, each expert's
 matrices multiply its own rows, and a token's products are weighted and added in float32.
 """
 from __future__ import annotations
@@ -164,7 +164,8 @@ class MixtureOfExperts(FeedForward):
 
     def sorted_takes(self, x) -> bool:
         """Whether the experts' matrices can be multiplied with the rows that chose them: whole tiles of 128 rows an expert, operands of the
-        tensor-core product."""
+        tensor-core product.  Clamped and ungated experts, and those beside a gated shared one, multiply every token as before: the product of sorted
+        rows has no epilogue for them (it is not built; the gain would be the same)."""
         return (self.gated and self.activation in api.GATE_ACTIVATIONS and not self.shared_gate and self.inter % 128 == 0 and self.shared_inter % 128 == 0
                 and self.hidden % 8 == 0 and api.gemm_tcgen05_usable(x, self.gate_up.fused.weight) and self.down.weight.dtype == torch.bfloat16
                 and self.down.weight.shape[1] % 8 == 0)
