@@ -71,7 +71,7 @@ def test_product_in_parts_at_tile_edges(m, n, k, pad, splits):
     assert bool((wide[:, :, n:] == 7.0).all()) and int(status) == 0
 
 
-@pytest.mark.parametrize("m,n,k", [(17, 4096, 64), (100, 1000, 100), (193, 2048, 512), (40, 1024, 2048)])
+@pytest.mark.parametrize("m,n,k", [(17, 4096, 64), (100, 1000, 100), (150, 3, 100), (193, 2048, 512), (40, 1024, 2048)])
 @pytest.mark.parametrize("kind", ["one sign", "cancelling", "few large", "one alone"])
 def test_product_in_parts_of_other_sums(m, n, k, kind):
     """Sums of one sign (the tensor cores truncate), sums that cancel to a thousandth, sums that one product in a few dozen dominates: no further from 64 bits than the
@@ -776,21 +776,23 @@ def test_chunks_scratch_is_what_the_kernels_lay_out(n_tokens, sequences, heads, 
 
 @pytest.mark.parametrize("heads,P,N,columns", [(70, 128, 128, 128), (70, 100, 64, 128), (70, 64, 128, 64), (70, 130, 64, 64), (100, 130, 64, 32), (100, 130, 128, 32), (1, 20, 128, 16)])
 @pytest.mark.parametrize("what", ["x", "c", "state"])
-def test_recurrence_in_chunks_keeps_other_columns(heads, P, N, columns, what):
-    """A number that is not finite, in the widths of a CTA's columns: what it does not reach keeps its bits, what it reaches is what it is token by token."""
+@pytest.mark.parametrize("decay,token", [(0.9, 100), (0.5, 100), (0.5, 125)])
+def test_recurrence_in_chunks_keeps_other_columns(heads, P, N, columns, what, decay, token):
+    """A number that is not finite, in the widths of a CTA's columns, ahead of a chunk's tail and in it: what it does not reach keeps its bits, what it reaches is what it
+    is token by token."""
     from thintensor_b200.kernels import api
 
     assert scan_columns(heads, 2, P, N) == columns
     news, inner = [150, 70], heads * P
     tokens = sum(news)
-    cu, slots, decays = i32([0, news[0], tokens]), i32([1, 0]), torch.full((heads,), 0.9, device=DEV)
+    cu, slots, decays = i32([0, news[0], tokens]), i32([1, 0]), torch.full((heads,), decay, device=DEV)
     outs = []
     for poisoned, chunks in ((False, True), (True, True), (True, False)):
         rows, state = randn(tokens, inner + 2 * heads * N, seed=130), randn(2, heads, P, N, seed=131)
         if poisoned and what == "state":
             state[1, 0, 5, 1] = float("inf")
         elif poisoned:
-            rows[100, 5 if what == "x" else inner + heads * N + 2] = float("nan")
+            rows[token, 5 if what == "x" else inner + heads * N + 2] = float("nan")
         y = torch.full((tokens, inner), 7.0, device=DEV)
         if chunks:
             scratch = torch.full(api.scan_chunks_scratch(tokens, 2, heads, heads, N), float("nan"), device=DEV)
@@ -802,12 +804,48 @@ def test_recurrence_in_chunks_keeps_other_columns(heads, P, N, columns, what):
     assert torch.equal(y.isfinite(), by_token.isfinite()) and torch.equal(state.isfinite(), by_token_state.isfinite())
     reached = torch.zeros(tokens, inner, dtype=torch.bool, device=DEV)
     if what == "c":
-        reached[100:news[0], :P] = True           # the token's outputs; the tokens behind it in the chunk are taken one by one
+        reached[token:news[0], :P] = True         # the token's outputs; the tokens behind it in the chunk are taken one by one
     else:
-        reached[100 if what == "x" else 0:news[0], 5] = True
+        reached[token if what == "x" else 0:news[0], 5] = True
     assert torch.equal(y[~reached], clean[~reached])
     keeps = torch.ones_like(state, dtype=torch.bool)
     keeps[1, 0, :P if what == "c" else 6] = False
+    assert torch.equal(state[keeps], clean_state[keeps])
+
+
+@pytest.mark.parametrize("heads,D,V,columns", [(70, 128, 64, 64), (70, 128, 60, 64), (70, 128, 32, 32), (70, 64, 64, 64), (70, 64, 32, 32), (2, 128, 20, 16)])
+@pytest.mark.parametrize("what,token", [("v", 100), ("v", 125), ("k", 100), ("k", 125), ("state", 0)])
+def test_delta_rule_in_chunks_keeps_other_columns(heads, D, V, columns, what, token):
+    """As for the scan, half of the heads with fast decays."""
+    from thintensor_b200.kernels import api
+
+    assert delta_columns(heads, 2, D, V) == columns
+    news, qk = [150, 70], heads * D
+    tokens = sum(news)
+    cu, slots = i32([0, news[0], tokens]), i32([1, 0])
+    dt_bias, a_log = torch.full((heads,), 0.5413, device=DEV), torch.tensor([-3.0, 0.5], device=DEV).repeat(heads // 2)
+    outs = []
+    for poisoned, chunks in ((False, True), (True, True), (True, False)):
+        qkv, raw, state = randn(tokens, 2 * qk + heads * V, seed=135), randn(1, tokens, 2 * heads, seed=136), randn(2, heads, V, D, seed=137)
+        raw[:, :, heads:] *= 0.1
+        if poisoned and what == "state":
+            state[1, 1, 5, 1] = float("inf")
+        elif poisoned:
+            qkv[token, 2 * qk + V + 5 if what == "v" else qk + D + 2] = float("nan")
+        out = torch.full((tokens, heads * V), 7.0, device=DEV)
+        if chunks:
+            scratch = torch.full(api.delta_chunks_scratch(tokens, 2, heads, D, V), float("nan"), device=DEV)
+            api.delta_chunks(qkv, raw, 0, heads, dt_bias, a_log, state, out, cu, slots, 2, heads, heads, D, V, scratch)
+        else:
+            api.delta_scan(qkv, raw, 0, heads, dt_bias, a_log, state, out, cu, slots, 2, heads, heads, D, V)
+        outs.append((out, state))
+    (clean, clean_state), (out, state), (by_token, by_token_state) = outs
+    assert torch.equal(out.isfinite(), by_token.isfinite()) and torch.equal(state.isfinite(), by_token_state.isfinite())
+    reached = torch.zeros(tokens, heads * V, dtype=torch.bool, device=DEV)
+    reached[token:news[0], slice(V, 2 * V) if what == "k" else V + 5] = True
+    assert torch.equal(out[~reached], clean[~reached])
+    keeps = torch.ones_like(state, dtype=torch.bool)
+    keeps[1, 1, slice(0, V) if what == "k" else 5] = False
     assert torch.equal(state[keeps], clean_state[keeps])
 
 
