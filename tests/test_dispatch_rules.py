@@ -2,6 +2,7 @@
 from __future__ import annotations
 
 import pytest
+import torch
 
 SMS = 148
 
@@ -59,3 +60,22 @@ def test_delta_rule_in_chunks(tokens, sequences, ctas, keys, pays):
     from thintensor_b200.parts.recurrent import delta_chunks_pay
 
     assert delta_chunks_pay(tokens, sequences, ctas, keys, SMS) is pays
+
+
+def test_tokens_are_sorted_where_the_kernels_take_them():
+    """Rows side by side, bfloat16, whole tiles of 128 rows an expert, plainly gated experts; everything else multiplies every token as before."""
+    from thintensor_b200.parts import moe
+
+    def mixture(**changes):
+        sizes = {"hidden": 256, "experts": 16, "top": 3, "inter": 128, "groups": 4, "keep": 2, "shared_inter": 0, **changes}
+        part = moe.MixtureOfExperts(**sizes)
+        part.bind({name: torch.zeros(*decl.shape, dtype=torch.bfloat16) for name, decl in part.weights().items()}, torch.bfloat16, torch.device("cpu"))
+        return part
+
+    wide = torch.zeros(40, 512, dtype=torch.bfloat16)
+    x = torch.zeros(40, 256, dtype=torch.bfloat16)
+    assert mixture().sorted_takes(x) and mixture(shared_inter=384).sorted_takes(x)
+    for rows in (wide[:, :256], wide[:, 8:264], wide[::2, :256], x.float()):
+        assert not mixture().sorted_takes(rows)
+    assert not mixture(inter=96).sorted_takes(x) and not mixture(shared_inter=100).sorted_takes(x)
+    assert not mixture(activation="clamped", limit=1.0).sorted_takes(x)

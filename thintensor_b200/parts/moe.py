@@ -167,7 +167,7 @@ class MixtureOfExperts(FeedForward):
         tensor-core product.  Clamped and ungated experts, and those beside a gated shared one, multiply every token as before: the product of sorted
         rows has no epilogue for them (it is not built; the gain would be the same)."""
         return (self.gated and self.activation in api.GATE_ACTIVATIONS and not self.shared_gate and self.inter % 128 == 0 and self.shared_inter % 128 == 0
-                and self.hidden % 8 == 0 and api.gemm_tcgen05_usable(x, self.gate_up.fused.weight) and self.down.weight.dtype == torch.bfloat16
+                and self.hidden % 8 == 0 and x.is_contiguous() and api.gemm_tcgen05_usable(x, self.gate_up.fused.weight) and self.down.weight.dtype == torch.bfloat16
                 and self.down.weight.shape[1] % 8 == 0)
 
     def by_expert(self, ctx, x, chosen, weights) -> Delta:
